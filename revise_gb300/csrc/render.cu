@@ -56,6 +56,25 @@ struct Dim {
 };
 __device__ __forceinline__ Dim dim_of(const BlockRay& r) { return Dim{r.n, r.pitch}; }
 
+// a / b correctly rounded from y = 1 / b correctly rounded (Markstein's quotient: one product, its exact
+// residual, one correction), for b and a / b well inside the normal range: three fused operations where the
+// divisor serves many quotients, against a division's reciprocal, refinement and range test each time.
+__device__ __forceinline__ float div_by(float a, float b, float y)
+{
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+}
+
+// floor(x) of |x| < 2^22 and the integer, by one addition rounded down that leaves the integer in the low
+// mantissa bits: the conversion unit, which float-to-integer, floor and the exponentials of a sample share,
+// runs at a fraction of the adders' rate.
+__device__ __forceinline__ float floor_small(float x, int& i)
+{
+    const float r = __fadd_rd(x, 12582912.f); // 1.5 * 2^23
+    i = __float_as_int(r) - 0x4b400000;
+    return __fsub_rn(r, 12582912.f);
+}
+
 __device__ __forceinline__ void pixel_ray(const s3r_view& v, uint32_t vx, uint32_t vy, float org[3], float dir[3])
 {
     const float x = __fmul_rn(__fadd_rn(-0.5f, __fdiv_rn(__fadd_rn((float)vx, 0.5f), (float)v.W)), v.cam.w);
@@ -74,10 +93,17 @@ __device__ __forceinline__ void pixel_ray(const s3r_view& v, uint32_t vx, uint32
     }
 }
 
+// 1 / dir per axis for block_ray and walk_blocks; an axis the ray hardly moves along is never divided by.
+__device__ __forceinline__ void ray_inverse(const float dir[3], float inv[3])
+{
+#pragma unroll
+    for (int d = 0; d < 3; ++d) inv[d] = __frcp_rn(dir[d]);
+}
+
 // Slab test and sample set-up (DenseFieldRenderer_cu.cu:81-181). Returns true
 // when the block is rendered for this ray.
 __device__ __forceinline__ bool block_ray(const s3r_view& v, const float org[3], const float dir[3],
-                                          const RenderBlock& rb, BlockRay& r)
+                                          const float inv[3], const RenderBlock& rb, BlockRay& r)
 {
     const float* c = rb.center;
     const float h = rb.half;
@@ -90,7 +116,7 @@ __device__ __forceinline__ bool block_ray(const s3r_view& v, const float org[3],
 #pragma unroll
         for (int side = 0; side < 2; ++side) {
             const float face = side ? __fadd_rn(c[a], h) : __fsub_rn(c[a], h);
-            const float tau = __fdiv_rn(__fsub_rn(face, org[a]), dir[a]);
+            const float tau = div_by(__fsub_rn(face, org[a]), dir[a], inv[a]);
             const float p1 = __fadd_rn(org[b1], __fmul_rn(dir[b1], tau));
             const float p2 = __fadd_rn(org[b2], __fmul_rn(dir[b2], tau));
             if (fabsf(__fsub_rn(p1, c[b1])) <= h && fabsf(__fsub_rn(p2, c[b2])) <= h) {
@@ -361,7 +387,9 @@ __global__ void render_block_argb_kernel(const s3r_view v, const float* __restri
     float org[3], dir[3];
     pixel_ray(v, vx, vy, org, dir);
     BlockRay r;
-    if (!block_ray(v, org, dir, rb, r)) return;
+    float inv[3];
+    ray_inverse(dir, inv);
+    if (!block_ray(v, org, dir, inv, rb, r)) return;
     const float span = v.field_max - v.field_min;
     const float of = (v.threshold - v.field_min) / span;
     const float il = layer_exponent(depth, v.level, v.quality);
@@ -814,7 +842,9 @@ __global__ void render_block_mode_kernel(const s3r_view v, const s3r_presentatio
     float org[3], dir[3];
     pixel_ray(v, vx, vy, org, dir);
     BlockRay r;
-    if (!block_ray(v, org, dir, rb, r)) return;
+    float inv[3];
+    ray_inverse(dir, inv);
+    if (!block_ray(v, org, dir, inv, rb, r)) return;
     const BrickSampler<kTex> smp{brick, brick2, dim_of(r), tf, v.tf_n};
     store_mode_pixel(&viewport[(size_t)(v.H - 1 - vy) * v.W + vx], march_block_mode(v, pr, smp, r, rb.depth));
 }
@@ -925,7 +955,8 @@ __global__ void render_block_texture_kernel(const s3r_view v, const s3r_presenta
 // (Amanatides-Woo); calls f(block_index, ix, iy, iz) for every block the ray
 // passes, in order; f returns false to stop.
 template <class F>
-__device__ __forceinline__ void walk_blocks(const float org[3], const float dir[3], uint32_t level, F&& f)
+__device__ __forceinline__ void walk_blocks(const float org[3], const float dir[3], const float inv[3],
+                                            uint32_t level, F&& f)
 {
     const int m = 1 << level;
     const float cell = (2.f * kTopHalf) / (float)m;
@@ -934,8 +965,7 @@ __device__ __forceinline__ void walk_blocks(const float org[3], const float dir[
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         if (fabsf(dir[a]) > 1e-10f) {
-            const float inv = 1.f / dir[a];
-            float ta = (-kTopHalf - org[a]) * inv, tb = (kTopHalf - org[a]) * inv;
+            float ta = (-kTopHalf - org[a]) * inv[a], tb = (kTopHalf - org[a]) * inv[a];
             if (ta > tb) { const float t = ta; ta = tb; tb = t; }
             t0 = fmaxf(t0, ta);
             t1 = fminf(t1, tb);
@@ -956,12 +986,12 @@ __device__ __forceinline__ void walk_blocks(const float org[3], const float dir[
         c = min(max((int)floorf((pm + kTopHalf) / cell), 0), m - 1);
         if (dir[a] > 1e-10f) {
             st = 1;
-            tmax = ((-kTopHalf + cell * (float)(c + 1)) - org[a]) / dir[a];
-            tdel = cell / dir[a];
+            tmax = div_by((-kTopHalf + cell * (float)(c + 1)) - org[a], dir[a], inv[a]);
+            tdel = div_by(cell, dir[a], inv[a]);
         } else if (dir[a] < -1e-10f) {
             st = -1;
-            tmax = ((-kTopHalf + cell * (float)c) - org[a]) / dir[a];
-            tdel = -cell / dir[a];
+            tmax = div_by((-kTopHalf + cell * (float)c) - org[a], dir[a], inv[a]);
+            tdel = div_by(-cell, dir[a], inv[a]);
         } else {
             st = 0;
             tmax = 3.4e38f;
@@ -1002,38 +1032,139 @@ struct Premul {
     float r, g, b, a;
 };
 
-// The 8 texels of sample k issued as independent loads (32-bit offsets: a brick
-// holds at most 513^3 vertices) with the cell's fractions.
+// The transfer function in shared memory as the batched kernels look it up: P holds tf_n + 2 entries, the
+// table with its first and last entry repeated, and D (tables of up to kTfDiff entries) the differences
+// P[j+1] - P[j], so that a lookup is one index, two 16-byte loads and four fmas, without clamping two indices.
+constexpr uint32_t kTfDiff = 1024;
+struct TfTable {
+    const float4* p;
+    const float4* d; // nullptr: a larger table, the difference formed at the lookup
+    __device__ const float4* raw() const { return p + 1; }
+};
+inline __host__ __device__ uint32_t tf_smem_entries(uint32_t tf_n)
+{
+    return tf_n <= kTfDiff ? 2 * tf_n + 3 : tf_n + 2;
+}
+
+// All threads of the CTA; ends with a barrier.
+__device__ __forceinline__ TfTable load_tf(float4* sm, const float* tf, uint32_t tf_n, uint32_t tid, uint32_t nthreads)
+{
+    const float4* g = reinterpret_cast<const float4*>(tf);
+    const bool diff = tf_n <= kTfDiff;
+    for (uint32_t j = tid; j < tf_n + 2; j += nthreads) {
+        const float4 a = g[min(max((int)j - 1, 0), (int)tf_n - 1)];
+        sm[j] = a;
+        if (diff && j <= tf_n) {
+            const float4 b = g[min(j, tf_n - 1)];
+            sm[tf_n + 2 + j] = make_float4(b.x - a.x, b.y - a.y, b.z - a.z, b.w - a.w);
+        }
+    }
+    __syncthreads();
+    return TfTable{sm, diff ? sm + tf_n + 2 : nullptr};
+}
+
+// tf_lookup's colour from the padded table: entry j = floor(u) + 1 within [0, tf_n] gives the clamped pair;
+// beyond the table the pair is one entry twice, so any finite fraction gives that entry.
+__device__ __forceinline__ float4 tf_colour(const TfTable& tf, uint32_t tfn, float v01)
+{
+    const float u = __fmaf_rn(v01, (float)tfn, -0.5f);
+    int j;
+    const float fl = floor_small(fminf(fmaxf(u, -1.f), (float)tfn - 0.5f), j);
+    const float f = u - fl;
+    const float4 p = tf.p[j + 1];
+    float4 d;
+    if (tf.d) {
+        d = tf.d[j + 1];
+    } else {
+        const float4 q = tf.p[j + 2];
+        d = make_float4(q.x - p.x, q.y - p.y, q.z - p.z, q.w - p.w);
+    }
+    return make_float4(__fmaf_rn(f, d.x, p.x), __fmaf_rn(f, d.y, p.y), __fmaf_rn(f, d.z, p.z), __fmaf_rn(f, d.w, p.w));
+}
+
+// The relative value (val - field_min) / span, correctly rounded: by the kept reciprocal where span is far
+// from the ends of the float range, else by a division.
+struct Relative {
+    float lo, span, y;
+    bool fast;
+    __device__ __forceinline__ float operator()(float val) const
+    {
+        const float a = __fsub_rn(val, lo);
+        return fast ? div_by(a, span, y) : __fdiv_rn(a, span);
+    }
+};
+__device__ __forceinline__ Relative relative_of(const s3r_view& v)
+{
+    const float span = v.field_max - v.field_min;
+    return Relative{v.field_min, span, __frcp_rn(span), span > 1e-18f && span < 1e18f};
+}
+
+// The 8 texels of a sample issued as independent loads (32-bit offsets: a brick holds at most 513^3 vertices)
+// with the cell's fractions: x fastest, then y, then z.
 template <int Fmt> struct Texels {
     float t[8];
     float f[3];
 };
 
-template <int Fmt>
-__device__ __forceinline__ void fetch_texels(const void* brick, const BlockRay& r, int k, Texels<Fmt>& x)
+// Sample kf (a whole number) of the ray in its block.  kTogether (the rays of a warp march one block): inside the
+// brick the cell's 8 texels are four pairs in four rows, and a sample in the outer half texel (a ray's first one, on
+// the block's face) takes the clamped indices.  Rays in different blocks meet their faces at different times, so
+// there every sample takes the clamped indices (320 x 240 pixels of a level-2 set: 109 us against 115 us).
+template <int Fmt, bool kTogether>
+__device__ __forceinline__ void fetch_texels(const void* brick, const BlockRay& r, float kf, Texels<Fmt>& x)
 {
-    Cell c;
-    sample_cell(r, k, c);
-    const uint32_t n = r.n;
+    const uint32_t hi = r.n - 1;
+    int a[3];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const uint32_t xi = (q & 1) ? c.i1[0] : c.i0[0];
-        const uint32_t yi = (q & 2) ? c.i1[1] : c.i0[1];
-        const uint32_t zi = (q & 4) ? c.i1[2] : c.i0[2];
-        x.t[q] = Brick<Fmt>::get(brick, (zi * n + yi) * r.pitch + xi);
+    for (int d = 0; d < 3; ++d) {
+        const float p = __fmaf_rn(r.step[d], kf, r.p0[d]);
+        const float tc = __fmul_rn(__fsub_rn(p, r.origin[d]), r.factor);
+        const float xb = __fsub_rn(tc, 0.5f);
+        x.f[d] = __fsub_rn(xb, floor_small(xb, a[d]));
     }
+    if (kTogether && (uint32_t)a[0] < hi && (uint32_t)a[1] < hi && (uint32_t)a[2] < hi) {
+        const uint32_t o = ((uint32_t)a[2] * r.n + (uint32_t)a[1]) * r.pitch + (uint32_t)a[0];
+        const uint32_t dz = r.n * r.pitch;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) x.f[d] = c.f[d];
+        for (int q = 0; q < 8; ++q)
+            x.t[q] = Brick<Fmt>::get(brick, (uint64_t)(o + ((q & 2) ? r.pitch : 0u) + ((q & 4) ? dz : 0u)) + (q & 1));
+    } else {
+        uint32_t i0[3], i1[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            i0[d] = (uint32_t)min(max(a[d], 0), (int)hi);
+            i1[d] = (uint32_t)min(max(a[d] + 1, 0), (int)hi);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t xi = (q & 1) ? i1[0] : i0[0];
+            const uint32_t yi = (q & 2) ? i1[1] : i0[1];
+            const uint32_t zi = (q & 4) ? i1[2] : i0[2];
+            x.t[q] = Brick<Fmt>::get(brick, (zi * r.n + yi) * r.pitch + xi);
+        }
+    }
+}
+
+// Whether one of 8 values is NaN, two values per comparison.
+__device__ __forceinline__ bool any_nan(const float t[8])
+{
+    uint32_t bad;
+    asm("{\n\t.reg .pred p;\n\t"
+        "setp.nan.f32 p, %1, %2;\n\t"
+        "setp.nan.or.f32 p, %3, %4, p;\n\t"
+        "setp.nan.or.f32 p, %5, %6, p;\n\t"
+        "setp.nan.or.f32 p, %7, %8, p;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(bad)
+        : "f"(t[0]), "f"(t[1]), "f"(t[2]), "f"(t[3]), "f"(t[4]), "f"(t[5]), "f"(t[6]), "f"(t[7]));
+    return bad != 0;
 }
 
 // Trilinear value of fetched texels; false when one of them is NaN (outside the domain).
 template <int Fmt> __device__ __forceinline__ bool filter_texels(const Texels<Fmt>& x, float& val)
 {
-    bool bad = false;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) bad |= isnan(x.t[q]);
-    if (bad) return false;
     const float* t = x.t;
+    if (any_nan(t)) return false;
     const float x00 = __fmaf_rn(x.f[0], t[1] - t[0], t[0]);
     const float x10 = __fmaf_rn(x.f[0], t[3] - t[2], t[2]);
     const float x01 = __fmaf_rn(x.f[0], t[5] - t[4], t[4]);
@@ -1045,39 +1176,49 @@ template <int Fmt> __device__ __forceinline__ bool filter_texels(const Texels<Fm
 }
 
 // March one block along a ray (premultiplied, block-local early termination).
-// Exact filter: software-pipelined -- sample k+1's texel loads are issued
-// before sample k is filtered, looked up and composited, so a ray keeps two
-// samples' loads in flight; the arithmetic and its order are unchanged.
-template <int Fmt, bool kTex>
+// Exact filter: software-pipelined over two sets of texels -- sample k+1's loads
+// are issued before sample k is filtered, looked up and composited, so a ray
+// keeps two samples' loads in flight; the arithmetic and its order are the
+// per-block kernel's.  What bounds it is the issue of the sample's instructions
+// (and, before floor_small and div_by, the conversion unit).
+template <int Fmt, bool kTex, bool kTogether>
 __device__ __forceinline__ Premul march_block(const s3r_view& v, const BlockRay& r, const void* brick, float scale,
-                                              float offset, uint32_t depth, const float4* tf, float of,
-                                              uint32_t& taken)
+                                              float offset, uint32_t depth, const TfTable& tf, const Relative& rel,
+                                              float of, uint32_t& taken)
 {
-    const float span = v.field_max - v.field_min;
     const float il = layer_exponent(depth, v.level, v.quality);
     Premul acc{0.f, 0.f, 0.f, 0.f};
+    auto blend = [&](float4 col) {
+        const float a = __fsub_rn(1.f, __powf(__fmaf_rn(-col.w, of, 1.f), il));
+        const float w = __fmul_rn(__fsub_rn(1.f, acc.a), a);
+        acc.r = __fmaf_rn(w, col.x, acc.r);
+        acc.g = __fmaf_rn(w, col.y, acc.g);
+        acc.b = __fmaf_rn(w, col.z, acc.b);
+        acc.a = __fadd_rn(acc.a, w);
+        return acc.a > kAlphaThreshold;
+    };
     if constexpr (!kTex) {
         if (r.samples < 2) return acc;
-        Texels<Fmt> cur, nxt;
-        fetch_texels<Fmt>(brick, r, 0, cur);
-        for (int i = 1; i < r.samples; ++i) {
-            ++taken;
-            if (i + 1 < r.samples) fetch_texels<Fmt>(brick, r, i, nxt);
+        Texels<Fmt> ca, cb;
+        // true: the block is opaque
+        auto sample = [&](const Texels<Fmt>& x) {
             float val;
-            if (filter_texels<Fmt>(cur, val)) {
-                if (Fmt != S3R_BRICK_F32) val = __fmaf_rn(scale, val, offset);
-                const float v01 = __fdiv_rn(__fsub_rn(val, v.field_min), span);
-                const float4 col = tf_lookup(tf, v.tf_n, v01).c;
-                const float a = __fsub_rn(1.f, __powf(__fmaf_rn(-col.w, of, 1.f), il));
-                const float w = __fmul_rn(__fsub_rn(1.f, acc.a), a);
-                acc.r = __fmaf_rn(w, col.x, acc.r);
-                acc.g = __fmaf_rn(w, col.y, acc.g);
-                acc.b = __fmaf_rn(w, col.z, acc.b);
-                acc.a = __fadd_rn(acc.a, w);
-                if (acc.a > kAlphaThreshold) break;
-            }
-            cur = nxt;
+            if (!filter_texels<Fmt>(x, val)) return false;
+            if (Fmt != S3R_BRICK_F32) val = __fmaf_rn(scale, val, offset);
+            return blend(tf_colour(tf, v.tf_n, rel(val)));
+        };
+        fetch_texels<Fmt, kTogether>(brick, r, 0.f, ca);
+        const float last = (float)(r.samples - 1); // samples 0 .. last-1
+        float k = 0.f; // the samples taken, a whole number
+        while (true) {
+            k += 1.f;
+            if (k < last) fetch_texels<Fmt, kTogether>(brick, r, k, cb);
+            if (sample(ca) || k >= last) break;
+            k += 1.f;
+            if (k < last) fetch_texels<Fmt, kTogether>(brick, r, k, ca);
+            if (sample(cb) || k >= last) break;
         }
+        taken += (uint32_t)k;
         return acc;
     } else {
         for (int i = 1; i < r.samples; ++i) {
@@ -1085,15 +1226,7 @@ __device__ __forceinline__ Premul march_block(const s3r_view& v, const BlockRay&
             float val;
             if (!tex_trilinear<Fmt>(brick, r, i - 1, val)) continue;
             if (Fmt != S3R_BRICK_F32) val = __fmaf_rn(scale, val, offset);
-            const float v01 = __fdiv_rn(__fsub_rn(val, v.field_min), span);
-            const float4 col = tex_tf_lookup(tf, v.tf_n, v01);
-            const float a = __fsub_rn(1.f, __powf(__fmaf_rn(-col.w, of, 1.f), il));
-            const float w = __fmul_rn(__fsub_rn(1.f, acc.a), a);
-            acc.r = __fmaf_rn(w, col.x, acc.r);
-            acc.g = __fmaf_rn(w, col.y, acc.g);
-            acc.b = __fmaf_rn(w, col.z, acc.b);
-            acc.a = __fadd_rn(acc.a, w);
-            if (acc.a > kAlphaThreshold) break;
+            if (blend(tex_tf_lookup(tf.raw(), v.tf_n, rel(val)))) break;
         }
         return acc;
     }
@@ -1107,7 +1240,7 @@ __device__ __forceinline__ Premul march_block(const s3r_view& v, const BlockRay&
 template <int Fmt, int R, bool kTex>
 __global__ void frame_render_kernel(FrameArgs fa)
 {
-    extern __shared__ float4 tf[];
+    extern __shared__ float4 tf_sm[];
     const s3r_view v = *fa.view;
     const uint32_t nthreads = blockDim.x * blockDim.y;
     const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x;
@@ -1128,19 +1261,21 @@ __global__ void frame_render_kernel(FrameArgs fa)
             return;
         }
     }
-    for (uint32_t i = tid; i < v.tf_n; i += nthreads) tf[i] = reinterpret_cast<const float4*>(fa.tf)[i];
-    __syncthreads();
+    const TfTable tf = load_tf(tf_sm, fa.tf, v.tf_n, tid, nthreads);
+    const Relative rel = relative_of(v);
     uint32_t taken = 0;
     Premul acc{0.f, 0.f, 0.f, 0.f};
     const bool inside = vx < v.W && vy < v.H;
     if (inside) {
         float org[3], dir[3];
         pixel_ray(v, vx, vy, org, dir);
+        float inv[3];
+        ray_inverse(dir, inv);
         const float of = (v.threshold - v.field_min) / (v.field_max - v.field_min);
         int lo = 0, hi = 1 << 30;
         if (R > 1) {
             int n = 0;
-            walk_blocks(org, dir, v.level, [&](uint32_t, uint32_t, uint32_t, uint32_t) {
+            walk_blocks(org, dir, inv, v.level, [&](uint32_t, uint32_t, uint32_t, uint32_t) {
                 ++n;
                 return true;
             });
@@ -1149,7 +1284,7 @@ __global__ void frame_render_kernel(FrameArgs fa)
             hi = lo + chunk;
         }
         int idx = 0;
-        walk_blocks(org, dir, v.level, [&](uint32_t b, uint32_t, uint32_t, uint32_t) {
+        walk_blocks(org, dir, inv, v.level, [&](uint32_t b, uint32_t, uint32_t, uint32_t) {
             if (idx >= hi) return false;
             if (idx++ < lo) return true;
             const RenderBlock* rb = &fa.table[b];
@@ -1159,7 +1294,7 @@ __global__ void frame_render_kernel(FrameArgs fa)
             const int32_t rca[4] = {rc.x, rc.y, rc.z, rc.w};
             if (!pixel_in_rect(rca, vx, vy)) return true;
             BlockRay r;
-            if (!block_ray(v, org, dir, *rb, r)) return true;
+            if (!block_ray(v, org, dir, inv, *rb, r)) return true;
             const char* base = reinterpret_cast<const char*>(fa.bricks);
             const size_t esz = Fmt == S3R_BRICK_F32 ? 4 : 2;
             float scale = 1.f, offset = 0.f;
@@ -1169,7 +1304,7 @@ __global__ void frame_render_kernel(FrameArgs fa)
                 offset = so.y;
             }
             const Premul p =
-                march_block<Fmt, kTex>(v, r, base + rb->brick_off * esz, scale, offset, depth, tf, of, taken);
+                march_block<Fmt, kTex, false>(v, r, base + rb->brick_off * esz, scale, offset, depth, tf, rel, of, taken);
             const float T = __fsub_rn(1.f, acc.a);
             acc.r = __fmaf_rn(T, p.r, acc.r);
             acc.g = __fmaf_rn(T, p.g, acc.g);
@@ -1255,12 +1390,12 @@ __device__ __forceinline__ uint32_t ray_rank(const float dir[3], uint32_t ix, ui
 template <int Fmt, bool kTex>
 __global__ void __launch_bounds__(128, 8) frame_segments_kernel(FrameArgs fa, SegArgs sa, uint32_t fx)
 {
-    extern __shared__ float4 tf[];
+    extern __shared__ float4 tf_sm[];
     const s3r_view v = *fa.view;
     const uint32_t nthreads = blockDim.x * blockDim.y;
     const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x;
-    for (uint32_t i = tid; i < v.tf_n; i += nthreads) tf[i] = reinterpret_cast<const float4*>(fa.tf)[i];
-    __syncthreads();
+    const TfTable tf = load_tf(tf_sm, fa.tf, v.tf_n, tid, nthreads);
+    const Relative rel = relative_of(v);
     const uint32_t lane = tid & 31u;
     const uint32_t fy = 32u / fx;
     const uint32_t total = *sa.count;
@@ -1295,8 +1430,10 @@ __global__ void __launch_bounds__(128, 8) frame_segments_kernel(FrameArgs fa, Se
         if (x < rc.x + rc.z && y < rc.y + rc.w && x >= 0 && y >= 0 && x < (int32_t)v.W && y < (int32_t)v.H) {
             float org[3], dir[3];
             pixel_ray(v, (uint32_t)x, (uint32_t)y, org, dir);
+            float inv[3];
+            ray_inverse(dir, inv);
             BlockRay r;
-            if (block_ray(v, org, dir, *rb, r)) {
+            if (block_ray(v, org, dir, inv, *rb, r)) {
                 const char* base = reinterpret_cast<const char*>(fa.bricks);
                 const size_t esz = Fmt == S3R_BRICK_F32 ? 4 : 2;
                 float scale = 1.f, offset = 0.f;
@@ -1305,8 +1442,8 @@ __global__ void __launch_bounds__(128, 8) frame_segments_kernel(FrameArgs fa, Se
                     scale = so.x;
                     offset = so.y;
                 }
-                const Premul p = march_block<Fmt, kTex>(v, r, base + rb->brick_off * esz, scale, offset, rb->depth,
-                                                        tf, of, taken);
+                const Premul p = march_block<Fmt, kTex, true>(v, r, base + rb->brick_off * esz, scale, offset, rb->depth,
+                                                        tf, rel, of, taken);
                 if (!(p.r == 0.f && p.g == 0.f && p.b == 0.f && p.a == 0.f)) {
                     const uint32_t ix = cell % m, iy = (cell / m) % m, iz = cell / (m * m);
                     const uint32_t k = ray_rank(dir, ix, iy, iz, m);
@@ -1391,8 +1528,10 @@ __global__ void frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr
     if ((int32_t)vx >= cv.x && (int32_t)vx < cv.z && (int32_t)vy >= cv.y && (int32_t)vy < cv.w) {
         float org[3], dir[3];
         pixel_ray(v, vx, vy, org, dir);
+        float inv[3];
+        ray_inverse(dir, inv);
         const float* bricks = reinterpret_cast<const float*>(fa.bricks);
-        walk_blocks(org, dir, v.level, [&](uint32_t b, uint32_t, uint32_t, uint32_t) {
+        walk_blocks(org, dir, inv, v.level, [&](uint32_t b, uint32_t, uint32_t, uint32_t) {
             const RenderBlock* rb = &fa.table[b];
             const uint32_t depth = rb->depth;
             if (depth == 0xffffffffu) return true;
@@ -1400,7 +1539,7 @@ __global__ void frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr
             const int32_t rca[4] = {rc.x, rc.y, rc.z, rc.w};
             if (!pixel_in_rect(rca, vx, vy)) return true;
             BlockRay r;
-            if (!block_ray(v, org, dir, *rb, r)) return true;
+            if (!block_ray(v, org, dir, inv, *rb, r)) return true;
             const BrickSampler<kTex> smp{bricks + rb->brick_off, bricks2 ? bricks2 + rb->brick_off : nullptr, dim_of(r),
                                          tf, v.tf_n};
             const ModeOut o = march_block_mode(v, pr, smp, r, depth);
@@ -1513,6 +1652,8 @@ __global__ void __launch_bounds__(128, 4) frame_backward_kernel(FrameArgs fa)
         if (active) {
             float org[3], dir[3];
             pixel_ray(v, vx, vy, org, dir);
+        float inv[3];
+        ray_inverse(dir, inv);
             const float span = v.field_max - v.field_min;
             const float inv_span = 1.f / span;
             const float of = (v.threshold - v.field_min) / span;
@@ -1530,7 +1671,7 @@ __global__ void __launch_bounds__(128, 4) frame_backward_kernel(FrameArgs fa)
                     tf_b[ch] = 0.f;
                 }
             };
-            walk_blocks(org, dir, v.level, [&](uint32_t b, uint32_t ix, uint32_t iy, uint32_t iz) {
+            walk_blocks(org, dir, inv, v.level, [&](uint32_t b, uint32_t ix, uint32_t iy, uint32_t iz) {
                 const RenderBlock* rb = &fa.table[b];
                 const uint32_t depth = rb->depth;
                 if (depth == 0xffffffffu) return true;
@@ -1538,7 +1679,7 @@ __global__ void __launch_bounds__(128, 4) frame_backward_kernel(FrameArgs fa)
                 const int32_t rca[4] = {rc.x, rc.y, rc.z, rc.w};
                 if (!pixel_in_rect(rca, vx, vy)) return true;
                 BlockRay r;
-                if (!block_ray(v, org, dir, *rb, r)) return true;
+                if (!block_ray(v, org, dir, inv, *rb, r)) return true;
                 const float* brick = reinterpret_cast<const float*>(fa.bricks) + rb->brick_off;
                 float* gdense = fa.ddense + rb->brick_off;
                 const float il = layer_exponent(depth, v.level, v.quality);
@@ -1760,7 +1901,7 @@ cudaError_t launch_frame_render(const FrameArgs& a, uint32_t W, uint32_t H, uint
     const int px = sx / (int)R > 0 ? sx / (int)R : 1;
     dim3 block(px * R, sy);
     dim3 grid((W + px - 1) / px, (H + sy - 1) / sy);
-    const size_t smem = tf_n * sizeof(float4);
+    const size_t smem = tf_smem_entries(tf_n) * sizeof(float4);
     const bool tex = filter == S3R_FILTER_TEXTURE;
     switch (fmt) {
     case S3R_BRICK_F32:
@@ -1799,7 +1940,7 @@ cudaError_t launch_frame_segments(const FrameArgs& a, const SegArgs& sa, uint32_
     shape %= kSegShapes;
     const uint32_t fx = (uint32_t)kSegShapeX[shape];
     const dim3 block(128); // four warps, each on its own items
-    const size_t smem = tf_n * sizeof(float4);
+    const size_t smem = tf_smem_entries(tf_n) * sizeof(float4);
     const bool tex = filter == S3R_FILTER_TEXTURE;
     cudaError_t err;
     switch (fmt) {
