@@ -99,9 +99,9 @@ uint64_t s3r_ctx_launch_count(const s3r_ctx* ctx);
  * node, the BlockTreeNodes<3> n2i layout); sparse (device): n values aligned
  * with n2i, S3R_NO_FIELD_VALUE where masked; dense (device): receives the grid,
  * x fastest (ordinal (z*e + y)*e + x with e = 2^depth+1), NaN outside the
- * domain.  Scratch: a (2^depth+1)^3 float grid owned by the context, grown on
- * demand (the call may allocate device memory the first time it sees a
- * larger depth).  Bit-identical to the reference CPU interpolator. */
+ * domain.  Scratch (depth 5 and up): a (2^depth+1)^3 float grid and a mask of as
+ * many bits (rows of whole words) owned by the context, grown on demand (the call
+ * may allocate device memory the first time it sees a larger depth).  Bit-identical to the reference CPU interpolator. */
 int s3r_interp_dense(s3r_ctx* ctx, const uint16_t* n2i_xyz, const float* sparse, uint32_t n, uint32_t depth,
                      float* dense, void* stream);
 
@@ -269,8 +269,8 @@ int s3r_texture_create(s3r_ctx* ctx, uint32_t depth, s3r_texture** out);
 int s3r_texture_destroy(s3r_texture* tex);
 /* Copies a dense grid (device, (2^depth+1)^3 floats in the s3r_interp_dense layout) into the texture. */
 int s3r_texture_fill(s3r_ctx* ctx, s3r_texture* tex, const float* dense, void* stream);
-/* s3r_interp_dense into the texture (DeviceField::makeField, DenseFieldRenderer_cu.cu:505-546): the grid
- * is interpolated into a context-owned linear grid (grown on demand) and copied into the array. */
+/* s3r_interp_dense into the texture (DeviceField::makeField, DenseFieldRenderer_cu.cu:505-546): the tiles are
+ * written to the array in place, with s3r_interp_dense's scratch. */
 int s3r_interp_dense_texture(s3r_ctx* ctx, const uint16_t* n2i_xyz, const float* sparse, uint32_t n,
                              s3r_texture* tex, void* stream);
 /* A transfer-function texture of tf_n entries (makeColorTransferTexture, DenseFieldRenderer_cu.cu:566-586:

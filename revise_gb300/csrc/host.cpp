@@ -28,8 +28,10 @@ thread_local std::string g_last_error;
 struct s3r_ctx {
     int device = 0;
     std::string err;
-    float* grid = nullptr; // single-block interpolation scratch
+    float* grid = nullptr; // block interpolation scratch: scattered node values, and their mask (rows of whole words)
     size_t grid_cap = 0;   // floats
+    uint32_t* grid_bits = nullptr;
+    size_t grid_bits_cap = 0; // words
     int32_t* rect_dev = nullptr;
     int32_t* rect_host = nullptr; // pinned
     s3r_image_part* parts_dev = nullptr;
@@ -38,11 +40,9 @@ struct s3r_ctx {
     float* worker_dense[2] = {nullptr, nullptr}; // s3r_render_scene_part: primary / secondary dense field
     size_t worker_cap[2] = {0, 0};
     // s3r_render_scene_part with the texture filter: per depth a primary / secondary field texture, the
-    // transfer-function texture, and the linear grid s3r_interp_dense_texture interpolates into
+    // transfer-function texture
     s3r_texture* worker_tex[2][S3R_MAX_DEPTH + 1] = {};
     s3r_tf_texture* worker_tf = nullptr;
-    float* tex_stage = nullptr;
-    size_t tex_stage_cap = 0;
     uint64_t launches = 0;
     int sms = 152;
 };
@@ -141,6 +141,7 @@ struct s3r_texture {
     uint32_t depth = 0, n = 0;
     cudaArray_t array = nullptr;
     cudaTextureObject_t tex = 0;
+    cudaSurfaceObject_t surf = 0; // the interpolation writes the array in place
 };
 
 // The transfer function as the reference's colour texture (makeColorTransferTexture,
@@ -978,6 +979,7 @@ int s3r_ctx_destroy(s3r_ctx* ctx)
     if (!ctx) return S3R_OK;
     cudaSetDevice(ctx->device);
     if (ctx->grid) cudaFree(ctx->grid);
+    if (ctx->grid_bits) cudaFree(ctx->grid_bits);
     if (ctx->rect_dev) cudaFree(ctx->rect_dev);
     if (ctx->rect_host) cudaFreeHost(ctx->rect_host);
     if (ctx->parts_dev) cudaFree(ctx->parts_dev);
@@ -987,8 +989,50 @@ int s3r_ctx_destroy(s3r_ctx* ctx)
     for (auto& per_field : ctx->worker_tex)
         for (s3r_texture* t : per_field) s3r_texture_destroy(t);
     s3r_tf_texture_destroy(ctx->worker_tf);
-    if (ctx->tex_stage) cudaFree(ctx->tex_stage);
     delete ctx;
+    return S3R_OK;
+}
+
+// The context's block interpolation scratch for this many scattered values and mask words (grown on demand).
+static int ensure_grid(s3r_ctx* ctx, uint64_t values, uint64_t words)
+{
+    if (ctx->grid_cap < values) {
+        if (ctx->grid) cudaFree(ctx->grid);
+        ctx->grid = nullptr;
+        ctx->grid_cap = 0;
+        S3R_CUDA(ctx, cudaMalloc(&ctx->grid, values * sizeof(float)));
+        ctx->grid_cap = values;
+    }
+    if (ctx->grid_bits_cap < words) {
+        if (ctx->grid_bits) cudaFree(ctx->grid_bits);
+        ctx->grid_bits = nullptr;
+        ctx->grid_bits_cap = 0;
+        S3R_CUDA(ctx, cudaMalloc(&ctx->grid_bits, words * sizeof(uint32_t)));
+        ctx->grid_bits_cap = words;
+    }
+    return S3R_OK;
+}
+
+// One subtree from its nodes into a dense grid, or into the 3-D array behind `surface` when dense is NULL.
+static int interp_block(s3r_ctx* ctx, const uint16_t* n2i, const float* sparse, uint32_t n, uint32_t depth, float* dense,
+                        unsigned long long surface, cudaStream_t s)
+{
+    GridArgs a{};
+    a.one = grid_block(n2i, sparse, n, depth);
+    a.one.out = dense;
+    a.one.surface = surface;
+    a.nblocks = 1;
+    a.tiles = grid_tiles(depth);
+    a.depth_max = depth;
+    const uint64_t words = a.one.direct ? 0 : grid_mask_words(depth);
+    if (words) {
+        if (int rc = ensure_grid(ctx, grid_vertices(depth), words)) return rc;
+        a.vals = ctx->grid;
+        a.bits = ctx->grid_bits;
+    }
+    uint32_t launches = 0;
+    S3R_CUDA(ctx, launch_interp_grid(a, dense == nullptr, words ? n : 0, words, s, &launches));
+    ctx->launches += launches;
     return S3R_OK;
 }
 
@@ -1000,22 +1044,7 @@ int s3r_interp_dense(s3r_ctx* ctx, const uint16_t* n2i_xyz, const float* sparse,
     if (!dense || (n > 0 && (!n2i_xyz || !sparse))) return fail(ctx, S3R_ERR_INVALID, "null pointer");
     int rc = set_device(ctx);
     if (rc) return rc;
-    const uint64_t e = (1ull << depth) + 1ull;
-    const uint64_t count = e * e * e;
-    if (ctx->grid_cap < count) {
-        if (ctx->grid) cudaFree(ctx->grid);
-        ctx->grid = nullptr;
-        ctx->grid_cap = 0;
-        S3R_CUDA(ctx, cudaMalloc(&ctx->grid, count * sizeof(float)));
-        ctx->grid_cap = count;
-    }
-    cudaStream_t s = as_stream(stream);
-    S3R_CUDA(ctx, launch_fill_f32(ctx->grid, count, __builtin_nanf(""), s));
-    S3R_CUDA(ctx, launch_scatter_nodes(ctx->grid, depth, n2i_xyz, sparse, n, s));
-    uint32_t launches = 0;
-    S3R_CUDA(ctx, launch_interp_grid(ctx->grid, depth, dense, s, &launches));
-    ctx->launches += 1 + (n > 0 ? 1 : 0) + launches;
-    return S3R_OK;
+    return interp_block(ctx, n2i_xyz, sparse, n, depth, dense, 0, as_stream(stream));
 }
 
 int s3r_camera_look_at(const double eye[3], const double center[3], const double up[3], double fovy_deg, uint32_t W,
@@ -1347,6 +1376,7 @@ int s3r_texture_create(s3r_ctx* ctx, uint32_t depth, s3r_texture** out)
         td.addressMode[0] = td.addressMode[1] = td.addressMode[2] = cudaAddressModeClamp;
         td.readMode = cudaReadModeElementType;
         e = cudaCreateTextureObject(&t->tex, &res, &td, nullptr);
+        if (e == cudaSuccess) e = cudaCreateSurfaceObject(&t->surf, &res);
     }
     if (e != cudaSuccess) {
         s3r_texture_destroy(t);
@@ -1361,6 +1391,7 @@ int s3r_texture_destroy(s3r_texture* t)
     if (!t) return S3R_OK;
     if (t->ctx) cudaSetDevice(t->ctx->device);
     if (t->tex) cudaDestroyTextureObject(t->tex);
+    if (t->surf) cudaDestroySurfaceObject(t->surf);
     if (t->array) cudaFreeArray(t->array);
     delete t;
     return S3R_OK;
@@ -1389,16 +1420,8 @@ int s3r_interp_dense_texture(s3r_ctx* ctx, const uint16_t* n2i_xyz, const float*
     if (t->ctx != ctx) return fail(ctx, S3R_ERR_INVALID, "texture belongs to another context");
     int rc = set_device(ctx);
     if (rc) return rc;
-    const uint64_t count = (uint64_t)t->n * t->n * t->n;
-    if (ctx->tex_stage_cap < count) {
-        if (ctx->tex_stage) cudaFree(ctx->tex_stage);
-        ctx->tex_stage = nullptr;
-        ctx->tex_stage_cap = 0;
-        S3R_CUDA(ctx, cudaMalloc(&ctx->tex_stage, count * sizeof(float)));
-        ctx->tex_stage_cap = count;
-    }
-    if ((rc = s3r_interp_dense(ctx, n2i_xyz, sparse, n, t->depth, ctx->tex_stage, stream))) return rc;
-    return s3r_texture_fill(ctx, t, ctx->tex_stage, stream);
+    if (n > 0 && (!n2i_xyz || !sparse)) return fail(ctx, S3R_ERR_INVALID, "null pointer");
+    return interp_block(ctx, n2i_xyz, sparse, n, t->depth, nullptr, t->surf, as_stream(stream));
 }
 
 int s3r_tf_texture_create(s3r_ctx* ctx, uint32_t tf_n, s3r_tf_texture** out)

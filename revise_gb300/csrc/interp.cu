@@ -34,57 +34,99 @@
 namespace s3r {
 namespace {
 
-__global__ void fill_f32_kernel(float* p, uint64_t n, float v)
-{
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        p[i] = v;
-}
-
 __global__ void fill_u32_kernel(uint32_t* p, uint64_t n, uint32_t v)
 {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         p[i] = v;
 }
 
-// dense[ord(n2i[i])] = sparse[i]  (scatterSparseFieldKernel, DenseFieldInterpolatorArr_cu_3.cu:38-51)
-__global__ void scatter_kernel(float* grid, uint32_t e, const uint16_t* n2i, const float* sparse, uint32_t n)
+// vals[ord(n2i[i])] = sparse[i] and the vertex's bit, for the scattered blocks of a set (block blockIdx.y)
+// (scatterSparseFieldKernel, DenseFieldInterpolatorArr_cu_3.cu:38-51)
+__global__ void scatter_kernel(GridArgs a)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t x = n2i[3 * i], y = n2i[3 * i + 1], z = n2i[3 * i + 2];
+    const GridBlock b = a.table ? a.table[blockIdx.y] : a.one;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b.direct || i >= b.n) return;
+    const uint32_t e = (1u << b.depth) + 1u, words = (e + 31) / 32;
+    const uint32_t x = b.n2i[3 * (size_t)i], y = b.n2i[3 * (size_t)i + 1], z = b.n2i[3 * (size_t)i + 2];
     if (x >= e || y >= e || z >= e) return; // out-of-range node: ignored (the reference asserts)
-    grid[((uint64_t)z * e + y) * e + x] = sparse[i];
+    const uint64_t row = (uint64_t)z * e + y;
+    a.vals[b.val_off + row * e + x] = b.sparse[i];
+    atomicOr(&a.bits[b.bit_off + row * words + (x >> 5)], 1u << (x & 31));
 }
 
-// Work item `item` of the batched plan (kGrid: tile `item` of the single grid) as the tile it names.
-template <bool kGrid> __device__ __forceinline__ TileItem decode_item(const TileArgs& a, uint32_t item)
+// The blocks of a set from their node lists, one CTA per tile (a set of one block: its tile is the CTA index; else
+// the block is found in the running tile counts).  kSurface: into 3-D arrays, else into plain grids.
+// Bound by the latency of a tile's phases, 8 CTAs per SM in flight; reading the mask instead of a NaN-filled grid
+// took the fill pass away and shortened the tile's first phase from 39 dependent grid loads a thread to a few.
+template <bool kSurface> __global__ void __launch_bounds__(kInterpThreads, 8) interp_grid_kernel(GridArgs a)
+{
+    extern __shared__ float4 s_tile[]; // tile_smem_bytes(): (2^k+1)^3 floats rounded up to whole float4s
+    float* s = reinterpret_cast<float*>(s_tile);
+    __shared__ float desc[27];                   // direct: the lattice of tile corners of a block of 8 tiles
+    __shared__ uint32_t row_mask[17 * 17];       // per row of the tile the vertices that hold a node
+    __shared__ uint32_t flags[(8 * 8 * 8) / 32]; // one bit per finest cube
+    uint32_t tile = blockIdx.x;
+    GridBlock b = a.one;
+    if (a.table) {
+        uint32_t lo = 0, hi = a.nblocks;
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (a.tile_off[mid] <= tile) lo = mid;
+            else hi = mid;
+        }
+        b = a.table[lo];
+        tile -= a.tile_off[lo];
+    }
+    const uint32_t k = b.depth < kGridTileLog2 ? b.depth : kGridTileLog2, L = b.depth - k, mL = 1u << L;
+    const uint32_t tx = tile & (mL - 1), ty = (tile >> L) & (mL - 1), tz = tile >> (2 * L);
+    const uint32_t e = (1u << b.depth) + 1u;
+    auto run = [&](auto size) {
+        constexpr uint32_t T = decltype(size)::value;
+        if constexpr (kSurface) {
+            run_grid_tile<T>(b, a.vals, a.bits, s, desc, row_mask, flags, tx, ty, tz,
+                             [&](uint32_t x, uint32_t y, uint32_t z) {
+                                 return SurfaceCursor{b.surface, (int)x, (int)y, (int)z};
+                             },
+                             [&](uint32_t x, uint32_t y, uint32_t z, float v) {
+                                 surf3Dwrite(v, (cudaSurfaceObject_t)b.surface, (int)x * 4, (int)y, (int)z);
+                             });
+        } else {
+            // (2^9+1)^3 elements: offsets fit 32 bits.  A cube's low corner has even coordinates, so its first row
+            // starts at an even element of the grid: the parities are the grid's own.
+            const uint32_t odd = (uint32_t)(reinterpret_cast<uintptr_t>(b.out) >> 2) & 1u;
+            run_grid_tile<T>(b, a.vals, a.bits, s, desc, row_mask, flags, tx, ty, tz,
+                             [&](uint32_t x, uint32_t y, uint32_t z) {
+                                 return GridCursor{b.out + ((z * e + y) * e + x), e, e * e, odd, x == 0};
+                             },
+                             [&](uint32_t x, uint32_t y, uint32_t z, float v) { b.out[(z * e + y) * e + x] = v; });
+        }
+    };
+    switch (k) {
+    case 0: run(std::integral_constant<uint32_t, 1>()); break;
+    case 1: run(std::integral_constant<uint32_t, 2>()); break;
+    case 2: run(std::integral_constant<uint32_t, 4>()); break;
+    case 3: run(std::integral_constant<uint32_t, 8>()); break;
+    default: run(std::integral_constant<uint32_t, 16>()); break;
+    }
+}
+
+// Work item `item` of the batched plan as the tile it names.
+__device__ __forceinline__ TileItem decode_item(const TileArgs& a, uint32_t item)
 {
     TileItem t;
-    uint32_t tile;
     t.item = item;
-    t.blk = 0;
-    t.slots = 1;
-    t.node_base = 0;
-    t.dense_off = 0;
-    if constexpr (kGrid) {
-        t.d = a.grid_depth;
-        t.k = a.grid_tile_log2 < t.d ? a.grid_tile_log2 : t.d;
-        t.L = t.d - t.k;
-        t.pitch = (1u << t.d) + 1u;
-        tile = item;
-    } else {
-        const uint2 it = a.items[item];
-        t.blk = it.x;
-        tile = it.y & 0x7fffffffu;
-        t.slots = it.y >> 31;
-        const PlanBlock b = a.blocks[t.blk];
-        t.d = b.depth;
-        t.k = b.tile_log2;
-        t.L = b.coarse_log2;
-        t.node_base = b.node_base;
-        t.dense_off = b.dense_off;
-        t.pitch = b.pitch;
-    }
+    const uint2 it = a.items[item];
+    t.blk = it.x;
+    const uint32_t tile = it.y & 0x7fffffffu;
+    t.slots = it.y >> 31;
+    const PlanBlock b = a.blocks[t.blk];
+    t.d = b.depth;
+    t.k = b.tile_log2;
+    t.L = b.coarse_log2;
+    t.node_base = b.node_base;
+    t.dense_off = b.dense_off;
+    t.pitch = b.pitch;
     const uint32_t mL = 1u << t.L;
     t.tx = tile & (mL - 1);
     t.ty = (tile >> t.L) & (mL - 1);
@@ -92,44 +134,40 @@ template <bool kGrid> __device__ __forceinline__ TileItem decode_item(const Tile
     return t;
 }
 
-template <bool kGrid, typename OutT>
+template <typename OutT>
 __global__ void __launch_bounds__(kInterpThreads, 8) interp_tiles_kernel(TileArgs a)
 {
     extern __shared__ float4 s_tile[]; // tile_smem_bytes(): (2^k+1)^3 floats rounded up to whole float4s
     float* s = reinterpret_cast<float*>(s_tile);
-    __shared__ float desc[27 * kMaxDescentLevels];
     __shared__ uint32_t flags[(16 * 16 * 16) / 32]; // one bit per finest cube, tiles up to 32 cells
     __shared__ uint32_t item_s, next_s[2];
     const uint32_t nitems = a.nitems;
     const Crew<kInterpThreads> cw{threadIdx.x};
-    // Work items come from the queue counter when there is one (zeroed before
-    // the launch), else item blockIdx.x once per CTA.  The next item is taken
-    // at the start of the current one so its entries can be prefetched.  The
-    // slot it goes to alternates: a warp still reading slot i & 1 after the
-    // loop's closing barrier must not see thread 0 refill it for item i + 2
-    // (the barriers inside the tile keep thread 0 from getting that far).
-    if (threadIdx.x == 0) item_s = a.queue ? atomicAdd(a.queue, 1u) : blockIdx.x;
+    // Work items come from the queue counter (zeroed before the launch).  The
+    // next item is taken at the start of the current one so its entries can be
+    // prefetched.  The slot it goes to alternates: a warp still reading slot
+    // i & 1 after the loop's closing barrier must not see thread 0 refill it for
+    // item i + 2 (the barriers inside the tile keep thread 0 from getting that far).
+    if (threadIdx.x == 0) item_s = atomicAdd(a.queue, 1u);
     __syncthreads();
     uint32_t item = item_s;
     Prefetch pf;
-    if constexpr (!kGrid) {
-        prefetch_head<kInterpThreads>(pf, a, item, threadIdx.x);
-        prefetch_index<kInterpThreads>(pf, a, threadIdx.x);
-        prefetch_values<kInterpThreads>(pf, a, threadIdx.x);
-    }
+    prefetch_head<kInterpThreads>(pf, a, item, threadIdx.x);
+    prefetch_index<kInterpThreads>(pf, a, threadIdx.x);
+    prefetch_values<kInterpThreads>(pf, a, threadIdx.x);
     for (uint32_t iter = 0;; ++iter) {
         if (item >= nitems) break;
         uint32_t* next_p = &next_s[iter & 1];
-        if (threadIdx.x == 0) *next_p = a.queue ? atomicAdd(a.queue, 1u) : nitems;
-        const TileItem t = decode_item<kGrid>(a, item);
+        if (threadIdx.x == 0) *next_p = atomicAdd(a.queue, 1u);
+        const TileItem t = decode_item(a, item);
         auto next = [next_p] { return *next_p; };
         switch (t.k) {
-        case 0: run_tile<1, kGrid, OutT>(a, s, desc, flags, t, pf, cw, next); break;
-        case 1: run_tile<2, kGrid, OutT>(a, s, desc, flags, t, pf, cw, next); break;
-        case 2: run_tile<4, kGrid, OutT>(a, s, desc, flags, t, pf, cw, next); break;
-        case 3: run_tile<8, kGrid, OutT>(a, s, desc, flags, t, pf, cw, next); break;
-        case 4: run_tile<16, kGrid, OutT>(a, s, desc, flags, t, pf, cw, next); break;
-        default: run_tile<32, kGrid, OutT>(a, s, desc, flags, t, pf, cw, next); break;
+        case 0: run_tile<1, OutT>(a, s, flags, t, pf, cw, next); break;
+        case 1: run_tile<2, OutT>(a, s, flags, t, pf, cw, next); break;
+        case 2: run_tile<4, OutT>(a, s, flags, t, pf, cw, next); break;
+        case 3: run_tile<8, OutT>(a, s, flags, t, pf, cw, next); break;
+        case 4: run_tile<16, OutT>(a, s, flags, t, pf, cw, next); break;
+        default: run_tile<32, OutT>(a, s, flags, t, pf, cw, next); break;
         }
         __syncthreads();
         item = *next_p;
@@ -160,13 +198,13 @@ template <typename OutT> __global__ void __launch_bounds__(kInterpThreads, 8) in
     prefetch_values<32>(pf, a, lane);
     while (item < nitems) {
         const uint32_t nxt = lane == 0 ? atomicAdd(a.queue, 1u) : 0u; // read by the warp once placed
-        const TileItem t = decode_item<false>(a, item);
+        const TileItem t = decode_item(a, item);
         auto next = [nxt] { return __shfl_sync(0xffffffffu, nxt, 0); };
         switch (t.k) {
-        case 0: run_tile<1, false, OutT>(a, s, nullptr, flags, t, pf, cw, next); break;
-        case 1: run_tile<2, false, OutT>(a, s, nullptr, flags, t, pf, cw, next); break;
-        case 2: run_tile<4, false, OutT>(a, s, nullptr, flags, t, pf, cw, next); break;
-        default: run_tile<8, false, OutT>(a, s, nullptr, flags, t, pf, cw, next); break;
+        case 0: run_tile<1, OutT>(a, s, flags, t, pf, cw, next); break;
+        case 1: run_tile<2, OutT>(a, s, flags, t, pf, cw, next); break;
+        case 2: run_tile<4, OutT>(a, s, flags, t, pf, cw, next); break;
+        default: run_tile<8, OutT>(a, s, flags, t, pf, cw, next); break;
         }
         __syncwarp();
         item = __shfl_sync(0xffffffffu, nxt, 0);
@@ -279,17 +317,15 @@ inline uint32_t ctas_for(uint64_t n, uint32_t threads)
     return c ? (uint32_t)c : 1u;
 }
 
-template <bool kGrid, typename OutT>
+template <typename OutT>
 cudaError_t launch_tiles(const TileArgs& a, uint32_t tile_log2_max, uint32_t grid_ctas, cudaStream_t s)
 {
-    if constexpr (!kGrid) {
-        if (tile_log2_max <= 3 && a.queue) {
-            interp_warp_tiles_kernel<OutT><<<grid_ctas, kInterpThreads, 0, s>>>(a);
-            return cudaGetLastError();
-        }
+    if (tile_log2_max <= 3) {
+        interp_warp_tiles_kernel<OutT><<<grid_ctas, kInterpThreads, 0, s>>>(a);
+        return cudaGetLastError();
     }
     const size_t smem = tile_smem_bytes(tile_log2_max);
-    auto kern = interp_tiles_kernel<kGrid, OutT>;
+    auto kern = interp_tiles_kernel<OutT>;
     if (smem > 48 * 1024) {
         cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return err;
@@ -300,37 +336,41 @@ cudaError_t launch_tiles(const TileArgs& a, uint32_t tile_log2_max, uint32_t gri
 
 } // namespace
 
-cudaError_t launch_fill_f32(float* p, uint64_t n, float v, cudaStream_t s)
-{
-    fill_f32_kernel<<<ctas_for(n, 256), 256, 0, s>>>(p, n, v);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_fill_u32(uint32_t* p, uint64_t n, uint32_t v, cudaStream_t s)
 {
     fill_u32_kernel<<<ctas_for(n, 256), 256, 0, s>>>(p, n, v);
     return cudaGetLastError();
 }
 
-cudaError_t launch_scatter_nodes(float* grid, uint32_t depth, const uint16_t* n2i, const float* sparse, uint32_t n,
-                                 cudaStream_t s)
+GridBlock grid_block(const uint16_t* n2i, const float* sparse, uint32_t n, uint32_t depth)
 {
-    if (n == 0) return cudaSuccess;
-    scatter_kernel<<<(n + 255) / 256, 256, 0, s>>>(grid, (1u << depth) + 1u, n2i, sparse, n);
-    return cudaGetLastError();
+    GridBlock b{};
+    b.n2i = n2i;
+    b.sparse = sparse;
+    b.n = n;
+    b.depth = depth;
+    b.direct = depth <= kGridTileLog2 || (depth == kGridTileLog2 + 1 && n <= kGridDirectNodes);
+    return b;
 }
 
-cudaError_t launch_interp_grid(const float* grid, uint32_t depth, float* dense, cudaStream_t s, uint32_t* launches)
+cudaError_t launch_interp_grid(const GridArgs& a, bool surface, uint32_t scattered_nodes, uint64_t bit_words,
+                               cudaStream_t s, uint32_t* launches)
 {
-    TileArgs a{};
-    a.grid = grid;
-    a.grid_depth = depth;
-    a.grid_tile_log2 = depth < 4 ? depth : 4;
-    const uint32_t L = depth - a.grid_tile_log2;
-    a.nitems = 1u << (3 * L);
-    a.out = dense;
-    if (launches) ++*launches;
-    return launch_tiles<true, float>(a, a.grid_tile_log2, a.nitems, s);
+    uint32_t count = 1, depth_max = a.depth_max;
+    cudaError_t err;
+    if (bit_words) {
+        if ((err = cudaMemsetAsync(a.bits, 0, bit_words * sizeof(uint32_t), s)) != cudaSuccess) return err;
+        if (scattered_nodes) {
+            scatter_kernel<<<dim3((scattered_nodes + 255) / 256, a.nblocks), 256, 0, s>>>(a);
+            if ((err = cudaGetLastError()) != cudaSuccess) return err;
+            ++count;
+        }
+    }
+    const size_t smem = tile_smem_bytes(depth_max < kGridTileLog2 ? depth_max : kGridTileLog2);
+    if (surface) interp_grid_kernel<true><<<a.tiles, kInterpThreads, smem, s>>>(a);
+    else interp_grid_kernel<false><<<a.tiles, kInterpThreads, smem, s>>>(a);
+    if (launches) *launches += count;
+    return cudaGetLastError();
 }
 
 uint32_t interp_plan_ctas_per_sm(uint32_t fmt, uint32_t tile_log2)
@@ -344,10 +384,10 @@ uint32_t interp_plan_ctas_per_sm(uint32_t fmt, uint32_t tile_log2)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kInterpThreads, smem);
     };
     switch (fmt) {
-    case S3R_BRICK_F32: warp ? occ(interp_warp_tiles_kernel<float>) : occ(interp_tiles_kernel<false, float>); break;
-    case S3R_BRICK_F16: warp ? occ(interp_warp_tiles_kernel<__half>) : occ(interp_tiles_kernel<false, __half>); break;
+    case S3R_BRICK_F32: warp ? occ(interp_warp_tiles_kernel<float>) : occ(interp_tiles_kernel<float>); break;
+    case S3R_BRICK_F16: warp ? occ(interp_warp_tiles_kernel<__half>) : occ(interp_tiles_kernel<__half>); break;
     case S3R_BRICK_BF16:
-        warp ? occ(interp_warp_tiles_kernel<__nv_bfloat16>) : occ(interp_tiles_kernel<false, __nv_bfloat16>);
+        warp ? occ(interp_warp_tiles_kernel<__nv_bfloat16>) : occ(interp_tiles_kernel<__nv_bfloat16>);
         break;
     default: break;
     }
@@ -359,9 +399,9 @@ cudaError_t launch_interp_plan(const TileArgs& a, uint32_t fmt, uint32_t tile_lo
 {
     if (a.nitems == 0) return cudaSuccess;
     switch (fmt) {
-    case S3R_BRICK_F32: return launch_tiles<false, float>(a, tile_log2_max, grid_ctas, s);
-    case S3R_BRICK_F16: return launch_tiles<false, __half>(a, tile_log2_max, grid_ctas, s);
-    case S3R_BRICK_BF16: return launch_tiles<false, __nv_bfloat16>(a, tile_log2_max, grid_ctas, s);
+    case S3R_BRICK_F32: return launch_tiles<float>(a, tile_log2_max, grid_ctas, s);
+    case S3R_BRICK_F16: return launch_tiles<__half>(a, tile_log2_max, grid_ctas, s);
+    case S3R_BRICK_BF16: return launch_tiles<__nv_bfloat16>(a, tile_log2_max, grid_ctas, s);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -91,8 +91,8 @@ __device__ __forceinline__ float inf_to_nan(float v) { return __fmaf_rn(0.f, v, 
 // before.  NaN keeps its meaning "not computed yet".
 __device__ __forceinline__ float to_internal(float v) { return v == kNoField ? __int_as_float(0x7f800000) : v; }
 
-// Descent slots: 27 points (3x3x3, x fastest) per coarse level.
-constexpr int kMaxDescentLevels = S3R_MAX_DEPTH;
+// Coarse levels above a tile of 2^kGridTileLog2 cells.
+constexpr uint32_t kMaxGridLevels = S3R_MAX_DEPTH - kGridTileLog2;
 
 // The threads that run one tile: a CTA of kInterpThreads (kN = kInterpThreads, CTA barriers) or one warp
 // (kN = 32, warp barriers; the warp-per-tile kernel for tiles of up to 8 cells).  tid is the thread's
@@ -143,19 +143,32 @@ __device__ __forceinline__ float level27(float v, uint32_t lane)
 
 // One warp, all lanes: walk from the block's root corners down L levels to the
 // tile's cube, each level's 27 points in registers (level27) with the sparse
-// values found in desc[27*l + p] (NaN where no node; at levels below the root
+// values from known(l, gx, gy, gz) (NaN where no node; at levels below the root
 // the corner points come from the level above).  Lanes 0-7 return the tile's 8
 // corners (lane & 1, lane >> 1 & 1, lane >> 2).
-__device__ __forceinline__ float descend_regs(const float* desc, uint32_t d, uint32_t L, uint32_t ox, uint32_t oy,
-                                              uint32_t oz, uint32_t lane)
+template <class Known>
+__device__ __forceinline__ float descend_regs(uint32_t d, uint32_t L, uint32_t ox, uint32_t oy, uint32_t oz,
+                                              uint32_t lane, Known&& known)
 {
     const uint32_t px = lane % 3, py = (lane / 3) % 3, pz = lane / 9;
     const bool is_corner = lane < 27 && !((px | py | pz) & 1);
     const uint32_t from = is_corner ? (px >> 1) + 2 * (py >> 1) + 4 * (pz >> 1) : lane;
+    // every level's values first: their loads are independent of one another
+    float val[kMaxGridLevels];
+#pragma unroll
+    for (uint32_t l = 0; l < kMaxGridLevels; ++l) {
+        val[l] = 0.f;
+        if (l < L && lane < 27) {
+            const uint32_t size = 1u << (d - l), hs = size >> 1;
+            val[l] = known((ox & ~(size - 1)) + hs * px, (oy & ~(size - 1)) + hs * py, (oz & ~(size - 1)) + hs * pz);
+        }
+    }
     uint32_t size = 1u << d, gx0 = 0, gy0 = 0, gz0 = 0;
     float corner = 0.f;
-    for (uint32_t l = 0; l < L; ++l) {
-        float v = lane < 27 ? desc[27 * l + lane] : 0.f;
+#pragma unroll
+    for (uint32_t l = 0; l < kMaxGridLevels; ++l) {
+        if (l >= L) break;
+        float v = val[l];
         if (l > 0) {
             const float cv = __shfl_sync(0xffffffffu, corner, from);
             if (is_corner) v = cv;
@@ -274,23 +287,6 @@ template <uint32_t T> __device__ __forceinline__ void tile_top(float* s, uint32_
     if (lane < 27 && ((px | py | pz) & 1)) s[off] = v;
 }
 
-// Marks the finest-level cubes holding a sparse value at one of their
-// midpoints (tile position (x, y, z), at least one coordinate odd): the cube
-// along each odd axis, both neighbours along each even one.
-__device__ __forceinline__ void flag_cubes(uint32_t* flags, uint32_t H, uint32_t x, uint32_t y, uint32_t z)
-{
-    if (!((x | y | z) & 1)) return;
-    const uint32_t x0 = (x & 1) ? x >> 1 : (x ? (x >> 1) - 1 : 0), x1 = (x & 1) ? x >> 1 : min(x >> 1, H - 1);
-    const uint32_t y0 = (y & 1) ? y >> 1 : (y ? (y >> 1) - 1 : 0), y1 = (y & 1) ? y >> 1 : min(y >> 1, H - 1);
-    const uint32_t z0 = (z & 1) ? z >> 1 : (z ? (z >> 1) - 1 : 0), z1 = (z & 1) ? z >> 1 : min(z >> 1, H - 1);
-    for (uint32_t k = z0; k <= z1; ++k)
-        for (uint32_t j = y0; j <= y1; ++j)
-            for (uint32_t i = x0; i <= x1; ++i) {
-                const uint32_t c = i + H * (j + H * k);
-                atomicOr(&flags[c >> 5], 1u << (c & 31));
-            }
-}
-
 // The 19 midpoints of one 2x2x2 cube from its 8 corners (v[p], p = a + 3b + 9c,
 // a, b, c in {0, 1, 2}); kSlots: v also holds sparse values (or NaN) at the
 // midpoints, which are kept.  Edges, then faces, then the centre, stencil sums
@@ -359,6 +355,75 @@ __device__ __forceinline__ void tile_levels(float* s, Crew<kN> cw)
     }
 }
 
+// Where a tile's finest level goes, masked values already NaN.  row: the cube's row (b, cc) of vertices, of which
+// v0 and v1 (x = 0, 1) are its own and v2 is the next cube's first; far_x: v2 of the block's last cube along x;
+// up: on to the next cube along z.
+//
+// A plan brick: rows padded to whole sectors, so a row's two vertices of a cube go out as one aligned store.
+template <typename OutT, bool kSector> struct BrickCursor {
+    OutT* p;
+    uint32_t e, pitch, e2;
+    float inv_scale, offset;
+    __device__ __forceinline__ void row(uint32_t b, uint32_t cc, float v0, float v1, float) const
+    {
+        Store2<OutT>::put_nan(p + b * pitch + cc * e2, v0, v1, inv_scale, offset);
+    }
+    __device__ __forceinline__ void far_x(uint32_t b, uint32_t cc, float v) const
+    {
+        if constexpr (std::is_same<OutT, float>::value && kSector) {
+            if (pitch >= e + 7) {
+                // a padded brick (plan layout, d >= 3): x = 2^d starts a sector of its own
+                // (rows are 32-byte aligned, 2^d is a multiple of 8, the pitch is 2^d + 8):
+                // write the whole sector, the padding as NaN
+                float4* q = reinterpret_cast<float4*>(p + 2 + b * pitch + cc * e2);
+                q[0] = make_float4(v, qnan(), qnan(), qnan());
+                q[1] = make_float4(qnan(), qnan(), qnan(), qnan());
+                return;
+            }
+        }
+        Store<OutT>::put_nan(p, 2 + b * pitch + cc * e2, v, inv_scale, offset);
+    }
+    __device__ __forceinline__ void up() { p += 2 * e2; }
+};
+// A plain (2^d+1)^3 grid: its rows are of odd length, so every other one starts in the middle of an 8-byte word.  In
+// those the cube stores v1 and v2 -- which the next cube, whose own first vertex v2 is, then leaves to it -- and the
+// row's first cube v0 besides, so that all rows go out in aligned pairs.
+struct GridCursor {
+    float* p;
+    uint32_t e, e2;
+    uint32_t odd;   // 1: the cube's first row starts in the middle of an 8-byte word
+    bool first;     // the block's first cube along x
+    __device__ __forceinline__ void row(uint32_t b, uint32_t cc, float v0, float v1, float v2) const
+    {
+        float* q = p + b * e + cc * e2;
+        if ((b + cc + odd) & 1) {
+            if (first) q[0] = v0;
+            *reinterpret_cast<float2*>(q + 1) = make_float2(v1, v2);
+        } else {
+            *reinterpret_cast<float2*>(q) = make_float2(v0, v1);
+        }
+    }
+    __device__ __forceinline__ void far_x(uint32_t b, uint32_t cc, float v) const
+    {
+        if (!((b + cc + odd) & 1)) p[2 + b * e + cc * e2] = v;
+    }
+    __device__ __forceinline__ void up() { p += 2 * e2; }
+};
+// A 3-D texture array, written in place through its surface: no linear grid and no copy into the array.
+struct SurfaceCursor {
+    cudaSurfaceObject_t s;
+    int x, y, z;
+    __device__ __forceinline__ void row(uint32_t b, uint32_t cc, float v0, float v1, float) const
+    {
+        surf3Dwrite(make_float2(v0, v1), s, x * 4, y + (int)b, z + (int)cc);
+    }
+    __device__ __forceinline__ void far_x(uint32_t b, uint32_t cc, float v) const
+    {
+        surf3Dwrite(v, s, (x + 2) * 4, y + (int)b, z + (int)cc);
+    }
+    __device__ __forceinline__ void up() { z += 2; }
+};
+
 // One finest-level cube (ci, cj, ck) of a tile: reads its corners from the even
 // sub-array -- kFirst: all 8; else the upper 4, its z = 0 face being the z = 2
 // face of the cube below it, already in v -- and, when flagged as holding a
@@ -371,12 +436,9 @@ __device__ __forceinline__ void tile_levels(float* s, Crew<kN> cw)
 // NaN ("no sparse value") before any slot is overwritten, then turn masked
 // sparse values to NaN.  A reused face went through the same steps in the cube
 // below, so every vertex gets the value a fresh cube would give it.
-// kPairs: plan bricks, whose rows are padded to whole sectors (aligned rows, even pitch): a row's two
-// vertices of a cube go out as one store.  A plain (2^d+1)^3 grid (odd pitch) stores them one by one.
-template <uint32_t T, typename OutT, bool kPairs, bool kFirst>
+template <uint32_t T, bool kFirst, class Cur>
 __device__ __forceinline__ void finest_cube(const float* s, bool has, uint32_t ci, uint32_t cj, uint32_t ck, float v[27],
-                                            OutT* base, uint32_t pitch, uint32_t e, uint32_t e2, bool lx, bool ly,
-                                            bool lz, float inv_scale, float offset)
+                                            const Cur& cur, bool lx, bool ly, bool lz)
 {
     using S = SplitTile<T>;
 #pragma unroll
@@ -402,78 +464,40 @@ __device__ __forceinline__ void finest_cube(const float* s, bool has, uint32_t c
     } else {
         fill_cube<false, !kFirst>(v);
     }
-    if constexpr (kPairs) {
+    auto row = [&](uint32_t b, uint32_t cc) {
+        const int p = 3 * (int)b + 9 * (int)cc;
+        cur.row(b, cc, v[p], v[p + 1], v[p + 2]);
+    };
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const uint32_t b = r & 1, cc = r >> 1;
-            Store2<OutT>::put_nan(base + b * pitch + cc * e2, v[3 * b + 9 * cc], v[1 + 3 * b + 9 * cc], inv_scale,
-                                  offset);
-        }
-    } else {
-#pragma unroll
-        for (int p = 0; p < 27; ++p) {
-            const uint32_t a = p % 3, b = (p / 3) % 3, cc = p / 9;
-            if (a < 2 && b < 2 && cc < 2) Store<OutT>::put_nan(base, a + b * pitch + cc * e2, v[p], inv_scale, offset);
-        }
-    }
+    for (uint32_t r = 0; r < 4; ++r) row(r & 1, r >> 1);
     // the far side where this is the block's last cube along an axis: the x = 2 face (with its
     // y = 2 / z = 2 edges where those are far too), then y = 2 (x < 2), then z = 2 (x, y < 2)
-    auto far_put = [&](int p) {
-        const uint32_t a = p % 3, b = (p / 3) % 3, cc = p / 9;
-        if constexpr (std::is_same<OutT, float>::value && T >= 8) {
-            if (a == 2 && pitch >= e + 7) {
-                // a padded brick (plan layout, d >= 3): x = 2^d starts a sector of its own
-                // (rows are 32-byte aligned, 2^d is a multiple of 8, the pitch is 2^d + 8):
-                // write the whole sector, the padding as NaN
-                float4* q = reinterpret_cast<float4*>(base + a + b * pitch + cc * e2);
-                q[0] = make_float4(v[p], qnan(), qnan(), qnan());
-                q[1] = make_float4(qnan(), qnan(), qnan(), qnan());
-                return;
-            }
-        }
-        Store<OutT>::put_nan(base, a + b * pitch + cc * e2, v[p], inv_scale, offset);
-    };
     if (lx) {
 #pragma unroll
-        for (int bb = 0; bb < 3; ++bb)
+        for (uint32_t b = 0; b < 3; ++b)
 #pragma unroll
-            for (int c2 = 0; c2 < 3; ++c2)
-                if ((bb < 2 || ly) && (c2 < 2 || lz)) far_put(2 + 3 * bb + 9 * c2);
+            for (uint32_t cc = 0; cc < 3; ++cc)
+                if ((b < 2 || ly) && (cc < 2 || lz)) cur.far_x(b, cc, v[2 + 3 * b + 9 * cc]);
     }
     if (ly) {
-#pragma unroll
-        for (int c2 = 0; c2 < 3; ++c2) {
-            if (c2 == 2 && !lz) continue;
-            if constexpr (kPairs) {
-                Store2<OutT>::put_nan(base + 2 * pitch + c2 * e2, v[6 + 9 * c2], v[7 + 9 * c2], inv_scale, offset);
-            } else {
-                far_put(6 + 9 * c2);
-                far_put(7 + 9 * c2);
-            }
-        }
+        row(2, 0);
+        row(2, 1);
+        if (lz) row(2, 2);
     }
     if (lz) {
-#pragma unroll
-        for (int b2 = 0; b2 < 2; ++b2) {
-            if constexpr (kPairs) {
-                Store2<OutT>::put_nan(base + b2 * pitch + 2 * e2, v[3 * b2 + 18], v[1 + 3 * b2 + 18], inv_scale,
-                                      offset);
-            } else {
-                far_put(3 * b2 + 18);
-                far_put(1 + 3 * b2 + 18);
-            }
-        }
+        row(0, 2);
+        row(1, 2);
     }
 }
 
-// The finest level of a tile, written straight to HBM: its H^3 2x2x2 cubes in
+// The finest level of a tile, written straight to its place: its H^3 2x2x2 cubes in
 // runs of Z along z, one run per thread (runs consecutive along x within a
 // warp), so that each cube after the first of a run takes its z = 0 face from
 // the one below; Z makes the runs about as many as the tile's threads (kN).
-template <uint32_t T, typename OutT, bool kPairs, uint32_t kN>
-__device__ __forceinline__ void finest_store(const float* s, const uint32_t* flags, OutT* out, uint32_t e,
-                                             uint32_t pitch, uint32_t ox, uint32_t oy, uint32_t oz, bool far_x,
-                                             bool far_y, bool far_z, float inv_scale, float offset, uint32_t tid)
+// at(x, y, z): the cursor of the cube whose low corner is vertex (x, y, z) of the tile.
+template <uint32_t T, uint32_t kN, class At>
+__device__ __forceinline__ void finest_store(const float* s, const uint32_t* flags, bool far_x, bool far_y, bool far_z,
+                                             uint32_t tid, At&& at)
 {
     using S = SplitTile<T>;
     constexpr uint32_t H = S::H;
@@ -482,18 +506,16 @@ __device__ __forceinline__ void finest_store(const float* s, const uint32_t* fla
     constexpr uint32_t Z = per >= H ? H : (per >= 1 ? per : 1);
     constexpr uint32_t lzr = 31 - __builtin_clz(Z);
     constexpr uint32_t nruns = H * H * H / Z;
-    const uint32_t e2 = e * pitch; // slab stride (a brick holds fewer than 2^32 elements)
 #pragma unroll 1
     for (uint32_t rr = tid; rr < nruns; rr += kN) {
         const uint32_t ci = rr & (H - 1), cj = (rr >> lh) & (H - 1), ck0 = (rr >> (2 * lh)) << lzr;
         const bool lx = far_x && ci == H - 1, ly = far_y && cj == H - 1;
         float v[27];
-        OutT* base = out + (((oz + 2 * ck0) * e + (oy + 2 * cj)) * pitch + (ox + 2 * ci));
+        auto cur = at(2 * ci, 2 * cj, 2 * ck0);
         {
             const uint32_t c = ci + H * (cj + H * ck0);
             const bool has = (flags[c >> 5] >> (c & 31)) & 1u;
-            finest_cube<T, OutT, kPairs, true>(s, has, ci, cj, ck0, v, base, pitch, e, e2, lx, ly,
-                                               far_z && ck0 == H - 1, inv_scale, offset);
+            finest_cube<T, true>(s, has, ci, cj, ck0, v, cur, lx, ly, far_z && ck0 == H - 1);
         }
 #pragma unroll 1
         for (uint32_t z = 1; z < Z; ++z) {
@@ -502,9 +524,8 @@ __device__ __forceinline__ void finest_store(const float* s, const uint32_t* fla
             const bool has = (flags[c >> 5] >> (c & 31)) & 1u;
 #pragma unroll
             for (int p = 0; p < 9; ++p) v[p] = v[p + 18];
-            base += 2 * e2;
-            finest_cube<T, OutT, kPairs, false>(s, has, ci, cj, ck, v, base, pitch, e, e2, lx, ly,
-                                                far_z && ck == H - 1, inv_scale, offset);
+            cur.up();
+            finest_cube<T, false>(s, has, ci, cj, ck, v, cur, lx, ly, far_z && ck == H - 1);
         }
     }
 }
@@ -581,13 +602,13 @@ struct TileItem {
     uint32_t item;
 };
 
-// One tile of T = 2^k cells.  Tiles of T >= 2 use the split layout; T = 1
+// One tile of T = 2^k cells of a plan.  Tiles of T >= 2 use the split layout; T = 1
 // (depth-0 blocks) is a plain 2x2x2 copy of the root corners.
 // cw: the CTA or the warp running the tile; next_item(): the next work item's number (read once the current
 // item's entries are placed, so that its first prefetch stage goes out behind this tile's work).
-template <uint32_t T, bool kGrid, typename OutT, uint32_t kN, class NextFn>
-__device__ __forceinline__ void run_tile(const TileArgs& a, float* s, float* desc, uint32_t* flags, const TileItem& t,
-                                         Prefetch& pf, Crew<kN> cw, NextFn next_item)
+template <uint32_t T, typename OutT, uint32_t kN, class NextFn>
+__device__ __forceinline__ void run_tile(const TileArgs& a, float* s, uint32_t* flags, const TileItem& t, Prefetch& pf,
+                                         Crew<kN> cw, NextFn next_item)
 {
     constexpr uint32_t E = T + 1, E3 = E * E * E;
     using S = SplitTile<T < 2 ? 2 : T>;
@@ -599,98 +620,248 @@ __device__ __forceinline__ void run_tile(const TileArgs& a, float* s, float* des
     const uint32_t ox = t.tx * T, oy = t.ty * T, oz = t.tz * T;
     const uint32_t e = (1u << d) + 1u;
     constexpr uint32_t nflags = T >= 2 ? (S::H * S::H * S::H + 31) / 32 : 0;
-    if constexpr (kGrid) {
-        for (uint32_t q = cw.tid; q < nflags; q += kN) flags[q] = 0u;
-    } else {
-        if (cw.tid < nflags) flags[cw.tid] = pf.flag; // the plan's flags, prefetched
-    }
-    // 1. the tile's sparse values (NaN elsewhere) and the descent's
-    if constexpr (kGrid) {
-        cw.sync(); // flags cleared
+    if (cw.tid < nflags) flags[cw.tid] = pf.flag; // the plan's flags, prefetched
+    // 1. the tile's sparse values, NaN elsewhere
+    {
+        const float4 nan4 = make_float4(qnan(), qnan(), qnan(), qnan());
+        float4* s4 = reinterpret_cast<float4*>(s);
+        // the even sub-array always (the coarse levels test it for NaN); the midpoint slots only
+        // where a flagged cube will read them
+        uint32_t n4 = (E3 + 3) / 4;
+        if constexpr (T >= 2) {
+            constexpr uint32_t G3 = S::G * S::G * S::G;
+            if (!t.slots) n4 = (G3 + 3) / 4;
+        }
 #pragma unroll 1
-        for (uint32_t p = cw.tid; p < E3; p += kN) {
-            const uint32_t lx = p % E, r = p / E, ly = r % E, lz = r / E;
-            const float v = to_internal(a.grid[((uint64_t)(oz + lz) * e + (oy + ly)) * e + (ox + lx)]);
-            s[at(lx, ly, lz)] = v;
-            if constexpr (T >= 2)
-                if (!isnan(v)) flag_cubes(flags, S::H, lx, ly, lz);
-        }
-        for (uint32_t q = cw.tid; q < 27 * L; q += kN) {
-            const uint32_t l = q / 27, p = q % 27;
-            const uint32_t size = 1u << (d - l), hs = size >> 1;
-            const uint32_t bx = ox & ~(size - 1), by = oy & ~(size - 1), bz = oz & ~(size - 1);
-            const uint32_t gx = bx + hs * (p % 3), gy = by + hs * ((p / 3) % 3), gz = bz + hs * (p / 9);
-            desc[q] = to_internal(a.grid[((uint64_t)gz * e + gy) * e + gx]);
-        }
-    } else {
-        {
-            const float4 nan4 = make_float4(qnan(), qnan(), qnan(), qnan());
-            float4* s4 = reinterpret_cast<float4*>(s);
-            // the even sub-array always (the coarse levels test it for NaN); the midpoint slots only
-            // where a flagged cube will read them
-            uint32_t n4 = (E3 + 3) / 4;
-            if constexpr (T >= 2) {
-                constexpr uint32_t G3 = S::G * S::G * S::G;
-                if (!t.slots) n4 = (G3 + 3) / 4;
-            }
-#pragma unroll 1
-            for (uint32_t p = cw.tid; p < n4; p += kN) s4[p] = nan4;
-        }
-        cw.sync();
-        auto place = [&](uint32_t loc, float v) {
-            if (loc < E3) s[loc] = v;
-        };
-        // the prefetched entries, then any beyond what the registers held
-#pragma unroll
-        for (uint32_t q = 0; q < kPrefetch; ++q)
-            if (pf.e0 + cw.tid + q * kN < pf.e1) place(pf.loc[q], to_internal(pf.val[q]));
-        for (uint32_t i = pf.e0 + cw.tid + kPrefetch * kN; i < pf.e1; i += kN)
-            place(a.entry_local[i], to_internal(a.sparse[t.node_base + a.entry_node[i]]));
-        // a tile of a block with coarse levels: its corners from the block's coarse grid
-        if (pf.cidx != 0xffffffffu)
-            s[at((cw.tid & 1) * T, ((cw.tid >> 1) & 1) * T, (cw.tid >> 2) * T)] = pf.corner;
-        prefetch_head<kN>(pf, a, next_item(), cw.tid); // the current item's entries are placed
+        for (uint32_t p = cw.tid; p < n4; p += kN) s4[p] = nan4;
     }
     cw.sync();
-    // 2. single-grid form: tile corners from the coarse levels; then the tile cube's own
-    //    midpoints (its first level): the first warp, each level's 27 points in registers
-    if ((kGrid && L > 0) || T >= 4) {
-        if (kN == 32 || cw.tid < 32) {
-            const uint32_t lane = cw.tid & 31;
-            if (kGrid && L > 0) {
-                const float corner = descend_regs(desc, d, L, ox, oy, oz, lane);
-                if (lane < 8) s[at((lane & 1) * T, ((lane >> 1) & 1) * T, (lane >> 2) * T)] = corner;
-                __syncwarp();
-            }
-            if constexpr (T >= 4) tile_top<T>(s, lane);
-        }
+    auto place = [&](uint32_t loc, float v) {
+        if (loc < E3) s[loc] = v;
+    };
+    // the prefetched entries, then any beyond what the registers held
+#pragma unroll
+    for (uint32_t q = 0; q < kPrefetch; ++q)
+        if (pf.e0 + cw.tid + q * kN < pf.e1) place(pf.loc[q], to_internal(pf.val[q]));
+    for (uint32_t i = pf.e0 + cw.tid + kPrefetch * kN; i < pf.e1; i += kN)
+        place(a.entry_local[i], to_internal(a.sparse[t.node_base + a.entry_node[i]]));
+    // a tile of a block with coarse levels: its corners from the block's coarse grid
+    if (pf.cidx != 0xffffffffu) s[at((cw.tid & 1) * T, ((cw.tid >> 1) & 1) * T, (cw.tid >> 2) * T)] = pf.corner;
+    prefetch_head<kN>(pf, a, next_item(), cw.tid); // the current item's entries are placed
+    cw.sync();
+    // 2. the tile cube's own midpoints (its first level): the first warp, its 27 points in registers
+    if constexpr (T >= 4) {
+        if (kN == 32 || cw.tid < 32) tile_top<T>(s, cw.tid & 31);
         cw.sync();
     }
-    if constexpr (!kGrid) prefetch_index<kN>(pf, a, cw.tid);
+    prefetch_index<kN>(pf, a, cw.tid);
     // 3. the remaining coarser levels on the even sub-array (a tile of T/2 cells)
     if constexpr (T >= 8) tile_levels<S::G, S::H, 1, 31 - __builtin_clz(T), kN>(s, cw);
     // 4. the finest level, straight to HBM, while the next item's entries load
-    if constexpr (!kGrid) prefetch_values<kN>(pf, a, cw.tid);
+    prefetch_values<kN>(pf, a, cw.tid);
     float inv_scale = 1.f, offset = 0.f;
-    if constexpr (!kGrid) {
-        if (a.scale_offset) {
-            const float2 so = a.scale_offset[t.blk];
-            inv_scale = 1.f / so.x;
-            offset = so.y;
-        }
+    if (a.scale_offset) {
+        const float2 so = a.scale_offset[t.blk];
+        inv_scale = 1.f / so.x;
+        offset = so.y;
     }
     const uint32_t mL = 1u << L;
     OutT* out = reinterpret_cast<OutT*>(a.out) + t.dense_off;
     const bool far_x = t.tx == mL - 1, far_y = t.ty == mL - 1, far_z = t.tz == mL - 1;
     if constexpr (T >= 2) {
-        finest_store<T, OutT, !kGrid, kN>(s, flags, out, e, t.pitch, ox, oy, oz, far_x, far_y, far_z, inv_scale,
-                                          offset, cw.tid);
+        const uint32_t pitch = t.pitch;
+        const uint32_t e2 = e * pitch; // slab stride (a brick holds fewer than 2^32 elements)
+        finest_store<T, kN>(s, flags, far_x, far_y, far_z, cw.tid, [&](uint32_t x, uint32_t y, uint32_t z) {
+            return BrickCursor<OutT, (T >= 8)>{out + (((oz + z) * e + (oy + y)) * pitch + (ox + x)), e, pitch, e2,
+                                               inv_scale, offset};
+        });
     } else {
         // depth-0 block: its 8 root corners
         for (uint32_t q = cw.tid; q < 8; q += kN) {
             const uint32_t x = q & 1, y = (q >> 1) & 1, z = q >> 2;
             Store<OutT>::put(out, ((uint64_t)(oz + z) * e + (oy + y)) * t.pitch + ox + x, s[at(x, y, z)],
                              inv_scale, offset);
+        }
+    }
+}
+
+// ---------------------------------------------------------------- blocks from their node lists
+//
+// A subtree's dense grid from its nodes as the caller holds them (vertex indices and values in any order), tile by
+// tile as above.  A block of up to kGridDirectTiles tiles and few nodes has every tile read the whole node list; else
+// the nodes were scattered beforehand, each value to its vertex's place in a grid and one bit into a mask of the
+// block's vertices (rows of whole words), so that a tile reads 17^2 mask rows and the values of the nodes it holds
+// instead of 17^3 grid values, and the grid itself is never cleared.
+
+// The tile's node values from the mask and grid, by kN threads: thread `tid` takes the rows tid, tid + kN, ... and
+// keeps up to 8 loads in flight; row_mask gets every row's bits.
+template <uint32_t T, uint32_t kN, class Put>
+__device__ __forceinline__ void gather_nodes(const uint32_t* bits, const float* vals, uint32_t e, uint32_t ox,
+                                             uint32_t oy, uint32_t oz, uint32_t tid, uint32_t* row_mask, Put&& put)
+{
+    constexpr uint32_t E = T + 1, kRows = E * E, kPer = (kRows + kN - 1) / kN;
+    const uint32_t words = (e + 31) / 32, w = ox >> 5, sh = ox & 31;
+    uint32_t mask[kPer];
+#pragma unroll
+    for (uint32_t r = 0; r < kPer; ++r) {
+        const uint32_t row = tid + r * kN;
+        mask[r] = 0;
+        if (row < kRows) {
+            const uint32_t* b = bits + ((uint64_t)(oz + row / E) * e + (oy + row % E)) * words + w;
+            const uint32_t lo = b[0], hi = sh + E > 32 ? b[1] : 0u;
+            mask[r] = __funnelshift_r(lo, hi, sh) & ((1u << E) - 1u);
+        }
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < kPer; ++r)
+        if (tid + r * kN < kRows) row_mask[tid + r * kN] = mask[r];
+#pragma unroll 1
+    for (uint32_t r = 0; r < kPer; ++r) {
+        // (a register array indexed by a loop variable would live in local memory)
+        uint32_t m = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kPer; ++q)
+            if (q == r) m = mask[q];
+        const uint32_t row = tid + r * kN, y = row % E, z = row / E;
+        const float* src = vals + ((uint64_t)(oz + z) * e + (oy + y)) * e + ox;
+        while (m) {
+            uint32_t x[8];
+            float v[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                x[q] = 32;
+                if (m) {
+                    x[q] = (uint32_t)__ffs((int)m) - 1;
+                    m &= m - 1;
+                    v[q] = src[x[q]];
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (x[q] < 32) put(x[q], y, z, to_internal(v[q]));
+        }
+    }
+}
+
+// The flags of the finest-level cubes that hold a node at one of their midpoints, from the rows' bits: along a row of
+// cubes, the rows with y or z odd count at all three positions of a cube, the four even ones at its middle.  By the
+// kInterpThreads - 32 threads after the first warp, tid counted from them.
+template <uint32_t T> __device__ __forceinline__ void flags_from_rows(const uint32_t* row_mask, uint32_t* flags,
+                                                                      uint32_t tid)
+{
+    constexpr uint32_t H = T / 2, E = T + 1;
+    for (uint32_t q = tid; q < H * H; q += kInterpThreads - 32) {
+        const uint32_t y = 2 * (q % H), z = 2 * (q / H);
+        const uint32_t* r = row_mask + y + E * z;
+        const uint32_t all = r[1] | r[E] | r[E + 1] | r[E + 2] | r[2 * E + 1];
+        const uint32_t mid = r[0] | r[2] | r[2 * E] | r[2 * E + 2];
+        const uint32_t odd = (all | (all << 1) | (all >> 1) | mid) & 0xaaaaaaaau; // bit 2i + 1: cube i
+        uint32_t f = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < H; ++i) f |= ((odd >> (2 * i + 1)) & 1u) << i;
+        if (f) atomicOr(&flags[(H * q) >> 5], f << ((H * q) & 31));
+    }
+}
+
+// One tile (tx, ty, tz) of T = 2^k cells of block b, by a CTA.  cursor(x, y, z): the output cursor of the cube whose
+// low corner is the block's vertex (x, y, z); put0(x, y, z, v): a vertex of a depth-0 block.
+template <uint32_t T, class At, class Put0>
+__device__ __forceinline__ void run_grid_tile(const GridBlock& b, const float* vals, const uint32_t* bits, float* s,
+                                              float* desc, uint32_t* row_mask, uint32_t* flags, uint32_t tx,
+                                              uint32_t ty, uint32_t tz, At&& cursor, Put0&& put0)
+{
+    constexpr uint32_t E = T + 1, E3 = E * E * E, kN = kInterpThreads;
+    constexpr uint32_t lt = 31 - __builtin_clz(T);
+    using S = SplitTile<T < 2 ? 2 : T>;
+    const uint32_t tid = threadIdx.x, d = b.depth, L = d - lt;
+    const uint32_t ox = tx * T, oy = ty * T, oz = tz * T, e = (1u << d) + 1u;
+    constexpr uint32_t nflags = T >= 2 ? (S::H * S::H * S::H + 31) / 32 : 0;
+    auto slot = [](uint32_t x, uint32_t y, uint32_t z) -> uint32_t {
+        if constexpr (T < 2) return x + 2 * (y + 2 * z);
+        else return S::at(x, y, z);
+    };
+    for (uint32_t q = tid; q < nflags; q += kN) flags[q] = 0u;
+    const float4 nan4 = make_float4(qnan(), qnan(), qnan(), qnan());
+    for (uint32_t p = tid; p < (E3 + 3) / 4; p += kN) reinterpret_cast<float4*>(s)[p] = nan4;
+    if (b.direct) {
+        for (uint32_t q = tid; q < E * E; q += kN) row_mask[q] = 0u;
+        if (tid < 27) desc[tid] = qnan();
+    }
+    __syncthreads();
+    float corner = 0.f; // lanes 0-7 of warp 0: the tile's corners from the coarse levels
+    if (b.direct) {
+        for (uint32_t i0 = tid; i0 < b.n; i0 += 4 * kN) {
+            uint32_t x[4], y[4], z[4];
+            float v[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t i = i0 + q * kN;
+                x[q] = 0xffffffffu;
+                if (i < b.n) {
+                    x[q] = b.n2i[3 * (size_t)i];
+                    y[q] = b.n2i[3 * (size_t)i + 1];
+                    z[q] = b.n2i[3 * (size_t)i + 2];
+                    v[q] = b.sparse[i];
+                }
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                if (x[q] >= e || y[q] >= e || z[q] >= e) continue; // no node, or one outside the block: ignored
+                const float w = to_internal(v[q]);
+                // L <= 1: the lattice of tile corners is the root cube's 27 points
+                if (L > 0 && ((x[q] | y[q] | z[q]) & (T - 1)) == 0)
+                    desc[(x[q] >> lt) + 3 * (y[q] >> lt) + 9 * (z[q] >> lt)] = w;
+                const uint32_t lx = x[q] - ox, ly = y[q] - oy, lz = z[q] - oz;
+                if (lx < E && ly < E && lz < E) {
+                    s[slot(lx, ly, lz)] = w;
+                    atomicOr(&row_mask[ly + E * lz], 1u << lx);
+                }
+            }
+        }
+    } else {
+        // the tile's corners by the first warp, its nodes by the others meanwhile
+        const float* bv = vals + b.val_off;
+        const uint32_t* bb = bits + b.bit_off;
+        if (tid < 32) {
+            const uint32_t words = (e + 31) / 32;
+            corner = descend_regs(d, L, ox, oy, oz, tid, [&](uint32_t gx, uint32_t gy, uint32_t gz) {
+                const uint64_t row = (uint64_t)gz * e + gy;
+                // both at once: the value means something only where the bit is set
+                const float v = bv[row * e + gx];
+                const uint32_t m = bb[row * words + (gx >> 5)];
+                return (m >> (gx & 31)) & 1u ? to_internal(v) : qnan();
+            });
+        } else {
+            gather_nodes<T, kN - 32>(bb, bv, e, ox, oy, oz, tid - 32, row_mask,
+                                     [&](uint32_t x, uint32_t y, uint32_t z, float v) { s[slot(x, y, z)] = v; });
+        }
+    }
+    __syncthreads();
+    if (tid < 32) {
+        // the corners, then the tile cube's own midpoints in registers; the flags by the other warps
+        if (L > 0) {
+            if (b.direct)
+                corner = descend_regs(d, L, ox, oy, oz, tid, [&](uint32_t gx, uint32_t gy, uint32_t gz) {
+                    return desc[(gx >> lt) + 3 * (gy >> lt) + 9 * (gz >> lt)];
+                });
+            if (tid < 8) s[slot((tid & 1) * T, ((tid >> 1) & 1) * T, (tid >> 2) * T)] = corner;
+            __syncwarp();
+        }
+        if constexpr (T >= 4) tile_top<T>(s, tid);
+    } else {
+        if constexpr (T >= 2) flags_from_rows<T>(row_mask, flags, tid - 32);
+    }
+    __syncthreads();
+    if constexpr (T >= 8) tile_levels<S::G, S::H, 1, lt, kN>(s, Crew<kN>{tid});
+    const uint32_t mL = 1u << L;
+    if constexpr (T >= 2) {
+        finest_store<T, kN>(s, flags, tx == mL - 1, ty == mL - 1, tz == mL - 1, tid,
+                            [&](uint32_t x, uint32_t y, uint32_t z) { return cursor(ox + x, oy + y, oz + z); });
+    } else {
+        for (uint32_t q = tid; q < 8; q += kN) {
+            const uint32_t x = q & 1, y = (q >> 1) & 1, z = q >> 2;
+            const float v = s[slot(x, y, z)];
+            put0(x, y, z, isinf(v) ? qnan() : v);
         }
     }
 }

@@ -12,9 +12,10 @@
 //
 // Limits and sharing:
 //   * depth <= S3R_NOALLOC_MAX_DEPTH (7): the scratch holds 129^3 floats (8.6 MB);
-//     deeper subtrees are rejected with S3R_ERR_INVALID.
-//   * All calls on a device share the one scratch array.  Each call re-fills the
-//     part it uses with NaN before scattering the nodes, so no state leaks from
+//     deeper subtrees are rejected with S3R_ERR_INVALID; 0.3 MB more hold the mask
+//     of the vertices that have a value in it.
+//   * All calls on a device share the one scratch array.  Each call clears the
+//     part of the mask it uses before scattering the nodes, so no state leaks from
 //     the previous call, but calls that overlap on the GPU (different streams,
 //     or host threads without ordering between them) race on the scratch and
 //     produce wrong grids: order them on one stream or serialize them.
@@ -37,12 +38,16 @@ constexpr size_t kNoAllocFloats = (size_t)kNoAllocEdge * kNoAllocEdge * kNoAlloc
 // The scratch grid.  In host code this name is only a host-side stand-in: its
 // device address comes from cudaGetSymbolAddress, per device.
 static __device__ __align__(256) float g_noalloc_grid[kNoAllocFloats];
+// The mask of the vertices the scratch holds a value for (rows of whole words).
+constexpr size_t kNoAllocWords = (size_t)kNoAllocEdge * kNoAllocEdge * ((kNoAllocEdge + 31) / 32);
+static __device__ __align__(256) uint32_t g_noalloc_bits[kNoAllocWords];
 
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 struct GridAddress {
     unsigned long long context_id = 0; // 0: none looked up yet
     float* grid = nullptr;
+    uint32_t* bits = nullptr;
 };
 GridAddress g_grid_on_device[kMaxDevices];
 
@@ -94,6 +99,7 @@ extern "C" int s3r_interp_dense_noalloc(const uint16_t* n2i_xyz, const float* sp
     if (dev < 0 || dev >= kMaxDevices)
         return record_error(S3R_ERR_UNSUPPORTED, "s3r_interp_dense_noalloc: device ordinal beyond 63");
     float* grid = nullptr;
+    uint32_t* bits = nullptr;
     {
         std::lock_guard<std::mutex> lock(g_setup_mutex);
         GridAddress& ga = g_grid_on_device[dev];
@@ -104,19 +110,28 @@ extern "C" int s3r_interp_dense_noalloc(const uint16_t* n2i_xyz, const float* sp
             void* p = nullptr;
             e = cudaGetSymbolAddress(&p, g_noalloc_grid);
             if (e != cudaSuccess) return record_cuda_error(e, "cudaGetSymbolAddress(g_noalloc_grid)");
+            void* q = nullptr;
+            e = cudaGetSymbolAddress(&q, g_noalloc_bits);
+            if (e != cudaSuccess) return record_cuda_error(e, "cudaGetSymbolAddress(g_noalloc_bits)");
             if (id == 0) id = current_context_id();
             ga.grid = static_cast<float*>(p);
+            ga.bits = static_cast<uint32_t*>(q);
             ga.context_id = id; // 0 (ids unavailable): looked up again on every call
         }
         grid = ga.grid;
+        bits = ga.bits;
     }
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    const uint64_t edge = (1ull << depth) + 1ull;
-    if ((e = launch_fill_f32(grid, edge * edge * edge, __builtin_nanf(""), s)) != cudaSuccess)
-        return record_cuda_error(e, "fill");
-    if ((e = launch_scatter_nodes(grid, depth, n2i_xyz, sparse, n, s)) != cudaSuccess)
-        return record_cuda_error(e, "scatter");
-    if ((e = launch_interp_grid(grid, depth, dense, s, nullptr)) != cudaSuccess)
+    GridArgs a{};
+    a.one = grid_block(n2i_xyz, sparse, n, depth);
+    a.one.out = dense;
+    a.nblocks = 1;
+    a.tiles = grid_tiles(depth);
+    a.depth_max = depth;
+    a.vals = grid;
+    a.bits = bits;
+    const uint64_t words = a.one.direct ? 0 : grid_mask_words(depth);
+    if ((e = launch_interp_grid(a, false, words ? n : 0, words, s, nullptr)) != cudaSuccess)
         return record_cuda_error(e, "interpolate");
     return S3R_OK;
 }

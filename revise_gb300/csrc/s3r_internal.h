@@ -36,10 +36,7 @@ inline __host__ __device__ uint32_t plan_brick_pitch(uint32_t depth, uint32_t el
     return (((1u << depth) + 1u + per - 1u) / per) * per;
 }
 
-// Arguments of the tile interpolation kernel.  Two node sources:
-//   grid   != nullptr: one block whose sparse values were scattered into a
-//                      NaN-filled (2^d+1)^3 grid (blocks/items unused);
-//   grid   == nullptr: a batched plan whose nodes are binned per tile.
+// Arguments of a batched plan's tile interpolation kernels: the nodes are binned per tile.
 struct TileArgs {
     const PlanBlock* blocks;
     const uint2* items;           // {block, tile} per work item
@@ -47,20 +44,51 @@ struct TileArgs {
     const uint64_t* entry_off;    // nitems+1 prefix offsets into local/node
     const uint16_t* entry_local;  // node position inside its tile (tile_offset)
     const uint32_t* entry_node;   // node index within its block
-    // entry_local >= (2^k+1)^3 addresses descent slot 27*level + point instead of the tile
     const uint32_t* flags;        // per item flag_words words: bit c set when finest cube c of the tile
-    uint32_t flag_words;          // holds a sparse value at one of its midpoints (plan form only)
+    uint32_t flag_words;          // holds a sparse value at one of its midpoints
     const float* sparse;          // node values
     const float2* scale_offset;   // per block {scale, offset} for 16-bit bricks
     void* out;                    // brick store
-    uint32_t* queue;              // work-queue counter, zeroed before the launch (nullptr: one item per CTA)
-    const float* coarse;          // plan form: per block cut into 2^L > 1 tiles per axis its coarse grid (the
+    uint32_t* queue;              // work-queue counter, zeroed before the launch
+    const float* coarse;          // per block cut into 2^L > 1 tiles per axis its coarse grid (the
                                   // (2^L+1)^3 vertices at multiples of the tile edge, internal values), from
                                   // block_prep_kernel: a tile reads its 8 corners there
-    // single-block form
-    const float* grid;
-    uint32_t grid_depth;
-    uint32_t grid_tile_log2;
+};
+
+// One subtree interpolated from its node list as the caller holds it (interp_tile.cuh, run_grid_tile).
+constexpr uint32_t kGridTileLog2 = 4; // tiles of up to 16 cells
+// A block of depth 5 (8 tiles) whose tiles read the whole node list: up to this many nodes that is less time than
+// the two launches that scatter them (at 8192 nodes a tile's scan takes about 4 us).
+constexpr uint32_t kGridDirectNodes = 8192;
+struct GridBlock {
+    const uint16_t* n2i; // n vertex indices (x, y, z)
+    const float* sparse; // n values
+    uint32_t n, depth;
+    uint32_t direct;     // every tile reads the node list (one tile, or a few and few nodes); else scattered
+    uint32_t pad;
+    uint64_t val_off;    // scattered: its (2^depth+1)^3 floats in GridArgs::vals
+    uint64_t bit_off;    // scattered: its mask in GridArgs::bits, rows of grid_mask_words(depth) words
+    float* out;          // the dense grid, or
+    unsigned long long surface; // the surface of a 3-D array
+};
+inline uint64_t grid_vertices(uint32_t depth)
+{
+    const uint64_t e = (1ull << depth) + 1;
+    return e * e * e;
+}
+inline uint64_t grid_mask_words(uint32_t depth)
+{
+    const uint64_t e = (1ull << depth) + 1;
+    return e * e * ((e + 31) / 32);
+}
+inline uint32_t grid_tiles(uint32_t depth) { return depth <= kGridTileLog2 ? 1u : 1u << (3 * (depth - kGridTileLog2)); }
+struct GridArgs {
+    GridBlock one;             // a set of one block
+    const GridBlock* table;    // device: nblocks blocks (nullptr: `one`)
+    const uint32_t* tile_off;  // device: nblocks + 1 running tile counts
+    uint32_t nblocks, tiles, depth_max;
+    float* vals;
+    uint32_t* bits;
 };
 
 // Position of vertex (x, y, z) inside the shared tile of T cells, as the
@@ -172,11 +200,13 @@ cudaError_t launch_divide(const float* sums, const float* weights, uint64_t n, f
 // Adds n to the context's launch counter (host.cpp).
 void count_launches(s3r_ctx* ctx, uint32_t n);
 
-cudaError_t launch_fill_f32(float* p, uint64_t n, float v, cudaStream_t s);
 cudaError_t launch_fill_u32(uint32_t* p, uint64_t n, uint32_t v, cudaStream_t s);
-cudaError_t launch_scatter_nodes(float* grid, uint32_t depth, const uint16_t* n2i, const float* sparse, uint32_t n,
-                                 cudaStream_t s);
-cudaError_t launch_interp_grid(const float* grid, uint32_t depth, float* dense, cudaStream_t s, uint32_t* launches);
+// The block of these nodes, direct or scattered by its size; the caller sets its offsets and output.
+GridBlock grid_block(const uint16_t* n2i, const float* sparse, uint32_t n, uint32_t depth);
+// Clears the first bit_words mask words, scatters the nodes of the set's scattered blocks (scattered_nodes: the
+// most any of them has) and interpolates the set's blocks into their grids or surfaces.
+cudaError_t launch_interp_grid(const GridArgs& a, bool surface, uint32_t scattered_nodes, uint64_t bit_words,
+                               cudaStream_t s, uint32_t* launches);
 cudaError_t launch_interp_plan(const TileArgs& a, uint32_t fmt, uint32_t tile_log2_max, uint32_t grid_ctas,
                                cudaStream_t s);
 uint32_t interp_plan_ctas_per_sm(uint32_t fmt, uint32_t tile_log2);
