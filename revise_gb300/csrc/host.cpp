@@ -32,17 +32,25 @@ struct s3r_ctx {
     size_t grid_cap = 0;   // floats
     uint32_t* grid_bits = nullptr;
     size_t grid_bits_cap = 0; // words
-    int32_t* rect_dev = nullptr;
+    int32_t* rect_dev = nullptr; // {bounding rectangle, a part's overflow flag}
     int32_t* rect_host = nullptr; // pinned
     s3r_image_part* parts_dev = nullptr;
     size_t parts_cap = 0;
     cudaStream_t capture = nullptr;
     float* worker_dense[2] = {nullptr, nullptr}; // s3r_render_scene_part: primary / secondary dense field
     size_t worker_cap[2] = {0, 0};
-    // s3r_render_scene_part with the texture filter: per depth a primary / secondary field texture, the
+    // s3r_render_scene_part with the texture filter: per depth field textures for a chunk of blocks (primary /
+    // secondary; kPartTextureBytes of them at most), the
     // transfer-function texture
-    s3r_texture* worker_tex[2][S3R_MAX_DEPTH + 1] = {};
+    std::vector<s3r_texture*> worker_tex[2][S3R_MAX_DEPTH + 1];
+    uint64_t worker_tex_bytes = 0;
     s3r_tf_texture* worker_tf = nullptr;
+    // a part's blocks at once: tables staged through pinned memory, and the pixels' result lists
+    char* part_host = nullptr;
+    char* part_dev = nullptr;
+    size_t part_cap = 0, part_used = 0;
+    char* part_lists = nullptr;
+    size_t part_lists_cap = 0;
     uint64_t launches = 0;
     int sms = 152;
 };
@@ -964,8 +972,8 @@ int s3r_ctx_create(int device, s3r_ctx** out)
     if (!c) return fail(nullptr, S3R_ERR_NOMEM, "out of host memory");
     c->device = device;
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
-    if ((e = cudaMalloc(&c->rect_dev, 4 * sizeof(int32_t))) != cudaSuccess ||
-        (e = cudaMallocHost(&c->rect_host, 4 * sizeof(int32_t))) != cudaSuccess ||
+    if ((e = cudaMalloc(&c->rect_dev, 5 * sizeof(int32_t))) != cudaSuccess ||
+        (e = cudaMallocHost(&c->rect_host, 5 * sizeof(int32_t))) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&c->capture, cudaStreamNonBlocking)) != cudaSuccess) {
         s3r_ctx_destroy(c);
         return cuda_fail(nullptr, e, "context allocation");
@@ -987,7 +995,11 @@ int s3r_ctx_destroy(s3r_ctx* ctx)
     for (float* d : ctx->worker_dense)
         if (d) cudaFree(d);
     for (auto& per_field : ctx->worker_tex)
-        for (s3r_texture* t : per_field) s3r_texture_destroy(t);
+        for (auto& per_depth : per_field)
+            for (s3r_texture* t : per_depth) s3r_texture_destroy(t);
+    if (ctx->part_host) cudaFreeHost(ctx->part_host);
+    if (ctx->part_dev) cudaFree(ctx->part_dev);
+    if (ctx->part_lists) cudaFree(ctx->part_lists);
     s3r_tf_texture_destroy(ctx->worker_tf);
     delete ctx;
     return S3R_OK;
@@ -1172,7 +1184,9 @@ static int render_block_argb_pitched(s3r_ctx* ctx, const s3r_view* view, const f
     block_sampling(view->level, idx, depth, rb);
     rb.pitch = pitch;
     for (int i = 0; i < 4; ++i) rb.rect[i] = rect[i];
-    S3R_CUDA(ctx, launch_render_block_argb(view, brick, rb, tf, viewport, as_stream(stream)));
+    s3r_presentation argb{};
+    argb.mode = S3R_MODE_ARGB;
+    S3R_CUDA(ctx, launch_render_block_mode(view, &argb, brick, nullptr, rb, tf, viewport, as_stream(stream)));
     if (rect[2] > 0 && rect[3] > 0) ++ctx->launches;
     return S3R_OK;
 }
@@ -1259,18 +1273,17 @@ int s3r_split_b2f(uint32_t level, uint32_t split_count, const double eye[3], uin
     return S3R_OK;
 }
 
-int s3r_bound_rect(s3r_ctx* ctx, const uint32_t* viewport, uint32_t W, uint32_t H, int32_t rect[4], void* stream)
+// overflow (optional): what a part's launches left in the flag beside the rectangle.
+static int bound_rect(s3r_ctx* ctx, const uint32_t* viewport, uint32_t W, uint32_t H, int32_t rect[4], int32_t* overflow,
+                      cudaStream_t s)
 {
-    if (!ctx || !viewport || !rect) return fail(ctx, S3R_ERR_INVALID, "null pointer");
-    int rc = set_device(ctx);
-    if (rc) return rc;
-    cudaStream_t s = as_stream(stream);
     int32_t init[4] = {(int32_t)W, (int32_t)H, -1, -1};
     std::memcpy(ctx->rect_host, init, sizeof(init));
     S3R_CUDA(ctx, cudaMemcpyAsync(ctx->rect_dev, ctx->rect_host, sizeof(init), cudaMemcpyHostToDevice, s));
     S3R_CUDA(ctx, launch_bound_rect(viewport, W, H, ctx->rect_dev, s));
     ++ctx->launches;
-    S3R_CUDA(ctx, cudaMemcpyAsync(ctx->rect_host, ctx->rect_dev, sizeof(init), cudaMemcpyDeviceToHost, s));
+    S3R_CUDA(ctx, cudaMemcpyAsync(ctx->rect_host, ctx->rect_dev, (overflow ? 5 : 4) * sizeof(int32_t),
+                                  cudaMemcpyDeviceToHost, s));
     S3R_CUDA(ctx, cudaStreamSynchronize(s));
     const int32_t* r = ctx->rect_host;
     if (r[2] < r[0] || r[3] < r[1]) {
@@ -1281,7 +1294,16 @@ int s3r_bound_rect(s3r_ctx* ctx, const uint32_t* viewport, uint32_t W, uint32_t 
         rect[2] = r[2] - r[0] + 1;
         rect[3] = r[3] - r[1] + 1;
     }
+    if (overflow) *overflow = r[4];
     return S3R_OK;
+}
+
+int s3r_bound_rect(s3r_ctx* ctx, const uint32_t* viewport, uint32_t W, uint32_t H, int32_t rect[4], void* stream)
+{
+    if (!ctx || !viewport || !rect) return fail(ctx, S3R_ERR_INVALID, "null pointer");
+    int rc = set_device(ctx);
+    if (rc) return rc;
+    return bound_rect(ctx, viewport, W, H, rect, nullptr, as_stream(stream));
 }
 
 int s3r_crop(s3r_ctx* ctx, const uint32_t* image, uint32_t W, const int32_t rect[4], uint32_t* dst, void* stream)
@@ -1309,6 +1331,16 @@ int s3r_default_light(const s3r_view* view, s3r_light* out)
     return S3R_OK;
 }
 
+static int check_presentation(s3r_ctx* ctx, const s3r_presentation& pr)
+{
+    if (pr.mode > S3R_MODE_VALUE_ON_ISOSURFACES) return fail(ctx, S3R_ERR_INVALID, "unknown field mode");
+    if (pr.level_count > S3R_MAX_LEVELS) return fail(ctx, S3R_ERR_INVALID, "more than S3R_MAX_LEVELS levels");
+    if (pr.light_count > S3R_MAX_LIGHTS) return fail(ctx, S3R_ERR_INVALID, "more than S3R_MAX_LIGHTS lights");
+    for (uint32_t i = 1; i < pr.level_count; ++i)
+        if (!(pr.levels[i] > pr.levels[i - 1])) return fail(ctx, S3R_ERR_INVALID, "levels must ascend strictly");
+    return S3R_OK;
+}
+
 static int render_block_pitched(s3r_ctx* ctx, const s3r_view* view, const s3r_presentation* pres,
                                 const float* brick, const float* brick2, uint32_t depth, uint32_t pitch,
                                 const uint32_t idx[3], const int32_t rect[4], const float* tf, uint32_t* viewport,
@@ -1318,12 +1350,7 @@ static int render_block_pitched(s3r_ctx* ctx, const s3r_view* view, const s3r_pr
     int rc = check_view(ctx, view);
     if (rc) return rc;
     if (!pres || !brick || !idx || !rect || !tf || !viewport) return fail(ctx, S3R_ERR_INVALID, "null pointer");
-    if (pres->mode > S3R_MODE_VALUE_ON_ISOSURFACES) return fail(ctx, S3R_ERR_INVALID, "unknown field mode");
-    if (pres->level_count > S3R_MAX_LEVELS) return fail(ctx, S3R_ERR_INVALID, "more than S3R_MAX_LEVELS levels");
-    if (pres->light_count > S3R_MAX_LIGHTS) return fail(ctx, S3R_ERR_INVALID, "more than S3R_MAX_LIGHTS lights");
-    for (uint32_t i = 1; i < pres->level_count; ++i)
-        if (!(pres->levels[i] > pres->levels[i - 1]))
-            return fail(ctx, S3R_ERR_INVALID, "levels must ascend strictly");
+    if ((rc = check_presentation(ctx, *pres))) return rc;
     const bool secondary = pres->mode == S3R_MODE_VALUE_ON_ISOSURFACE || pres->mode == S3R_MODE_VALUE_ON_ISOSURFACES;
     if (secondary && !brick2) return fail(ctx, S3R_ERR_INVALID, "this mode needs the secondary field's brick");
     if (secondary && !(pres->secondary_max > pres->secondary_min))
@@ -1493,11 +1520,7 @@ int s3r_render_block_texture(s3r_ctx* ctx, const s3r_view* view, const s3r_prese
     s3r_presentation argb{};
     argb.mode = S3R_MODE_ARGB;
     const s3r_presentation* pr = pres ? pres : &argb;
-    if (pr->mode > S3R_MODE_VALUE_ON_ISOSURFACES) return fail(ctx, S3R_ERR_INVALID, "unknown field mode");
-    if (pr->level_count > S3R_MAX_LEVELS) return fail(ctx, S3R_ERR_INVALID, "more than S3R_MAX_LEVELS levels");
-    if (pr->light_count > S3R_MAX_LIGHTS) return fail(ctx, S3R_ERR_INVALID, "more than S3R_MAX_LIGHTS lights");
-    for (uint32_t i = 1; i < pr->level_count; ++i)
-        if (!(pr->levels[i] > pr->levels[i - 1])) return fail(ctx, S3R_ERR_INVALID, "levels must ascend strictly");
+    if ((rc = check_presentation(ctx, *pr))) return rc;
     const bool secondary = pr->mode == S3R_MODE_VALUE_ON_ISOSURFACE || pr->mode == S3R_MODE_VALUE_ON_ISOSURFACES;
     if (secondary && (!field2 || field2->depth != field->depth))
         return fail(ctx, S3R_ERR_INVALID, "this mode needs the secondary field's texture, of the same depth");
@@ -2252,6 +2275,290 @@ int s3r_render_argb_backward(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view,
 
 } // extern "C"
 
+// ------------------------------------------------------------------ worker loop
+
+namespace {
+
+// A part's blocks are marched by one launch per chunk (part_blocks_kernel) where a pixel's list of results stays
+// short: index boxes of up to kPartSpan blocks along their three axes together (a level of 16^3 blocks: 48), since a
+// ray passes at most that many.  Larger boxes, single blocks, and a part in which some pixel's list overflowed (rays
+// along the faces of blocks meet more) go block by block.
+constexpr uint32_t kPartSpan = 64;
+// Blocks interpolated for one launch and the bytes of their dense fields: enough to fill the GPU several times.
+constexpr uint32_t kPartChunkBlocks = 256;
+constexpr uint64_t kPartChunkBytes = 512ull << 20;
+constexpr uint64_t kPartTextureBytes = 1ull << 30;
+// The lists of a strip of the part's pixels.
+constexpr uint64_t kPartListBytes = 256ull << 20;
+
+bool part_secondary(const s3r_presentation* pres)
+{
+    return pres && (pres->mode == S3R_MODE_VALUE_ON_ISOSURFACE || pres->mode == S3R_MODE_VALUE_ON_ISOSURFACES);
+}
+
+bool part_at_once(const uint32_t bmin[3], const uint32_t bmax[3], size_t blocks)
+{
+    uint64_t span = 0;
+    for (int a = 0; a < 3; ++a) span += bmax[a] > bmin[a] ? bmax[a] - bmin[a] : 0;
+    return blocks > 1 && span <= kPartSpan;
+}
+
+// `bytes` of the context's table buffer: where to write on the host, and where part_upload puts it on the device.
+int part_table(s3r_ctx* ctx, size_t bytes, cudaStream_t s, char** host, char** dev)
+{
+    bytes = (bytes + 255) & ~(size_t)255;
+    if (ctx->part_used + bytes > ctx->part_cap) {
+        // what was staged before has to be on the device, and used, before its memory is used again
+        S3R_CUDA(ctx, cudaStreamSynchronize(s));
+        ctx->part_used = 0;
+        if (bytes > ctx->part_cap) {
+            if (ctx->part_host) cudaFreeHost(ctx->part_host);
+            if (ctx->part_dev) cudaFree(ctx->part_dev);
+            ctx->part_host = ctx->part_dev = nullptr;
+            ctx->part_cap = 0;
+            const size_t cap = std::max<size_t>(2 * bytes, 1 << 20);
+            S3R_CUDA(ctx, cudaMallocHost(&ctx->part_host, cap));
+            S3R_CUDA(ctx, cudaMalloc(&ctx->part_dev, cap));
+            ctx->part_cap = cap;
+        }
+    }
+    *host = ctx->part_host + ctx->part_used;
+    *dev = ctx->part_dev + ctx->part_used;
+    ctx->part_used += bytes;
+    return S3R_OK;
+}
+
+// One chunk of a part: the blocks `refs` (back to front, rectangles not empty) blended onto the viewport.
+int part_blend(s3r_ctx* ctx, const s3r_view* view, const s3r_presentation* pres, std::vector<PartRef>& refs,
+               uint32_t span, const float* tf, unsigned long long tf_tex, bool texture, uint32_t* viewport, cudaStream_t s)
+{
+    if (refs.empty()) return S3R_OK;
+    const uint32_t n = (uint32_t)refs.size();
+    int32_t x0 = INT32_MAX, y0 = INT32_MAX, x1 = INT32_MIN, y1 = INT32_MIN;
+    for (uint32_t i = 0; i < n; ++i) {
+        const int32_t* r = refs[i].rb.rect;
+        x0 = std::min(x0, r[0]);
+        y0 = std::min(y0, r[1]);
+        x1 = std::max(x1, r[0] + r[2]);
+        y1 = std::max(y1, r[1] + r[3]);
+        refs[i].order = i;
+    }
+    // the deepest blocks' rays take the most samples: their CTAs start first
+    std::stable_sort(refs.begin(), refs.end(),
+                     [](const PartRef& a, const PartRef& b) { return a.rb.depth > b.rb.depth; });
+    PartArgs a{};
+    a.nblocks = n;
+    a.cap = std::min(n, span + 1);
+    a.tf = tf;
+    a.tf_tex = tf_tex;
+    a.x0 = x0;
+    a.w = x1 - x0;
+    a.overflow = ctx->rect_dev + 4;
+    const uint64_t per_pixel = sizeof(uint32_t) + a.cap * (sizeof(float4) + sizeof(uint16_t));
+    const int32_t rows = (int32_t)std::max<uint64_t>(
+        1, std::min<uint64_t>((uint64_t)(y1 - y0), kPartListBytes / (per_pixel * (uint64_t)a.w)));
+    const size_t lists = (size_t)rows * a.w * per_pixel;
+    if (ctx->part_lists_cap < lists) {
+        if (ctx->part_lists) cudaFree(ctx->part_lists);
+        ctx->part_lists = nullptr;
+        ctx->part_lists_cap = 0;
+        S3R_CUDA(ctx, cudaMalloc(&ctx->part_lists, lists));
+        ctx->part_lists_cap = lists;
+    }
+    const size_t npix = (size_t)rows * a.w;
+    a.result = reinterpret_cast<float4*>(ctx->part_lists);
+    a.count = reinterpret_cast<uint32_t*>(a.result + a.cap * npix);
+    a.order = reinterpret_cast<uint16_t*>(a.count + npix);
+    const uint32_t strips = (uint32_t)((y1 - y0 + rows - 1) / rows);
+    char *host, *dev;
+    const size_t refs_bytes = n * sizeof(PartRef), first_bytes = (n + 1) * sizeof(uint32_t);
+    if (int rc = part_table(ctx, refs_bytes + strips * first_bytes, s, &host, &dev)) return rc;
+    std::memcpy(host, refs.data(), refs_bytes);
+    uint32_t tw, th;
+    part_tile(pres->mode, texture, tw, th);
+    for (uint32_t k = 0; k < strips; ++k) {
+        uint32_t* first = reinterpret_cast<uint32_t*>(host + refs_bytes + k * first_bytes);
+        const int32_t s0 = y0 + (int32_t)k * rows, s1 = std::min(s0 + rows, y1);
+        uint64_t at = 0;
+        for (uint32_t i = 0; i < n; ++i) {
+            const int32_t* r = refs[i].rb.rect;
+            const int32_t h = std::min(r[1] + r[3], s1) - std::max(r[1], s0);
+            first[i] = (uint32_t)at;
+            if (h > 0) at += (uint64_t)(((uint32_t)r[2] + tw - 1) / tw) * (((uint32_t)h + th - 1) / th);
+        }
+        if (at > 0x7fffffffull) return fail(ctx, S3R_ERR_INVALID, "the part's rectangles are too large");
+        first[n] = (uint32_t)at;
+    }
+    S3R_CUDA(ctx, cudaMemcpyAsync(dev, host, refs_bytes + strips * first_bytes, cudaMemcpyHostToDevice, s));
+    a.refs = reinterpret_cast<const PartRef*>(dev);
+    for (uint32_t k = 0; k < strips; ++k) {
+        a.first = reinterpret_cast<const uint32_t*>(dev + refs_bytes + k * first_bytes);
+        a.y0 = y0 + (int32_t)k * rows;
+        a.h = std::min(rows, y1 - a.y0);
+        const uint32_t ctas = reinterpret_cast<const uint32_t*>(host + refs_bytes + k * first_bytes)[n];
+        S3R_CUDA(ctx, launch_part(view, pres, a, ctas, texture, viewport, s));
+        ctx->launches += 2;
+    }
+    return S3R_OK;
+}
+
+// Field textures for `need[d]` blocks of each depth (per field), kept by the context for the next chunk and call.
+int part_textures(s3r_ctx* ctx, const uint32_t need[S3R_MAX_DEPTH + 1], int fields, cudaStream_t s)
+{
+    auto bytes_of = [](uint32_t d) { return grid_vertices(d) * sizeof(float); };
+    uint64_t more = 0;
+    for (int f = 0; f < fields; ++f)
+        for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d)
+            if (need[d] > ctx->worker_tex[f][d].size()) more += (need[d] - ctx->worker_tex[f][d].size()) * bytes_of(d);
+    if (more && ctx->worker_tex_bytes + more > kPartTextureBytes) {
+        S3R_CUDA(ctx, cudaStreamSynchronize(s));
+        for (auto& per_field : ctx->worker_tex)
+            for (auto& per_depth : per_field) {
+                for (s3r_texture* t : per_depth) s3r_texture_destroy(t);
+                per_depth.clear();
+            }
+        ctx->worker_tex_bytes = 0;
+    }
+    for (int f = 0; f < fields; ++f)
+        for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d)
+            while (ctx->worker_tex[f][d].size() < need[d]) {
+                s3r_texture* t = nullptr;
+                if (int rc = s3r_texture_create(ctx, d, &t)) return rc;
+                ctx->worker_tex[f][d].push_back(t);
+                ctx->worker_tex_bytes += bytes_of(d);
+            }
+    return S3R_OK;
+}
+
+// A block of the part: its index in the caller's list and its view rectangle.
+struct PartBlock {
+    uint32_t b;
+    int32_t rect[4];
+};
+
+// s3r_render_scene_part's blocks, back to front, in chunks: each chunk's blocks interpolated by one set of launches
+// (into the context's field textures, or into dense grids), then blended.
+int part_from_nodes(s3r_ctx* ctx, const s3r_view* view, const s3r_presentation* pres, const s3r_worker_blocks* wb,
+                    const std::vector<PartBlock>& blocks, uint32_t span, const float* tf, uint32_t* viewport,
+                    cudaStream_t s)
+{
+    const bool tex = view->filter == S3R_FILTER_TEXTURE, secondary = part_secondary(pres);
+    const int fields = secondary ? 2 : 1;
+    size_t at = 0;
+    while (at < blocks.size()) {
+        uint64_t vertices = 0;
+        size_t end = at;
+        while (end < blocks.size() && end - at < kPartChunkBlocks) {
+            const uint64_t more = grid_vertices(wb->blocks[4 * blocks[end].b + 3]);
+            if (end > at && (vertices + more) * sizeof(float) > kPartChunkBytes) break;
+            vertices += more;
+            ++end;
+        }
+        const uint32_t n = (uint32_t)(end - at);
+        uint32_t need[S3R_MAX_DEPTH + 1] = {};
+        for (size_t i = at; i < end; ++i) ++need[wb->blocks[4 * blocks[i].b + 3]];
+        if (tex) {
+            if (int rc = part_textures(ctx, need, fields, s)) return rc;
+        } else {
+            for (int f = 0; f < fields; ++f)
+                if (ctx->worker_cap[f] < vertices) {
+                    if (ctx->worker_dense[f]) cudaFree(ctx->worker_dense[f]);
+                    ctx->worker_dense[f] = nullptr;
+                    ctx->worker_cap[f] = 0;
+                    S3R_CUDA(ctx, cudaMalloc(&ctx->worker_dense[f], vertices * sizeof(float)));
+                    ctx->worker_cap[f] = vertices;
+                }
+        }
+        char *host, *dev;
+        const uint32_t ng = n * (uint32_t)fields;
+        if (int rc = part_table(ctx, ng * sizeof(GridBlock) + (ng + 1) * sizeof(uint32_t), s, &host, &dev)) return rc;
+        GridBlock* gb = reinterpret_cast<GridBlock*>(host);
+        uint32_t* tile_off = reinterpret_cast<uint32_t*>(host + ng * sizeof(GridBlock));
+        std::vector<PartRef> refs(n);
+        uint64_t vals = 0, words = 0;
+        uint32_t tiles = 0, scattered = 0, depth_max = 0, g = 0;
+        for (int f = 0; f < fields; ++f) {
+            uint32_t used[S3R_MAX_DEPTH + 1] = {};
+            uint64_t dense = 0;
+            for (uint32_t i = 0; i < n; ++i, ++g) {
+                const PartBlock& pb = blocks[at + i];
+                const uint32_t* bl = wb->blocks + 4 * pb.b;
+                const uint64_t o = wb->node_off[pb.b], nn = wb->node_off[pb.b + 1] - o;
+                GridBlock q = grid_block(wb->n2i + 3 * o, (f ? wb->sparse2 : wb->sparse) + o, (uint32_t)nn, bl[3]);
+                if (!q.direct) {
+                    q.val_off = vals;
+                    q.bit_off = words;
+                    vals += grid_vertices(bl[3]);
+                    words += grid_mask_words(bl[3]);
+                    scattered = std::max(scattered, (uint32_t)nn);
+                }
+                unsigned long long src;
+                if (tex) {
+                    s3r_texture* t = ctx->worker_tex[f][bl[3]][used[bl[3]]++];
+                    q.surface = t->surf;
+                    src = t->tex;
+                } else {
+                    q.out = ctx->worker_dense[f] + dense;
+                    src = (unsigned long long)(uintptr_t)q.out;
+                    dense += grid_vertices(bl[3]);
+                }
+                gb[g] = q;
+                tile_off[g] = tiles;
+                tiles += grid_tiles(bl[3]);
+                depth_max = std::max(depth_max, bl[3]);
+                PartRef& r = refs[i];
+                if (f == 0) {
+                    r = PartRef{};
+                    block_sampling(view->level, bl, bl[3], r.rb);
+                    std::memcpy(r.rb.rect, pb.rect, sizeof(pb.rect));
+                    r.src1 = src;
+                } else {
+                    r.src2 = src;
+                }
+            }
+        }
+        tile_off[ng] = tiles;
+        if (words)
+            if (int rc = ensure_grid(ctx, vals, words)) return rc;
+        S3R_CUDA(ctx, cudaMemcpyAsync(dev, host, ng * sizeof(GridBlock) + (ng + 1) * sizeof(uint32_t),
+                                      cudaMemcpyHostToDevice, s));
+        GridArgs a{};
+        a.table = reinterpret_cast<const GridBlock*>(dev);
+        a.tile_off = reinterpret_cast<const uint32_t*>(dev + ng * sizeof(GridBlock));
+        a.nblocks = ng;
+        a.tiles = tiles;
+        a.depth_max = depth_max;
+        a.vals = ctx->grid;
+        a.bits = ctx->grid_bits;
+        uint32_t launches = 0;
+        S3R_CUDA(ctx, launch_interp_grid(a, tex, scattered, words, s, &launches));
+        ctx->launches += launches;
+        if (int rc = part_blend(ctx, view, pres, refs, span, tf, tex ? ctx->worker_tf->tex : 0, tex, viewport, s))
+            return rc;
+        at = end;
+    }
+    return S3R_OK;
+}
+
+// The checks that the per-block calls make before they launch.
+int check_part(s3r_ctx* ctx, const s3r_view* view, const s3r_presentation* pres, const uint32_t* blocks,
+               const std::vector<PartBlock>& list)
+{
+    if (pres) {
+        if (int rc = check_presentation(ctx, *pres)) return rc;
+        if (part_secondary(pres) && !(pres->secondary_max > pres->secondary_min))
+            return fail(ctx, S3R_ERR_INVALID, "secondary field range is empty");
+    }
+    const uint32_t m = 1u << view->level;
+    for (const PartBlock& p : list) {
+        const uint32_t* bl = blocks + 4 * p.b;
+        if (bl[0] >= m || bl[1] >= m || bl[2] >= m) return fail(ctx, S3R_ERR_INVALID, "block index outside level");
+    }
+    return S3R_OK;
+}
+
+} // namespace
+
 extern "C" {
 
 int s3r_render_scene_part(s3r_ctx* ctx, const s3r_view* view, const s3r_presentation* pres,
@@ -2264,8 +2571,7 @@ int s3r_render_scene_part(s3r_ctx* ctx, const s3r_view* view, const s3r_presenta
     if (!wb || !box_min || !box_max || !tf || !viewport || !rect) return fail(ctx, S3R_ERR_INVALID, "null pointer");
     if (wb->nblocks && (!wb->blocks || !wb->node_off || !wb->n2i || !wb->sparse))
         return fail(ctx, S3R_ERR_INVALID, "null block data");
-    const bool secondary = pres && (pres->mode == S3R_MODE_VALUE_ON_ISOSURFACE ||
-                                    pres->mode == S3R_MODE_VALUE_ON_ISOSURFACES);
+    const bool secondary = part_secondary(pres);
     if (secondary && !wb->sparse2) return fail(ctx, S3R_ERR_INVALID, "this mode needs the secondary field");
     if ((rc = set_device(ctx))) return rc;
     const cudaStream_t s = as_stream(stream);
@@ -2294,70 +2600,78 @@ int s3r_render_scene_part(s3r_ctx* ctx, const s3r_view* view, const s3r_presenta
         const uint32_t* bl = wb->blocks + 4 * b;
         where[(uint64_t)bl[0] | ((uint64_t)bl[1] << 21) | ((uint64_t)bl[2] << 42)] = b;
     }
+    // the blocks that can show, back to front
+    std::vector<PartBlock> list;
     b2f_traverse(sp, [&](const uint32_t q[3]) {
         if (rc) return;
         auto it = where.find((uint64_t)q[0] | ((uint64_t)q[1] << 21) | ((uint64_t)q[2] << 42));
         if (it == where.end()) return; // not a block of this set
-        const uint32_t b = it->second;
-        const uint32_t depth = wb->blocks[4 * b + 3];
-        if (depth > S3R_MAX_DEPTH) {
+        PartBlock p;
+        p.b = it->second;
+        if (wb->blocks[4 * p.b + 3] > S3R_MAX_DEPTH) {
             rc = fail(ctx, S3R_ERR_INVALID, "depth exceeds S3R_MAX_DEPTH");
             return;
         }
-        const uint64_t o = wb->node_off[b], n = wb->node_off[b + 1] - o;
+        view_rect(*view, wb->blocks + 4 * p.b, p.rect);
+        if (p.rect[2] > 0 && p.rect[3] > 0) list.push_back(p);
+    });
+    if (rc) return rc;
+    if (!list.empty() && (rc = check_part(ctx, view, pres, wb->blocks, list))) return rc;
+    if (part_at_once(box_min, box_max, list.size())) {
+        uint32_t span = 0;
+        for (int a = 0; a < 3; ++a) span += box_max[a] - box_min[a];
+        s3r_presentation argb{};
+        argb.mode = S3R_MODE_ARGB;
+        ctx->part_used = 0; // every call ends with its stream drained
+        S3R_CUDA(ctx, cudaMemsetAsync(ctx->rect_dev + 4, 0, sizeof(int32_t), s));
+        if ((rc = part_from_nodes(ctx, view, pres ? pres : &argb, wb, list, span, tf, viewport, s))) {
+            cudaStreamSynchronize(s); // the staged tables may still be read
+            return rc;
+        }
+        int32_t overflow = 0;
+        if ((rc = bound_rect(ctx, viewport, view->W, view->H, rect, &overflow, s)) || !overflow) return rc;
+        if ((rc = s3r_clear_viewport(ctx, viewport, view->W, view->H, clear, stream))) return rc;
+    }
+    for (const PartBlock& p : list) {
+        const uint32_t* bl = wb->blocks + 4 * p.b;
+        const uint32_t depth = bl[3];
+        const uint64_t o = wb->node_off[p.b], n = wb->node_off[p.b + 1] - o;
         if (tex) {
             // DeviceField::makeField: the block's dense field interpolated into the depth's field texture
-            for (int f = 0; f < (secondary ? 2 : 1); ++f) {
-                if (!ctx->worker_tex[f][depth] && (rc = s3r_texture_create(ctx, depth, &ctx->worker_tex[f][depth])))
-                    return;
+            uint32_t need[S3R_MAX_DEPTH + 1] = {};
+            need[depth] = 1;
+            if ((rc = part_textures(ctx, need, secondary ? 2 : 1, s))) return rc;
+            for (int f = 0; f < (secondary ? 2 : 1); ++f)
                 if ((rc = s3r_interp_dense_texture(ctx, wb->n2i + 3 * o, (f ? wb->sparse2 : wb->sparse) + o,
-                                                   (uint32_t)n, ctx->worker_tex[f][depth], stream)))
-                    return;
-            }
-            int32_t r[4];
-            view_rect(*view, wb->blocks + 4 * b, r);
-            if (r[2] <= 0 || r[3] <= 0) return;
-            rc = s3r_render_block_texture(ctx, view, pres, ctx->worker_tex[0][depth],
-                                          secondary ? ctx->worker_tex[1][depth] : nullptr, wb->blocks + 4 * b, r,
-                                          ctx->worker_tf, viewport, stream);
-            return;
+                                                   (uint32_t)n, ctx->worker_tex[f][depth][0], stream)))
+                    return rc;
+            if ((rc = s3r_render_block_texture(ctx, view, pres, ctx->worker_tex[0][depth][0],
+                                               secondary ? ctx->worker_tex[1][depth][0] : nullptr, bl, p.rect,
+                                               ctx->worker_tf, viewport, stream)))
+                return rc;
+            continue;
         }
-        const uint64_t e = (1ull << depth) + 1, count = e * e * e;
+        const uint64_t count = grid_vertices(depth);
         for (int f = 0; f < (secondary ? 2 : 1); ++f)
             if (ctx->worker_cap[f] < count) {
                 if (ctx->worker_dense[f]) cudaFree(ctx->worker_dense[f]);
                 ctx->worker_dense[f] = nullptr;
                 ctx->worker_cap[f] = 0;
-                const cudaError_t err = cudaMalloc(&ctx->worker_dense[f], count * sizeof(float));
-                if (err != cudaSuccess) {
-                    rc = cuda_fail(ctx, err, "cudaMalloc(worker dense field)");
-                    return;
-                }
+                S3R_CUDA(ctx, cudaMalloc(&ctx->worker_dense[f], count * sizeof(float)));
                 ctx->worker_cap[f] = count;
             }
         // DeviceField::makeField: the block's dense field from its nodes
-        if ((rc = s3r_interp_dense(ctx, wb->n2i + 3 * o, wb->sparse + o, (uint32_t)n, depth, ctx->worker_dense[0],
-                                   stream)))
-            return;
-        if (secondary && (rc = s3r_interp_dense(ctx, wb->n2i + 3 * o, wb->sparse2 + o, (uint32_t)n, depth,
-                                                ctx->worker_dense[1], stream)))
-            return;
-        int32_t r[4];
-        view_rect(*view, wb->blocks + 4 * b, r);
-        if (r[2] <= 0 || r[3] <= 0) return;
+        for (int f = 0; f < (secondary ? 2 : 1); ++f)
+            if ((rc = s3r_interp_dense(ctx, wb->n2i + 3 * o, (f ? wb->sparse2 : wb->sparse) + o, (uint32_t)n, depth,
+                                       ctx->worker_dense[f], stream)))
+                return rc;
         rc = pres ? s3r_render_block(ctx, view, pres, ctx->worker_dense[0], secondary ? ctx->worker_dense[1] : nullptr,
-                                     depth, wb->blocks + 4 * b, r, tf, viewport, stream)
-                  : s3r_render_block_argb(ctx, view, ctx->worker_dense[0], depth, wb->blocks + 4 * b, r, tf, viewport,
-                                          stream);
-    });
-    if (rc) return rc;
-    (void)s;
+                                     depth, bl, p.rect, tf, viewport, stream)
+                  : s3r_render_block_argb(ctx, view, ctx->worker_dense[0], depth, bl, p.rect, tf, viewport, stream);
+        if (rc) return rc;
+    }
     return s3r_bound_rect(ctx, viewport, view->W, view->H, rect, stream);
 }
-
-} // extern "C"
-
-extern "C" {
 
 int s3r_render_scene_part_bricks(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const s3r_presentation* pres,
                                  const void* bricks2, const uint32_t box_min[3], const uint32_t box_max[3],
@@ -2370,10 +2684,10 @@ int s3r_render_scene_part_bricks(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* v
     if (view->level != plan->level) return fail(ctx, S3R_ERR_INVALID, "view level differs from the plan level");
     if (!box_min || !box_max || !tf || !viewport || !rect) return fail(ctx, S3R_ERR_INVALID, "null pointer");
     if (plan->fmt != S3R_BRICK_F32) return fail(ctx, S3R_ERR_UNSUPPORTED, "the per-block renderer reads F32 bricks");
-    const bool secondary = pres && (pres->mode == S3R_MODE_VALUE_ON_ISOSURFACE ||
-                                    pres->mode == S3R_MODE_VALUE_ON_ISOSURFACES);
+    const bool secondary = part_secondary(pres);
     if (secondary && !bricks2) return fail(ctx, S3R_ERR_INVALID, "this mode needs the secondary bricks");
     if ((rc = set_device(ctx))) return rc;
+    const cudaStream_t s = as_stream(stream);
     const uint32_t clear = pres && pres->mode == S3R_MODE_MAX_INTENSITY ? 0x7fc00000u : 0u;
     if ((rc = s3r_clear_viewport(ctx, viewport, view->W, view->H, clear, stream))) return rc;
     double cmin[3], cmax[3];
@@ -2382,29 +2696,53 @@ int s3r_render_scene_part_bricks(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* v
     for (int a = 0; a < 3; ++a)
         sp[a] = split_range(box_min[a], box_max[a], (float)cmin[a], (float)cmax[a], view->cam.eye[a]);
     const uint32_t m = 1u << plan->level;
-    std::vector<int32_t> where((size_t)m * m * m, -1);
-    for (uint32_t b = 0; b < plan->nblocks; ++b) {
-        const uint32_t* bl = &plan->blocks[4 * b];
-        where[bl[0] + m * (bl[1] + (size_t)m * bl[2])] = (int32_t)b;
-    }
+    std::vector<PartBlock> list;
+    b2f_traverse(sp, [&](const uint32_t q[3]) {
+        if (q[0] >= m || q[1] >= m || q[2] >= m) return;
+        const RenderBlock& t = plan->table_host[q[0] + m * (q[1] + (size_t)m * q[2])];
+        if (t.depth == 0xffffffffu) return;
+        PartBlock p;
+        p.b = t.block;
+        view_rect(*view, &plan->blocks[4 * p.b], p.rect);
+        if (p.rect[2] > 0 && p.rect[3] > 0) list.push_back(p);
+    });
+    if (!list.empty() && (rc = check_part(ctx, view, pres, plan->blocks.data(), list))) return rc;
     const float* bricks = static_cast<const float*>(plan->bricks);
     const float* b2 = static_cast<const float*>(bricks2);
-    b2f_traverse(sp, [&](const uint32_t q[3]) {
-        if (rc) return;
-        if (q[0] >= m || q[1] >= m || q[2] >= m) return;
-        const int32_t b = where[q[0] + m * (q[1] + (size_t)m * q[2])];
-        if (b < 0) return;
-        const uint32_t* bl = &plan->blocks[4 * b];
-        int32_t r[4];
-        view_rect(*view, bl, r);
-        if (r[2] <= 0 || r[3] <= 0) return;
-        const uint64_t o = plan->vertex_off[b];
-        const uint32_t pitch = plan->pitch[b];
+    if (part_at_once(box_min, box_max, list.size())) {
+        uint32_t span = 0;
+        for (int a = 0; a < 3; ++a) span += box_max[a] - box_min[a];
+        s3r_presentation argb{};
+        argb.mode = S3R_MODE_ARGB;
+        std::vector<PartRef> refs(list.size());
+        for (size_t i = 0; i < list.size(); ++i) {
+            const uint32_t* bl = &plan->blocks[4 * list[i].b];
+            PartRef& r = refs[i];
+            r.rb = plan->table_host[bl[0] + m * (bl[1] + (size_t)m * bl[2])];
+            std::memcpy(r.rb.rect, list[i].rect, sizeof(r.rb.rect));
+            const uint64_t o = plan->vertex_off[list[i].b];
+            r.src1 = (unsigned long long)(uintptr_t)(bricks + o);
+            r.src2 = secondary ? (unsigned long long)(uintptr_t)(b2 + o) : 0;
+        }
+        ctx->part_used = 0; // every call ends with its stream drained
+        S3R_CUDA(ctx, cudaMemsetAsync(ctx->rect_dev + 4, 0, sizeof(int32_t), s));
+        if ((rc = part_blend(ctx, view, pres ? pres : &argb, refs, span, tf, 0, false, viewport, s))) {
+            cudaStreamSynchronize(s); // the staged tables may still be read
+            return rc;
+        }
+        int32_t overflow = 0;
+        if ((rc = bound_rect(ctx, viewport, view->W, view->H, rect, &overflow, s)) || !overflow) return rc;
+        if ((rc = s3r_clear_viewport(ctx, viewport, view->W, view->H, clear, stream))) return rc;
+    }
+    for (const PartBlock& p : list) {
+        const uint32_t* bl = &plan->blocks[4 * p.b];
+        const uint64_t o = plan->vertex_off[p.b];
+        const uint32_t pitch = plan->pitch[p.b];
         rc = pres ? render_block_pitched(ctx, view, pres, bricks + o, secondary ? b2 + o : nullptr, bl[3], pitch, bl,
-                                         r, tf, viewport, stream)
-                  : render_block_argb_pitched(ctx, view, bricks + o, bl[3], pitch, bl, r, tf, viewport, stream);
-    });
-    if (rc) return rc;
+                                         p.rect, tf, viewport, stream)
+                  : render_block_argb_pitched(ctx, view, bricks + o, bl[3], pitch, bl, p.rect, tf, viewport, stream);
+        if (rc) return rc;
+    }
     return s3r_bound_rect(ctx, viewport, view->W, view->H, rect, stream);
 }
 

@@ -233,8 +233,31 @@ cudaError_t launch_render_block_texture(const s3r_view* view_host, const s3r_pre
 cudaError_t launch_render_block_mode(const s3r_view* view_host, const s3r_presentation* pres, const float* brick,
                                      const float* brick2, const RenderBlock& rb, const float* tf, uint32_t* viewport,
                                      cudaStream_t s);
-cudaError_t launch_render_block_argb(const s3r_view* view_host, const float* brick, const RenderBlock& rb,
-                                     const float* tf, uint32_t* viewport, cudaStream_t s);
+// The blocks of a worker's part at once (part_blocks_kernel, part_composite_kernel), for the strip of pixels
+// [x0, x0 + w) x [y0, y0 + h).
+struct PartRef {
+    RenderBlock rb;
+    unsigned long long src1, src2; // primary / secondary field: the brick's address or the texture object
+    uint32_t order;                // place in the back-to-front order, below 65536
+    uint32_t pad;
+};
+struct PartArgs {
+    const PartRef* refs;    // nblocks blocks, the longest marches first
+    const uint32_t* first;  // nblocks + 1: running counts of the blocks' CTAs in this strip
+    uint32_t nblocks;
+    uint32_t cap;           // results a pixel's list holds
+    const float* tf;
+    unsigned long long tf_tex;
+    int32_t x0, y0, w, h;
+    uint32_t* count;        // per pixel: results appended
+    float4* result;         // [slot][pixel]
+    uint16_t* order;        // [slot][pixel]
+    int32_t* overflow;      // set when a pixel's list is too short
+};
+// Pixels of a part_blocks_kernel CTA.
+void part_tile(uint32_t mode, bool texture, uint32_t& w, uint32_t& h);
+cudaError_t launch_part(const s3r_view* view_host, const s3r_presentation* pres, const PartArgs& a, uint32_t ctas,
+                        bool texture, uint32_t* viewport, cudaStream_t s);
 cudaError_t launch_frame_render(const FrameArgs& a, uint32_t W, uint32_t H, uint32_t tf_n, uint32_t fmt,
                                 uint32_t tile_shape, uint32_t filter, cudaStream_t s);
 // The block-major form: segment kernel (persistent grid of ctas CTAs, 0: as many as fit on sms SMs) over
