@@ -32,7 +32,7 @@ struct s3r_ctx {
     size_t grid_cap = 0;   // floats
     uint32_t* grid_bits = nullptr;
     size_t grid_bits_cap = 0; // words
-    int32_t* rect_dev = nullptr; // {bounding rectangle, a part's overflow flag}
+    int32_t* rect_dev = nullptr; // launch_bound_rect's accumulators, a part's overflow flag among them
     int32_t* rect_host = nullptr; // pinned
     s3r_image_part* parts_dev = nullptr;
     size_t parts_cap = 0;
@@ -972,7 +972,8 @@ int s3r_ctx_create(int device, s3r_ctx** out)
     if (!c) return fail(nullptr, S3R_ERR_NOMEM, "out of host memory");
     c->device = device;
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
-    if ((e = cudaMalloc(&c->rect_dev, 5 * sizeof(int32_t))) != cudaSuccess ||
+    if ((e = cudaMalloc(&c->rect_dev, 6 * sizeof(int32_t))) != cudaSuccess ||
+        (e = cudaMemset(c->rect_dev, 0, 6 * sizeof(int32_t))) != cudaSuccess ||
         (e = cudaMallocHost(&c->rect_host, 5 * sizeof(int32_t))) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&c->capture, cudaStreamNonBlocking)) != cudaSuccess) {
         s3r_ctx_destroy(c);
@@ -1277,22 +1278,17 @@ int s3r_split_b2f(uint32_t level, uint32_t split_count, const double eye[3], uin
 static int bound_rect(s3r_ctx* ctx, const uint32_t* viewport, uint32_t W, uint32_t H, int32_t rect[4], int32_t* overflow,
                       cudaStream_t s)
 {
-    int32_t init[4] = {(int32_t)W, (int32_t)H, -1, -1};
-    std::memcpy(ctx->rect_host, init, sizeof(init));
-    S3R_CUDA(ctx, cudaMemcpyAsync(ctx->rect_dev, ctx->rect_host, sizeof(init), cudaMemcpyHostToDevice, s));
-    S3R_CUDA(ctx, launch_bound_rect(viewport, W, H, ctx->rect_dev, s));
+    S3R_CUDA(ctx, launch_bound_rect(viewport, W, H, ctx->rect_dev, ctx->rect_host, s));
     ++ctx->launches;
-    S3R_CUDA(ctx, cudaMemcpyAsync(ctx->rect_host, ctx->rect_dev, (overflow ? 5 : 4) * sizeof(int32_t),
-                                  cudaMemcpyDeviceToHost, s));
     S3R_CUDA(ctx, cudaStreamSynchronize(s));
     const int32_t* r = ctx->rect_host;
-    if (r[2] < r[0] || r[3] < r[1]) {
+    if (r[2] == 0) {
         rect[0] = rect[1] = rect[2] = rect[3] = 0;
     } else {
-        rect[0] = r[0];
-        rect[1] = r[1];
-        rect[2] = r[2] - r[0] + 1;
-        rect[3] = r[3] - r[1] + 1;
+        rect[0] = (int32_t)W - r[0];
+        rect[1] = (int32_t)H - r[1];
+        rect[2] = r[2] - rect[0];
+        rect[3] = r[3] - rect[1];
     }
     if (overflow) *overflow = r[4];
     return S3R_OK;
@@ -1603,17 +1599,21 @@ int s3r_compose_parts(s3r_ctx* ctx, const s3r_image_part* parts, uint32_t nparts
     int rc = set_device(ctx);
     if (rc) return rc;
     if (nparts == 0) return S3R_OK;
-    if (ctx->parts_cap < nparts) {
-        if (ctx->parts_dev) cudaFree(ctx->parts_dev);
-        ctx->parts_dev = nullptr;
-        ctx->parts_cap = 0;
-        S3R_CUDA(ctx, cudaMalloc(&ctx->parts_dev, sizeof(s3r_image_part) * nparts));
-        ctx->parts_cap = nparts;
-    }
     cudaStream_t s = as_stream(stream);
-    S3R_CUDA(ctx, cudaMemcpyAsync(ctx->parts_dev, parts, sizeof(s3r_image_part) * nparts, cudaMemcpyHostToDevice, s));
-    S3R_CUDA(ctx, launch_compose(ctx->parts_dev, nparts, just_copy_first, dst, dw, dh, offx, offy, s));
-    // the parts array is pageable host memory copied asynchronously: finish before returning
+    if (nparts > kComposeInline) {
+        if (ctx->parts_cap < nparts) {
+            if (ctx->parts_dev) cudaFree(ctx->parts_dev);
+            ctx->parts_dev = nullptr;
+            ctx->parts_cap = 0;
+            S3R_CUDA(ctx, cudaMalloc(&ctx->parts_dev, sizeof(s3r_image_part) * nparts));
+            ctx->parts_cap = nparts;
+        }
+        S3R_CUDA(ctx, cudaMemcpyAsync(ctx->parts_dev, parts, sizeof(s3r_image_part) * nparts, cudaMemcpyHostToDevice, s));
+    }
+    S3R_CUDA(ctx, launch_compose(parts, nparts > kComposeInline ? ctx->parts_dev : nullptr, nparts, just_copy_first, dst,
+                                 dw, dh, offx, offy, s));
+    // callers may release the parts' pixels on return (and a longer list is pageable host memory copied
+    // asynchronously): finish first
     S3R_CUDA(ctx, cudaStreamSynchronize(s));
     ++ctx->launches;
     return S3R_OK;
@@ -2623,7 +2623,6 @@ int s3r_render_scene_part(s3r_ctx* ctx, const s3r_view* view, const s3r_presenta
         s3r_presentation argb{};
         argb.mode = S3R_MODE_ARGB;
         ctx->part_used = 0; // every call ends with its stream drained
-        S3R_CUDA(ctx, cudaMemsetAsync(ctx->rect_dev + 4, 0, sizeof(int32_t), s));
         if ((rc = part_from_nodes(ctx, view, pres ? pres : &argb, wb, list, span, tf, viewport, s))) {
             cudaStreamSynchronize(s); // the staged tables may still be read
             return rc;
@@ -2725,7 +2724,6 @@ int s3r_render_scene_part_bricks(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* v
             r.src2 = secondary ? (unsigned long long)(uintptr_t)(b2 + o) : 0;
         }
         ctx->part_used = 0; // every call ends with its stream drained
-        S3R_CUDA(ctx, cudaMemsetAsync(ctx->rect_dev + 4, 0, sizeof(int32_t), s));
         if ((rc = part_blend(ctx, view, pres ? pres : &argb, refs, span, tf, 0, false, viewport, s))) {
             cudaStreamSynchronize(s); // the staged tables may still be read
             return rc;

@@ -34,10 +34,13 @@
 namespace s3r {
 namespace {
 
-__global__ void fill_u32_kernel(uint32_t* p, uint64_t n, uint32_t v)
+// p: 16-byte aligned up to the last n % 4 words, or (vec false) anywhere
+__global__ void fill_u32_kernel(uint32_t* p, uint64_t n, uint32_t v, bool vec)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        p[i] = v;
+    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, step = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t n4 = vec ? n / 4 : 0;
+    for (uint64_t i = t; i < n4; i += step) reinterpret_cast<uint4*>(p)[i] = make_uint4(v, v, v, v);
+    for (uint64_t i = 4 * n4 + t; i < n; i += step) p[i] = v;
 }
 
 // vals[ord(n2i[i])] = sparse[i] and the vertex's bit, for the scattered blocks of a set (block blockIdx.y)
@@ -338,7 +341,8 @@ cudaError_t launch_tiles(const TileArgs& a, uint32_t tile_log2_max, uint32_t gri
 
 cudaError_t launch_fill_u32(uint32_t* p, uint64_t n, uint32_t v, cudaStream_t s)
 {
-    fill_u32_kernel<<<ctas_for(n, 256), 256, 0, s>>>(p, n, v);
+    const bool vec = reinterpret_cast<uintptr_t>(p) % 16 == 0;
+    fill_u32_kernel<<<ctas_for(vec ? (n + 3) / 4 : n, 256), 256, 0, s>>>(p, n, v, vec);
     return cudaGetLastError();
 }
 

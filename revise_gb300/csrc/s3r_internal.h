@@ -270,10 +270,16 @@ cudaError_t launch_frame_backward(const FrameArgs& a, uint32_t W, uint32_t H, ui
 // dtf[i] += sum over the kDtfParts copies of part[. * n + i], n = 4 * tf_n
 cudaError_t launch_dtf_reduce(const float* part, float* dtf, uint32_t n, cudaStream_t s);
 
-cudaError_t launch_bound_rect(const uint32_t* img, uint32_t W, uint32_t H, int32_t* rect_dev, cudaStream_t s);
+// acc: six zeros (again afterwards); acc[4] is a flag that travels along.  host (pinned): {W - min x, H - min y,
+// max x + 1, max y + 1, flag}, the bounds 0 when no pixel is opaque.
+cudaError_t launch_bound_rect(const uint32_t* img, uint32_t W, uint32_t H, int32_t* acc, int32_t* host,
+                              cudaStream_t s);
 cudaError_t launch_crop(const uint32_t* img, uint32_t W, const int32_t rect[4], uint32_t* dst, cudaStream_t s);
-cudaError_t launch_compose(const s3r_image_part* parts_dev, uint32_t nparts, int32_t just_copy_first, uint32_t* dst,
-                           int32_t dw, int32_t dh, int32_t offx, int32_t offy, cudaStream_t s);
+// Up to kComposeInline parts are passed by value (parts_dev null), more by their device copy.
+constexpr uint32_t kComposeInline = 8;
+cudaError_t launch_compose(const s3r_image_part* parts, const s3r_image_part* parts_dev, uint32_t nparts,
+                           int32_t just_copy_first, uint32_t* dst, int32_t dw, int32_t dh, int32_t offx, int32_t offy,
+                           cudaStream_t s);
 
 // Render CTA pixel shapes the autotuner chooses from: {x, y} pixels.  A render
 // tile id below kRenderWalkTiles is a per-ray walk (frame_render_kernel), shape +
