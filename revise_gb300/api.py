@@ -20,20 +20,34 @@ from . import _lib, host
 from ._lib import FrameDesc, ImagePart, PlanInfo, View, WorkerBlocks, arr, check, ptr
 
 
+_torch_module = None
+
+
 def _torch():
-    import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("revise_gb300 needs a CUDA device (no CPU fallback)")
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        if not torch.cuda.is_available():
+            raise RuntimeError("revise_gb300 needs a CUDA device (no CPU fallback)")
+        torch.cuda.init()
+        _torch_module = torch
+    return _torch_module
 
 
 def _stream(stream):
-    torch = _torch()
+    """A stream argument as the address the C calls take (None: torch's current stream, its raw handle -- building a
+    torch.cuda.Stream object for it took as long as a small kernel)."""
     if stream is None:
-        return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        c = _torch()._C
+        return C.c_void_p(c._cuda_getCurrentRawStream(c._cuda_getDevice()))
     if hasattr(stream, "cuda_stream"):
         return C.c_void_p(stream.cuda_stream)
     return C.c_void_p(int(stream))
+
+
+def _never() -> bool:
+    """The default `cancelled` callback: a render that nothing can cancel."""
+    return False
 
 
 class _CudaArray:
@@ -397,7 +411,7 @@ class DenseFieldRenderer:
         s = self.state
         self.ctx.clear_viewport(viewport, s.view.W, s.view.H, 0)
 
-    def render_dense_field(self, viewport, level: int, index, cancelled=lambda: False):
+    def render_dense_field(self, viewport, level: int, index, cancelled=_never):
         torch = _torch()
         s = self.state
         b = s.block_index[(int(index[0]), int(index[1]), int(index[2]))]
@@ -479,7 +493,7 @@ class VsWorker:
     def update_state(self, flags: int = ~0):
         pass
 
-    def render_scene_part(self, level: int, index_box_min, index_box_max, cancelled=lambda: False):
+    def render_scene_part(self, level: int, index_box_min, index_box_max, cancelled=_never):
         part = self.render_scene_part_device(level, index_box_min, index_box_max, cancelled)
         if part is None:
             return None
@@ -544,9 +558,12 @@ class VsWorker:
         self.ctx.crop(self.viewport, W, list(rect), crop)
         return (int(rect[0]), int(rect[1])), (int(rect[2]), int(rect[3])), crop
 
-    def render_scene_part_device(self, level: int, index_box_min, index_box_max, cancelled=lambda: False):
+    def render_scene_part_device(self, level: int, index_box_min, index_box_max, cancelled=_never):
         """renderScenePart with the cropped part left in device memory: (origin, size, int32 tensor),
-        size (0, 0) when nothing was drawn; None when cancelled."""
+        size (0, 0) when nothing was drawn; None when cancelled.  A render that nothing can cancel is one native
+        call; `cancelled` is asked between blocks, so with it they go one by one."""
+        if cancelled is _never:
+            return self.render_scene_part_native(level, index_box_min, index_box_max)
         torch = _torch()
         s = self.state
         W, H = s.view.W, s.view.H

@@ -214,6 +214,10 @@ int clampi(int x, int lo, int hi) { return x < lo ? lo : (x > hi ? hi : x); }
 
 // DenseFieldRenderer_cu.cu:374-409: bounding box of the projected cube corners,
 // truncated toward zero, clamped to the viewport; {x, y, w, h} with w = max - min.
+// Every block of a level goes through this whenever the camera moves, so the 8
+// corners are worked out side by side (arrays the compiler vectorizes) from the
+// products of the 2 coordinates they have per axis; each corner's sums and
+// quotients are rounded as the one-by-one form rounds them.
 void view_rect(const s3r_view& v, const uint32_t idx[3], int32_t rect[4])
 {
     float c[3], h;
@@ -222,43 +226,44 @@ void view_rect(const s3r_view& v, const uint32_t idx[3], int32_t rect[4])
     const float pixel = v.cam.h / (float)v.H;
     const float* r = v.cam.view_r;
     const float* t = v.cam.view_t;
-    bool have = false, full = false;
-    int xmin = 0, xmax = 0, ymin = 0, ymax = 0;
-    for (int i = 0; i < 8; ++i) {
-        float p[3];
-        for (int d = 0; d < 3; ++d)
-            p[d] = c[d] + (float)((int)(((i >> d) & 1) << 1) - 1) * h;
-        float q[3];
-        for (int a = 0; a < 3; ++a)
-            q[a] = r[3 * a] * p[0] + r[3 * a + 1] * p[1] + r[3 * a + 2] * p[2] + t[a];
-        int sx, sy;
-        if (v.cam.ortho) {
-            sx = clampi((int)(q[0] / pixel) + (int)(v.W >> 1), 0, (int)v.W - 1);
-            sy = clampi((int)(q[1] / pixel) + (int)(v.H >> 1), 0, (int)v.H - 1);
-        } else {
-            if (q[2] >= 0) {
-                full = true;
-                break;
-            }
-            sx = clampi((int)(-q[0] / q[2] * lcam / pixel) + (int)(v.W >> 1), 0, (int)v.W - 1);
-            sy = clampi((int)(-q[1] / q[2] * lcam / pixel) + (int)(v.H >> 1), 0, (int)v.H - 1);
+    float q[3][8];
+    for (int a = 0; a < 3; ++a) {
+        float prod[3][2];
+        for (int d = 0; d < 3; ++d) {
+            prod[d][0] = r[3 * a + d] * (c[d] - h);
+            prod[d][1] = r[3 * a + d] * (c[d] + h);
         }
-        if (!have) {
-            xmin = xmax = sx;
-            ymin = ymax = sy;
-            have = true;
-        } else {
-            xmin = std::min(xmin, sx);
-            xmax = std::max(xmax, sx);
-            ymin = std::min(ymin, sy);
-            ymax = std::max(ymax, sy);
+        for (int i = 0; i < 8; ++i) q[a][i] = prod[0][i & 1] + prod[1][(i >> 1) & 1] + prod[2][i >> 2] + t[a];
+    }
+    float fx[8], fy[8];
+    bool full = false;
+    if (v.cam.ortho) {
+        for (int i = 0; i < 8; ++i) {
+            fx[i] = q[0][i] / pixel;
+            fy[i] = q[1][i] / pixel;
+        }
+    } else {
+        for (int i = 0; i < 8; ++i) full |= q[2][i] >= 0;
+        for (int i = 0; i < 8 && !full; ++i) {
+            fx[i] = -q[0][i] / q[2][i] * lcam / pixel;
+            fy[i] = -q[1][i] / q[2][i] * lcam / pixel;
         }
     }
     if (full) {
         // a corner behind the eye: the whole viewport (bb << {0,0} << viewportSize)
-        xmin = ymin = 0;
-        xmax = (int)v.W;
-        ymax = (int)v.H;
+        rect[0] = rect[1] = 0;
+        rect[2] = (int)v.W;
+        rect[3] = (int)v.H;
+        return;
+    }
+    int xmin = INT32_MAX, xmax = INT32_MIN, ymin = INT32_MAX, ymax = INT32_MIN;
+    for (int i = 0; i < 8; ++i) {
+        const int sx = clampi((int)fx[i] + (int)(v.W >> 1), 0, (int)v.W - 1);
+        const int sy = clampi((int)fy[i] + (int)(v.H >> 1), 0, (int)v.H - 1);
+        xmin = std::min(xmin, sx);
+        xmax = std::max(xmax, sx);
+        ymin = std::min(ymin, sy);
+        ymax = std::max(ymax, sy);
     }
     rect[0] = xmin;
     rect[1] = ymin;
@@ -2343,9 +2348,6 @@ int part_blend(s3r_ctx* ctx, const s3r_view* view, const s3r_presentation* pres,
         y1 = std::max(y1, r[1] + r[3]);
         refs[i].order = i;
     }
-    // the deepest blocks' rays take the most samples: their CTAs start first
-    std::stable_sort(refs.begin(), refs.end(),
-                     [](const PartRef& a, const PartRef& b) { return a.rb.depth > b.rb.depth; });
     PartArgs a{};
     a.nblocks = n;
     a.cap = std::min(n, span + 1);
@@ -2373,7 +2375,12 @@ int part_blend(s3r_ctx* ctx, const s3r_view* view, const s3r_presentation* pres,
     char *host, *dev;
     const size_t refs_bytes = n * sizeof(PartRef), first_bytes = (n + 1) * sizeof(uint32_t);
     if (int rc = part_table(ctx, refs_bytes + strips * first_bytes, s, &host, &dev)) return rc;
-    std::memcpy(host, refs.data(), refs_bytes);
+    // the deepest blocks' rays take the most samples: their CTAs start first
+    PartRef* sorted = reinterpret_cast<PartRef*>(host);
+    uint32_t put = 0;
+    for (int d = S3R_MAX_DEPTH; d >= 0; --d)
+        for (uint32_t i = 0; i < n; ++i)
+            if (refs[i].rb.depth == (uint32_t)d) sorted[put++] = refs[i];
     uint32_t tw, th;
     part_tile(pres->mode, texture, tw, th);
     for (uint32_t k = 0; k < strips; ++k) {
@@ -2381,7 +2388,7 @@ int part_blend(s3r_ctx* ctx, const s3r_view* view, const s3r_presentation* pres,
         const int32_t s0 = y0 + (int32_t)k * rows, s1 = std::min(s0 + rows, y1);
         uint64_t at = 0;
         for (uint32_t i = 0; i < n; ++i) {
-            const int32_t* r = refs[i].rb.rect;
+            const int32_t* r = sorted[i].rb.rect;
             const int32_t h = std::min(r[1] + r[3], s1) - std::max(r[1], s0);
             first[i] = (uint32_t)at;
             if (h > 0) at += (uint64_t)(((uint32_t)r[2] + tw - 1) / tw) * (((uint32_t)h + th - 1) / th);
@@ -2594,20 +2601,38 @@ int s3r_render_scene_part(s3r_ctx* ctx, const s3r_view* view, const s3r_presenta
         if (!ctx->worker_tf && (rc = s3r_tf_texture_create(ctx, view->tf_n, &ctx->worker_tf))) return rc;
         if ((rc = s3r_tf_texture_set(ctx, ctx->worker_tf, tf, stream))) return rc;
     }
+    // the set's blocks by their place in the box
+    const uint64_t ex = box_max[0] > box_min[0] ? box_max[0] - box_min[0] : 0,
+                   ey = box_max[1] > box_min[1] ? box_max[1] - box_min[1] : 0,
+                   ez = box_max[2] > box_min[2] ? box_max[2] - box_min[2] : 0;
+    const bool flat = ex * ey * ez <= (1u << 18);
+    std::vector<int32_t> place(flat ? ex * ey * ez : 0, -1);
     std::unordered_map<uint64_t, uint32_t> where;
-    where.reserve(wb->nblocks * 2 + 1);
+    if (!flat) where.reserve(wb->nblocks * 2 + 1);
     for (uint32_t b = 0; b < wb->nblocks; ++b) {
         const uint32_t* bl = wb->blocks + 4 * b;
-        where[(uint64_t)bl[0] | ((uint64_t)bl[1] << 21) | ((uint64_t)bl[2] << 42)] = b;
+        if (!flat) {
+            where[(uint64_t)bl[0] | ((uint64_t)bl[1] << 21) | ((uint64_t)bl[2] << 42)] = b;
+        } else {
+            const uint64_t x = (uint64_t)bl[0] - box_min[0], y = (uint64_t)bl[1] - box_min[1],
+                           z = (uint64_t)bl[2] - box_min[2];
+            if (x < ex && y < ey && z < ez) place[x + ex * (y + ey * z)] = (int32_t)b;
+        }
     }
     // the blocks that can show, back to front
     std::vector<PartBlock> list;
     b2f_traverse(sp, [&](const uint32_t q[3]) {
         if (rc) return;
-        auto it = where.find((uint64_t)q[0] | ((uint64_t)q[1] << 21) | ((uint64_t)q[2] << 42));
-        if (it == where.end()) return; // not a block of this set
         PartBlock p;
-        p.b = it->second;
+        if (flat) {
+            const int32_t b = place[(q[0] - box_min[0]) + ex * ((q[1] - box_min[1]) + ey * (uint64_t)(q[2] - box_min[2]))];
+            if (b < 0) return; // not a block of this set
+            p.b = (uint32_t)b;
+        } else {
+            auto it = where.find((uint64_t)q[0] | ((uint64_t)q[1] << 21) | ((uint64_t)q[2] << 42));
+            if (it == where.end()) return;
+            p.b = it->second;
+        }
         if (wb->blocks[4 * p.b + 3] > S3R_MAX_DEPTH) {
             rc = fail(ctx, S3R_ERR_INVALID, "depth exceeds S3R_MAX_DEPTH");
             return;

@@ -258,7 +258,9 @@ class VsRenderer:
         self.last_parts = {}
 
     def continue_rendering(self, eye, min_level: int = 0, level_count: int | None = None, render_level: int = -1,
-                           cancelled=lambda: False):
+                           cancelled=None):
+        from .api import _never
+        cancelled = cancelled or _never
         levels = sorted(self.states)
         level_count = (max(levels) + 1) if level_count is None else level_count
         if render_level >= 0:
