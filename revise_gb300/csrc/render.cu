@@ -1101,75 +1101,99 @@ __global__ void __launch_bounds__(kCompositeThreads) part_composite_kernel(const
 
 // ---------------------------------------------------------------- batched form
 
-// Front-to-back walk of the (2^level)^3 block grid along one ray
-// (Amanatides-Woo); calls f(block_index, ix, iy, iz) for every block the ray
-// passes, in order; f returns false to stop.
+// Front-to-back walk of the (2^level)^3 block grid along one ray (Amanatides-Woo).
+struct BlockWalk {
+    int m;
+    int c0, c1, c2, s0, s1, s2;
+    float tx0, tx1, tx2, td0, td1, td2, t1;
+
+    // The ray's first block; false when it misses the grid.
+    __device__ __forceinline__ bool begin(const float org[3], const float dir[3], const float inv[3], uint32_t level)
+    {
+        m = 1 << level;
+        const float cell = (2.f * kTopHalf) / (float)m;
+        // entry/exit of the whole cube [-5, 5]^3, restricted to tau >= 1 (the screen plane)
+        float t0 = 1.f;
+        t1 = 3.4e38f;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            if (fabsf(dir[a]) > 1e-10f) {
+                float ta = (-kTopHalf - org[a]) * inv[a], tb = (kTopHalf - org[a]) * inv[a];
+                if (ta > tb) { const float t = ta; ta = tb; tb = t; }
+                t0 = fmaxf(t0, ta);
+                t1 = fminf(t1, tb);
+            } else if (org[a] < -kTopHalf || org[a] > kTopHalf) {
+                return false;
+            }
+        }
+        if (!(t1 > t0)) return false;
+        // start cell: the one holding the entry point itself (clamped onto the grid);
+        // starting any distance inside would skip the first block's segment on rays
+        // that enter close to a block boundary
+        const float tm = t0;
+        // start cell, step direction, next boundary crossing and crossing period per axis
+        auto setup = [&](int a, int& c, int& st, float& tmax, float& tdel) {
+            const float pm = __fmaf_rn(dir[a], tm, org[a]);
+            c = min(max((int)floorf((pm + kTopHalf) / cell), 0), m - 1);
+            if (dir[a] > 1e-10f) {
+                st = 1;
+                tmax = div_by((-kTopHalf + cell * (float)(c + 1)) - org[a], dir[a], inv[a]);
+                tdel = div_by(cell, dir[a], inv[a]);
+            } else if (dir[a] < -1e-10f) {
+                st = -1;
+                tmax = div_by((-kTopHalf + cell * (float)c) - org[a], dir[a], inv[a]);
+                tdel = div_by(-cell, dir[a], inv[a]);
+            } else {
+                st = 0;
+                tmax = 3.4e38f;
+                tdel = 3.4e38f;
+            }
+        };
+        setup(0, c0, s0, tx0, td0);
+        setup(1, c1, s1, tx1, td1);
+        setup(2, c2, s2, tx2, td2);
+        return true;
+    }
+
+    __device__ __forceinline__ uint32_t cell() const
+    {
+        return (uint32_t)c0 + (uint32_t)m * ((uint32_t)c1 + (uint32_t)m * (uint32_t)c2);
+    }
+
+    // On to the next block of the ray; false when it has left the grid.  (Every step moves one index towards
+    // its end of the grid, an axis the ray does not move along never being chosen before the exit, so a walk
+    // visits at most 3 m - 2 blocks.)
+    __device__ __forceinline__ bool next()
+    {
+        if (tx0 <= tx1 && tx0 <= tx2) {
+            if (tx0 >= t1) return false;
+            c0 += s0;
+            tx0 += td0;
+            return c0 >= 0 && c0 < m;
+        }
+        if (tx1 <= tx2) {
+            if (tx1 >= t1) return false;
+            c1 += s1;
+            tx1 += td1;
+            return c1 >= 0 && c1 < m;
+        }
+        if (tx2 >= t1) return false;
+        c2 += s2;
+        tx2 += td2;
+        return c2 >= 0 && c2 < m;
+    }
+};
+
+// Calls f(block cell) for every block one ray passes, front to back; f returns false to stop.
 template <class F>
 __device__ __forceinline__ void walk_blocks(const float org[3], const float dir[3], const float inv[3],
                                             uint32_t level, F&& f)
 {
-    const int m = 1 << level;
-    const float cell = (2.f * kTopHalf) / (float)m;
-    // entry/exit of the whole cube [-5, 5]^3, restricted to tau >= 1 (the screen plane)
-    float t0 = 1.f, t1 = 3.4e38f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (fabsf(dir[a]) > 1e-10f) {
-            float ta = (-kTopHalf - org[a]) * inv[a], tb = (kTopHalf - org[a]) * inv[a];
-            if (ta > tb) { const float t = ta; ta = tb; tb = t; }
-            t0 = fmaxf(t0, ta);
-            t1 = fminf(t1, tb);
-        } else if (org[a] < -kTopHalf || org[a] > kTopHalf) {
-            return;
-        }
-    }
-    if (!(t1 > t0)) return;
-    // start cell: the one holding the entry point itself (clamped onto the grid);
-    // starting any distance inside would skip the first block's segment on rays
-    // that enter close to a block boundary
-    const float tm = t0;
-    // start cell, step direction, next boundary crossing and crossing period per axis
-    int c0, c1, c2, s0, s1, s2;
-    float tx0, tx1, tx2, td0, td1, td2;
-    auto setup = [&](int a, int& c, int& st, float& tmax, float& tdel) {
-        const float pm = __fmaf_rn(dir[a], tm, org[a]);
-        c = min(max((int)floorf((pm + kTopHalf) / cell), 0), m - 1);
-        if (dir[a] > 1e-10f) {
-            st = 1;
-            tmax = div_by((-kTopHalf + cell * (float)(c + 1)) - org[a], dir[a], inv[a]);
-            tdel = div_by(cell, dir[a], inv[a]);
-        } else if (dir[a] < -1e-10f) {
-            st = -1;
-            tmax = div_by((-kTopHalf + cell * (float)c) - org[a], dir[a], inv[a]);
-            tdel = div_by(-cell, dir[a], inv[a]);
-        } else {
-            st = 0;
-            tmax = 3.4e38f;
-            tdel = 3.4e38f;
-        }
-    };
-    setup(0, c0, s0, tx0, td0);
-    setup(1, c1, s1, tx1, td1);
-    setup(2, c2, s2, tx2, td2);
-    for (int guard = 0; guard < 3 * m + 3; ++guard) {
-        const uint32_t b = (uint32_t)c0 + (uint32_t)m * ((uint32_t)c1 + (uint32_t)m * (uint32_t)c2);
-        if (!f(b, (uint32_t)c0, (uint32_t)c1, (uint32_t)c2)) return;
-        if (tx0 <= tx1 && tx0 <= tx2) {
-            if (tx0 >= t1) return;
-            c0 += s0;
-            if (c0 < 0 || c0 >= m) return;
-            tx0 += td0;
-        } else if (tx1 <= tx2) {
-            if (tx1 >= t1) return;
-            c1 += s1;
-            if (c1 < 0 || c1 >= m) return;
-            tx1 += td1;
-        } else {
-            if (tx2 >= t1) return;
-            c2 += s2;
-            if (c2 < 0 || c2 >= m) return;
-            tx2 += td2;
-        }
+    BlockWalk w;
+    if (!w.begin(org, dir, inv, level)) return;
+    for (int guard = 0; guard < 3 * w.m + 3; ++guard) {
+        if (!f(w.cell())) return;
+        if (!w.next()) return;
     }
 }
 
@@ -1343,7 +1367,7 @@ __global__ void frame_render_kernel(FrameArgs fa)
         int lo = 0, hi = 1 << 30;
         if (R > 1) {
             int n = 0;
-            walk_blocks(org, dir, inv, v.level, [&](uint32_t, uint32_t, uint32_t, uint32_t) {
+            walk_blocks(org, dir, inv, v.level, [&](uint32_t) {
                 ++n;
                 return true;
             });
@@ -1352,7 +1376,7 @@ __global__ void frame_render_kernel(FrameArgs fa)
             hi = lo + chunk;
         }
         int idx = 0;
-        walk_blocks(org, dir, inv, v.level, [&](uint32_t b, uint32_t, uint32_t, uint32_t) {
+        walk_blocks(org, dir, inv, v.level, [&](uint32_t b) {
             if (idx >= hi) return false;
             if (idx++ < lo) return true;
             const RenderBlock* rb = &fa.table[b];
@@ -1598,7 +1622,7 @@ __global__ void frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr
         float inv[3];
         ray_inverse(dir, inv);
         const float* bricks = reinterpret_cast<const float*>(fa.bricks);
-        walk_blocks(org, dir, inv, v.level, [&](uint32_t b, uint32_t, uint32_t, uint32_t) {
+        walk_blocks(org, dir, inv, v.level, [&](uint32_t b) {
             const RenderBlock* rb = &fa.table[b];
             const uint32_t depth = rb->depth;
             if (depth == 0xffffffffu) return true;
@@ -1638,57 +1662,176 @@ __global__ void frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr
 
 // ---------------------------------------------------------------- adjoint
 
-// The 8 texels of a cell (F32 brick, 32-bit offsets), their offsets, and the trilinear value (false on a NaN).
-__device__ __forceinline__ void cell_offsets(const Cell& c, Dim g, uint32_t off[8])
+__device__ __forceinline__ bool filter_cell(const float f[3], const float t[8], float& val)
+{
+    if (any_nan(t)) return false;
+    const float x00 = __fmaf_rn(f[0], t[1] - t[0], t[0]);
+    const float x10 = __fmaf_rn(f[0], t[3] - t[2], t[2]);
+    const float x01 = __fmaf_rn(f[0], t[5] - t[4], t[4]);
+    const float x11 = __fmaf_rn(f[0], t[7] - t[6], t[6]);
+    const float y0 = __fmaf_rn(f[1], x10 - x00, x00);
+    const float y1 = __fmaf_rn(f[1], x11 - x01, x01);
+    val = __fmaf_rn(f[2], y1 - y0, y0);
+    return true;
+}
+
+// A sample's cell in an F32 brick: its low corner (before clamping) and fractions, and its 8 texels.
+struct GradCell {
+    int a[3];
+    float f[3];
+    float t[8];
+};
+
+__device__ __forceinline__ bool inside_brick(const int a[3], uint32_t hi)
+{
+    return (uint32_t)a[0] < hi && (uint32_t)a[1] < hi && (uint32_t)a[2] < hi;
+}
+
+// Offset of corner q (x | y << 1 | z << 2) of a cell that reaches over the brick's edge, by the clamped indices.
+__device__ __forceinline__ uint32_t clamped_corner(const int a[3], Dim g, int q)
+{
+    const int hi = (int)g.n - 1;
+    const int x = min(max(a[0] + (q & 1), 0), hi), y = min(max(a[1] + ((q >> 1) & 1), 0), hi),
+              z = min(max(a[2] + (q >> 2), 0), hi);
+    return ((uint32_t)z * g.n + (uint32_t)y) * g.pitch + (uint32_t)x;
+}
+
+__device__ __forceinline__ void fetch_grad_cell(const float* brick, const BlockRay& r, float kf, GradCell& c)
 {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const uint32_t x = (q & 1) ? c.i1[0] : c.i0[0];
-        const uint32_t y = (q & 2) ? c.i1[1] : c.i0[1];
-        const uint32_t z = (q & 4) ? c.i1[2] : c.i0[2];
-        off[q] = (z * g.n + y) * g.pitch + x;
+    for (int d = 0; d < 3; ++d) {
+        const float p = __fmaf_rn(r.step[d], kf, r.p0[d]);
+        const float tc = __fmul_rn(__fsub_rn(p, r.origin[d]), r.factor);
+        const float xb = __fsub_rn(tc, 0.5f);
+        c.f[d] = __fsub_rn(xb, floor_small(xb, c.a[d]));
+    }
+    if (inside_brick(c.a, r.n - 1)) {
+        const uint32_t o = ((uint32_t)c.a[2] * r.n + (uint32_t)c.a[1]) * r.pitch + (uint32_t)c.a[0];
+        const uint32_t dz = r.n * r.pitch;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            c.t[q] = __ldg(brick + (uint64_t)(o + ((q & 2) ? r.pitch : 0u) + ((q & 4) ? dz : 0u)) + (q & 1));
+    } else {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) c.t[q] = __ldg(brick + clamped_corner(c.a, dim_of(r), q));
     }
 }
 
-__device__ __forceinline__ void fetch_cell(const float* brick, const Cell& c, Dim g, float t[8])
-{
-    uint32_t off[8];
-    cell_offsets(c, g, off);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) t[q] = __ldg(brick + off[q]);
-}
+// The dense-value gradients of a ray's current cell, kept in registers while the ray moves from cell to cell: a step
+// of one along an axis hands the shared face's four sums on and only the face left behind goes to memory, so that a
+// sample costs four to seven reductions instead of eight.  A ray moves one way along each axis, so corners are counted
+// along the ray: bit a of q is 0 for the face it entered by, and stride[a] leads from that face to the other one.
+struct CellGradient {
+    float g[8];
+    int a[3];       // the cell's low corner
+    float* p;       // corner 0
+    int stride[3];
+    bool have;
 
-__device__ __forceinline__ bool filter_cell(const Cell& c, const float t[8], float& val)
-{
-    bool bad = false;
+    __device__ __forceinline__ void begin(const float step[3], int pitch, int dz)
+    {
+        have = false;
+        stride[0] = step[0] < 0.f ? -1 : 1;
+        stride[1] = step[1] < 0.f ? -pitch : pitch;
+        stride[2] = step[2] < 0.f ? -dz : dz;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) bad |= isnan(t[q]);
-    if (bad) return false;
-    const float x00 = __fmaf_rn(c.f[0], t[1] - t[0], t[0]);
-    const float x10 = __fmaf_rn(c.f[0], t[3] - t[2], t[2]);
-    const float x01 = __fmaf_rn(c.f[0], t[5] - t[4], t[4]);
-    const float x11 = __fmaf_rn(c.f[0], t[7] - t[6], t[6]);
-    const float y0 = __fmaf_rn(c.f[1], x10 - x00, x00);
-    const float y1 = __fmaf_rn(c.f[1], x11 - x01, x01);
-    val = __fmaf_rn(c.f[2], y1 - y0, y0);
-    return true;
-}
+        for (int q = 0; q < 8; ++q) g[q] = 0.f;
+    }
+    __device__ __forceinline__ float* corner(int q) const
+    {
+        return p + (((q & 1) ? stride[0] : 0) + ((q & 2) ? stride[1] : 0) + ((q & 4) ? stride[2] : 0));
+    }
+    __device__ __forceinline__ void put(int q) const
+    {
+        if (g[q] != 0.f) atomicAdd(corner(q), g[q]);
+    }
+    __device__ __forceinline__ void flush()
+    {
+        if (!have) return;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            put(q);
+            g[q] = 0.f;
+        }
+        have = false;
+    }
+    template <int B> __device__ __forceinline__ void step(int axis)
+    {
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (!(q & B)) {
+                put(q);
+                g[q] = g[q | B];
+                g[q | B] = 0.f;
+            }
+        p += stride[axis];
+    }
+    // The ray is now in the (inside) cell `to` of the brick whose gradients start at `dense`.
+    __device__ __forceinline__ void move(const int to[3], float* dense, uint32_t n, uint32_t pitch)
+    {
+        // steps along the ray: 0 or 1 per axis, or the cell is left altogether
+        const int dx = stride[0] < 0 ? a[0] - to[0] : to[0] - a[0], dy = stride[1] < 0 ? a[1] - to[1] : to[1] - a[1],
+                  dz = stride[2] < 0 ? a[2] - to[2] : to[2] - a[2];
+        if (have && (uint32_t)(dx | dy | dz) <= 1u) {
+            if (dx) step<1>(0);
+            if (dy) step<2>(1);
+            if (dz) step<4>(2);
+        } else {
+            flush();
+            p = dense + (((uint32_t)to[2] * n + (uint32_t)to[1]) * pitch + (uint32_t)to[0]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                if (stride[d] < 0) p -= stride[d];
+            have = true;
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) a[d] = to[d];
+    }
+    // Adds the sample's gradient by its trilinear weights.
+    __device__ __forceinline__ void add(float v, const float f[3])
+    {
+        float w[3][2];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            w[d][1] = stride[d] < 0 ? 1.f - f[d] : f[d];
+            w[d][0] = stride[d] < 0 ? f[d] : 1.f - f[d];
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) g[q] = __fmaf_rn(v, w[0][q & 1] * w[1][(q >> 1) & 1] * w[2][q >> 2], g[q]);
+    }
+};
 
 // For L = 1/2 sum (I - target)^2 with I = (C/A, A) the premultiplied composite
 // of the kept samples (front to back, T_k = prod_{j<k} (1 - a_k)):
 //   dC/dc_k = T_k a_k,  dC/da_k = T_k c_k - (C - C_{<=k}) / (1 - a_k),
 //   dA/da_k = (1 - A) / (1 - a_k),
 // a_k = 1 - (1 - alpha_tf * of)^il, c_k / alpha_tf linear in the table
-// entries around v01, v01 linear in the trilinear value.
-__global__ void __launch_bounds__(128, 4) frame_backward_kernel(FrameArgs fa)
+// entries around v01, v01 linear in the trilinear value.  With s_k = gC . c_k
+// the gradient of a_k is T_k s_k + Q_k / (1 - a_k), Q_k = gA (1 - A) - gC . (C -
+// C_{<=k}), and Q grows by T_k a_k s_k from one sample to the next: one number a
+// ray where the composite has three.
+//
+// What bounds it: the reductions into the dense gradient (about a third of the
+// time) and the latency of a ray's chain of samples, at the warps that the
+// registers leave room for; the ray, its walk and what only a new block needs are
+// kept in shared memory.
+constexpr uint32_t kBackwardThreads = 64;
+struct BackwardShared {
+    BlockWalk walk[kBackwardThreads];
+    float ray[9][kBackwardThreads]; // origin, direction, 1 / direction
+};
+
+__global__ void __launch_bounds__(kBackwardThreads, 8) frame_backward_kernel(FrameArgs fa)
 {
     extern __shared__ float4 sm[];
-    const s3r_view v = *fa.view;
-    float4* tf = sm;
-    const uint32_t nthreads = blockDim.x * blockDim.y;
+    __shared__ BackwardShared sh;
+    __shared__ s3r_view view_sm;
     const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x;
-    for (uint32_t i = tid; i < v.tf_n; i += nthreads) tf[i] = reinterpret_cast<const float4*>(fa.tf)[i];
+    for (uint32_t i = tid; i < sizeof(s3r_view) / 4; i += kBackwardThreads)
+        reinterpret_cast<uint32_t*>(&view_sm)[i] = reinterpret_cast<const uint32_t*>(fa.view)[i];
     __syncthreads();
+    const s3r_view& v = view_sm;
+    const TfTable tf = load_tf(sm, fa.tf, v.tf_n, tid, kBackwardThreads);
     // The transfer-function gradient goes to one of kDtfParts copies in global
     // memory, an RGBA float4 reduction per table entry (fire and forget).  The copy
     // is picked by CTA (modulo kDtfCtaGroups) and by lane (modulo kDtfLaneGroups):
@@ -1700,14 +1843,15 @@ __global__ void __launch_bounds__(128, 4) frame_backward_kernel(FrameArgs fa)
                             (tid & 31) % kDtfLaneGroups) * v.tf_n;
     const uint32_t vx = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t vy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (vx < v.W && vy < v.H) {
+    if (vx >= v.W || vy >= v.H) return;
+    float gC[3] = {0.f, 0.f, 0.f};
+    float Q;
+    {
         const size_t o = (size_t)(v.H - 1 - vy) * v.W + vx;
         const float4 I = reinterpret_cast<const float4*>(fa.fwd_rgba)[o];
         const float4 gI = reinterpret_cast<const float4*>(fa.dl_drgba)[o];
         const float A = I.w;
-        float gC[3] = {0.f, 0.f, 0.f};
         float gA = gI.w;
-        const float Ct[3] = {I.x * A, I.y * A, I.z * A};
         if (A > 0.f) {
             const float inv = 1.f / A;
             gC[0] = gI.x * inv;
@@ -1715,162 +1859,174 @@ __global__ void __launch_bounds__(128, 4) frame_backward_kernel(FrameArgs fa)
             gC[2] = gI.z * inv;
             gA -= (gI.x * I.x + gI.y * I.y + gI.z * I.z) * inv;
         }
-        const bool active = (gC[0] != 0.f || gC[1] != 0.f || gC[2] != 0.f || gA != 0.f);
-        if (active) {
-            float org[3], dir[3];
-            pixel_ray(v, vx, vy, org, dir);
-        float inv[3];
+        if (gC[0] == 0.f && gC[1] == 0.f && gC[2] == 0.f && gA == 0.f) return;
+        Q = gA * (1.f - A) - (gC[0] * (I.x * A) + gC[1] * (I.y * A) + gC[2] * (I.z * A));
+    }
+    {
+        float org[3], dir[3], inv[3];
+        pixel_ray(v, vx, vy, org, dir);
         ray_inverse(dir, inv);
-            const float span = v.field_max - v.field_min;
-            const float inv_span = 1.f / span;
-            const float of = (v.threshold - v.field_min) / span;
-            float T = 1.f, Cpre[3] = {0.f, 0.f, 0.f};
-            float accA = 0.f;
-            uint32_t tf_i0 = 0xffffffffu, tf_i1 = 0xffffffffu;
-            float tf_a[4] = {0.f, 0.f, 0.f, 0.f}, tf_b[4] = {0.f, 0.f, 0.f, 0.f};
-            auto flush_tf = [&]() {
-                if (tf_i0 == 0xffffffffu) return;
-                atomicAdd(&dtf4[tf_i0], make_float4(tf_a[0], tf_a[1], tf_a[2], tf_a[3]));
-                atomicAdd(&dtf4[tf_i1], make_float4(tf_b[0], tf_b[1], tf_b[2], tf_b[3]));
 #pragma unroll
-                for (int ch = 0; ch < 4; ++ch) {
-                    tf_a[ch] = 0.f;
-                    tf_b[ch] = 0.f;
+        for (int d = 0; d < 3; ++d) {
+            sh.ray[d][tid] = org[d];
+            sh.ray[3 + d][tid] = dir[d];
+            sh.ray[6 + d][tid] = inv[d];
+        }
+        BlockWalk w;
+        if (!w.begin(org, dir, inv, v.level)) return;
+        sh.walk[tid] = w;
+    }
+    const float inv_span = 1.f / (v.field_max - v.field_min);
+    const float of = (v.threshold - v.field_min) / (v.field_max - v.field_min);
+    float T = 1.f, accA = 0.f;
+    int tf_j = -2; // the table interval of the two sums: entries max(j, 0) and min(j + 1, tf_n - 1); -2: none yet
+    float tf_a[4] = {0.f, 0.f, 0.f, 0.f}, tf_b[4] = {0.f, 0.f, 0.f, 0.f};
+    auto put_a = [&]() { atomicAdd(&dtf4[max(tf_j, 0)], make_float4(tf_a[0], tf_a[1], tf_a[2], tf_a[3])); };
+    auto put_b = [&]() {
+        atomicAdd(&dtf4[min(tf_j + 1, (int)v.tf_n - 1)], make_float4(tf_b[0], tf_b[1], tf_b[2], tf_b[3]));
+    };
+    while (true) {
+        asm volatile("" ::: "memory"); // the walk is read back from shared memory, not kept in registers
+        const RenderBlock* rb = &fa.table[sh.walk[tid].cell()];
+        const uint32_t depth = rb->depth;
+        const int4 rc = *reinterpret_cast<const int4*>(rb->rect);
+        const int32_t rca[4] = {rc.x, rc.y, rc.z, rc.w};
+        BlockRay r;
+        bool hit = depth != 0xffffffffu && pixel_in_rect(rca, vx, vy);
+        if (hit) {
+            const float org[3] = {sh.ray[0][tid], sh.ray[1][tid], sh.ray[2][tid]};
+            const float dir[3] = {sh.ray[3][tid], sh.ray[4][tid], sh.ray[5][tid]};
+            const float inv[3] = {sh.ray[6][tid], sh.ray[7][tid], sh.ray[8][tid]};
+            hit = block_ray(v, org, dir, inv, *rb, r);
+        }
+        if (hit) {
+            const float* brick = reinterpret_cast<const float*>(fa.bricks) + rb->brick_off;
+            float* gdense = fa.ddense + rb->brick_off;
+            const float il = layer_exponent(depth, v.level, v.quality);
+            float Ab = 0.f;
+            CellGradient cg;
+            cg.begin(r.step, (int)r.pitch, (int)(r.n * r.pitch));
+            // one sample's gradients from its cell; false once the block is opaque
+            auto step_sample = [&](const GradCell& cell) -> bool {
+                float val;
+                if (!filter_cell(cell.f, cell.t, val)) return true;
+                // the forward's v01 up to the last ulp (a reciprocal instead of the division), and its colour
+                const float u = __fmaf_rn(__fmul_rn(__fsub_rn(val, v.field_min), inv_span), (float)v.tf_n, -0.5f);
+                int j;
+                const float f = u - floor_small(fminf(fmaxf(u, -1.f), (float)v.tf_n - 0.5f), j);
+                const float4 p = tf.p[j + 1];
+                float4 d;
+                if (tf.d) {
+                    d = tf.d[j + 1];
+                } else {
+                    const float4 q = tf.p[j + 2];
+                    d = make_float4(q.x - p.x, q.y - p.y, q.z - p.z, q.w - p.w);
                 }
-            };
-            walk_blocks(org, dir, inv, v.level, [&](uint32_t b, uint32_t ix, uint32_t iy, uint32_t iz) {
-                const RenderBlock* rb = &fa.table[b];
-                const uint32_t depth = rb->depth;
-                if (depth == 0xffffffffu) return true;
-                const int4 rc = *reinterpret_cast<const int4*>(rb->rect);
-                const int32_t rca[4] = {rc.x, rc.y, rc.z, rc.w};
-                if (!pixel_in_rect(rca, vx, vy)) return true;
-                BlockRay r;
-                if (!block_ray(v, org, dir, inv, *rb, r)) return true;
-                const float* brick = reinterpret_cast<const float*>(fa.bricks) + rb->brick_off;
-                float* gdense = fa.ddense + rb->brick_off;
-                const float il = layer_exponent(depth, v.level, v.quality);
-                float Ab = 0.f;
-                // one sample's gradients from its cell and texels; false once the block is opaque
-                auto step_sample = [&](const Cell& cell, const float* tcur) -> bool {
-                    float val;
-                    if (!filter_cell(cell, tcur, val)) return true;
-                    uint32_t off[8];
-                    cell_offsets(cell, dim_of(r), off);
-                    const float fx = cell.f[0], fy = cell.f[1], fz = cell.f[2];
-                    // the forward's v01 up to the last ulp (a reciprocal instead of the division)
-                    const float v01 = __fmul_rn(__fsub_rn(val, v.field_min), inv_span);
-                    const TfSample ts = tf_lookup(tf, v.tf_n, v01);
-                    const float base = __fmaf_rn(-ts.c.w, of, 1.f);
-                    const float pw = __powf(base, il);
-                    const float a = __fsub_rn(1.f, pw);
-                    // derivatives need no correctly rounded divisions: fast reciprocals
-                    const float dadc = base > 0.f ? __fdividef(il * pw, base) * of : 0.f;
-                    const float wa = T * a;
-                    const float col[3] = {ts.c.x, ts.c.y, ts.c.z};
-                    float g_col[4];
-                    float g_a = 0.f;
-                    const float om = 1.f - a;
-                    const float inv_om = om > 1e-12f ? __fdividef(1.f, om) : 0.f;
-#pragma unroll
-                    for (int ch = 0; ch < 3; ++ch) {
-                        const float cpost = __fmaf_rn(wa, col[ch], Cpre[ch]);
-                        g_col[ch] = gC[ch] * wa;
-                        g_a += gC[ch] * (T * col[ch] - (Ct[ch] - cpost) * inv_om);
-                        Cpre[ch] = cpost;
-                    }
-                    g_a += gA * (1.f - A) * inv_om;
-                    g_col[3] = g_a * dadc;
-                    // transfer-function table: accumulate the two entries of the current
-                    // pair in registers; when the pair changes, an entry the new pair
-                    // shares (a ray moving to the next interval) keeps its sum and only
-                    // the other one goes to shared memory
-                    const float f = ts.f;
-                    if (ts.i0 != tf_i0 || ts.i1 != tf_i1) {
-                        if (tf_i0 != 0xffffffffu && ts.i0 == tf_i1 && ts.i0 != ts.i1) {
-                            // moving up: old i1 becomes new i0
-                            atomicAdd(&dtf4[tf_i0], make_float4(tf_a[0], tf_a[1], tf_a[2], tf_a[3]));
-#pragma unroll
-                            for (int ch = 0; ch < 4; ++ch) {
-                                tf_a[ch] = tf_b[ch];
-                                tf_b[ch] = 0.f;
-                            }
-                        } else if (tf_i0 != 0xffffffffu && ts.i1 == tf_i0 && ts.i0 != ts.i1) {
-                            // moving down: old i0 becomes new i1
-                            atomicAdd(&dtf4[tf_i1], make_float4(tf_b[0], tf_b[1], tf_b[2], tf_b[3]));
-#pragma unroll
-                            for (int ch = 0; ch < 4; ++ch) {
-                                tf_b[ch] = tf_a[ch];
-                                tf_a[ch] = 0.f;
-                            }
-                        } else {
-                            flush_tf();
-                        }
-                        tf_i0 = ts.i0;
-                        tf_i1 = ts.i1;
+                const float base = __fmaf_rn(-__fmaf_rn(f, d.w, p.w), of, 1.f);
+                const float pw = __powf(base, il);
+                const float a = __fsub_rn(1.f, pw);
+                // derivatives need no correctly rounded divisions: fast reciprocals
+                const float dadc = base > 0.f ? __fdividef(il * pw, base) * of : 0.f;
+                const float wa = T * a;
+                const float om = 1.f - a;
+                const float inv_om = om > 1e-12f ? __fdividef(1.f, om) : 0.f;
+                const float s = gC[0] * __fmaf_rn(f, d.x, p.x) + gC[1] * __fmaf_rn(f, d.y, p.y) +
+                                gC[2] * __fmaf_rn(f, d.z, p.z);
+                Q = __fmaf_rn(wa, s, Q);
+                const float g_col[4] = {gC[0] * wa, gC[1] * wa, gC[2] * wa, (T * s + Q * inv_om) * dadc};
+                // transfer-function table: accumulate the two entries of the current
+                // interval in registers; when it changes, an entry that the new interval
+                // shares (a ray moving to the next one) keeps its sum and only the other
+                // one goes to memory
+                if (j != tf_j) {
+                    const bool up = j == tf_j + 1, down = j == tf_j - 1;
+                    if (tf_j != -2) {
+                        if (!down) put_a();
+                        if (!up) put_b();
                     }
 #pragma unroll
                     for (int ch = 0; ch < 4; ++ch) {
-                        tf_a[ch] = __fmaf_rn(g_col[ch], 1.f - f, tf_a[ch]);
-                        tf_b[ch] = __fmaf_rn(g_col[ch], f, tf_b[ch]);
+                        const float ta = tf_a[ch], tb = tf_b[ch];
+                        tf_a[ch] = up ? tb : 0.f;
+                        tf_b[ch] = down ? ta : 0.f;
                     }
-                    // dense values
-                    if (!ts.clamped) {
-                        const float4 p = tf[ts.i0], q = tf[ts.i1];
-                        const float g_v01 = (g_col[0] * (q.x - p.x) + g_col[1] * (q.y - p.y) +
-                                             g_col[2] * (q.z - p.z) + g_col[3] * (q.w - p.w)) *
-                                            (float)v.tf_n;
-                        const float g_val = g_v01 * inv_span;
-                        if (g_val != 0.f) {
+                    tf_j = j;
+                }
 #pragma unroll
-                            for (int qn = 0; qn < 8; ++qn) {
-                                const float w = ((qn & 1) ? fx : 1.f - fx) * ((qn & 2) ? fy : 1.f - fy) *
-                                                ((qn & 4) ? fz : 1.f - fz);
-                                atomicAdd(&gdense[off[qn]], g_val * w);
+                for (int ch = 0; ch < 4; ++ch) {
+                    tf_a[ch] = __fmaf_rn(g_col[ch], 1.f - f, tf_a[ch]);
+                    tf_b[ch] = __fmaf_rn(g_col[ch], f, tf_b[ch]);
+                }
+                // dense values; at the table's ends the colour does not depend on them
+                if ((uint32_t)j < v.tf_n - 1) {
+                    const float g_v01 = (g_col[0] * d.x + g_col[1] * d.y + g_col[2] * d.z + g_col[3] * d.w) *
+                                        (float)v.tf_n;
+                    const float g_val = g_v01 * inv_span;
+                    if (g_val != 0.f) {
+                        if (inside_brick(cell.a, r.n - 1)) {
+                            cg.move(cell.a, gdense, r.n, r.pitch);
+                            cg.add(g_val, cell.f);
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) {
+                                const float w = ((q & 1) ? cell.f[0] : 1.f - cell.f[0]) *
+                                                ((q & 2) ? cell.f[1] : 1.f - cell.f[1]) *
+                                                ((q & 4) ? cell.f[2] : 1.f - cell.f[2]);
+                                atomicAdd(&gdense[clamped_corner(cell.a, dim_of(r), q)], g_val * w);
                             }
                         }
                     }
-                    T *= om;
-                    Ab = __fadd_rn(Ab, __fmul_rn(__fsub_rn(1.f, Ab), a));
-                    return !(Ab > kAlphaThreshold);
-                };
-                // software-pipelined as the forward march, unrolled by two with two
-                // buffers: sample i's texels load while sample i-1's gradients form
-                Cell ca, cb;
-                float ta[8], tb[8];
-                if (r.samples > 1) {
-                    sample_cell(r, 0, ca);
-                    fetch_cell(brick, ca, dim_of(r), ta);
                 }
-                for (int i = 1; i < r.samples; i += 2) {
-                    if (i + 1 < r.samples) {
-                        sample_cell(r, i, cb);
-                        fetch_cell(brick, cb, dim_of(r), tb);
-                    }
-                    if (!step_sample(ca, ta)) break;
-                    if (i + 1 >= r.samples) break;
-                    if (i + 2 < r.samples) {
-                        sample_cell(r, i + 1, ca);
-                        fetch_cell(brick, ca, dim_of(r), ta);
-                    }
-                    if (!step_sample(cb, tb)) break;
-                }
-                // block composite exactly as the forward kernel forms it
-                accA = __fmaf_rn(__fsub_rn(1.f, accA), Ab, accA);
-                return !(accA > v.alpha_stop);
-            });
-            flush_tf();
+                T *= om;
+                Ab = __fadd_rn(Ab, __fmul_rn(__fsub_rn(1.f, Ab), a));
+                return !(Ab > kAlphaThreshold);
+            };
+            // software-pipelined as the forward march, unrolled by two with two
+            // buffers: sample i's texels load while sample i-1's gradients form
+            GradCell ca, cb;
+            if (r.samples > 1) fetch_grad_cell(brick, r, 0.f, ca);
+            const float last = (float)(r.samples - 1);
+            for (float k = 1.f; k <= last;) {
+                if (k < last) fetch_grad_cell(brick, r, k, cb);
+                if (!step_sample(ca) || k >= last) break;
+                k += 1.f;
+                if (k < last) fetch_grad_cell(brick, r, k, ca);
+                if (!step_sample(cb)) break;
+                k += 1.f;
+            }
+            cg.flush();
+            // block composite exactly as the forward kernel forms it
+            accA = __fmaf_rn(__fsub_rn(1.f, accA), Ab, accA);
+            if (accA > v.alpha_stop) break;
         }
+        asm volatile("" ::: "memory");
+        BlockWalk w = sh.walk[tid];
+        if (!w.next()) break;
+        sh.walk[tid] = w;
+    }
+    if (tf_j != -2) {
+        put_a();
+        put_b();
     }
 }
 
-__global__ void dtf_reduce_kernel(const float* __restrict__ part, float* __restrict__ dtf, uint32_t n)
+// dtf[i] += the sum of its kDtfParts copies, one warp per entry-channel of 32 columns: lane l of warp w sums copies
+// w, w + 8, ... of column i, so that reads stay coalesced and a column's 512 additions are 8 chains of 64.
+__global__ void __launch_bounds__(256) dtf_reduce_kernel(const float* __restrict__ part, float* __restrict__ dtf, uint32_t n)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    __shared__ float sums[8][32];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
     float g = 0.f;
-    for (uint32_t p = 0; p < kDtfParts; ++p) g += part[(size_t)p * n + i];
-    dtf[i] += g;
+    if (i < n) {
+#pragma unroll 8
+        for (uint32_t p = w; p < kDtfParts; p += 8) g += part[(size_t)p * n + i];
+    }
+    sums[w][lane] = g;
+    __syncthreads();
+    if (w == 0 && i < n) {
+        for (uint32_t q = 1; q < 8; ++q) g += sums[q][lane];
+        dtf[i] += g;
+    }
 }
 
 } // namespace
@@ -2057,12 +2213,12 @@ cudaError_t launch_frame_render_mode(const FrameArgs& a, const s3r_presentation&
 
 cudaError_t launch_frame_backward(const FrameArgs& a, uint32_t W, uint32_t H, uint32_t tf_n, cudaStream_t s)
 {
-    // 32x2-pixel CTAs: measured 2-3 % faster than 32x4 on cfg5 (the rays' work is uneven; smaller CTAs
-    // leave less idle at the end)
-    dim3 block(32, 2);
-    dim3 grid((W + 31) / 32, (H + 1) / 2);
-    const size_t smem = tf_n * sizeof(float4);
-    if (smem > 48 * 1024) {
+    // 8x8-pixel CTAs: 8x4 pixels a warp share most of the cells they add to (337 us with 32x2, 318 with this on 8
+    // blocks of depth 6 at 512x512); larger CTAs leave more idle at the end, the rays' work being uneven
+    dim3 block(8, 8);
+    dim3 grid((W + 7) / 8, (H + 7) / 8);
+    const size_t smem = tf_smem_entries(tf_n) * sizeof(float4);
+    if (smem + sizeof(BackwardShared) > 47 * 1024) {
         cudaError_t err =
             cudaFuncSetAttribute(frame_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return err;
@@ -2073,7 +2229,7 @@ cudaError_t launch_frame_backward(const FrameArgs& a, uint32_t W, uint32_t H, ui
 
 cudaError_t launch_dtf_reduce(const float* part, float* dtf, uint32_t n, cudaStream_t s)
 {
-    dtf_reduce_kernel<<<(n + 255) / 256, 256, 0, s>>>(part, dtf, n);
+    dtf_reduce_kernel<<<(n + 31) / 32, 256, 0, s>>>(part, dtf, n);
     return cudaGetLastError();
 }
 
