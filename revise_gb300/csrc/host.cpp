@@ -59,7 +59,7 @@ struct s3r_ctx {
 struct FrameGraph {
     cudaGraphExec_t exec = nullptr;
     const void* key[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    uint32_t dims[4] = {0, 0, 0, 0}; // W, H, tf_n, filter the launches were sized for
+    uint32_t dims[5] = {0, 0, 0, 0, 0}; // W, H, tf_n, filter and block-major variant of the launches
     uint32_t kernels = 0;
 };
 
@@ -123,6 +123,7 @@ struct s3r_plan {
     uint32_t* seg_count_pinned = nullptr;
     uint32_t* seg_count_dev = nullptr;  // items staged
     int seg_staged_shape = -1;          // the footprint the staged items are cut for
+    bool seg_lanes = false;             // some of them have several lanes to a ray
     uint32_t* seg_queue = nullptr;      // 2 counters
     float4* seg_buf[2] = {nullptr, nullptr};
     unsigned long long* seg_mask[2] = {nullptr, nullptr};
@@ -776,6 +777,56 @@ int plan_ensure_segments(s3r_plan* p, uint32_t W, uint32_t H)
     return S3R_OK;
 }
 
+// Lanes to a ray (log2) for the block-major items of every depth.  A frame takes about its work spread over all warps
+// plus the longest item's chain of samples; sharing a ray among lanes shortens the chains of deep blocks at the price
+// of more items and instructions.  In units of a sample's time, measured on GB300: an item's set-up about 20, a ray of
+// a block of 2^d cells 1.3 q 2^d on average, six tenths of a view rectangle's pixels hit the block, shared rays cost
+// 1.35 as much, and the kernel that can share marches the others 1.2 times slower -- so sharing has to win clearly
+// (level 2 of depths 3-7 at 800x600: 178 us without, 125 with; 64 blocks of depth 6 there: 157 without, 197 with).
+void seg_lanes_by_depth(const s3r_plan* p, const RenderBlock* table, uint32_t fx, uint32_t fy, float quality,
+                        uint32_t log_lanes[S3R_MAX_DEPTH + 1])
+{
+    constexpr double kSetup = 20, kHit = 0.6, kShared = 1.35, kSlower = 1.2, kMargin = 1.15;
+    const double warps = 32.0 * p->ctx->sms;
+    double items[S3R_MAX_DEPTH + 1] = {}, chain[S3R_MAX_DEPTH + 1];
+    for (uint32_t cell : p->seg_order) {
+        const RenderBlock& t = table[cell];
+        if (t.rect[2] > 0 && t.rect[3] > 0)
+            items[t.depth] += (double)(((uint32_t)t.rect[2] + fx - 1) / fx) * (((uint32_t)t.rect[3] + fy - 1) / fy);
+    }
+    for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d) {
+        log_lanes[d] = 0;
+        chain[d] = 1.3 * quality * (1u << d);
+    }
+    double best = 0;
+    for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d) {
+        best += items[d] * (kSetup + kHit * chain[d]) / warps;
+    }
+    double longest = 0;
+    for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d)
+        if (items[d] > 0) longest = std::max(longest, kSetup + chain[d]);
+    best += longest;
+    // every chain length that some depth can have is tried as the longest one
+    for (uint32_t d0 = 0; d0 <= S3R_MAX_DEPTH; ++d0)
+        for (uint32_t l0 = 1; l0 <= 3 && items[d0] > 0; ++l0) {
+            const double limit = chain[d0] / (1u << l0);
+            uint32_t l[S3R_MAX_DEPTH + 1];
+            double work = 0, top = 0;
+            for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d) {
+                l[d] = 0;
+                while (l[d] < 3 && chain[d] / (1u << l[d]) > limit * 1.001) ++l[d];
+                const double own = chain[d] / (1u << l[d]);
+                work += items[d] * (1u << l[d]) * (kSetup + kHit * own * (l[d] ? kShared : kSlower));
+                if (items[d] > 0) top = std::max(top, kSetup + own);
+            }
+            const double t = (work / warps + top) * kMargin;
+            if (t < best) {
+                best = t;
+                std::memcpy(log_lanes, l, sizeof(l));
+            }
+        }
+}
+
 int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s)
 {
     s3r_ctx* ctx = p->ctx;
@@ -806,11 +857,22 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s)
     // block-major render: the warp-sized tiles of every block's view rectangle, deepest blocks first
     if (p->render_tile >= (uint32_t)kRenderWalkTiles) {
         const int f = (int)(p->render_tile - (uint32_t)kRenderWalkTiles);
-        const int fx = kSegShapeX[f], fy = kSegShapeY[f];
+        const uint32_t fx = (uint32_t)kSegShapeX[f], fy = (uint32_t)kSegShapeY[f];
+        uint32_t log_lanes[S3R_MAX_DEPTH + 1];
+        seg_lanes_by_depth(p, tb, fx, fy, view->quality, log_lanes);
+        auto tiles_of = [&](const RenderBlock& t) -> uint64_t {
+            if (t.rect[2] <= 0 || t.rect[3] <= 0) return 0;
+            uint32_t w, h;
+            seg_footprint(fx, log_lanes[t.depth], w, h);
+            return (uint64_t)(((uint32_t)t.rect[2] + w - 1) / w) * (((uint32_t)t.rect[3] + h - 1) / h);
+        };
         uint64_t n = 0;
+        p->seg_lanes = false;
         for (uint32_t i = 0; i < p->nblocks; ++i) {
-            const int32_t* r = tb[p->seg_order[i]].rect;
-            if (r[2] > 0 && r[3] > 0) n += (uint64_t)((r[2] + fx - 1) / fx) * ((r[3] + fy - 1) / fy);
+            const RenderBlock& t = tb[p->seg_order[i]];
+            const uint64_t tiles = tiles_of(t);
+            n += tiles;
+            p->seg_lanes |= tiles > 0 && log_lanes[t.depth] > 0;
         }
         if (n > 0xffffffffull) return fail(ctx, S3R_ERR_INVALID, "too many block-major render items");
         cudaError_t e;
@@ -836,10 +898,9 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s)
         uint2* it = p->seg_items_pinned;
         for (uint32_t i = 0; i < p->nblocks; ++i) {
             const uint32_t cell = p->seg_order[i];
-            const int32_t* r = tb[cell].rect;
-            if (r[2] <= 0 || r[3] <= 0) continue;
-            const uint32_t tiles = (uint32_t)(((r[2] + fx - 1) / fx) * ((r[3] + fy - 1) / fy));
-            for (uint32_t t = 0; t < tiles; ++t) *it++ = make_uint2(cell, t);
+            const uint32_t tiles = (uint32_t)tiles_of(tb[cell]);
+            const uint32_t key = cell | log_lanes[tb[cell].depth] << kSegLanesShift;
+            for (uint32_t t = 0; t < tiles; ++t) *it++ = make_uint2(key, t);
         }
         *p->seg_count_pinned = (uint32_t)n;
         if (n) S3R_CUDA(ctx, cudaMemcpyAsync(p->seg_items_dev, p->seg_items_pinned, n * sizeof(uint2),
@@ -921,6 +982,7 @@ int plan_launch_render(s3r_plan* p, const float* tf, float* rgba, uint32_t* argb
             return fail(p->ctx, S3R_ERR_INVALID, "block-major render items not staged for this render tile");
         sa.items = p->seg_items_dev;
         sa.count = p->seg_count_dev;
+        sa.lanes = p->seg_lanes;
         sa.words = p->seg_words;
         sa.seg = p->seg_buf[data];
         sa.mask = p->seg_mask[data];
@@ -1941,7 +2003,7 @@ static int plan_launch_frame(s3r_plan* plan, int slot, const s3r_view* view, con
     s3r_ctx* ctx = plan->ctx;
     FrameGraph& G = plan->graphs[slot];
     const void* key[5] = {sparse, tf, rgba, argb, samples};
-    const uint32_t dims[4] = {view->W, view->H, view->tf_n, view->filter};
+    const uint32_t dims[5] = {view->W, view->H, view->tf_n, view->filter, plan->seg_lanes ? 1u : 0u};
     const bool same = G.exec && std::memcmp(key, G.key, sizeof(key)) == 0 && std::memcmp(dims, G.dims, sizeof(dims)) == 0;
     if (!same) {
         if (G.exec) cudaGraphExecDestroy(G.exec);

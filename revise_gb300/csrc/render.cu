@@ -1324,6 +1324,61 @@ __device__ __forceinline__ Premul march_block(const s3r_view& v, const BlockRay&
     }
 }
 
+// march_block with `lanes` consecutive lanes (2, 4 or 8) to a ray: lane `sub` fetches, filters and looks up samples
+// sub, sub + lanes, ...; the samples' colours then go around by shuffles and every lane of the ray composites them in
+// order, so the result is march_block's bit for bit.  A ray's chain of samples is that much shorter, for a third more
+// instructions in all; a warp's 32 lanes call it together (last: samples to take, 0 for no ray).
+template <int Fmt, bool kTex>
+__device__ __forceinline__ Premul march_block_lanes(const s3r_view& v, const BlockRay& r, float last, const void* brick,
+                                                    float scale, float offset, uint32_t depth, const TfTable& tf,
+                                                    const Relative& rel, float of, uint32_t lanes, uint32_t sub,
+                                                    uint32_t& taken)
+{
+    const float il = layer_exponent(depth, v.level, v.quality);
+    Premul acc{0.f, 0.f, 0.f, 0.f};
+    bool open = last > 0.f;
+    float k0 = 0.f; // the group's first sample
+    const float fsub = (float)sub, flanes = (float)lanes;
+    Texels<Fmt> cur, nxt;
+    if constexpr (!kTex)
+        if (fsub < last) fetch_texels<Fmt, true>(brick, r, fsub, cur);
+    while (__any_sync(0xffffffffu, open)) {
+        const float k = k0 + fsub;
+        if constexpr (!kTex)
+            if (open && k + flanes < last) fetch_texels<Fmt, true>(brick, r, k + flanes, nxt);
+        // a sample outside the domain blends as nothing: all zero
+        float4 col = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (open && k < last) {
+            float val;
+            bool in;
+            if constexpr (kTex) in = tex_trilinear<Fmt>(brick, r, (int)k, val);
+            else in = filter_texels<Fmt>(cur, val);
+            if (in) {
+                if (Fmt != S3R_BRICK_F32) val = __fmaf_rn(scale, val, offset);
+                col = kTex ? tex_tf_lookup(tf.raw(), v.tf_n, rel(val)) : tf_colour(tf, v.tf_n, rel(val));
+                col.w = __fsub_rn(1.f, __powf(__fmaf_rn(-col.w, of, 1.f), il));
+            }
+        }
+#pragma unroll 2
+        for (uint32_t j = 0; j < lanes; ++j) {
+            const float cr = __shfl_sync(0xffffffffu, col.x, j, lanes), cg = __shfl_sync(0xffffffffu, col.y, j, lanes),
+                        cb = __shfl_sync(0xffffffffu, col.z, j, lanes), a = __shfl_sync(0xffffffffu, col.w, j, lanes);
+            if (open) {
+                const float w = __fmul_rn(__fsub_rn(1.f, acc.a), a);
+                acc.r = __fmaf_rn(w, cr, acc.r);
+                acc.g = __fmaf_rn(w, cg, acc.g);
+                acc.b = __fmaf_rn(w, cb, acc.b);
+                acc.a = __fadd_rn(acc.a, w);
+                k0 += 1.f;
+                if (sub == 0) ++taken;
+                open = !(acc.a > kAlphaThreshold) && k0 < last;
+            }
+        }
+        if constexpr (!kTex) cur = nxt;
+    }
+    return acc;
+}
+
 // One pixel ray per R consecutive lanes: the ray's block sequence (the DDA
 // order) is cut into R contiguous runs, lane r composites run r, and the R
 // premultiplied partial results are merged front to back with shuffles (the
@@ -1479,7 +1534,11 @@ __device__ __forceinline__ uint32_t ray_rank(const float dir[3], uint32_t ix, ui
 // and the deep blocks' items spread over every SM -- the per-ray walk's lanes
 // instead each hold their own block sequence.  frame_composite_kernel then blends
 // every pixel's results in rank order with frame_render_kernel's arithmetic.
-template <int Fmt, bool kTex>
+// kLanes: an item of a block whose rays would take longer than the whole frame's
+// share of a warp has 2, 4 or 8 lanes to a ray (SegArgs::items).  A kernel of its
+// own: with both marches in it the one with one lane to a ray has too few
+// registers (64 blocks of depth 6 at 1920x1080: 336 us instead of 278).
+template <int Fmt, bool kTex, bool kLanes>
 __global__ void __launch_bounds__(128, 8) frame_segments_kernel(FrameArgs fa, SegArgs sa, uint32_t fx)
 {
     extern __shared__ float4 tf_sm[];
@@ -1489,7 +1548,6 @@ __global__ void __launch_bounds__(128, 8) frame_segments_kernel(FrameArgs fa, Se
     const TfTable tf = load_tf(tf_sm, fa.tf, v.tf_n, tid, nthreads);
     const Relative rel = relative_of(v);
     const uint32_t lane = tid & 31u;
-    const uint32_t fy = 32u / fx;
     const uint32_t total = *sa.count;
     const uint32_t m = 1u << v.level;
     const uint64_t npix = (uint64_t)v.W * v.H;
@@ -1513,37 +1571,46 @@ __global__ void __launch_bounds__(128, 8) frame_segments_kernel(FrameArgs fa, Se
         uint32_t next;
         uint2 ndesc;
         take(next, ndesc); // in flight while this item is marched
-        const uint32_t cell = desc.x, tile = desc.y;
+        const uint32_t cell = desc.x & kSegCellMask, tile = desc.y,
+                       log_lanes = kLanes ? desc.x >> kSegLanesShift : 0u;
         const RenderBlock* rb = &fa.table[cell];
         const int4 rc = *reinterpret_cast<const int4*>(rb->rect);
-        const uint32_t tiles_x = ((uint32_t)rc.z + fx - 1) / fx;
-        const int32_t x = rc.x + (int32_t)((tile % tiles_x) * fx + lane % fx);
-        const int32_t y = rc.y + (int32_t)((tile / tiles_x) * fy + lane / fx);
+        uint32_t w, h;
+        seg_footprint(fx, log_lanes, w, h);
+        const uint32_t p = lane >> log_lanes, tiles_x = ((uint32_t)rc.z + w - 1) / w;
+        const int32_t x = rc.x + (int32_t)((tile % tiles_x) * w + p % w);
+        const int32_t y = rc.y + (int32_t)((tile / tiles_x) * h + p / w);
+        float org[3], dir[3];
+        BlockRay r;
+        bool hit = false;
         if (x < rc.x + rc.z && y < rc.y + rc.w && x >= 0 && y >= 0 && x < (int32_t)v.W && y < (int32_t)v.H) {
-            float org[3], dir[3];
             pixel_ray(v, (uint32_t)x, (uint32_t)y, org, dir);
             float inv[3];
             ray_inverse(dir, inv);
-            BlockRay r;
-            if (block_ray(v, org, dir, inv, *rb, r)) {
-                const char* base = reinterpret_cast<const char*>(fa.bricks);
-                const size_t esz = Fmt == S3R_BRICK_F32 ? 4 : 2;
-                float scale = 1.f, offset = 0.f;
-                if (Fmt != S3R_BRICK_F32) {
-                    const float2 so = fa.scale_offset[rb->block];
-                    scale = so.x;
-                    offset = so.y;
-                }
-                const Premul p = march_block<Fmt, kTex, true>(v, r, base + rb->brick_off * esz, scale, offset, rb->depth,
-                                                        tf, rel, of, taken);
-                if (!(p.r == 0.f && p.g == 0.f && p.b == 0.f && p.a == 0.f)) {
-                    const uint32_t ix = cell % m, iy = (cell / m) % m, iz = cell / (m * m);
-                    const uint32_t k = ray_rank(dir, ix, iy, iz, m);
-                    const uint64_t pix = (uint64_t)y * v.W + (uint32_t)x;
-                    sa.seg[(uint64_t)k * npix + pix] = make_float4(p.r, p.g, p.b, p.a);
-                    atomicOr(&sa.mask[(uint64_t)(k >> 6) * npix + pix], 1ull << (k & 63));
-                }
-            }
+            hit = block_ray(v, org, dir, inv, *rb, r);
+        }
+        const char* brick = reinterpret_cast<const char*>(fa.bricks) + rb->brick_off * (Fmt == S3R_BRICK_F32 ? 4 : 2);
+        float scale = 1.f, offset = 0.f;
+        if (Fmt != S3R_BRICK_F32) {
+            const float2 so = fa.scale_offset[rb->block];
+            scale = so.x;
+            offset = so.y;
+        }
+        Premul acc{0.f, 0.f, 0.f, 0.f};
+        if (kLanes && log_lanes) {
+            const uint32_t lanes = 1u << log_lanes, sub = lane & (lanes - 1);
+            acc = march_block_lanes<Fmt, kTex>(v, r, hit ? (float)(r.samples - 1) : 0.f, brick, scale, offset,
+                                               rb->depth, tf, rel, of, lanes, sub, taken);
+            hit = hit && sub == 0;
+        } else if (hit) {
+            acc = march_block<Fmt, kTex, true>(v, r, brick, scale, offset, rb->depth, tf, rel, of, taken);
+        }
+        if (hit && !(acc.r == 0.f && acc.g == 0.f && acc.b == 0.f && acc.a == 0.f)) {
+            const uint32_t ix = cell % m, iy = (cell / m) % m, iz = cell / (m * m);
+            const uint32_t k = ray_rank(dir, ix, iy, iz, m);
+            const uint64_t pix = (uint64_t)y * v.W + (uint32_t)x;
+            sa.seg[(uint64_t)k * npix + pix] = make_float4(acc.r, acc.g, acc.b, acc.a);
+            atomicOr(&sa.mask[(uint64_t)(k >> 6) * npix + pix], 1ull << (k & 63));
         }
         item = __shfl_sync(0xffffffffu, next, 0);
         desc.x = __shfl_sync(0xffffffffu, ndesc.x, 0);
@@ -2157,7 +2224,7 @@ template <int Fmt, bool kTex>
 cudaError_t launch_frame_segments_fmt(const FrameArgs& a, const SegArgs& sa, uint32_t fx, dim3 block, size_t smem,
                                       uint32_t sms, cudaStream_t s)
 {
-    auto kernel = frame_segments_kernel<Fmt, kTex>;
+    auto kernel = sa.lanes ? frame_segments_kernel<Fmt, kTex, true> : frame_segments_kernel<Fmt, kTex, false>;
     if (smem > 48 * 1024) {
         cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (err != cudaSuccess) return err;

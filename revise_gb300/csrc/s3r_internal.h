@@ -147,10 +147,18 @@ struct FrameArgs {
 // The block-major frame render (render tile ids kRenderWalkTiles and up): its work
 // items and per-pixel block results.
 constexpr uint32_t kSegMaskWords = 6; // rank masks of up to 384 ranks: levels <= 7
+constexpr uint32_t kSegLanesShift = 28, kSegCellMask = (1u << kSegLanesShift) - 1;
+// Pixels of an item: fx x (32 / fx) with one lane to a ray, halved along x, then y, then x again with 2, 4, 8 lanes.
+inline __host__ __device__ void seg_footprint(uint32_t fx, uint32_t log_lanes, uint32_t& w, uint32_t& h)
+{
+    w = fx >> ((log_lanes + 1) / 2);
+    h = (32u / fx) >> (log_lanes / 2);
+}
 struct SegArgs {
-    const uint2* items;         // {block cell, tile} per warp work item: the footprint-sized tiles of every
-                                // block's view rectangle, deepest blocks first
+    const uint2* items;         // {block cell | log2(lanes to a ray) << kSegLanesShift, tile} per warp work item: the
+                                // footprint-sized tiles of every block's view rectangle, deepest blocks first
     const uint32_t* count;      // items
+    bool lanes;                 // some items have several lanes to a ray
     uint32_t words;             // mask words per pixel: ceil((3m - 2) / 64)
     float4* seg;                // [rank][pixel] premultiplied block results
     unsigned long long* mask;   // [word][pixel] ranks holding a result
