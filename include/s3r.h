@@ -392,10 +392,15 @@ int s3r_make_color_transfer(const double* xs, const double* rgba, uint32_t npoin
  *   ids below S3R_RENDER_TILES_WALK: one thread (or 2, 4, 8 lanes) per pixel ray walks the block grid
  *     front to back and composites every block it passes (4 CTA pixel shapes x 4 lane counts; several
  *     lanes per ray merge partial composites in another association order, within 1e-5);
- *   ids S3R_RENDER_TILES_WALK .. S3R_RENDER_TILES-1: block-major -- CTAs take pixel tiles of the
- *     blocks' view rectangles (deepest blocks first) and march one block each, the per-block results
- *     are blended per pixel in front-to-back order afterwards; the same image bit for bit as id 0, for
- *     levels up to 7, at the cost of (3 * 2^level - 2) x W x H x 16 bytes of device memory per data slot.
+ *   ids S3R_RENDER_TILES_WALK .. S3R_RENDER_TILES-1: block-major -- warps take pixel tiles of the
+ *     blocks' view rectangles (deepest blocks first) and march one block each, a deep block's rays with several
+ *     lanes where few of them would set the time; the per-block results are blended per pixel in front-to-back
+ *     order afterwards.  The same image bit for bit as id 0 but on rays that run in a plane between two blocks
+ *     (the walk takes one of them, this form both); for levels up to 7, at the cost of (3 * 2^level - 2) x 16
+ *     bytes of device memory per pixel that the blocks cover and data slot.
+ *   One thread per ray (ids 0-3): a view for which block-major is the faster one (64 blocks and more with rays of
+ *     some length in each; at most 1 GB of results) renders in that form, restricted to the blocks that the walk
+ *     meets -- the walk's image bit for bit.
  * The autotuner times every form. */
 #define S3R_RENDER_TILES_WALK 16u
 #define S3R_RENDER_TILES 19u

@@ -122,7 +122,8 @@ struct s3r_plan {
     uint64_t seg_items_cap = 0, seg_items_dev_cap = 0;
     uint32_t* seg_count_pinned = nullptr;
     uint32_t* seg_count_dev = nullptr;  // items staged
-    int seg_staged_shape = -1;          // the footprint the staged items are cut for
+    int staged_tile = -1;               // the render tile the view is staged for (-1: the table alone)
+    bool seg_now = false;               // the staged view renders block-major
     bool seg_lanes = false;             // some of them have several lanes to a ray
     uint32_t* seg_queue = nullptr;      // 2 counters
     float4* seg_buf[2] = {nullptr, nullptr};
@@ -734,9 +735,9 @@ int plan_bin(s3r_plan* p, uint32_t tile_log2, const uint8_t* by_depth = nullptr)
     return S3R_OK;
 }
 
-// The block-major render's per-rank results and rank masks for W x H pixels, in both data slots; called
-// before a frame is launched (or captured) with a block-major render tile.  Reallocation drops the captured
-// frames (they hold the old buffers).
+// The block-major render's per-rank results and rank masks for `npix` covered pixels in data slots 0 .. slots-1;
+// called before a frame is launched (or captured) in the block-major form.  Reallocation drops the captured frames
+// (they hold the old buffers).
 void plan_free_segments(s3r_plan* p)
 {
     for (int b = 0; b < 2; ++b) {
@@ -748,22 +749,22 @@ void plan_free_segments(s3r_plan* p)
     p->seg_pixels = 0;
 }
 
-int plan_ensure_segments(s3r_plan* p, uint32_t W, uint32_t H)
+uint64_t seg_pixel_bytes(const s3r_plan* p) { return (3ull * (1u << p->level) - 2) * sizeof(float4); }
+
+int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t most)
 {
-    if (p->render_tile < (uint32_t)kRenderWalkTiles) return S3R_OK;
     s3r_ctx* ctx = p->ctx;
-    const uint64_t npix = (uint64_t)W * H;
-    const uint32_t m = 1u << p->level;
-    const uint32_t words = (3 * m - 2 + 63) / 64;
-    if (words > kSegMaskWords)
-        return fail(ctx, S3R_ERR_UNSUPPORTED, "the block-major render covers levels up to 7");
-    if (p->seg_buf[0] && p->seg_pixels >= npix && p->seg_words == words) return S3R_OK;
+    const int slots = p->hs_h2d ? 2 : 1; // the second one only for the host-buffer pipeline
+    const uint32_t words = (3 * (1u << p->level) - 2 + 63) / 64;
+    if (p->seg_buf[slots - 1] && p->seg_pixels >= npix) return S3R_OK;
     S3R_CUDA(ctx, cudaDeviceSynchronize());
+    // some room to move closer in, up to the whole viewport
+    npix = std::max(p->seg_pixels, std::min(npix + npix / 2, most));
     plan_free_segments(p);
     plan_drop_graph(p);
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < slots; ++b) {
         cudaError_t e;
-        if ((e = cudaMalloc(&p->seg_buf[b], (size_t)(3 * m - 2) * npix * sizeof(float4))) != cudaSuccess ||
+        if ((e = cudaMalloc(&p->seg_buf[b], npix * seg_pixel_bytes(p))) != cudaSuccess ||
             (e = cudaMalloc(&p->seg_mask[b], (size_t)words * npix * sizeof(unsigned long long))) != cudaSuccess ||
             (e = cudaMemset(p->seg_mask[b], 0, (size_t)words * npix * sizeof(unsigned long long))) != cudaSuccess) {
             plan_free_segments(p);
@@ -783,8 +784,9 @@ int plan_ensure_segments(s3r_plan* p, uint32_t W, uint32_t H)
 // a block of 2^d cells 1.3 q 2^d on average, six tenths of a view rectangle's pixels hit the block, shared rays cost
 // 1.35 as much, and the kernel that can share marches the others 1.2 times slower -- so sharing has to win clearly
 // (level 2 of depths 3-7 at 800x600: 178 us without, 125 with; 64 blocks of depth 6 there: 157 without, 197 with).
-void seg_lanes_by_depth(const s3r_plan* p, const RenderBlock* table, uint32_t fx, uint32_t fy, float quality,
-                        uint32_t log_lanes[S3R_MAX_DEPTH + 1])
+// Returns the samples of an item's ray, averaged over the items.
+double seg_lanes_by_depth(const s3r_plan* p, const RenderBlock* table, uint32_t fx, uint32_t fy, float quality,
+                          uint32_t log_lanes[S3R_MAX_DEPTH + 1])
 {
     constexpr double kSetup = 20, kHit = 0.6, kShared = 1.35, kSlower = 1.2, kMargin = 1.15;
     const double warps = 32.0 * p->ctx->sms;
@@ -798,11 +800,12 @@ void seg_lanes_by_depth(const s3r_plan* p, const RenderBlock* table, uint32_t fx
         log_lanes[d] = 0;
         chain[d] = 1.3 * quality * (1u << d);
     }
-    double best = 0;
+    double best = 0, all = 0, samples = 0, longest = 0;
     for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d) {
         best += items[d] * (kSetup + kHit * chain[d]) / warps;
+        all += items[d];
+        samples += items[d] * chain[d];
     }
-    double longest = 0;
     for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d)
         if (items[d] > 0) longest = std::max(longest, kSetup + chain[d]);
     best += longest;
@@ -825,15 +828,40 @@ void seg_lanes_by_depth(const s3r_plan* p, const RenderBlock* table, uint32_t fx
                 std::memcpy(log_lanes, l, sizeof(l));
             }
         }
+    return all > 0 ? samples / all : 0;
 }
 
-int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s)
+// Whether a plan left to the render form's default (ids below kRenderShapes: one image from all of them) goes
+// block-major for this view.  The measured line (depths 3-7 and 4 to 6, 200x150 to 1920x1080, from close up to far):
+// with 64 blocks and more the walk's lanes sit in different blocks and wait for each other, and block-major is up to
+// seven times faster (level 3, 200x150: 550 against 79 us); short segments in a large part of the image favour the
+// walk, which writes no block results (level 4 of depth 3, close up: 711 against 878 us); of 8 blocks only small views
+// of mixed depths gain (66 against 42 us), and a single one is the walk's.
+constexpr uint64_t kSegAutoBytes = 1ull << 30; // of block results
+bool seg_pays(const s3r_plan* p, uint64_t covered, double samples, const uint32_t log_lanes[S3R_MAX_DEPTH + 1])
+{
+    if (p->level < 1 || p->level > 7 || covered == 0 || covered * seg_pixel_bytes(p) > kSegAutoBytes) return false;
+    if (p->level == 1) {
+        bool lanes = false;
+        for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d) lanes |= log_lanes[d] > 0;
+        return lanes && covered < 60000;
+    }
+    return samples >= 30 || covered < 100000 || (samples >= 18 && covered < 1000000);
+}
+
+// frame: for s3r_frame_render and the frames of s3r_frame_run(_host), whose render may go block-major; the field modes
+// and the adjoint read the table alone.
+int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool frame)
 {
     s3r_ctx* ctx = p->ctx;
-    if (int rc = plan_ensure_segments(p, view->W, view->H)) return rc;
-    const bool seg = p->render_tile >= (uint32_t)kRenderWalkTiles;
+    const bool asked = p->render_tile >= (uint32_t)kRenderWalkTiles; // block-major by its id
+    if (asked && (3 * (1u << p->level) - 2 + 63) / 64 > kSegMaskWords)
+        return fail(ctx, S3R_ERR_UNSUPPORTED, "the block-major render covers levels up to 7");
+    const int shape = asked ? (int)(p->render_tile - (uint32_t)kRenderWalkTiles) : 0;
+    // a view staged for another form (the autotuner's) or, since then, for fewer data slots is staged again
     const bool same = p->have_view && std::memcmp(&p->last_view, view, sizeof(s3r_view)) == 0 &&
-                      (!seg || p->seg_staged_shape == (int)(p->render_tile - (uint32_t)kRenderWalkTiles));
+                      (!frame || (p->staged_tile == (int)p->render_tile &&
+                                  (!p->seg_now || p->seg_buf[p->hs_h2d ? 1 : 0])));
     if (same) return S3R_OK;
     // the staging buffers may still feed an earlier copy
     S3R_CUDA(ctx, cudaEventSynchronize(p->staged));
@@ -855,11 +883,28 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s)
     }
     if (cover[0] > cover[2]) cover[0] = cover[1] = cover[2] = cover[3] = 0;
     // block-major render: the warp-sized tiles of every block's view rectangle, deepest blocks first
-    if (p->render_tile >= (uint32_t)kRenderWalkTiles) {
-        const int f = (int)(p->render_tile - (uint32_t)kRenderWalkTiles);
-        const uint32_t fx = (uint32_t)kSegShapeX[f], fy = (uint32_t)kSegShapeY[f];
-        uint32_t log_lanes[S3R_MAX_DEPTH + 1];
-        seg_lanes_by_depth(p, tb, fx, fy, view->quality, log_lanes);
+    const uint64_t covered = (uint64_t)(cover[2] - cover[0]) * (uint64_t)(cover[3] - cover[1]);
+    const uint32_t fx = (uint32_t)kSegShapeX[shape], fy = (uint32_t)kSegShapeY[shape];
+    uint32_t log_lanes[S3R_MAX_DEPTH + 1];
+    bool seg = false;
+    if (frame && (asked || p->render_tile < (uint32_t)kRenderShapes)) {
+        const double samples = seg_lanes_by_depth(p, tb, fx, fy, view->quality, log_lanes);
+        seg = asked || seg_pays(p, covered, samples, log_lanes);
+    }
+    if (seg) {
+        const uint64_t most = (uint64_t)view->W * view->H;
+        const int rc = plan_ensure_segments(p, std::max<uint64_t>(covered, 1),
+                                            asked ? most : std::min(most, kSegAutoBytes / seg_pixel_bytes(p)));
+        if (rc && asked) return rc;
+        if (rc) {
+            // no room: the walk gives the same image
+            seg = false;
+            ctx->err.clear();
+            set_thread_error("");
+        }
+    }
+    p->seg_now = seg;
+    if (seg) {
         auto tiles_of = [&](const RenderBlock& t) -> uint64_t {
             if (t.rect[2] <= 0 || t.rect[3] <= 0) return 0;
             uint32_t w, h;
@@ -907,8 +952,8 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s)
                                              cudaMemcpyHostToDevice, s));
         S3R_CUDA(ctx, cudaMemcpyAsync(p->seg_count_dev, p->seg_count_pinned, sizeof(uint32_t), cudaMemcpyHostToDevice,
                                       s));
-        p->seg_staged_shape = f;
     }
+    p->staged_tile = frame ? (int)p->render_tile : -1;
     std::memcpy(p->cover_pinned, cover, sizeof(cover));
     S3R_CUDA(ctx, cudaMemcpyAsync(p->cover_dev, p->cover_pinned, sizeof(cover), cudaMemcpyHostToDevice, s));
     *p->view_pinned = *view;
@@ -972,17 +1017,19 @@ int plan_launch_render(s3r_plan* p, const float* tf, float* rgba, uint32_t* argb
     fa.samples = samples;
     fa.scale_offset = p->fmt == S3R_BRICK_F32 ? nullptr : (slot ? p->scale_offset_1 : p->scale_offset_dev);
     fa.cover = p->cover_dev;
-    if (p->render_tile >= (uint32_t)kRenderWalkTiles) {
+    if (p->staged_tile != (int)p->render_tile)
+        return fail(p->ctx, S3R_ERR_INVALID, "view not staged for this render tile");
+    if (p->seg_now) {
         const int data = slot ? 1 : 0;
-        if (!p->seg_buf[data] || p->seg_pixels < (uint64_t)p->last_view.W * p->last_view.H)
+        if (!p->seg_buf[data] || !p->seg_items_dev)
             return fail(p->ctx, S3R_ERR_INVALID, "block-major render buffers not allocated for this view");
-        const uint32_t shape = p->render_tile - (uint32_t)kRenderWalkTiles;
+        const bool asked = p->render_tile >= (uint32_t)kRenderWalkTiles;
+        const uint32_t shape = asked ? p->render_tile - (uint32_t)kRenderWalkTiles : 0u;
         SegArgs sa{};
-        if (p->seg_staged_shape != (int)shape || !p->seg_items_dev)
-            return fail(p->ctx, S3R_ERR_INVALID, "block-major render items not staged for this render tile");
         sa.items = p->seg_items_dev;
         sa.count = p->seg_count_dev;
         sa.lanes = p->seg_lanes;
+        sa.walk = !asked;
         sa.words = p->seg_words;
         sa.seg = p->seg_buf[data];
         sa.mask = p->seg_mask[data];
@@ -1941,7 +1988,7 @@ int s3r_frame_render(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const f
     if (view->level != plan->level) return fail(ctx, S3R_ERR_INVALID, "view level differs from the plan level");
     if ((rc = set_device(ctx))) return rc;
     cudaStream_t s = as_stream(stream);
-    if ((rc = plan_stage_view(plan, view, s))) return rc;
+    if ((rc = plan_stage_view(plan, view, s, true))) return rc;
     uint32_t k = 0;
     rc = plan_launch_render(plan, tf, rgba, argb, samples, s, &k);
     ctx->launches += k;
@@ -1964,7 +2011,7 @@ int s3r_frame_render_mode(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, co
     if (plan->fmt != S3R_BRICK_F32) return fail(ctx, S3R_ERR_UNSUPPORTED, "field modes need F32 bricks");
     if ((rc = set_device(ctx))) return rc;
     cudaStream_t s = as_stream(stream);
-    if ((rc = plan_stage_view(plan, view, s))) return rc;
+    if ((rc = plan_stage_view(plan, view, s, false))) return rc;
     FrameArgs fa{};
     fa.view = plan->view_dev;
     fa.table = plan->table_dev;
@@ -1992,7 +2039,7 @@ int s3r_frame_run(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const floa
     if (view->level != plan->level) return fail(ctx, S3R_ERR_INVALID, "view level differs from the plan level");
     if ((rc = set_device(ctx))) return rc;
     cudaStream_t s = as_stream(stream);
-    if ((rc = plan_stage_view(plan, view, s))) return rc;
+    if ((rc = plan_stage_view(plan, view, s, true))) return rc;
     return plan_launch_frame(plan, 0, view, sparse, tf, rgba, argb, samples, s);
 }
 
@@ -2003,7 +2050,7 @@ static int plan_launch_frame(s3r_plan* plan, int slot, const s3r_view* view, con
     s3r_ctx* ctx = plan->ctx;
     FrameGraph& G = plan->graphs[slot];
     const void* key[5] = {sparse, tf, rgba, argb, samples};
-    const uint32_t dims[5] = {view->W, view->H, view->tf_n, view->filter, plan->seg_lanes ? 1u : 0u};
+    const uint32_t dims[5] = {view->W, view->H, view->tf_n, view->filter, (plan->seg_now ? 2u : 0u) | (plan->seg_lanes ? 1u : 0u)};
     const bool same = G.exec && std::memcmp(key, G.key, sizeof(key)) == 0 && std::memcmp(dims, G.dims, sizeof(dims)) == 0;
     if (!same) {
         if (G.exec) cudaGraphExecDestroy(G.exec);
@@ -2105,11 +2152,12 @@ static int frame_host_submit(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view,
     S3R_CUDA(ctx, cudaStreamWaitEvent(cb, plan->hs_entry, 0));
     S3R_CUDA(ctx, cudaStreamWaitEvent(cb, plan->hs_copied[b], 0));
     S3R_CUDA(ctx, cudaStreamWaitEvent(cb, plan->hs_read[b], 0));
-    if (!plan->have_view || std::memcmp(&plan->last_view, view, sizeof(s3r_view)) != 0) {
+    if (!plan->have_view || plan->staged_tile != (int)plan->render_tile ||
+        std::memcmp(&plan->last_view, view, sizeof(s3r_view)) != 0) {
         // the render table both slots read changes: let the frames in flight finish first
         for (int q = 0; q < 2; ++q) S3R_CUDA(ctx, cudaStreamSynchronize(plan->hs_comp[q]));
     }
-    if ((rc = plan_stage_view(plan, view, cb))) return rc;
+    if ((rc = plan_stage_view(plan, view, cb, true))) return rc;
     // the table upload may have been queued on the other slot's stream
     S3R_CUDA(ctx, cudaStreamWaitEvent(cb, plan->staged, 0));
     if ((rc = plan_launch_frame(plan, 1 + b, view, plan->hs_sparse[b], plan->hs_tf[b], nullptr, plan->hs_argb[b],
@@ -2267,16 +2315,15 @@ int s3r_plan_autotune(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const 
     uint32_t k = 0;
     if ((rc = plan_launch_interp(plan, sparse, s, &k))) return cleanup(rc);
     ctx->launches += k;
-    if ((rc = plan_stage_view(plan, view, s))) return cleanup(rc);
     uint32_t best_shape = plan->render_tile;
     best = 3.4e38f;
     for (uint32_t shape = 0; shape < (uint32_t)kRenderTiles; ++shape) {
         // several lanes per ray only where rays composite every block (alpha_stop >= 1)
         if (shape >= (uint32_t)kRenderShapes && shape < (uint32_t)kRenderWalkTiles && view->alpha_stop < 1.f) continue;
         plan->render_tile = shape;
-        // the block-major forms' buffers and their footprint's work items
-        if (shape >= (uint32_t)kRenderWalkTiles && plan_stage_view(plan, view, s) != S3R_OK) {
-            // no room for the block-major buffers: keep to the per-ray walk
+        if ((rc = plan_stage_view(plan, view, s, true)) != S3R_OK) {
+            if (shape < (uint32_t)kRenderWalkTiles) return cleanup(rc);
+            // no room for the block-major buffers, or a level they do not cover: keep to the others
             ctx->err.clear();
             set_thread_error("");
             continue;
@@ -2291,8 +2338,8 @@ int s3r_plan_autotune(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const 
     }
     plan->render_tile = best_shape;
     plan_drop_graph(plan);
-    if (best_shape < (uint32_t)kRenderWalkTiles) {
-        // the per-ray walk won: release the block-major buffers
+    if (best_shape >= (uint32_t)kRenderShapes && best_shape < (uint32_t)kRenderWalkTiles) {
+        // several lanes per ray won: release the block-major buffers
         cudaStreamSynchronize(s);
         plan_free_segments(plan);
     }
@@ -2312,7 +2359,7 @@ int s3r_render_argb_backward(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view,
     if (view->level != plan->level) return fail(ctx, S3R_ERR_INVALID, "view level differs from the plan level");
     if ((rc = set_device(ctx))) return rc;
     cudaStream_t s = as_stream(stream);
-    if ((rc = plan_stage_view(plan, view, s))) return rc;
+    if ((rc = plan_stage_view(plan, view, s, false))) return rc;
     FrameArgs fa{};
     fa.view = plan->view_dev;
     fa.table = plan->table_dev;

@@ -355,25 +355,28 @@ __device__ __forceinline__ TfSample tf_lookup(const float4* tf, uint32_t tfn, fl
     return s;
 }
 
-// The transfer function in shared memory as the kernels look it up: P holds tf_n + 2 entries, the
-// table with its first and last entry repeated, and D (tables of up to kTfDiff entries) the differences
-// P[j+1] - P[j], so that a lookup is one index, two 16-byte loads and four fmas, without clamping two indices.
+// The transfer function in shared memory as the kernels look it up: P holds tf_n + 2 entries, the table with its first
+// and last entry repeated, so that a lookup is one index and two 16-byte loads, without clamping two indices.  Shared
+// memory is taken from the L1, which the texels need: kernels whose CTAs fill an SM two at a time also keep D, the
+// differences P[j+1] - P[j] (tables of up to kTfDiff entries), the others form them at the lookup.  (8 CTAs with 1000
+// entries and their differences each left no L1: 606 -> 1197 us for level 3, depths 3-7, at 1920x1080.)
 constexpr uint32_t kTfDiff = 1024;
 struct TfTable {
     const float4* p;
-    const float4* d; // nullptr: a larger table, the difference formed at the lookup
+    const float4* d; // nullptr: the difference is formed at the lookup
     __device__ const float4* raw() const { return p + 1; }
 };
-inline __host__ __device__ uint32_t tf_smem_entries(uint32_t tf_n)
+inline __host__ __device__ uint32_t tf_smem_entries(uint32_t tf_n, bool diff)
 {
-    return tf_n <= kTfDiff ? 2 * tf_n + 3 : tf_n + 2;
+    return diff && tf_n <= kTfDiff ? 2 * tf_n + 3 : tf_n + 2;
 }
 
 // All threads of the CTA; ends with a barrier.
+template <bool kDiff>
 __device__ __forceinline__ TfTable load_tf(float4* sm, const float* tf, uint32_t tf_n, uint32_t tid, uint32_t nthreads)
 {
     const float4* g = reinterpret_cast<const float4*>(tf);
-    const bool diff = tf_n <= kTfDiff;
+    const bool diff = kDiff && tf_n <= kTfDiff;
     for (uint32_t j = tid; j < tf_n + 2; j += nthreads) {
         const float4 a = g[min(max((int)j - 1, 0), (int)tf_n - 1)];
         sm[j] = a;
@@ -874,7 +877,7 @@ __global__ void render_block_mode_kernel(const s3r_view v, const s3r_presentatio
                                          const float* __restrict__ tf_g, uint32_t* __restrict__ viewport)
 {
     extern __shared__ float4 tf_sm[];
-    const TfTable tf = load_tf(tf_sm, tf_g, v.tf_n, threadIdx.y * blockDim.x + threadIdx.x, blockDim.x * blockDim.y);
+    const TfTable tf = load_tf<false>(tf_sm, tf_g, v.tf_n, threadIdx.y * blockDim.x + threadIdx.x, blockDim.x * blockDim.y);
     const int32_t xx = blockIdx.x * blockDim.x + threadIdx.x;
     const int32_t yy = blockIdx.y * blockDim.y + threadIdx.y;
     if (xx >= rb.rect[2] || yy >= rb.rect[3]) return;
@@ -1027,7 +1030,7 @@ __global__ void part_blocks_kernel(const s3r_view v, const s3r_presentation pr, 
     const PartRef ref = a.refs[b];
     const RenderBlock rb = ref.rb;
     TfTable tf{nullptr, nullptr};
-    if constexpr (kFilter != 2) tf = load_tf(tf_sm, a.tf, v.tf_n, tid, blockDim.x * blockDim.y);
+    if constexpr (kFilter != 2) tf = load_tf<false>(tf_sm, a.tf, v.tf_n, tid, blockDim.x * blockDim.y);
     // the rows of the block's rectangle that fall into this strip of the part
     const int32_t y0 = max(rb.rect[1], a.y0), y1 = min(rb.rect[1] + rb.rect[3], a.y0 + a.h);
     const uint32_t tile = blockIdx.x - a.first[b];
@@ -1408,7 +1411,7 @@ __global__ void frame_render_kernel(FrameArgs fa)
             return;
         }
     }
-    const TfTable tf = load_tf(tf_sm, fa.tf, v.tf_n, tid, nthreads);
+    const TfTable tf = load_tf<false>(tf_sm, fa.tf, v.tf_n, tid, nthreads);
     const Relative rel = relative_of(v);
     uint32_t taken = 0;
     Premul acc{0.f, 0.f, 0.f, 0.f};
@@ -1522,6 +1525,26 @@ __device__ __forceinline__ uint32_t ray_rank(const float dir[3], uint32_t ix, ui
     return (dir[0] < 0.f ? m - 1 - ix : ix) + (dir[1] < 0.f ? m - 1 - iy : iy) + (dir[2] < 0.f ? m - 1 - iz : iz);
 }
 
+// Whether the per-ray walk (walk_blocks) meets this block on the ray, block_ray having found that the ray passes it.
+// It does wherever the middle of the ray's segment lies inside the block by more than the walk's rounding (its
+// crossing times are summed up over as many blocks as it has passed); only a ray that grazes the block -- along a
+// face, past an edge -- is walked to see which of the blocks around it the walk takes.
+__device__ __forceinline__ bool on_walk(const s3r_view& v, const float org[3], const float dir[3], const float inv[3],
+                                        const RenderBlock& rb, const BlockRay& r, uint32_t cell)
+{
+    const float tm = 0.5f * (r.tau_enter + r.tau_exit), room = rb.half - (2e-4f + 1e-5f * (float)(1u << v.level));
+    bool inside = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) inside &= fabsf(__fmaf_rn(dir[d], tm, org[d]) - rb.center[d]) < room;
+    if (inside) return true;
+    bool met = false;
+    walk_blocks(org, dir, inv, v.level, [&](uint32_t b) {
+        met = b == cell;
+        return !met;
+    });
+    return met;
+}
+
 // Block-major ray cast: the work items are the warp-sized pixel tiles of every
 // block's view rectangle, blocks in decreasing depth (most samples per ray
 // first); each warp of a persistent grid takes items from a work-queue counter on
@@ -1538,19 +1561,22 @@ __device__ __forceinline__ uint32_t ray_rank(const float dir[3], uint32_t ix, ui
 // share of a warp has 2, 4 or 8 lanes to a ray (SegArgs::items).  A kernel of its
 // own: with both marches in it the one with one lane to a ray has too few
 // registers (64 blocks of depth 6 at 1920x1080: 336 us instead of 278).
+constexpr uint32_t kSegThreads = 512; // warps on their own items, sharing a transfer-function table
 template <int Fmt, bool kTex, bool kLanes>
-__global__ void __launch_bounds__(128, 8) frame_segments_kernel(FrameArgs fa, SegArgs sa, uint32_t fx)
+__global__ void __launch_bounds__(kSegThreads, 2) frame_segments_kernel(FrameArgs fa, SegArgs sa, uint32_t fx)
 {
     extern __shared__ float4 tf_sm[];
     const s3r_view v = *fa.view;
     const uint32_t nthreads = blockDim.x * blockDim.y;
     const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const TfTable tf = load_tf(tf_sm, fa.tf, v.tf_n, tid, nthreads);
+    const TfTable tf = load_tf<true>(tf_sm, fa.tf, v.tf_n, tid, nthreads);
     const Relative rel = relative_of(v);
     const uint32_t lane = tid & 31u;
     const uint32_t total = *sa.count;
     const uint32_t m = 1u << v.level;
-    const uint64_t npix = (uint64_t)v.W * v.H;
+    const int4 cv = *reinterpret_cast<const int4*>(fa.cover);
+    const uint32_t cw = (uint32_t)(cv.z - cv.x);
+    const uint64_t npix = (uint64_t)cw * (uint32_t)(cv.w - cv.y);
     const float of = (v.threshold - v.field_min) / (v.field_max - v.field_min);
     uint32_t taken = 0;
     auto take = [&](uint32_t& item, uint2& desc) {
@@ -1588,6 +1614,7 @@ __global__ void __launch_bounds__(128, 8) frame_segments_kernel(FrameArgs fa, Se
             float inv[3];
             ray_inverse(dir, inv);
             hit = block_ray(v, org, dir, inv, *rb, r);
+            if (hit && sa.walk) hit = on_walk(v, org, dir, inv, *rb, r, cell);
         }
         const char* brick = reinterpret_cast<const char*>(fa.bricks) + rb->brick_off * (Fmt == S3R_BRICK_F32 ? 4 : 2);
         float scale = 1.f, offset = 0.f;
@@ -1608,7 +1635,7 @@ __global__ void __launch_bounds__(128, 8) frame_segments_kernel(FrameArgs fa, Se
         if (hit && !(acc.r == 0.f && acc.g == 0.f && acc.b == 0.f && acc.a == 0.f)) {
             const uint32_t ix = cell % m, iy = (cell / m) % m, iz = cell / (m * m);
             const uint32_t k = ray_rank(dir, ix, iy, iz, m);
-            const uint64_t pix = (uint64_t)y * v.W + (uint32_t)x;
+            const uint64_t pix = (uint64_t)(y - cv.y) * cw + (uint32_t)(x - cv.x);
             sa.seg[(uint64_t)k * npix + pix] = make_float4(acc.r, acc.g, acc.b, acc.a);
             atomicOr(&sa.mask[(uint64_t)(k >> 6) * npix + pix], 1ull << (k & 63));
         }
@@ -1630,15 +1657,20 @@ __global__ void __launch_bounds__(128, 8) frame_segments_kernel(FrameArgs fa, Se
 __global__ void frame_composite_kernel(FrameArgs fa, SegArgs sa)
 {
     const s3r_view v = *fa.view;
-    const uint64_t npix = (uint64_t)v.W * v.H;
-    const uint64_t pix = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (pix == 0) *sa.queue = 0u;
-    if (pix >= npix) return;
+    const uint64_t at = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (at == 0) *sa.queue = 0u;
+    if (at >= (uint64_t)v.W * v.H) return;
+    const uint32_t x = (uint32_t)(at % v.W), y = (uint32_t)(at / v.W);
+    const int4 cv = *reinterpret_cast<const int4*>(fa.cover);
+    const uint32_t cw = (uint32_t)(cv.z - cv.x);
+    const uint64_t npix = (uint64_t)cw * (uint32_t)(cv.w - cv.y);
+    const uint64_t pix = (uint64_t)((int32_t)y - cv.y) * cw + (uint32_t)((int32_t)x - cv.x);
+    const bool covered = (int32_t)x >= cv.x && (int32_t)x < cv.z && (int32_t)y >= cv.y && (int32_t)y < cv.w;
     unsigned long long bits[kSegMaskWords];
 #pragma unroll
     for (uint32_t w = 0; w < kSegMaskWords; ++w) {
         bits[w] = 0ull;
-        if (w < sa.words) {
+        if (covered && w < sa.words) {
             bits[w] = sa.mask[w * npix + pix];
             if (bits[w]) sa.mask[w * npix + pix] = 0ull;
         }
@@ -1657,7 +1689,7 @@ __global__ void frame_composite_kernel(FrameArgs fa, SegArgs sa)
             acc.a = __fmaf_rn(T, p.w, acc.a);
         }
     }
-    write_pixel(fa, v, (uint32_t)(pix % v.W), (uint32_t)(pix / v.W), acc);
+    write_pixel(fa, v, x, y, acc);
 }
 
 // Batched field modes (F32 bricks): one lane per ray walks the blocks front
@@ -1674,7 +1706,7 @@ __global__ void frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr
     const s3r_view v = *fa.view;
     const uint32_t nthreads = blockDim.x * blockDim.y;
     const uint32_t tid = threadIdx.y * blockDim.x + threadIdx.x;
-    const TfTable tf = load_tf(tf_sm, fa.tf, v.tf_n, tid, nthreads);
+    const TfTable tf = load_tf<false>(tf_sm, fa.tf, v.tf_n, tid, nthreads);
     const uint32_t vx = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t vy = blockIdx.y * blockDim.y + threadIdx.y;
     if (vx >= v.W || vy >= v.H) return;
@@ -1898,7 +1930,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 8) frame_backward_kernel(Fra
         reinterpret_cast<uint32_t*>(&view_sm)[i] = reinterpret_cast<const uint32_t*>(fa.view)[i];
     __syncthreads();
     const s3r_view& v = view_sm;
-    const TfTable tf = load_tf(sm, fa.tf, v.tf_n, tid, kBackwardThreads);
+    const TfTable tf = load_tf<false>(sm, fa.tf, v.tf_n, tid, kBackwardThreads);
     // The transfer-function gradient goes to one of kDtfParts copies in global
     // memory, an RGBA float4 reduction per table entry (fire and forget).  The copy
     // is picked by CTA (modulo kDtfCtaGroups) and by lane (modulo kDtfLaneGroups):
@@ -2120,7 +2152,7 @@ cudaError_t launch_render_block_mode(const s3r_view* view_host, const s3r_presen
     if (rb.rect[2] <= 0 || rb.rect[3] <= 0) return cudaSuccess;
     dim3 block(16, 8);
     dim3 grid((rb.rect[2] + 15) / 16, (rb.rect[3] + 7) / 8);
-    const size_t smem = tf_smem_entries(view_host->tf_n) * sizeof(float4);
+    const size_t smem = tf_smem_entries(view_host->tf_n, false) * sizeof(float4);
     if (view_host->filter == S3R_FILTER_TEXTURE)
         render_block_mode_kernel<true, -1><<<grid, block, smem, s>>>(*view_host, *pres, brick, brick2, rb, tf, viewport);
     else if (pres->mode == S3R_MODE_ARGB)
@@ -2146,7 +2178,7 @@ cudaError_t launch_part(const s3r_view* view_host, const s3r_presentation* pres,
     uint32_t tw, th;
     part_tile(pres->mode, texture, tw, th);
     const dim3 block(tw, th);
-    const size_t smem = texture ? 0 : tf_smem_entries(view_host->tf_n) * sizeof(float4);
+    const size_t smem = texture ? 0 : tf_smem_entries(view_host->tf_n, false) * sizeof(float4);
     with_mode(pres->mode, [&](auto mode) {
         constexpr int m = decltype(mode)::value;
         if (texture) part_blocks_kernel<2, m><<<ctas, block, 0, s>>>(*view_host, *pres, a);
@@ -2204,7 +2236,7 @@ cudaError_t launch_frame_render(const FrameArgs& a, uint32_t W, uint32_t H, uint
     const int px = sx / (int)R > 0 ? sx / (int)R : 1;
     dim3 block(px * R, sy);
     dim3 grid((W + px - 1) / px, (H + sy - 1) / sy);
-    const size_t smem = tf_smem_entries(tf_n) * sizeof(float4);
+    const size_t smem = tf_smem_entries(tf_n, false) * sizeof(float4);
     const bool tex = filter == S3R_FILTER_TEXTURE;
     switch (fmt) {
     case S3R_BRICK_F32:
@@ -2242,8 +2274,8 @@ cudaError_t launch_frame_segments(const FrameArgs& a, const SegArgs& sa, uint32_
     if (sa.words > kSegMaskWords) return cudaErrorInvalidValue;
     shape %= kSegShapes;
     const uint32_t fx = (uint32_t)kSegShapeX[shape];
-    const dim3 block(128); // four warps, each on its own items
-    const size_t smem = tf_smem_entries(tf_n) * sizeof(float4);
+    const dim3 block(kSegThreads);
+    const size_t smem = tf_smem_entries(tf_n, true) * sizeof(float4);
     const bool tex = filter == S3R_FILTER_TEXTURE;
     cudaError_t err;
     switch (fmt) {
@@ -2272,7 +2304,7 @@ cudaError_t launch_frame_render_mode(const FrameArgs& a, const s3r_presentation&
 {
     dim3 block(16, 8);
     dim3 grid((W + 15) / 16, (H + 7) / 8);
-    const size_t smem = tf_smem_entries(tf_n) * sizeof(float4);
+    const size_t smem = tf_smem_entries(tf_n, false) * sizeof(float4);
     if (filter == S3R_FILTER_TEXTURE) frame_render_mode_kernel<true><<<grid, block, smem, s>>>(a, pres, bricks2);
     else frame_render_mode_kernel<false><<<grid, block, smem, s>>>(a, pres, bricks2);
     return cudaGetLastError();
@@ -2284,7 +2316,7 @@ cudaError_t launch_frame_backward(const FrameArgs& a, uint32_t W, uint32_t H, ui
     // blocks of depth 6 at 512x512); larger CTAs leave more idle at the end, the rays' work being uneven
     dim3 block(8, 8);
     dim3 grid((W + 7) / 8, (H + 7) / 8);
-    const size_t smem = tf_smem_entries(tf_n) * sizeof(float4);
+    const size_t smem = tf_smem_entries(tf_n, false) * sizeof(float4);
     if (smem + sizeof(BackwardShared) > 47 * 1024) {
         cudaError_t err =
             cudaFuncSetAttribute(frame_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -159,9 +159,10 @@ struct SegArgs {
                                 // footprint-sized tiles of every block's view rectangle, deepest blocks first
     const uint32_t* count;      // items
     bool lanes;                 // some items have several lanes to a ray
+    bool walk;                  // only the blocks that the per-ray walk meets (render tiles below kRenderShapes)
     uint32_t words;             // mask words per pixel: ceil((3m - 2) / 64)
-    float4* seg;                // [rank][pixel] premultiplied block results
-    unsigned long long* mask;   // [word][pixel] ranks holding a result
+    float4* seg;                // [rank][covered pixel] premultiplied block results
+    unsigned long long* mask;   // [word][covered pixel] ranks holding a result
     uint32_t* queue;            // work-queue counter: 0 before the segment launch, zeroed again by the composite
 };
 
