@@ -463,53 +463,56 @@ __device__ __forceinline__ uint32_t rgba_to_argb(float4 c)
 // renderKernel<mode> with the reference's render functions (render*.hpp) and
 // lighting (cuda_lighting.hpp), on the plain form's ray set-up and sampling.
 
-// Field value at texel coordinate (x, y, z) -- the reference's fetch
-// coordinate -- filtered as kTex says; NaN where the filter gives NaN.
-template <bool kTex>
-__device__ __forceinline__ float field_at(const float* brick, Dim n, float x, float y, float z)
+// Trilinear value of 8 texels (x fastest, then y, then z) at the cell's fractions.
+__device__ __forceinline__ float lerp_cell(const float t[8], const float f[3])
 {
-    float val;
-    if constexpr (kTex) {
-        if (!tex_trilinear_at<S3R_BRICK_F32>(brick, n, x, y, z, val)) return __int_as_float(0x7fc00000);
-        return val;
+    const float x00 = __fmaf_rn(f[0], t[1] - t[0], t[0]);
+    const float x10 = __fmaf_rn(f[0], t[3] - t[2], t[2]);
+    const float x01 = __fmaf_rn(f[0], t[5] - t[4], t[4]);
+    const float x11 = __fmaf_rn(f[0], t[7] - t[6], t[6]);
+    const float y0 = __fmaf_rn(f[1], x10 - x00, x00);
+    const float y1 = __fmaf_rn(f[1], x11 - x01, x01);
+    return __fmaf_rn(f[2], y1 - y0, y0);
+}
+
+// The 8 texels and fractions of the exact filter at a texel coordinate -- the reference's fetch coordinate: loads
+// issued by fetch_cell, value (NaN where one texel is NaN) by cell_value.
+struct FieldCell {
+    float t[8], f[3];
+};
+__device__ __forceinline__ void fetch_cell(const float* brick, Dim n, float x, float y, float z, FieldCell& c)
+{
+    const uint32_t hi = n.n - 1;
+    const float tc[3] = {x, y, z};
+    int a[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const float xb = __fsub_rn(tc[d], 0.5f);
+        c.f[d] = __fsub_rn(xb, floor_small(xb, a[d]));
+    }
+    if ((uint32_t)a[0] < hi && (uint32_t)a[1] < hi && (uint32_t)a[2] < hi) {
+        // the cell lies in the brick: four pairs in four rows (32-bit offsets: a brick holds at most 513^3)
+        const uint32_t o = ((uint32_t)a[2] * n.n + (uint32_t)a[1]) * n.pitch + (uint32_t)a[0];
+        const uint32_t dz = n.n * n.pitch;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            c.t[q] = __ldg(brick + (uint64_t)(o + ((q & 2) ? n.pitch : 0u) + ((q & 4) ? dz : 0u)) + (q & 1));
     } else {
-        const uint32_t hi = n.n - 1;
-        const float tc[3] = {x, y, z};
-        int a[3];
-        float f[3], t[8];
+        uint32_t i0[3], i1[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const float xb = __fsub_rn(tc[d], 0.5f);
-            f[d] = __fsub_rn(xb, floor_small(xb, a[d]));
+            i0[d] = (uint32_t)min(max(a[d], 0), (int)hi);
+            i1[d] = (uint32_t)min(max(a[d], -1) + 1, (int)hi);
         }
-        if ((uint32_t)a[0] < hi && (uint32_t)a[1] < hi && (uint32_t)a[2] < hi) {
-            // the cell lies in the brick: four pairs in four rows (32-bit offsets: a brick holds at most 513^3)
-            const uint32_t o = ((uint32_t)a[2] * n.n + (uint32_t)a[1]) * n.pitch + (uint32_t)a[0];
-            const uint32_t dz = n.n * n.pitch;
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-                t[q] = __ldg(brick + (uint64_t)(o + ((q & 2) ? n.pitch : 0u) + ((q & 4) ? dz : 0u)) + (q & 1));
-        } else {
-            uint32_t i0[3], i1[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                i0[d] = (uint32_t)min(max(a[d], 0), (int)hi);
-                i1[d] = (uint32_t)min(max(a[d], -1) + 1, (int)hi);
-            }
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                t[q] = __ldg(brick + ((((q & 4) ? i1[2] : i0[2]) * n.n + ((q & 2) ? i1[1] : i0[1])) * n.pitch +
-                                      ((q & 1) ? i1[0] : i0[0])));
-        }
-        if (any_nan(t)) return __int_as_float(0x7fc00000);
-        const float x00 = __fmaf_rn(f[0], t[1] - t[0], t[0]);
-        const float x10 = __fmaf_rn(f[0], t[3] - t[2], t[2]);
-        const float x01 = __fmaf_rn(f[0], t[5] - t[4], t[4]);
-        const float x11 = __fmaf_rn(f[0], t[7] - t[6], t[6]);
-        const float y0 = __fmaf_rn(f[1], x10 - x00, x00);
-        const float y1 = __fmaf_rn(f[1], x11 - x01, x01);
-        return __fmaf_rn(f[2], y1 - y0, y0);
+        for (int q = 0; q < 8; ++q)
+            c.t[q] = __ldg(brick + ((((q & 4) ? i1[2] : i0[2]) * n.n + ((q & 2) ? i1[1] : i0[1])) * n.pitch +
+                                  ((q & 1) ? i1[0] : i0[0])));
     }
+}
+__device__ __forceinline__ float cell_value(const FieldCell& c)
+{
+    return any_nan(c.t) ? __int_as_float(0x7fc00000) : lerp_cell(c.t, c.f);
 }
 
 template <bool kTex> __device__ __forceinline__ float4 tf_rgba(const TfTable& tf, uint32_t tfn, float v01)
@@ -551,7 +554,8 @@ __device__ __forceinline__ F3 blinn(F3 N, F3 V, F3 L, const s3r_light& light, F3
     return f3(light.ambient) + kd * f3(light.diffuse) * diff + F3{0.5f, 0.5f, 0.5f} * f3(light.specular) * spec;
 }
 
-// Where a field-mode march takes its samples from.
+// Where a field-mode march takes its samples from: fetch starts a sample's loads at a texel coordinate (from the
+// second field's brick, or the first's), value gives its field value, NaN outside the domain.
 //   BrickSampler<kTex>: linear bricks in HBM, filtered in software (kTex: the
 //     texture unit's rule, else exact trilinear); the table in shared memory.
 //   TextureSampler: the GPU's texture unit itself, as the reference samples --
@@ -572,9 +576,16 @@ template <bool kTex> struct BrickSampler {
     TfTable tf;
     uint32_t tfn;
     static constexpr bool kStepwise = kTex, kContracted = false;
-    __device__ float field(int second, float x, float y, float z) const
+    using Sample = std::conditional_t<kTex, float, FieldCell>;
+    __device__ void fetch(int second, F3 p, Sample& x) const
     {
-        return field_at<kTex>(second ? b2 : b1, n, x, y, z);
+        if constexpr (!kTex) fetch_cell(second ? b2 : b1, n, p.x, p.y, p.z, x);
+        else if (!tex_trilinear_at<S3R_BRICK_F32>(second ? b2 : b1, n, p.x, p.y, p.z, x)) x = __int_as_float(0x7fc00000);
+    }
+    static __device__ float value(const Sample& x)
+    {
+        if constexpr (kTex) return x;
+        else return cell_value(x);
     }
     __device__ float4 colour(float v01) const { return tf_rgba<kTex>(tf, tfn, v01); }
 };
@@ -582,10 +593,9 @@ template <bool kTex> struct BrickSampler {
 struct TextureSampler {
     cudaTextureObject_t t1, t2, tf;
     static constexpr bool kStepwise = true, kContracted = true;
-    __device__ float field(int second, float x, float y, float z) const
-    {
-        return tex3D<float>(second ? t2 : t1, x, y, z);
-    }
+    using Sample = float;
+    __device__ void fetch(int second, F3 p, Sample& x) const { x = tex3D<float>(second ? t2 : t1, p.x, p.y, p.z); }
+    static __device__ float value(const Sample& x) { return x; }
     __device__ float4 colour(float v01) const { return tex1D<float4>(tf, v01); }
 };
 
@@ -596,10 +606,13 @@ __device__ __forceinline__ float4 frag_color(const S& smp, float4 diffuse, F3 ey
                                              const s3r_presentation& pr)
 {
     constexpr float d = 0.1f;
-    const F3 a{smp.field(0, tc.x - d, tc.y, tc.z), smp.field(0, tc.x, tc.y - d, tc.z),
-               smp.field(0, tc.x, tc.y, tc.z - d)};
-    const F3 b{smp.field(0, tc.x + d, tc.y, tc.z), smp.field(0, tc.x, tc.y + d, tc.z),
-               smp.field(0, tc.x, tc.y, tc.z + d)};
+    auto field = [&](float x, float y, float z) {
+        typename S::Sample c;
+        smp.fetch(0, F3{x, y, z}, c);
+        return S::value(c);
+    };
+    const F3 a{field(tc.x - d, tc.y, tc.z), field(tc.x, tc.y - d, tc.z), field(tc.x, tc.y, tc.z - d)};
+    const F3 b{field(tc.x + d, tc.y, tc.z), field(tc.x, tc.y + d, tc.z), field(tc.x, tc.y, tc.z + d)};
     F3 N = normalize3(a - b);
     const F3 V = normalize3(eye - surf);
     F3 c{0.f, 0.f, 0.f};
@@ -710,9 +723,12 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
         return F3{__fmul_rn(__fsub_rn(p.x, r.origin[0]), r.factor), __fmul_rn(__fsub_rn(p.y, r.origin[1]), r.factor),
                   __fmul_rn(__fsub_rn(p.z, r.origin[2]), r.factor)};
     };
-    auto value = [&](int second, F3 p) {
-        const F3 tc = tc_of(p);
-        return smp.field(second, tc.x, tc.y, tc.z);
+    // the sample that comes next: its position and its loads in flight
+    F3 pn;
+    typename S::Sample ahead;
+    auto open = [&](int k) {
+        pn = pos_of(k);
+        smp.fetch(0, tc_of(pn), ahead);
     };
     constexpr float kMax = 0.996f; // AlphaThreshold / AlphaMaxThreshold
     // kMode >= 0: the mode is fixed at compile time (one kernel per mode, as renderKernel<mode> is), so
@@ -721,8 +737,14 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
     if (mode == S3R_MODE_MAX_INTENSITY) {
         // renderMaxIntensityProjection.hpp:30-50; the pixel holds float bits
         float maxv = v.field_min - span;
-        for (int i = 1; i < r.samples; ++i, advance()) {
-            const float val = value(0, pos_of(i - 1));
+        open(0);
+        for (int i = 1; i < r.samples; ++i) {
+            const typename S::Sample x = ahead;
+            if (i + 1 < r.samples) {
+                advance();
+                open(i);
+            }
+            const float val = S::value(x);
             if (val >= v.threshold && maxv < val) maxv = val;
         }
         if (maxv < v.field_min) return out;
@@ -740,9 +762,15 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
             dom = smp.colour(0.5f);
             dom.w = 1.f - powf(1.f - dom.w * of, il);
         }
-        for (int i = 1; i < r.samples; ++i, advance()) {
-            const F3 p = pos_of(i - 1);
-            const float val = value(0, p);
+        open(0);
+        for (int i = 1; i < r.samples; ++i) {
+            const F3 p = pn;
+            const typename S::Sample x = ahead;
+            if (i + 1 < r.samples) {
+                advance();
+                open(i);
+            }
+            const float val = S::value(x);
             if (isnan(val)) continue;
             float4 col;
             if (mode == S3R_MODE_DOMAIN_VOXELS) {
@@ -775,7 +803,9 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
     auto surface_colour = [&](float level, F3 xpos) {
         float4 dif;
         if (secondary) {
-            const float vs = value(1, xpos);
+            typename S::Sample x;
+            smp.fetch(1, tc_of(xpos), x);
+            const float vs = S::value(x);
             dif = smp.colour((vs - pr.secondary_min) / (pr.secondary_max - pr.secondary_min));
         } else {
             dif = smp.colour((level - v.field_min) / span);
@@ -789,13 +819,22 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
             return F3{__fadd_rn(p.x, __fmul_rn(step.x, t)), __fadd_rn(p.y, __fmul_rn(step.y, t)),
                       __fadd_rn(p.z, __fmul_rn(step.z, t))};
     };
-    float v1 = value(0, pos_of(0));
+    open(0);
+    float v1 = S::value(ahead);
+    if (r.samples > 1) {
+        advance();
+        open(1);
+    }
     if (!multi) {
         const float thr = v.threshold;
         for (int i = 1; i < r.samples; ++i) {
-            advance();
-            const F3 p = pos_of(i);
-            const float v2 = value(0, p);
+            const F3 p = pn;
+            const typename S::Sample x = ahead;
+            if (i + 1 < r.samples) {
+                advance();
+                open(i + 1);
+            }
+            const float v2 = S::value(x);
             if (!isnan(v1) && !isnan(v2) && (v1 - thr) * (v2 - thr) < 0.f) {
                 const float t = (thr - v1) / (v2 - v1);
                 blend_behind(acc, surface_colour(thr, xpos_of(p, t)));
@@ -807,9 +846,13 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
         // renderIsosurfaces.hpp:34-106 / renderValueOnIsosurfaces.hpp
         int iint = isnan(v1) ? -1 : find_interval(v1, pr.levels, nl);
         for (int i = 1; i < r.samples; ++i) {
-            advance();
-            const F3 p = pos_of(i);
-            const float v2 = value(0, p);
+            const F3 p = pn;
+            const typename S::Sample x = ahead;
+            if (i + 1 < r.samples) {
+                advance();
+                open(i + 1);
+            }
+            const float v2 = S::value(x);
             if (isnan(v2)) {
                 iint = -1;
                 v1 = __int_as_float(0x7fc00000);
@@ -1258,15 +1301,8 @@ __device__ __forceinline__ void fetch_texels(const void* brick, const BlockRay& 
 // Trilinear value of fetched texels; false when one of them is NaN (outside the domain).
 template <int Fmt> __device__ __forceinline__ bool filter_texels(const Texels<Fmt>& x, float& val)
 {
-    const float* t = x.t;
-    if (any_nan(t)) return false;
-    const float x00 = __fmaf_rn(x.f[0], t[1] - t[0], t[0]);
-    const float x10 = __fmaf_rn(x.f[0], t[3] - t[2], t[2]);
-    const float x01 = __fmaf_rn(x.f[0], t[5] - t[4], t[4]);
-    const float x11 = __fmaf_rn(x.f[0], t[7] - t[6], t[6]);
-    const float y0 = __fmaf_rn(x.f[1], x10 - x00, x00);
-    const float y1 = __fmaf_rn(x.f[1], x11 - x01, x01);
-    val = __fmaf_rn(x.f[2], y1 - y0, y0);
+    if (any_nan(x.t)) return false;
+    val = lerp_cell(x.t, x.f);
     return true;
 }
 
@@ -1699,8 +1735,9 @@ __global__ void frame_composite_kernel(FrameArgs fa, SegArgs sa)
 // no ARGB8 rounding between blocks, max intensity the maximum over the
 // blocks, and a multi-level mode without levels clears the pixel (what lies
 // behind the first block it meets is erased, as the per-block path erases it).
-template <bool kTex>
-__global__ void frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr, const float* __restrict__ bricks2)
+// A kernel per mode and filter, as renderKernel<mode> is: with the mode known at run time it needed 128 registers.
+template <bool kTex, int kMode>
+__global__ void __launch_bounds__(128, 4) frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr, const float* __restrict__ bricks2)
 {
     extern __shared__ float4 tf_sm[];
     const s3r_view v = *fa.view;
@@ -1710,7 +1747,7 @@ __global__ void frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr
     const uint32_t vx = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t vy = blockIdx.y * blockDim.y + threadIdx.y;
     if (vx >= v.W || vy >= v.H) return;
-    const bool mip = pr.mode == S3R_MODE_MAX_INTENSITY;
+    constexpr bool mip = kMode == S3R_MODE_MAX_INTENSITY;
     Premul acc{0.f, 0.f, 0.f, 0.f};
     bool have_max = false;
     float best = 0.f;
@@ -1732,7 +1769,7 @@ __global__ void frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr
             if (!block_ray(v, org, dir, inv, *rb, r)) return true;
             const BrickSampler<kTex> smp{bricks + rb->brick_off, bricks2 ? bricks2 + rb->brick_off : nullptr, dim_of(r),
                                          tf, v.tf_n};
-            const ModeOut o = march_block_mode(v, pr, smp, r, depth);
+            const ModeOut o = march_block_mode<BrickSampler<kTex>, kMode>(v, pr, smp, r, depth);
             if (o.kind == ModeOut::kMax) {
                 if (!have_max || o.t > best) best = o.t;
                 have_max = true;
@@ -1764,13 +1801,7 @@ __global__ void frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr
 __device__ __forceinline__ bool filter_cell(const float f[3], const float t[8], float& val)
 {
     if (any_nan(t)) return false;
-    const float x00 = __fmaf_rn(f[0], t[1] - t[0], t[0]);
-    const float x10 = __fmaf_rn(f[0], t[3] - t[2], t[2]);
-    const float x01 = __fmaf_rn(f[0], t[5] - t[4], t[4]);
-    const float x11 = __fmaf_rn(f[0], t[7] - t[6], t[6]);
-    const float y0 = __fmaf_rn(f[1], x10 - x00, x00);
-    const float y1 = __fmaf_rn(f[1], x11 - x01, x01);
-    val = __fmaf_rn(f[2], y1 - y0, y0);
+    val = lerp_cell(t, f);
     return true;
 }
 
@@ -2302,11 +2333,14 @@ cudaError_t launch_frame_segments(const FrameArgs& a, const SegArgs& sa, uint32_
 cudaError_t launch_frame_render_mode(const FrameArgs& a, const s3r_presentation& pres, const float* bricks2,
                                      uint32_t W, uint32_t H, uint32_t tf_n, uint32_t filter, cudaStream_t s)
 {
-    dim3 block(16, 8);
-    dim3 grid((W + 15) / 16, (H + 7) / 8);
+    const dim3 block(8, 16); // 8 x 4 pixels a warp
+    const dim3 grid((W + 7) / 8, (H + 15) / 16);
     const size_t smem = tf_smem_entries(tf_n, false) * sizeof(float4);
-    if (filter == S3R_FILTER_TEXTURE) frame_render_mode_kernel<true><<<grid, block, smem, s>>>(a, pres, bricks2);
-    else frame_render_mode_kernel<false><<<grid, block, smem, s>>>(a, pres, bricks2);
+    with_mode(pres.mode, [&](auto mode) {
+        constexpr int m = decltype(mode)::value;
+        if (filter == S3R_FILTER_TEXTURE) frame_render_mode_kernel<true, m><<<grid, block, smem, s>>>(a, pres, bricks2);
+        else frame_render_mode_kernel<false, m><<<grid, block, smem, s>>>(a, pres, bricks2);
+    });
     return cudaGetLastError();
 }
 
