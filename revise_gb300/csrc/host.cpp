@@ -97,15 +97,21 @@ struct s3r_plan {
     void* bricks_1 = nullptr;
     float2* scale_offset_1 = nullptr;
     void* bricks = nullptr;
+    // what is staged with a view, one allocation and one copy: the table, the view, the cover and the block list
+    void* stage_dev = nullptr;
+    void* stage_pinned = nullptr;
+    size_t stage_bytes = 0;
     RenderBlock* table_dev = nullptr;
     s3r_view* view_dev = nullptr;
     int32_t* cover_dev = nullptr;    // union of the present blocks' view rectangles {x0, y0, x1, y1}
-    int32_t* cover_pinned = nullptr;
+    uint2* seg_list_dev = nullptr;   // the blocks' {key, first item}, deepest first, and {0, items}
     uint32_t grid_ctas = 0;
     // host render table (rects depend on the view)
     std::vector<RenderBlock> table_host;
     RenderBlock* table_pinned = nullptr;
     s3r_view* view_pinned = nullptr;
+    int32_t* cover_pinned = nullptr;
+    uint2* seg_list_pinned = nullptr;
     cudaEvent_t staged = nullptr;
     bool have_view = false;
     s3r_view last_view{};
@@ -113,21 +119,17 @@ struct s3r_plan {
     FrameGraph graphs[3];
     float* dtf_part = nullptr; // adjoint: kDtfParts copies of the transfer-function gradient
     size_t dtf_part_floats = 0;
-    // block-major render: the block cells deepest first, per item footprint the running tile counts over
-    // them (staged with the view), per data slot the per-rank block results and rank masks, and one
-    // work-queue counter per data slot
+    // block-major render: the block cells deepest first, the work items of the staged view, per data slot the
+    // per-rank block results and rank masks, and one work-queue counter per data slot
     std::vector<uint32_t> seg_order;
-    uint2* seg_items_pinned = nullptr;  // {cell, tile} per warp work item, staged with the view
-    uint2* seg_items_dev = nullptr;
-    uint64_t seg_items_cap = 0, seg_items_dev_cap = 0;
-    uint32_t* seg_count_pinned = nullptr;
-    uint32_t* seg_count_dev = nullptr;  // items staged
+    uint2* seg_items_dev = nullptr;     // SegArgs::items, expanded from the block list
+    uint64_t seg_items_cap = 0;
     int staged_tile = -1;               // the render tile the view is staged for (-1: the table alone)
     bool seg_now = false;               // the staged view renders block-major
     bool seg_lanes = false;             // some of them have several lanes to a ray
     uint32_t* seg_queue = nullptr;      // 2 counters
     float4* seg_buf[2] = {nullptr, nullptr};
-    unsigned long long* seg_mask[2] = {nullptr, nullptr};
+    unsigned long long* seg_mask[2] = {nullptr, nullptr}; // behind seg_buf, in its allocation
     uint64_t seg_pixels = 0;            // pixels the buffers hold
     uint32_t seg_words = 0;
     // s3r_frame_run_host: per slot a device copy of the frame's sparse values and its image, and the
@@ -742,7 +744,6 @@ void plan_free_segments(s3r_plan* p)
 {
     for (int b = 0; b < 2; ++b) {
         if (p->seg_buf[b]) cudaFree(p->seg_buf[b]);
-        if (p->seg_mask[b]) cudaFree(p->seg_mask[b]);
         p->seg_buf[b] = nullptr;
         p->seg_mask[b] = nullptr;
     }
@@ -757,16 +758,19 @@ int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t most)
     const int slots = p->hs_h2d ? 2 : 1; // the second one only for the host-buffer pipeline
     const uint32_t words = (3 * (1u << p->level) - 2 + 63) / 64;
     if (p->seg_buf[slots - 1] && p->seg_pixels >= npix) return S3R_OK;
-    S3R_CUDA(ctx, cudaDeviceSynchronize());
+    if (p->seg_buf[0]) S3R_CUDA(ctx, cudaDeviceSynchronize()); // frames in flight
     // some room to move closer in, up to the whole viewport
     npix = std::max(p->seg_pixels, std::min(npix + npix / 2, most));
     plan_free_segments(p);
     plan_drop_graph(p);
     for (int b = 0; b < slots; ++b) {
-        cudaError_t e;
-        if ((e = cudaMalloc(&p->seg_buf[b], npix * seg_pixel_bytes(p))) != cudaSuccess ||
-            (e = cudaMalloc(&p->seg_mask[b], (size_t)words * npix * sizeof(unsigned long long))) != cudaSuccess ||
-            (e = cudaMemset(p->seg_mask[b], 0, (size_t)words * npix * sizeof(unsigned long long))) != cudaSuccess) {
+        const size_t results = npix * seg_pixel_bytes(p), masks = (size_t)words * npix * sizeof(unsigned long long);
+        cudaError_t e = cudaMalloc(&p->seg_buf[b], results + masks);
+        if (e == cudaSuccess) {
+            p->seg_mask[b] = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(p->seg_buf[b]) + results);
+            e = cudaMemset(p->seg_mask[b], 0, masks);
+        }
+        if (e != cudaSuccess) {
             plan_free_segments(p);
             (void)cudaGetLastError(); // an allocation failure leaves no error behind for later launches
             return cuda_fail(ctx, e, "cudaMalloc(block-major render buffers)");
@@ -914,53 +918,37 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
         uint64_t n = 0;
         p->seg_lanes = false;
         for (uint32_t i = 0; i < p->nblocks; ++i) {
-            const RenderBlock& t = tb[p->seg_order[i]];
+            const uint32_t cell = p->seg_order[i];
+            const RenderBlock& t = tb[cell];
             const uint64_t tiles = tiles_of(t);
+            p->seg_list_pinned[i] = make_uint2(cell | log_lanes[t.depth] << kSegLanesShift, (uint32_t)n);
             n += tiles;
             p->seg_lanes |= tiles > 0 && log_lanes[t.depth] > 0;
         }
+        p->seg_list_pinned[p->nblocks] = make_uint2(0, (uint32_t)n);
         if (n > 0xffffffffull) return fail(ctx, S3R_ERR_INVALID, "too many block-major render items");
-        cudaError_t e;
         if (n > p->seg_items_cap) {
-            if (p->seg_items_pinned) cudaFreeHost(p->seg_items_pinned);
-            p->seg_items_pinned = nullptr;
-            p->seg_items_cap = 0;
-            if ((e = cudaMallocHost(&p->seg_items_pinned, n * sizeof(uint2))) != cudaSuccess)
-                return cuda_fail(ctx, e, "cudaMallocHost(block-major items)");
-            p->seg_items_cap = n;
-        }
-        if (n > p->seg_items_dev_cap) {
             // frames in flight or captured may hold the old list
-            S3R_CUDA(ctx, cudaDeviceSynchronize());
+            if (p->seg_items_dev) S3R_CUDA(ctx, cudaDeviceSynchronize());
             plan_drop_graph(p);
             if (p->seg_items_dev) cudaFree(p->seg_items_dev);
             p->seg_items_dev = nullptr;
-            p->seg_items_dev_cap = 0;
-            if ((e = cudaMalloc(&p->seg_items_dev, n * sizeof(uint2))) != cudaSuccess)
-                return cuda_fail(ctx, e, "cudaMalloc(block-major items)");
-            p->seg_items_dev_cap = n;
+            p->seg_items_cap = 0;
+            const uint64_t cap = n + n / 4; // some room for other views
+            const cudaError_t e = cudaMalloc(&p->seg_items_dev, cap * sizeof(uint2));
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(block-major items)");
+            p->seg_items_cap = cap;
         }
-        uint2* it = p->seg_items_pinned;
-        for (uint32_t i = 0; i < p->nblocks; ++i) {
-            const uint32_t cell = p->seg_order[i];
-            const uint32_t tiles = (uint32_t)tiles_of(tb[cell]);
-            const uint32_t key = cell | log_lanes[tb[cell].depth] << kSegLanesShift;
-            for (uint32_t t = 0; t < tiles; ++t) *it++ = make_uint2(key, t);
-        }
-        *p->seg_count_pinned = (uint32_t)n;
-        if (n) S3R_CUDA(ctx, cudaMemcpyAsync(p->seg_items_dev, p->seg_items_pinned, n * sizeof(uint2),
-                                             cudaMemcpyHostToDevice, s));
-        S3R_CUDA(ctx, cudaMemcpyAsync(p->seg_count_dev, p->seg_count_pinned, sizeof(uint32_t), cudaMemcpyHostToDevice,
-                                      s));
     }
     p->staged_tile = frame ? (int)p->render_tile : -1;
     std::memcpy(p->cover_pinned, cover, sizeof(cover));
-    S3R_CUDA(ctx, cudaMemcpyAsync(p->cover_dev, p->cover_pinned, sizeof(cover), cudaMemcpyHostToDevice, s));
     *p->view_pinned = *view;
-    S3R_CUDA(ctx, cudaMemcpyAsync(p->table_dev, tb, sizeof(RenderBlock) * p->table_host.size(),
-                                  cudaMemcpyHostToDevice, s));
-    S3R_CUDA(ctx, cudaMemcpyAsync(p->view_dev, p->view_pinned, sizeof(s3r_view), cudaMemcpyHostToDevice, s));
+    S3R_CUDA(ctx, cudaMemcpyAsync(p->stage_dev, p->stage_pinned, p->stage_bytes, cudaMemcpyHostToDevice, s));
     S3R_CUDA(ctx, cudaEventRecord(p->staged, s));
+    if (seg) {
+        S3R_CUDA(ctx, launch_seg_items(p->seg_list_dev, p->nblocks, p->seg_items_dev, s));
+        ++ctx->launches;
+    }
     p->last_view = *view;
     p->have_view = true;
     return S3R_OK;
@@ -1027,7 +1015,7 @@ int plan_launch_render(s3r_plan* p, const float* tf, float* rgba, uint32_t* argb
         const uint32_t shape = asked ? p->render_tile - (uint32_t)kRenderWalkTiles : 0u;
         SegArgs sa{};
         sa.items = p->seg_items_dev;
-        sa.count = p->seg_count_dev;
+        sa.count = &p->seg_list_dev[p->nblocks].y;
         sa.lanes = p->seg_lanes;
         sa.walk = !asked;
         sa.words = p->seg_words;
@@ -1851,18 +1839,24 @@ int s3r_frame_plan(s3r_ctx* ctx, const s3r_frame_desc* desc, s3r_plan** out)
         return bail(cuda_fail(ctx, e, "cudaMalloc(queue)"));
     if ((e = cudaMalloc(&p->scale_offset_dev, sizeof(float2) * p->nblocks)) != cudaSuccess)
         return bail(cuda_fail(ctx, e, "cudaMalloc(scales)"));
-    if ((e = cudaMalloc(&p->table_dev, sizeof(RenderBlock) * p->table_host.size())) != cudaSuccess)
-        return bail(cuda_fail(ctx, e, "cudaMalloc(table)"));
-    if ((e = cudaMalloc(&p->view_dev, sizeof(s3r_view))) != cudaSuccess)
-        return bail(cuda_fail(ctx, e, "cudaMalloc(view)"));
-    if ((e = cudaMallocHost(&p->table_pinned, sizeof(RenderBlock) * p->table_host.size())) != cudaSuccess)
-        return bail(cuda_fail(ctx, e, "cudaMallocHost(table)"));
-    if ((e = cudaMallocHost(&p->view_pinned, sizeof(s3r_view))) != cudaSuccess)
-        return bail(cuda_fail(ctx, e, "cudaMallocHost(view)"));
-    if ((e = cudaMalloc(&p->cover_dev, 4 * sizeof(int32_t))) != cudaSuccess)
-        return bail(cuda_fail(ctx, e, "cudaMalloc(cover)"));
-    if ((e = cudaMallocHost(&p->cover_pinned, 4 * sizeof(int32_t))) != cudaSuccess)
-        return bail(cuda_fail(ctx, e, "cudaMallocHost(cover)"));
+    {
+        auto round = [](size_t n) { return (n + 255) & ~(size_t)255; };
+        const size_t view_off = round(sizeof(RenderBlock) * p->table_host.size()),
+                     cover_off = view_off + round(sizeof(s3r_view)), list_off = cover_off + 256;
+        p->stage_bytes = list_off + sizeof(uint2) * ((size_t)p->nblocks + 1);
+        if ((e = cudaMalloc(&p->stage_dev, p->stage_bytes)) != cudaSuccess ||
+            (e = cudaMallocHost(&p->stage_pinned, p->stage_bytes)) != cudaSuccess)
+            return bail(cuda_fail(ctx, e, "cudaMalloc(view and table)"));
+        auto place = [&](void* base, RenderBlock*& table, s3r_view*& view, int32_t*& cover, uint2*& list) {
+            char* c = static_cast<char*>(base);
+            table = reinterpret_cast<RenderBlock*>(c);
+            view = reinterpret_cast<s3r_view*>(c + view_off);
+            cover = reinterpret_cast<int32_t*>(c + cover_off);
+            list = reinterpret_cast<uint2*>(c + list_off);
+        };
+        place(p->stage_dev, p->table_dev, p->view_dev, p->cover_dev, p->seg_list_dev);
+        place(p->stage_pinned, p->table_pinned, p->view_pinned, p->cover_pinned, p->seg_list_pinned);
+    }
     if ((e = cudaEventCreateWithFlags(&p->staged, cudaEventDisableTiming)) != cudaSuccess)
         return bail(cuda_fail(ctx, e, "cudaEventCreate"));
     // block-major render: blocks deepest first (most samples per ray), so that the longest work items start first
@@ -1876,9 +1870,7 @@ int s3r_frame_plan(s3r_ctx* ctx, const s3r_frame_desc* desc, s3r_plan** out)
             const uint32_t* bl = &p->blocks[4 * idx[i]];
             p->seg_order[i] = bl[0] + m * (bl[1] + m * bl[2]);
         }
-        if ((e = cudaMalloc(&p->seg_count_dev, sizeof(uint32_t))) != cudaSuccess ||
-            (e = cudaMallocHost(&p->seg_count_pinned, sizeof(uint32_t))) != cudaSuccess ||
-            (e = cudaMalloc(&p->seg_queue, 2 * sizeof(uint32_t))) != cudaSuccess ||
+        if ((e = cudaMalloc(&p->seg_queue, 2 * sizeof(uint32_t))) != cudaSuccess ||
             (e = cudaMemset(p->seg_queue, 0, 2 * sizeof(uint32_t))) != cudaSuccess)
             return bail(cuda_fail(ctx, e, "cudaMalloc(block-major render)"));
     }
@@ -1903,18 +1895,11 @@ int s3r_plan_destroy(s3r_plan* p)
     f(p->node_off_dev);
     f(p->queue_dev);
     f(p->scale_offset_dev);
-    f(p->table_dev);
-    f(p->view_dev);
-    if (p->table_pinned) cudaFreeHost(p->table_pinned);
-    if (p->view_pinned) cudaFreeHost(p->view_pinned);
-    if (p->cover_pinned) cudaFreeHost(p->cover_pinned);
-    f(p->cover_dev);
+    f(p->stage_dev);
+    if (p->stage_pinned) cudaFreeHost(p->stage_pinned);
     f(p->dtf_part);
     f(p->seg_items_dev);
-    f(p->seg_count_dev);
     f(p->seg_queue);
-    if (p->seg_items_pinned) cudaFreeHost(p->seg_items_pinned);
-    if (p->seg_count_pinned) cudaFreeHost(p->seg_count_pinned);
     plan_free_segments(p);
     if (p->staged) cudaEventDestroy(p->staged);
     delete p;

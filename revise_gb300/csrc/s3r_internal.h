@@ -273,6 +273,8 @@ cudaError_t launch_frame_render(const FrameArgs& a, uint32_t W, uint32_t H, uint
 // the work items of footprint `shape`, then the composite kernel over all W x H pixels.
 cudaError_t launch_frame_segments(const FrameArgs& a, const SegArgs& sa, uint32_t W, uint32_t H, uint32_t tf_n,
                                   uint32_t fmt, uint32_t shape, uint32_t filter, uint32_t sms, cudaStream_t s);
+// Expands the staged block list {key, first item}, closed by {0, items}, to SegArgs::items.
+cudaError_t launch_seg_items(const uint2* list, uint32_t nblocks, uint2* items, cudaStream_t s);
 cudaError_t launch_frame_render_mode(const FrameArgs& a, const s3r_presentation& pres, const float* bricks2,
                                      uint32_t W, uint32_t H, uint32_t tf_n, uint32_t filter, cudaStream_t s);
 cudaError_t launch_frame_backward(const FrameArgs& a, uint32_t W, uint32_t H, uint32_t tf_n, cudaStream_t s);
