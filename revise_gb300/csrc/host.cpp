@@ -67,6 +67,7 @@ struct s3r_plan {
     s3r_ctx* ctx = nullptr;
     s3r_frame_desc desc{};
     uint32_t nblocks = 0, level = 0, fmt = 0;
+    uint32_t max_nodes = 0; // of one block
     uint32_t tile_log2 = 4;             // the largest tile edge (log2 cells) over the blocks
     uint8_t tile_by_depth[S3R_MAX_DEPTH + 1] = {}; // per block depth: its tile edge (log2), capped by the depth
     uint32_t render_tile = 0;
@@ -969,7 +970,7 @@ int plan_launch_interp(s3r_plan* p, const float* sparse, cudaStream_t s, uint32_
         pa.coarse = p->coarse_dev[slot ? 1 : 0];
         pa.centry_off = p->centry_off_dev;
         pa.centry = p->centry_dev;
-        S3R_CUDA(ctx, launch_block_prep(pa, p->nblocks, s));
+        S3R_CUDA(ctx, launch_block_prep(pa, p->nblocks, p->max_nodes, (uint32_t)ctx->sms, s));
         ++*kernels;
     }
     TileArgs a{};
@@ -1813,6 +1814,7 @@ int s3r_frame_plan(s3r_ctx* ctx, const s3r_frame_desc* desc, s3r_plan** out)
         if (p->node_off[b + 1] < p->node_off[b]) return bail(fail(ctx, S3R_ERR_INVALID, "node offsets decrease"));
         if (p->node_off[b + 1] - p->node_off[b] > 0xffffffffull)
             return bail(fail(ctx, S3R_ERR_INVALID, "too many nodes in one block"));
+        p->max_nodes = std::max(p->max_nodes, (uint32_t)(p->node_off[b + 1] - p->node_off[b]));
         const uint64_t e = (1ull << bl[3]) + 1;
         const uint32_t pitch = plan_brick_pitch(bl[3], elem_bytes);
         p->pitch[b] = pitch;

@@ -214,79 +214,51 @@ template <typename OutT> __global__ void __launch_bounds__(kInterpThreads, 8) in
     }
 }
 
-// Per block {scale, offset} of its valid sparse values (16-bit bricks). All
-// dense values are means of sparse values, so they stay inside this range.
-__global__ void block_range_kernel(const PlanBlock* blocks, const uint64_t* node_off, const float* sparse,
-                                   float2* so)
-{
-    const uint32_t b = blockIdx.x;
-    const uint64_t n0 = node_off[b], n1 = node_off[b + 1];
-    float lo = INFINITY, hi = -INFINITY;
-    for (uint64_t i = n0 + threadIdx.x; i < n1; i += blockDim.x) {
-        const float v = sparse[i];
-        if (v != kNoField && !isnan(v)) {
-            lo = fminf(lo, v);
-            hi = fmaxf(hi, v);
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    __shared__ float slo[32], shi[32];
-    const uint32_t w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
-        slo[w] = lo;
-        shi[w] = hi;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (uint32_t i = 1; i < blockDim.x / 32; ++i) {
-            lo = fminf(lo, slo[i]);
-            hi = fmaxf(hi, shi[i]);
-        }
-        float scale = hi - lo;
-        if (!(scale > 0.f) || !isfinite(scale)) scale = 1.f;
-        if (!isfinite(lo)) lo = 0.f;
-        so[b] = make_float2(scale, lo);
-    }
-}
-
-// Per-block preparation of a plan frame, one CTA of kInterpThreads per block:
-//  * 16-bit bricks: the {scale, offset} of the block's valid sparse values (as block_range_kernel);
+// Per-block preparation of a plan frame, one CTA per block:
+//  * 16-bit bricks: the {scale, offset} of the block's valid sparse values; all dense values are means of
+//    sparse values, so they stay inside this range;
 //  * a block cut into 2^L > 1 tiles per axis: its coarse grid, the (2^L+1)^3 vertices at multiples of
-//    the tile edge, from the sparse nodes on it, filled level by level exactly as cube_level fills a
-//    tile (the reference's midpoint rules, sums in its order).  A midpoint of a coarse level depends
-//    only on the points of that level's cube, so the full grid holds the values a descent from the
-//    block's root along any one tile's path computes -- each tile then reads its 8 corners from it
-//    instead of descending itself, and the plan carries the coarse nodes once per block instead of
-//    once per tile.
-__global__ void __launch_bounds__(kInterpThreads) block_prep_kernel(PrepArgs a)
+//    the tile edge, from the sparse nodes on it, filled level by level exactly as a tile is filled (the
+//    reference's midpoint rules, sums in its order).  A midpoint of a coarse level depends only on the
+//    points of that level's cube, so the full grid holds the values a descent from the block's root
+//    along any one tile's path computes -- each tile then reads its 8 corners from it instead of
+//    descending itself, and the plan carries the coarse nodes once per block instead of once per tile.
+// What bounds it is latency: the rounds of a thread's loads of the values and the levels of the coarse grid.  So 8
+// loads are in flight, grids of up to 9^3 are filled in shared memory, and few blocks of many nodes get wider CTAs
+// (launch_block_prep).
+constexpr uint32_t kPrepGrid = 9 * 9 * 9;
+__global__ void __launch_bounds__(1024) block_prep_kernel(PrepArgs a)
 {
-    const uint32_t b = blockIdx.x;
+    __shared__ float s_grid[kPrepGrid];
+    __shared__ float slo[32], shi[32];
+    const uint32_t b = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
     const PlanBlock B = a.blocks[b];
+    const uint32_t L = B.coarse_log2, T = 1u << L, E = T + 1, E3 = E * E * E;
     if (a.scale_offset) {
         const uint64_t n0 = a.node_off[b], n1 = a.node_off[b + 1];
         float lo = INFINITY, hi = -INFINITY;
-        for (uint64_t i = n0 + threadIdx.x; i < n1; i += kInterpThreads) {
-            const float v = a.sparse[i];
-            if (v != kNoField && !isnan(v)) {
-                lo = fminf(lo, v);
-                hi = fmaxf(hi, v);
-            }
+        for (uint64_t i = n0 + tid; i < n1; i += 8 * nt) {
+            float v[8];
+#pragma unroll
+            for (uint32_t q = 0; q < 8; ++q) v[q] = i + q * nt < n1 ? a.sparse[i + q * nt] : kNoField;
+#pragma unroll
+            for (uint32_t q = 0; q < 8; ++q)
+                if (v[q] != kNoField) { // a NaN changes neither
+                    lo = fminf(lo, v[q]);
+                    hi = fmaxf(hi, v[q]);
+                }
         }
         for (int o = 16; o > 0; o >>= 1) {
             lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
             hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
         }
-        __shared__ float slo[kInterpThreads / 32], shi[kInterpThreads / 32];
-        if ((threadIdx.x & 31) == 0) {
-            slo[threadIdx.x >> 5] = lo;
-            shi[threadIdx.x >> 5] = hi;
+        if ((tid & 31) == 0) {
+            slo[tid >> 5] = lo;
+            shi[tid >> 5] = hi;
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            for (uint32_t i = 1; i < kInterpThreads / 32; ++i) {
+        if (tid == 0) {
+            for (uint32_t i = 1; i < nt / 32; ++i) {
                 lo = fminf(lo, slo[i]);
                 hi = fmaxf(hi, shi[i]);
             }
@@ -296,20 +268,26 @@ __global__ void __launch_bounds__(kInterpThreads) block_prep_kernel(PrepArgs a)
             a.scale_offset[b] = make_float2(scale, lo);
         }
     }
-    const uint32_t L = B.coarse_log2;
     if (L == 0) return;
-    const uint32_t T = 1u << L, E = T + 1, E3 = E * E * E;
-    float* g = a.coarse + B.coarse_off;
-    for (uint32_t p = threadIdx.x; p < E3; p += kInterpThreads) g[p] = qnan();
-    __syncthreads();
-    for (uint32_t i = a.centry_off[b] + threadIdx.x; i < a.centry_off[b + 1]; i += kInterpThreads) {
-        const uint2 ce = a.centry[i];
-        if (ce.x < E3) g[ce.x] = to_internal(a.sparse[B.node_base + ce.y]);
-    }
-    __syncthreads();
-    for (uint32_t j = 0; j < L; ++j) {
-        cube_level(g, E, T, j);
+    auto fill = [&](float* g) {
+        for (uint32_t p = tid; p < E3; p += nt) g[p] = qnan();
         __syncthreads();
+        for (uint32_t i = a.centry_off[b] + tid; i < a.centry_off[b + 1]; i += nt) {
+            const uint2 ce = a.centry[i];
+            if (ce.x < E3) g[ce.x] = to_internal(a.sparse[B.node_base + ce.y]);
+        }
+        __syncthreads();
+        for (uint32_t j = 0; j < L; ++j) {
+            cube_level(g, E, T, j);
+            __syncthreads();
+        }
+    };
+    float* out = a.coarse + B.coarse_off;
+    if (E3 <= kPrepGrid) {
+        fill(s_grid);
+        for (uint32_t p = tid; p < E3; p += nt) out[p] = s_grid[p];
+    } else {
+        fill(out);
     }
 }
 
@@ -410,18 +388,15 @@ cudaError_t launch_interp_plan(const TileArgs& a, uint32_t fmt, uint32_t tile_lo
     }
 }
 
-cudaError_t launch_block_prep(const PrepArgs& a, uint32_t nblocks, cudaStream_t s)
+// Wider CTAs while every block's is resident at once and a thread is left two rounds of loads.
+cudaError_t launch_block_prep(const PrepArgs& a, uint32_t nblocks, uint32_t max_nodes, uint32_t sms, cudaStream_t s)
 {
     if (nblocks == 0) return cudaSuccess;
-    block_prep_kernel<<<nblocks, kInterpThreads, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_block_ranges(const PlanBlock* blocks, uint32_t nblocks, const float* sparse,
-                                const uint64_t* node_off_dev, float2* scale_offset, cudaStream_t s)
-{
-    if (nblocks == 0) return cudaSuccess;
-    block_range_kernel<<<nblocks, 256, 0, s>>>(blocks, node_off_dev, sparse, scale_offset);
+    uint32_t threads = kInterpThreads;
+    if (a.scale_offset)
+        while (threads < 1024 && 2 * threads * 16 <= max_nodes && (uint64_t)nblocks * 2 * threads <= 2048ull * sms)
+            threads *= 2;
+    block_prep_kernel<<<nblocks, threads, 0, s>>>(a);
     return cudaGetLastError();
 }
 

@@ -203,7 +203,7 @@ __device__ __forceinline__ void cube_level(float* s, uint32_t E, uint32_t T, uin
     const uint32_t st0 = hs, st1 = E * hs, st2 = E * E * hs;
     const uint32_t ncubes = 1u << (3 * j);
 #pragma unroll 1
-    for (uint32_t c = threadIdx.x; c < ncubes; c += kInterpThreads) {
+    for (uint32_t c = threadIdx.x; c < ncubes; c += blockDim.x) {
         const uint32_t ci = c & (m - 1), cj = (c >> j) & (m - 1), ck = c >> (2 * j);
         const uint32_t base = ci * sz + E * (cj * sz + E * (ck * sz));
         float v[27];

@@ -230,9 +230,8 @@ struct PrepArgs {
     const uint32_t* centry_off;   // nblocks + 1: the sparse nodes on each block's coarse grid
     const uint2* centry;          // {coarse grid index, node index within the block}
 };
-cudaError_t launch_block_prep(const PrepArgs& a, uint32_t nblocks, cudaStream_t s);
-cudaError_t launch_block_ranges(const PlanBlock* blocks, uint32_t nblocks, const float* sparse,
-                                const uint64_t* node_off_dev, float2* scale_offset, cudaStream_t s);
+// max_nodes: of one block, at most.
+cudaError_t launch_block_prep(const PrepArgs& a, uint32_t nblocks, uint32_t max_nodes, uint32_t sms, cudaStream_t s);
 
 // One block in any field mode (pres) sampled through the texture unit: field / field2 / tf_tex are
 // cudaTextureObject_t handles (3-D float field arrays, 1-D RGBA transfer-function array).
