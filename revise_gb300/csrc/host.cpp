@@ -123,14 +123,14 @@ struct s3r_plan {
     // block-major render: the block cells deepest first, the work items of the staged view, per data slot the
     // per-rank block results and rank masks, and one work-queue counter per data slot
     std::vector<uint32_t> seg_order;
-    uint2* seg_items_dev = nullptr;     // SegArgs::items, expanded from the block list
-    uint64_t seg_items_cap = 0;
     int staged_tile = -1;               // the render tile the view is staged for (-1: the table alone)
     bool seg_now = false;               // the staged view renders block-major
     bool seg_lanes = false;             // some of them have several lanes to a ray
     uint32_t* seg_queue = nullptr;      // 2 counters
     float4* seg_buf[2] = {nullptr, nullptr};
     unsigned long long* seg_mask[2] = {nullptr, nullptr}; // behind seg_buf, in its allocation
+    uint2* seg_items_dev = nullptr;     // SegArgs::items, expanded from the block list; behind seg_mask[0]
+    uint64_t seg_items_cap = 0;
     uint64_t seg_pixels = 0;            // pixels the buffers hold
     uint32_t seg_words = 0;
     // s3r_frame_run_host: per slot a device copy of the frame's sparse values and its image, and the
@@ -738,9 +738,9 @@ int plan_bin(s3r_plan* p, uint32_t tile_log2, const uint8_t* by_depth = nullptr)
     return S3R_OK;
 }
 
-// The block-major render's per-rank results and rank masks for `npix` covered pixels in data slots 0 .. slots-1;
-// called before a frame is launched (or captured) in the block-major form.  Reallocation drops the captured frames
-// (they hold the old buffers).
+// The block-major render's per-rank results and rank masks for `npix` covered pixels in data slots 0 .. slots-1, and
+// room for `items` work items; called before a frame is launched (or captured) in the block-major form.  Reallocation
+// drops the captured frames (they hold the old buffers).
 void plan_free_segments(s3r_plan* p)
 {
     for (int b = 0; b < 2; ++b) {
@@ -748,28 +748,32 @@ void plan_free_segments(s3r_plan* p)
         p->seg_buf[b] = nullptr;
         p->seg_mask[b] = nullptr;
     }
-    p->seg_pixels = 0;
+    p->seg_items_dev = nullptr;
+    p->seg_pixels = p->seg_items_cap = 0;
 }
 
 uint64_t seg_pixel_bytes(const s3r_plan* p) { return (3ull * (1u << p->level) - 2) * sizeof(float4); }
 
-int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t most)
+int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t most, uint64_t items)
 {
     s3r_ctx* ctx = p->ctx;
     const int slots = p->hs_h2d ? 2 : 1; // the second one only for the host-buffer pipeline
     const uint32_t words = (3 * (1u << p->level) - 2 + 63) / 64;
-    if (p->seg_buf[slots - 1] && p->seg_pixels >= npix) return S3R_OK;
+    if (p->seg_buf[slots - 1] && p->seg_pixels >= npix && p->seg_items_cap >= items) return S3R_OK;
     if (p->seg_buf[0]) S3R_CUDA(ctx, cudaDeviceSynchronize()); // frames in flight
     // some room to move closer in, up to the whole viewport
-    npix = std::max(p->seg_pixels, std::min(npix + npix / 2, most));
+    npix = p->seg_pixels >= npix ? p->seg_pixels : std::max(p->seg_pixels, std::min(npix + npix / 2, most));
+    items = p->seg_items_cap >= items ? p->seg_items_cap : items + items / 4;
     plan_free_segments(p);
     plan_drop_graph(p);
     for (int b = 0; b < slots; ++b) {
         const size_t results = npix * seg_pixel_bytes(p), masks = (size_t)words * npix * sizeof(unsigned long long);
-        cudaError_t e = cudaMalloc(&p->seg_buf[b], results + masks);
+        cudaError_t e = cudaMalloc(&p->seg_buf[b], results + masks + (b ? 0 : items * sizeof(uint2)));
         if (e == cudaSuccess) {
-            p->seg_mask[b] = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(p->seg_buf[b]) + results);
-            e = cudaMemset(p->seg_mask[b], 0, masks);
+            char* mask = reinterpret_cast<char*>(p->seg_buf[b]) + results;
+            p->seg_mask[b] = reinterpret_cast<unsigned long long*>(mask);
+            if (b == 0) p->seg_items_dev = reinterpret_cast<uint2*>(mask + masks);
+            e = cudaMemset(mask, 0, masks);
         }
         if (e != cudaSuccess) {
             plan_free_segments(p);
@@ -779,6 +783,7 @@ int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t most)
     }
     S3R_CUDA(ctx, cudaDeviceSynchronize());
     p->seg_pixels = npix;
+    p->seg_items_cap = items;
     p->seg_words = words;
     return S3R_OK;
 }
@@ -897,9 +902,23 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
         seg = asked || seg_pays(p, covered, samples, log_lanes);
     }
     if (seg) {
+        uint64_t n = 0;
+        p->seg_lanes = false;
+        for (uint32_t i = 0; i < p->nblocks; ++i) {
+            const uint32_t cell = p->seg_order[i];
+            const RenderBlock& t = tb[cell];
+            p->seg_list_pinned[i] = make_uint2(cell | log_lanes[t.depth] << kSegLanesShift, (uint32_t)n);
+            if (t.rect[2] <= 0 || t.rect[3] <= 0) continue;
+            uint32_t w, h;
+            seg_footprint(fx, log_lanes[t.depth], w, h);
+            n += (uint64_t)(((uint32_t)t.rect[2] + w - 1) / w) * (((uint32_t)t.rect[3] + h - 1) / h);
+            p->seg_lanes |= log_lanes[t.depth] > 0;
+        }
+        p->seg_list_pinned[p->nblocks] = make_uint2(0, (uint32_t)n);
+        if (n > 0xffffffffull) return fail(ctx, S3R_ERR_INVALID, "too many block-major render items");
         const uint64_t most = (uint64_t)view->W * view->H;
         const int rc = plan_ensure_segments(p, std::max<uint64_t>(covered, 1),
-                                            asked ? most : std::min(most, kSegAutoBytes / seg_pixel_bytes(p)));
+                                            asked ? most : std::min(most, kSegAutoBytes / seg_pixel_bytes(p)), n);
         if (rc && asked) return rc;
         if (rc) {
             // no room: the walk gives the same image
@@ -909,38 +928,6 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
         }
     }
     p->seg_now = seg;
-    if (seg) {
-        auto tiles_of = [&](const RenderBlock& t) -> uint64_t {
-            if (t.rect[2] <= 0 || t.rect[3] <= 0) return 0;
-            uint32_t w, h;
-            seg_footprint(fx, log_lanes[t.depth], w, h);
-            return (uint64_t)(((uint32_t)t.rect[2] + w - 1) / w) * (((uint32_t)t.rect[3] + h - 1) / h);
-        };
-        uint64_t n = 0;
-        p->seg_lanes = false;
-        for (uint32_t i = 0; i < p->nblocks; ++i) {
-            const uint32_t cell = p->seg_order[i];
-            const RenderBlock& t = tb[cell];
-            const uint64_t tiles = tiles_of(t);
-            p->seg_list_pinned[i] = make_uint2(cell | log_lanes[t.depth] << kSegLanesShift, (uint32_t)n);
-            n += tiles;
-            p->seg_lanes |= tiles > 0 && log_lanes[t.depth] > 0;
-        }
-        p->seg_list_pinned[p->nblocks] = make_uint2(0, (uint32_t)n);
-        if (n > 0xffffffffull) return fail(ctx, S3R_ERR_INVALID, "too many block-major render items");
-        if (n > p->seg_items_cap) {
-            // frames in flight or captured may hold the old list
-            if (p->seg_items_dev) S3R_CUDA(ctx, cudaDeviceSynchronize());
-            plan_drop_graph(p);
-            if (p->seg_items_dev) cudaFree(p->seg_items_dev);
-            p->seg_items_dev = nullptr;
-            p->seg_items_cap = 0;
-            const uint64_t cap = n + n / 4; // some room for other views
-            const cudaError_t e = cudaMalloc(&p->seg_items_dev, cap * sizeof(uint2));
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(block-major items)");
-            p->seg_items_cap = cap;
-        }
-    }
     p->staged_tile = frame ? (int)p->render_tile : -1;
     std::memcpy(p->cover_pinned, cover, sizeof(cover));
     *p->view_pinned = *view;
@@ -1010,7 +997,7 @@ int plan_launch_render(s3r_plan* p, const float* tf, float* rgba, uint32_t* argb
         return fail(p->ctx, S3R_ERR_INVALID, "view not staged for this render tile");
     if (p->seg_now) {
         const int data = slot ? 1 : 0;
-        if (!p->seg_buf[data] || !p->seg_items_dev)
+        if (!p->seg_buf[data])
             return fail(p->ctx, S3R_ERR_INVALID, "block-major render buffers not allocated for this view");
         const bool asked = p->render_tile >= (uint32_t)kRenderWalkTiles;
         const uint32_t shape = asked ? p->render_tile - (uint32_t)kRenderWalkTiles : 0u;
@@ -1900,7 +1887,6 @@ int s3r_plan_destroy(s3r_plan* p)
     f(p->stage_dev);
     if (p->stage_pinned) cudaFreeHost(p->stage_pinned);
     f(p->dtf_part);
-    f(p->seg_items_dev);
     f(p->seg_queue);
     plan_free_segments(p);
     if (p->staged) cudaEventDestroy(p->staged);
