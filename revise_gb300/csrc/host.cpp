@@ -899,7 +899,8 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
     bool seg = false;
     if (frame && (asked || p->render_tile < (uint32_t)kRenderShapes)) {
         const double samples = seg_lanes_by_depth(p, tb, fx, fy, view->quality, log_lanes);
-        seg = asked || seg_pays(p, covered, samples, log_lanes);
+        // a table that the walk refuses stays refused
+        seg = asked || (view->tf_n <= kTfPlain && seg_pays(p, covered, samples, log_lanes));
     }
     if (seg) {
         uint64_t n = 0;

@@ -158,28 +158,7 @@ __device__ __forceinline__ bool block_ray(const s3r_view& v, const float org[3],
     return true;
 }
 
-struct Cell {
-    uint32_t i0[3], i1[3];
-    float f[3];
-};
-
-__device__ __forceinline__ void sample_cell(const BlockRay& r, int k, Cell& c)
-{
-    const int hi = (int)r.n - 1;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const float p = __fmaf_rn(r.step[d], (float)k, r.p0[d]);
-        const float tc = __fmul_rn(__fsub_rn(p, r.origin[d]), r.factor);
-        const float xb = __fsub_rn(tc, 0.5f);
-        const float fl = floorf(xb);
-        c.f[d] = __fsub_rn(xb, fl);
-        const int a = (int)fl, b = a + 1;
-        c.i0[d] = (uint32_t)min(max(a, 0), hi);
-        c.i1[d] = (uint32_t)min(max(b, 0), hi);
-    }
-}
-
-// 8 texels of a cell from a brick of format Fmt, decoded to float.
+// A texel of a brick of format Fmt, decoded to float.
 template <int Fmt> struct Brick;
 template <> struct Brick<S3R_BRICK_F32> {
     __device__ static float get(const void* b, uint64_t i) { return __ldg(reinterpret_cast<const float*>(b) + i); }
@@ -196,33 +175,6 @@ template <> struct Brick<S3R_BRICK_BF16> {
         return __bfloat162float(__ldg(reinterpret_cast<const __nv_bfloat16*>(b) + i));
     }
 };
-
-template <int Fmt>
-__device__ __forceinline__ bool trilinear(const void* brick, const Cell& c, Dim g, float& val, float t[8],
-                                          uint64_t off[8])
-{
-    const uint64_t n64 = g.n, p64 = g.pitch;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-        const uint64_t x = (q & 1) ? c.i1[0] : c.i0[0];
-        const uint64_t y = (q & 2) ? c.i1[1] : c.i0[1];
-        const uint64_t z = (q & 4) ? c.i1[2] : c.i0[2];
-        off[q] = (z * n64 + y) * p64 + x;
-        t[q] = Brick<Fmt>::get(brick, off[q]);
-    }
-    bool bad = false;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) bad |= isnan(t[q]);
-    if (bad) return false;
-    const float x00 = __fmaf_rn(c.f[0], t[1] - t[0], t[0]);
-    const float x10 = __fmaf_rn(c.f[0], t[3] - t[2], t[2]);
-    const float x01 = __fmaf_rn(c.f[0], t[5] - t[4], t[4]);
-    const float x11 = __fmaf_rn(c.f[0], t[7] - t[6], t[6]);
-    const float y0 = __fmaf_rn(c.f[1], x10 - x00, x00);
-    const float y1 = __fmaf_rn(c.f[1], x11 - x01, x01);
-    val = __fmaf_rn(c.f[2], y1 - y0, y0);
-    return true;
-}
 
 // ---------------------------------------------------------------- texture-unit filtering
 //
@@ -315,13 +267,6 @@ __device__ __forceinline__ bool tex_trilinear(const void* brick, const BlockRay&
     return tex_trilinear_at<Fmt>(brick, dim_of(r), sample_tc(r, k, 0), sample_tc(r, k, 1), sample_tc(r, k, 2), val);
 }
 
-struct TfSample {
-    float4 c;
-    uint32_t i0, i1;
-    float f;
-    bool clamped;
-};
-
 __device__ __forceinline__ float4 tex_tf_lookup(const float4* tf, uint32_t tfn, float v01)
 {
     const TexAxis u = tex_axis(__fmul_rn(v01, (float)tfn), (int)tfn - 1);
@@ -333,26 +278,6 @@ __device__ __forceinline__ float4 tex_tf_lookup(const float4* tf, uint32_t tfn, 
     c.z = __fmul_rn(__fmaf_rn(wh, q.z, __fmul_rn(wl, p.z)), 0.00390625f);
     c.w = __fmul_rn(__fmaf_rn(wh, q.w, __fmul_rn(wl, p.w)), 0.00390625f);
     return c;
-}
-
-// tex1D with normalized coordinates, linear filtering, clamp addressing.
-__device__ __forceinline__ TfSample tf_lookup(const float4* tf, uint32_t tfn, float v01)
-{
-    TfSample s;
-    const float u = __fmaf_rn(v01, (float)tfn, -0.5f);
-    const float fl = floorf(u);
-    s.f = u - fl;
-    const int hi = (int)tfn - 1;
-    const int a = (int)fmaxf(fminf(fl, 1e9f), -1e9f), b = a + 1;
-    s.clamped = a < 0 || b > hi;
-    s.i0 = (uint32_t)min(max(a, 0), hi);
-    s.i1 = (uint32_t)min(max(b, 0), hi);
-    const float4 p = tf[s.i0], q = tf[s.i1];
-    s.c.x = __fmaf_rn(s.f, q.x - p.x, p.x);
-    s.c.y = __fmaf_rn(s.f, q.y - p.y, p.y);
-    s.c.z = __fmaf_rn(s.f, q.z - p.z, p.z);
-    s.c.w = __fmaf_rn(s.f, q.w - p.w, p.w);
-    return s;
 }
 
 // The transfer function in shared memory as the kernels look it up: P holds tf_n + 2 entries, the table with its first
@@ -389,7 +314,7 @@ __device__ __forceinline__ TfTable load_tf(float4* sm, const float* tf, uint32_t
     return TfTable{sm, diff ? sm + tf_n + 2 : nullptr};
 }
 
-// tf_lookup's colour from the padded table: entry j = floor(u) + 1 within [0, tf_n] gives the clamped pair;
+// The colour from the padded table: entry j = floor(u) + 1 within [0, tf_n] gives the clamped pair;
 // beyond the table the pair is one entry twice, so any finite fraction gives that entry.
 __device__ __forceinline__ float4 tf_colour(const TfTable& tf, uint32_t tfn, float v01)
 {
@@ -2170,6 +2095,15 @@ __global__ void __launch_bounds__(256) dtf_reduce_kernel(const float* __restrict
 
 } // namespace
 
+// The walk, the field modes and the per-block kernels take tables of up to kTfPlain entries: 48 KB of shared memory
+// and the two repeated entries.  The launch refuses larger ones.
+template <class K> cudaError_t allow_table(K kernel, size_t smem)
+{
+    if (smem <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(tf_smem_entries(kTfPlain, false) * sizeof(float4)));
+}
+
 // f(std::integral_constant<int, mode>) for a field mode known at run time.
 template <class F> auto with_mode(uint32_t mode, F&& f)
 {
@@ -2193,14 +2127,15 @@ cudaError_t launch_render_block_mode(const s3r_view* view_host, const s3r_presen
     dim3 block(16, 8);
     dim3 grid((rb.rect[2] + 15) / 16, (rb.rect[3] + 7) / 8);
     const size_t smem = tf_smem_entries(view_host->tf_n, false) * sizeof(float4);
-    if (view_host->filter == S3R_FILTER_TEXTURE)
-        render_block_mode_kernel<true, -1><<<grid, block, smem, s>>>(*view_host, *pres, brick, brick2, rb, tf, viewport);
-    else if (pres->mode == S3R_MODE_ARGB)
-        render_block_mode_kernel<false, S3R_MODE_ARGB>
-            <<<grid, block, smem, s>>>(*view_host, *pres, brick, brick2, rb, tf, viewport);
-    else
-        render_block_mode_kernel<false, -1><<<grid, block, smem, s>>>(*view_host, *pres, brick, brick2, rb, tf, viewport);
-    return cudaGetLastError();
+    auto launch = [&](auto kernel) {
+        const cudaError_t err = allow_table(kernel, smem);
+        if (err != cudaSuccess) return err;
+        kernel<<<grid, block, smem, s>>>(*view_host, *pres, brick, brick2, rb, tf, viewport);
+        return cudaGetLastError();
+    };
+    if (view_host->filter == S3R_FILTER_TEXTURE) return launch(render_block_mode_kernel<true, -1>);
+    if (pres->mode == S3R_MODE_ARGB) return launch(render_block_mode_kernel<false, S3R_MODE_ARGB>);
+    return launch(render_block_mode_kernel<false, -1>);
 }
 
 void part_tile(uint32_t mode, bool texture, uint32_t& w, uint32_t& h)
@@ -2219,14 +2154,19 @@ cudaError_t launch_part(const s3r_view* view_host, const s3r_presentation* pres,
     part_tile(pres->mode, texture, tw, th);
     const dim3 block(tw, th);
     const size_t smem = texture ? 0 : tf_smem_entries(view_host->tf_n, false) * sizeof(float4);
-    with_mode(pres->mode, [&](auto mode) {
+    auto launch = [&](auto kernel) {
+        const cudaError_t e = allow_table(kernel, smem);
+        if (e != cudaSuccess) return e;
+        kernel<<<ctas, block, smem, s>>>(*view_host, *pres, a);
+        return cudaGetLastError();
+    };
+    err = with_mode(pres->mode, [&](auto mode) {
         constexpr int m = decltype(mode)::value;
-        if (texture) part_blocks_kernel<2, m><<<ctas, block, 0, s>>>(*view_host, *pres, a);
-        else if (view_host->filter != S3R_FILTER_TEXTURE)
-            part_blocks_kernel<0, m><<<ctas, block, smem, s>>>(*view_host, *pres, a);
-        else part_blocks_kernel<1, -1><<<ctas, block, smem, s>>>(*view_host, *pres, a);
+        if (texture) return launch(part_blocks_kernel<2, m>);
+        return view_host->filter != S3R_FILTER_TEXTURE ? launch(part_blocks_kernel<0, m>)
+                                                       : launch(part_blocks_kernel<1, -1>);
     });
-    if ((err = cudaGetLastError()) != cudaSuccess) return err;
+    if (err != cudaSuccess) return err;
     const bool multi = pres->mode == S3R_MODE_ISOSURFACES || pres->mode == S3R_MODE_VALUE_ON_ISOSURFACES;
     const uint32_t kind = pres->mode == S3R_MODE_MAX_INTENSITY ? ModeOut::kMax
                           : multi && pres->level_count < 1     ? ModeOut::kClear
@@ -2256,13 +2196,18 @@ cudaError_t launch_render_block_texture(const s3r_view* view_host, const s3r_pre
 template <int Fmt, bool kTex>
 cudaError_t launch_frame_render_fmt(const FrameArgs& a, dim3 grid, dim3 block, size_t smem, uint32_t R, cudaStream_t s)
 {
+    auto launch = [&](auto kernel) {
+        const cudaError_t err = allow_table(kernel, smem);
+        if (err != cudaSuccess) return err;
+        kernel<<<grid, block, smem, s>>>(a);
+        return cudaGetLastError();
+    };
     switch (R) {
-    case 1: frame_render_kernel<Fmt, 1, kTex><<<grid, block, smem, s>>>(a); break;
-    case 2: frame_render_kernel<Fmt, 2, kTex><<<grid, block, smem, s>>>(a); break;
-    case 4: frame_render_kernel<Fmt, 4, kTex><<<grid, block, smem, s>>>(a); break;
-    default: frame_render_kernel<Fmt, 8, kTex><<<grid, block, smem, s>>>(a); break;
+    case 1: return launch(frame_render_kernel<Fmt, 1, kTex>);
+    case 2: return launch(frame_render_kernel<Fmt, 2, kTex>);
+    case 4: return launch(frame_render_kernel<Fmt, 4, kTex>);
+    default: return launch(frame_render_kernel<Fmt, 8, kTex>);
     }
-    return cudaGetLastError();
 }
 
 cudaError_t launch_frame_render(const FrameArgs& a, uint32_t W, uint32_t H, uint32_t tf_n, uint32_t fmt,
@@ -2351,12 +2296,17 @@ cudaError_t launch_frame_render_mode(const FrameArgs& a, const s3r_presentation&
     const dim3 block(8, 16); // 8 x 4 pixels a warp
     const dim3 grid((W + 7) / 8, (H + 15) / 16);
     const size_t smem = tf_smem_entries(tf_n, false) * sizeof(float4);
-    with_mode(pres.mode, [&](auto mode) {
+    auto launch = [&](auto kernel) {
+        const cudaError_t err = allow_table(kernel, smem);
+        if (err != cudaSuccess) return err;
+        kernel<<<grid, block, smem, s>>>(a, pres, bricks2);
+        return cudaGetLastError();
+    };
+    return with_mode(pres.mode, [&](auto mode) {
         constexpr int m = decltype(mode)::value;
-        if (filter == S3R_FILTER_TEXTURE) frame_render_mode_kernel<true, m><<<grid, block, smem, s>>>(a, pres, bricks2);
-        else frame_render_mode_kernel<false, m><<<grid, block, smem, s>>>(a, pres, bricks2);
+        return filter == S3R_FILTER_TEXTURE ? launch(frame_render_mode_kernel<true, m>)
+                                            : launch(frame_render_mode_kernel<false, m>);
     });
-    return cudaGetLastError();
 }
 
 cudaError_t launch_frame_backward(const FrameArgs& a, uint32_t W, uint32_t H, uint32_t tf_n, cudaStream_t s)

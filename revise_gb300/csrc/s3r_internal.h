@@ -146,6 +146,7 @@ struct FrameArgs {
 
 // The block-major frame render (render tile ids kRenderWalkTiles and up): its work
 // items and per-pixel block results.
+constexpr uint32_t kTfPlain = 3072; // table entries that the renders other than block-major and adjoint take
 constexpr uint32_t kSegMaskWords = 6; // rank masks of up to 384 ranks: levels <= 7
 constexpr uint32_t kSegLanesShift = 28, kSegCellMask = (1u << kSegLanesShift) - 1;
 // Pixels of an item: fx x (32 / fx) with one lane to a ray, halved along x, then y, then x again with 2, 4, 8 lanes.
