@@ -1790,66 +1790,57 @@ struct CellGradient {
     int a[3];       // the cell's low corner
     float* p;       // corner 0
     int stride[3];
-    bool have;
 
-    __device__ __forceinline__ void begin(const float step[3], int pitch, int dz)
+    __device__ __forceinline__ void begin(const float step[3], float* dense, int pitch, int dz)
     {
-        have = false;
+        p = dense;
         stride[0] = step[0] < 0.f ? -1 : 1;
         stride[1] = step[1] < 0.f ? -pitch : pitch;
         stride[2] = step[2] < 0.f ? -dz : dz;
 #pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (stride[d] < 0) p -= stride[d];
+            a[d] = 0;
+        }
+#pragma unroll
         for (int q = 0; q < 8; ++q) g[q] = 0.f;
     }
-    __device__ __forceinline__ float* corner(int q) const
-    {
-        return p + (((q & 1) ? stride[0] : 0) + ((q & 2) ? stride[1] : 0) + ((q & 4) ? stride[2] : 0));
-    }
-    __device__ __forceinline__ void put(int q) const
-    {
-        if (g[q] != 0.f) atomicAdd(corner(q), g[q]);
-    }
-    __device__ __forceinline__ void flush()
-    {
-        if (!have) return;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            put(q);
-            g[q] = 0.f;
-        }
-        have = false;
-    }
-    template <int B> __device__ __forceinline__ void step(int axis)
+    // The corners in `which` (bit q) go to memory.
+    __device__ __forceinline__ void put(uint32_t which) const
     {
 #pragma unroll
         for (int q = 0; q < 8; ++q)
-            if (!(q & B)) {
-                put(q);
-                g[q] = g[q | B];
-                g[q | B] = 0.f;
-            }
-        p += stride[axis];
+            if (((which >> q) & 1u) && g[q] != 0.f)
+                atomicAdd(p + (((q & 1) ? stride[0] : 0) + ((q & 2) ? stride[1] : 0) + ((q & 4) ? stride[2] : 0)), g[q]);
     }
-    // The ray is now in the (inside) cell `to` of the brick whose gradients start at `dense`.
+    // The ray is now in the (inside) cell `to` of the brick whose gradients start at `dense`: the corners left behind
+    // go out, the others move up, without a branch on the axes (a warp's rays cross their faces at different samples;
+    // with branches 267 us where this takes 254, and 220 where it takes 201).
     __device__ __forceinline__ void move(const int to[3], float* dense, uint32_t n, uint32_t pitch)
     {
         // steps along the ray: 0 or 1 per axis, or the cell is left altogether
         const int dx = stride[0] < 0 ? a[0] - to[0] : to[0] - a[0], dy = stride[1] < 0 ? a[1] - to[1] : to[1] - a[1],
                   dz = stride[2] < 0 ? a[2] - to[2] : to[2] - a[2];
-        if (have && (uint32_t)(dx | dy | dz) <= 1u) {
-            if (dx) step<1>(0);
-            if (dy) step<2>(1);
-            if (dz) step<4>(2);
-        } else {
-            flush();
-            p = dense + (((uint32_t)to[2] * n + (uint32_t)to[1]) * pitch + (uint32_t)to[0]);
+        if ((dx | dy | dz) == 0) return;
+        const bool all = (uint32_t)(dx | dy | dz) > 1u;
+        put(all ? 0xffu : ((dx ? 0x55u : 0u) | (dy ? 0x33u : 0u) | (dz ? 0x0fu : 0u)));
 #pragma unroll
-            for (int d = 0; d < 3; ++d)
-                if (stride[d] < 0) p -= stride[d];
-            have = true;
+        for (int d = 0; d < 3; ++d) {
+            const bool moved = all || (d == 0 ? dx : d == 1 ? dy : dz) != 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (!(q & (1 << d))) {
+                    g[q] = moved ? g[q | (1 << d)] : g[q];
+                    g[q | (1 << d)] = moved ? 0.f : g[q | (1 << d)];
+                }
         }
+        if (all) g[0] = 0.f; // corner 7, out already
+        p = dense + (((uint32_t)to[2] * n + (uint32_t)to[1]) * pitch + (uint32_t)to[0]);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) a[d] = to[d];
+        for (int d = 0; d < 3; ++d) {
+            if (stride[d] < 0) p -= stride[d];
+            a[d] = to[d];
+        }
     }
     // Adds the sample's gradient by its trilinear weights.
     __device__ __forceinline__ void add(float v, const float f[3])
@@ -1969,7 +1960,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 8) frame_backward_kernel(Fra
             const float il = layer_exponent(depth, v.level, v.quality);
             float Ab = 0.f;
             CellGradient cg;
-            cg.begin(r.step, (int)r.pitch, (int)(r.n * r.pitch));
+            cg.begin(r.step, gdense, (int)r.pitch, (int)(r.n * r.pitch));
             // one sample's gradients from its cell; false once the block is opaque
             auto step_sample = [&](const GradCell& cell) -> bool {
                 float val;
@@ -2058,7 +2049,7 @@ __global__ void __launch_bounds__(kBackwardThreads, 8) frame_backward_kernel(Fra
                 if (!step_sample(cb)) break;
                 k += 1.f;
             }
-            cg.flush();
+            cg.put(0xffu);
             // block composite exactly as the forward kernel forms it
             accA = __fmaf_rn(__fsub_rn(1.f, accA), Ab, accA);
             if (accA > v.alpha_stop) break;
@@ -2311,10 +2302,11 @@ cudaError_t launch_frame_render_mode(const FrameArgs& a, const s3r_presentation&
 
 cudaError_t launch_frame_backward(const FrameArgs& a, uint32_t W, uint32_t H, uint32_t tf_n, cudaStream_t s)
 {
-    // 8x8-pixel CTAs: 8x4 pixels a warp share most of the cells they add to (337 us with 32x2, 318 with this on 8
-    // blocks of depth 6 at 512x512); larger CTAs leave more idle at the end, the rays' work being uneven
-    dim3 block(8, 8);
-    dim3 grid((W + 7) / 8, (H + 7) / 8);
+    // 16x4-pixel CTAs, 16x2 pixels a warp.  8 blocks of depth 6 at 512x512: long transparent rays take 254 us with 8x8
+    // (8x4 a warp: its rays share most of the cells they add to), 264 with this, 274 with 32x2; rays that end early in
+    // opaque blocks 201, 186 and 188 us, where 32x2 with eight reductions a sample took 199 (342 for the long rays)
+    dim3 block(16, 4);
+    dim3 grid((W + 15) / 16, (H + 3) / 4);
     const size_t smem = tf_smem_entries(tf_n, false) * sizeof(float4);
     if (smem + sizeof(BackwardShared) > 47 * 1024) {
         cudaError_t err =
