@@ -739,7 +739,7 @@ int plan_bin(s3r_plan* p, uint32_t tile_log2, const uint8_t* by_depth = nullptr)
 }
 
 // The block-major render's per-rank results and rank masks for `npix` covered pixels in data slots 0 .. slots-1, and
-// room for `items` work items; called before a frame is launched (or captured) in the block-major form.  Reallocation
+// room for `items` work items (not while the stream `unless_capturing` is being captured); called before a frame is launched (or captured) in the block-major form.  Reallocation
 // drops the captured frames (they hold the old buffers).
 void plan_free_segments(s3r_plan* p)
 {
@@ -754,12 +754,15 @@ void plan_free_segments(s3r_plan* p)
 
 uint64_t seg_pixel_bytes(const s3r_plan* p) { return (3ull * (1u << p->level) - 2) * sizeof(float4); }
 
-int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t most, uint64_t items)
+int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t most, uint64_t items, cudaStream_t unless_capturing)
 {
     s3r_ctx* ctx = p->ctx;
     const int slots = p->hs_h2d ? 2 : 1; // the second one only for the host-buffer pipeline
     const uint32_t words = (3 * (1u << p->level) - 2 + 63) / 64;
     if (p->seg_buf[slots - 1] && p->seg_pixels >= npix && p->seg_items_cap >= items) return S3R_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (unless_capturing) S3R_CUDA(ctx, cudaStreamIsCapturing(unless_capturing, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return fail(ctx, S3R_ERR_UNSUPPORTED, "allocation in a stream capture");
     if (p->seg_buf[0]) S3R_CUDA(ctx, cudaDeviceSynchronize()); // frames in flight
     // some room to move closer in, up to the whole viewport
     npix = p->seg_pixels >= npix ? p->seg_pixels : std::max(p->seg_pixels, std::min(npix + npix / 2, most));
@@ -845,18 +848,22 @@ double seg_lanes_by_depth(const s3r_plan* p, const RenderBlock* table, uint32_t 
 // block-major for this view.  The measured line (depths 3-7 and 4 to 6, 200x150 to 1920x1080, from close up to far):
 // with 64 blocks and more the walk's lanes sit in different blocks and wait for each other, and block-major is up to
 // seven times faster (level 3, 200x150: 550 against 79 us); short segments in a large part of the image favour the
-// walk, which writes no block results (level 4 of depth 3, close up: 711 against 878 us); of 8 blocks only small views
-// of mixed depths gain (66 against 42 us), and a single one is the walk's.
+// walk, which writes no block results (level 4 of depth 3, close up: 711 against 878 us; level 2 of depths 3-7 with 19
+// samples a ray, 783x588: 152 against 168; with 5 samples the second launch is not won back, 22 against 23); of 8 blocks only small views of deep ones gain (66 against 42 us; of depth 3
+// the second launch costs more, 19 against 21), and a single one is the walk's.  Where rays may stop before their last block
+// (alpha_stop below 1) it is the walk's too: block-major marches what lies behind opaque blocks (64 FP16 blocks of depth
+// 6, 233x238: 74 against 157 us), and how opaque the data are is not known here.
 constexpr uint64_t kSegAutoBytes = 1ull << 30; // of block results
-bool seg_pays(const s3r_plan* p, uint64_t covered, double samples, const uint32_t log_lanes[S3R_MAX_DEPTH + 1])
+bool seg_pays(const s3r_plan* p, uint64_t covered, double samples, float quality,
+              const uint32_t log_lanes[S3R_MAX_DEPTH + 1])
 {
     if (p->level < 1 || p->level > 7 || covered == 0 || covered * seg_pixel_bytes(p) > kSegAutoBytes) return false;
     if (p->level == 1) {
-        bool lanes = false;
-        for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d) lanes |= log_lanes[d] > 0;
+        bool lanes = false; // shared rays of at least 32 samples
+        for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d) lanes |= log_lanes[d] > 0 && 1.3 * quality * (1u << d) >= 32;
         return lanes && covered < 60000;
     }
-    return samples >= 30 || covered < 100000 || (samples >= 18 && covered < 1000000);
+    return samples >= 30 || (samples >= 8 && covered < 100000) || (samples >= 22 && covered < 1000000);
 }
 
 // frame: for s3r_frame_render and the frames of s3r_frame_run(_host), whose render may go block-major; the field modes
@@ -900,7 +907,8 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
     if (frame && (asked || p->render_tile < (uint32_t)kRenderShapes)) {
         const double samples = seg_lanes_by_depth(p, tb, fx, fy, view->quality, log_lanes);
         // a table that the walk refuses stays refused
-        seg = asked || (view->tf_n <= kTfPlain && seg_pays(p, covered, samples, log_lanes));
+        seg = asked || (view->tf_n <= kTfPlain && view->alpha_stop >= 1.f &&
+                        seg_pays(p, covered, samples, view->quality, log_lanes));
     }
     if (seg) {
         uint64_t n = 0;
@@ -919,10 +927,11 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
         if (n > 0xffffffffull) return fail(ctx, S3R_ERR_INVALID, "too many block-major render items");
         const uint64_t most = (uint64_t)view->W * view->H;
         const int rc = plan_ensure_segments(p, std::max<uint64_t>(covered, 1),
-                                            asked ? most : std::min(most, kSegAutoBytes / seg_pixel_bytes(p)), n);
+                                            asked ? most : std::min(most, kSegAutoBytes / seg_pixel_bytes(p)), n,
+                                            asked ? nullptr : s);
         if (rc && asked) return rc;
         if (rc) {
-            // no room: the walk gives the same image
+            // no room, or none to be had in a caller's capture: the walk gives the same image
             seg = false;
             ctx->err.clear();
             set_thread_error("");
