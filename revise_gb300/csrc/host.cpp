@@ -849,10 +849,11 @@ double seg_lanes_by_depth(const s3r_plan* p, const RenderBlock* table, uint32_t 
 // with 64 blocks and more the walk's lanes sit in different blocks and wait for each other, and block-major is up to
 // seven times faster (level 3, 200x150: 550 against 79 us); short segments in a large part of the image favour the
 // walk, which writes no block results (level 4 of depth 3, close up: 711 against 878 us; level 2 of depths 3-7 with 19
-// samples a ray, 783x588: 152 against 168; with 5 samples the second launch is not won back, 22 against 23); of 8 blocks only small views of deep ones gain (66 against 42 us; of depth 3
-// the second launch costs more, 19 against 21), and a single one is the walk's.  Where rays may stop before their last block
-// (alpha_stop below 1) it is the walk's too: block-major marches what lies behind opaque blocks (64 FP16 blocks of depth
-// 6, 233x238: 74 against 157 us), and how opaque the data are is not known here.
+// samples a ray, 783x588: 152 against 168; with 5 samples the second launch is not won back, 22 against 23); of 8
+// blocks only small views of deep ones gain (66 against 42 us; of depth 3 the second launch costs more, 19 against 21),
+// and a single one is the walk's.  Where rays may stop before their last block (alpha_stop below 1) it is the walk's
+// too: block-major marches what lies behind opaque blocks (64 FP16 blocks of depth 6, 233x238: 74 against 157 us), and
+// how opaque the data are is not known here.
 constexpr uint64_t kSegAutoBytes = 1ull << 30; // of block results
 bool seg_pays(const s3r_plan* p, uint64_t covered, double samples, float quality,
               const uint32_t log_lanes[S3R_MAX_DEPTH + 1])

@@ -494,13 +494,16 @@ __device__ __forceinline__ F3 blinn(F3 N, F3 V, F3 L, const s3r_light& light, F3
 // kContracted: the crossing positions of the isosurface modes written as the
 // reference writes them (pos + step * t, which nvcc fuses into one fma), else
 // rounded twice as the oracle rounds them.
+// kAhead: sample k + 1 is fetched before sample k is used.  The texture unit's
+// rule in software filters in its fetch, and a sample ahead only costs it
+// registers (lit volume, 64 blocks of depth 6: 10.0 against 11.0 ms).
 template <bool kTex> struct BrickSampler {
     const float* b1;
     const float* b2;
     Dim n;
     TfTable tf;
     uint32_t tfn;
-    static constexpr bool kStepwise = kTex, kContracted = false;
+    static constexpr bool kStepwise = kTex, kContracted = false, kAhead = !kTex;
     using Sample = std::conditional_t<kTex, float, FieldCell>;
     __device__ void fetch(int second, F3 p, Sample& x) const
     {
@@ -517,7 +520,7 @@ template <bool kTex> struct BrickSampler {
 
 struct TextureSampler {
     cudaTextureObject_t t1, t2, tf;
-    static constexpr bool kStepwise = true, kContracted = true;
+    static constexpr bool kStepwise = true, kContracted = true, kAhead = true;
     using Sample = float;
     __device__ void fetch(int second, F3 p, Sample& x) const { x = tex3D<float>(second ? t2 : t1, p.x, p.y, p.z); }
     static __device__ float value(const Sample& x) { return x; }
@@ -648,12 +651,16 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
         return F3{__fmul_rn(__fsub_rn(p.x, r.origin[0]), r.factor), __fmul_rn(__fsub_rn(p.y, r.origin[1]), r.factor),
                   __fmul_rn(__fsub_rn(p.z, r.origin[2]), r.factor)};
     };
-    // the sample that comes next: its position and its loads in flight
+    // the sample that comes next: its position and, where a fetch is loads alone, these in flight
     F3 pn;
     typename S::Sample ahead;
     auto open = [&](int k) {
         pn = pos_of(k);
-        smp.fetch(0, tc_of(pn), ahead);
+        if constexpr (S::kAhead) smp.fetch(0, tc_of(pn), ahead);
+    };
+    auto value = [&](typename S::Sample& x, F3 p) {
+        if constexpr (!S::kAhead) smp.fetch(0, tc_of(p), x);
+        return S::value(x);
     };
     constexpr float kMax = 0.996f; // AlphaThreshold / AlphaMaxThreshold
     // kMode >= 0: the mode is fixed at compile time (one kernel per mode, as renderKernel<mode> is), so
@@ -662,13 +669,11 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
     if (mode == S3R_MODE_MAX_INTENSITY) {
         // renderMaxIntensityProjection.hpp:30-50; the pixel holds float bits
         float maxv = v.field_min - span;
-        open(0);
-        for (int i = 1; i < r.samples; ++i) {
-            const typename S::Sample x = ahead;
-            if (i + 1 < r.samples) {
-                advance();
-                open(i);
-            }
+        // nothing ends this loop early: the compiler unrolls it and issues several samples' loads at once (64 blocks of
+        // depth 6 through textures, 64 launches: 0.58 ms, 1.31 with the next sample opened by hand)
+        for (int i = 1; i < r.samples; ++i, advance()) {
+            typename S::Sample x;
+            smp.fetch(0, tc_of(pos_of(i - 1)), x);
             const float val = S::value(x);
             if (val >= v.threshold && maxv < val) maxv = val;
         }
@@ -690,12 +695,12 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
         open(0);
         for (int i = 1; i < r.samples; ++i) {
             const F3 p = pn;
-            const typename S::Sample x = ahead;
+            typename S::Sample x = ahead;
             if (i + 1 < r.samples) {
                 advance();
                 open(i);
             }
-            const float val = S::value(x);
+            const float val = value(x, p);
             if (isnan(val)) continue;
             float4 col;
             if (mode == S3R_MODE_DOMAIN_VOXELS) {
@@ -745,7 +750,7 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
                       __fadd_rn(p.z, __fmul_rn(step.z, t))};
     };
     open(0);
-    float v1 = S::value(ahead);
+    float v1 = value(ahead, pn);
     if (r.samples > 1) {
         advance();
         open(1);
@@ -754,12 +759,12 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
         const float thr = v.threshold;
         for (int i = 1; i < r.samples; ++i) {
             const F3 p = pn;
-            const typename S::Sample x = ahead;
+            typename S::Sample x = ahead;
             if (i + 1 < r.samples) {
                 advance();
                 open(i + 1);
             }
-            const float v2 = S::value(x);
+            const float v2 = value(x, p);
             if (!isnan(v1) && !isnan(v2) && (v1 - thr) * (v2 - thr) < 0.f) {
                 const float t = (thr - v1) / (v2 - v1);
                 blend_behind(acc, surface_colour(thr, xpos_of(p, t)));
@@ -772,12 +777,12 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
         int iint = isnan(v1) ? -1 : find_interval(v1, pr.levels, nl);
         for (int i = 1; i < r.samples; ++i) {
             const F3 p = pn;
-            const typename S::Sample x = ahead;
+            typename S::Sample x = ahead;
             if (i + 1 < r.samples) {
                 advance();
                 open(i + 1);
             }
-            const float v2 = S::value(x);
+            const float v2 = value(x, p);
             if (isnan(v2)) {
                 iint = -1;
                 v1 = __int_as_float(0x7fc00000);
