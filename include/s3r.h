@@ -399,8 +399,8 @@ int s3r_make_color_transfer(const double* xs, const double* rgba, uint32_t npoin
  *     (the walk takes one of them, this form both); for levels up to 7, at the cost of (3 * 2^level - 2) x 16
  *     bytes of device memory per pixel that the blocks cover and data slot.
  *   One thread per ray (ids 0-3): a view for which block-major is the faster one (64 blocks and more with rays of
- *     some length in each; at most 1 GB of results) renders in that form, restricted to the blocks that the walk
- *     meets -- the walk's image bit for bit.
+ *     some length in each; at most 1 GB of results; alpha_stop of 1 or more) renders in that form, restricted to
+ *     the blocks that the walk meets -- the walk's image bit for bit.
  * The autotuner times every form. */
 #define S3R_RENDER_TILES_WALK 16u
 #define S3R_RENDER_TILES 19u

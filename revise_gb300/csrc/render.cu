@@ -1674,7 +1674,10 @@ __global__ void frame_composite_kernel(FrameArgs fa, SegArgs sa)
 // no ARGB8 rounding between blocks, max intensity the maximum over the
 // blocks, and a multi-level mode without levels clears the pixel (what lies
 // behind the first block it meets is erased, as the per-block path erases it).
-// A kernel per mode and filter, as renderKernel<mode> is: with the mode known at run time it needed 128 registers.
+// A kernel per mode and filter, as renderKernel<mode> is (with the mode known at run time: 128 registers and spills).
+// What bounds it is the march's instructions and rays of a warp that meet surfaces at different samples; lit
+// isosurfaces, 64 blocks of depth 6, 1280x720: 557 us at first, 314 with the cell's fast path, 304 per mode with 8 x 4
+// pixels a warp (16 x 2: 343), 275 with the next sample in flight; 5 and 6 CTAs an SM 292 and 303.
 template <bool kTex, int kMode>
 __global__ void __launch_bounds__(128, 4) frame_render_mode_kernel(FrameArgs fa, const s3r_presentation pr, const float* __restrict__ bricks2)
 {
