@@ -943,11 +943,12 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
     std::memcpy(p->cover_pinned, cover, sizeof(cover));
     *p->view_pinned = *view;
     S3R_CUDA(ctx, cudaMemcpyAsync(p->stage_dev, p->stage_pinned, p->stage_bytes, cudaMemcpyHostToDevice, s));
-    S3R_CUDA(ctx, cudaEventRecord(p->staged, s));
     if (seg) {
         S3R_CUDA(ctx, launch_seg_items(p->seg_list_dev, p->nblocks, p->seg_items_dev, s));
         ++ctx->launches;
     }
+    // after the expansion: the host pipeline orders its other slot's stream by this event alone
+    S3R_CUDA(ctx, cudaEventRecord(p->staged, s));
     p->last_view = *view;
     p->have_view = true;
     return S3R_OK;
