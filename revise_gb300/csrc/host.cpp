@@ -131,7 +131,7 @@ struct s3r_plan {
     unsigned long long* seg_mask[2] = {nullptr, nullptr}; // behind seg_buf, in its allocation
     uint2* seg_items_dev = nullptr;     // SegArgs::items, expanded from the block list; behind seg_mask[0]
     uint64_t seg_items_cap = 0;
-    uint64_t seg_pixels = 0;            // pixels the buffers hold
+    uint64_t seg_pixels[2] = {0, 0};    // pixels the buffers hold
     uint32_t seg_words = 0;
     // s3r_frame_run_host: per slot a device copy of the frame's sparse values and its image, and the
     // streams and events that overlap frame k's copies with frames k-1 and k+1
@@ -738,40 +738,48 @@ int plan_bin(s3r_plan* p, uint32_t tile_log2, const uint8_t* by_depth = nullptr)
     return S3R_OK;
 }
 
-// The block-major render's per-rank results and rank masks for `npix` covered pixels in data slots 0 .. slots-1, and
-// room for `items` work items (not while the stream `unless_capturing` is being captured); called before a frame is launched (or captured) in the block-major form.  Reallocation
-// drops the captured frames (they hold the old buffers).
+// Whether the caller is capturing this stream (the legacy stream cannot be captured, nor asked about while another is).
+bool capturing(cudaStream_t s)
+{
+    if (!s || s == cudaStreamLegacy) return false;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) != cudaSuccess) (void)cudaGetLastError();
+    return status != cudaStreamCaptureStatusNone;
+}
+
 void plan_free_segments(s3r_plan* p)
 {
     for (int b = 0; b < 2; ++b) {
         if (p->seg_buf[b]) cudaFree(p->seg_buf[b]);
         p->seg_buf[b] = nullptr;
         p->seg_mask[b] = nullptr;
+        p->seg_pixels[b] = 0;
     }
     p->seg_items_dev = nullptr;
-    p->seg_pixels = p->seg_items_cap = 0;
+    p->seg_items_cap = 0;
 }
 
 uint64_t seg_pixel_bytes(const s3r_plan* p) { return (3ull * (1u << p->level) - 2) * sizeof(float4); }
 
-int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t most, uint64_t items, cudaStream_t unless_capturing)
+// The block-major render's per-rank results and rank masks for `npix` pixels, in the second data slot too once there is
+// a host-buffer pipeline, and behind those of the first slot room for `items` work items.  Called before a frame is
+// launched (or captured) in the block-major form.  A slot that is too small is allocated again, which drops the plan's
+// captured frames (they hold the old buffers).
+int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t items)
 {
     s3r_ctx* ctx = p->ctx;
-    const int slots = p->hs_h2d ? 2 : 1; // the second one only for the host-buffer pipeline
     const uint32_t words = (3 * (1u << p->level) - 2 + 63) / 64;
-    if (p->seg_buf[slots - 1] && p->seg_pixels >= npix && p->seg_items_cap >= items) return S3R_OK;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (unless_capturing) S3R_CUDA(ctx, cudaStreamIsCapturing(unless_capturing, &capture));
-    if (capture != cudaStreamCaptureStatusNone) return fail(ctx, S3R_ERR_UNSUPPORTED, "allocation in a stream capture");
-    if (p->seg_buf[0]) S3R_CUDA(ctx, cudaDeviceSynchronize()); // frames in flight
-    // some room to move closer in, up to the whole viewport
-    npix = p->seg_pixels >= npix ? p->seg_pixels : std::max(p->seg_pixels, std::min(npix + npix / 2, most));
-    items = p->seg_items_cap >= items ? p->seg_items_cap : items + items / 4;
-    plan_free_segments(p);
-    plan_drop_graph(p);
-    for (int b = 0; b < slots; ++b) {
-        const size_t results = npix * seg_pixel_bytes(p), masks = (size_t)words * npix * sizeof(unsigned long long);
-        cudaError_t e = cudaMalloc(&p->seg_buf[b], results + masks + (b ? 0 : items * sizeof(uint2)));
+    for (int b = 0; b < (p->hs_h2d ? 2 : 1); ++b) {
+        if (p->seg_buf[b] && p->seg_pixels[b] >= npix && (b || p->seg_items_cap >= items)) continue;
+        S3R_CUDA(ctx, cudaDeviceSynchronize()); // frames in flight
+        plan_drop_graph(p);
+        if (p->seg_buf[b]) cudaFree(p->seg_buf[b]);
+        p->seg_buf[b] = nullptr;
+        const uint64_t pixels = std::max(npix, p->seg_pixels[b]),
+                       room = b ? 0 : (p->seg_items_cap >= items ? p->seg_items_cap : items + items / 4);
+        p->seg_pixels[b] = 0;
+        const size_t results = pixels * seg_pixel_bytes(p), masks = (size_t)words * pixels * sizeof(unsigned long long);
+        cudaError_t e = cudaMalloc(&p->seg_buf[b], results + masks + room * sizeof(uint2));
         if (e == cudaSuccess) {
             char* mask = reinterpret_cast<char*>(p->seg_buf[b]) + results;
             p->seg_mask[b] = reinterpret_cast<unsigned long long*>(mask);
@@ -783,10 +791,10 @@ int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t most, uint64_t ite
             (void)cudaGetLastError(); // an allocation failure leaves no error behind for later launches
             return cuda_fail(ctx, e, "cudaMalloc(block-major render buffers)");
         }
+        S3R_CUDA(ctx, cudaDeviceSynchronize());
+        p->seg_pixels[b] = pixels;
+        if (b == 0) p->seg_items_cap = room;
     }
-    S3R_CUDA(ctx, cudaDeviceSynchronize());
-    p->seg_pixels = npix;
-    p->seg_items_cap = items;
     p->seg_words = words;
     return S3R_OK;
 }
@@ -868,7 +876,7 @@ bool seg_pays(const s3r_plan* p, uint64_t covered, double samples, float quality
 }
 
 // frame: for s3r_frame_render and the frames of s3r_frame_run(_host), whose render may go block-major; the field modes
-// and the adjoint read the table alone.
+// and the adjoint read the table alone (with a block-major id the items are staged all the same, for a caller's graph).
 int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool frame)
 {
     s3r_ctx* ctx = p->ctx;
@@ -905,7 +913,7 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
     const uint32_t fx = (uint32_t)kSegShapeX[shape], fy = (uint32_t)kSegShapeY[shape];
     uint32_t log_lanes[S3R_MAX_DEPTH + 1];
     bool seg = false;
-    if (frame && (asked || p->render_tile < (uint32_t)kRenderShapes)) {
+    if (asked || (frame && p->render_tile < (uint32_t)kRenderShapes && !capturing(s))) {
         const double samples = seg_lanes_by_depth(p, tb, fx, fy, view->quality, log_lanes);
         // a table that the walk refuses stays refused
         seg = asked || (view->tf_n <= kTfPlain && view->alpha_stop >= 1.f &&
@@ -926,20 +934,21 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
         }
         p->seg_list_pinned[p->nblocks] = make_uint2(0, (uint32_t)n);
         if (n > 0xffffffffull) return fail(ctx, S3R_ERR_INVALID, "too many block-major render items");
-        const uint64_t most = (uint64_t)view->W * view->H;
-        const int rc = plan_ensure_segments(p, std::max<uint64_t>(covered, 1),
-                                            asked ? most : std::min(most, kSegAutoBytes / seg_pixel_bytes(p)), n,
-                                            asked ? nullptr : s);
+        // Asked for by its id, the form may be in a caller's graph, which is replayed after views of the same size that
+        // cover more of it: room for the whole viewport.  Else some room to move closer in.
+        const uint64_t most = (uint64_t)view->W * view->H,
+                       some = std::min({covered + covered / 2, most, kSegAutoBytes / seg_pixel_bytes(p)});
+        const int rc = plan_ensure_segments(p, asked ? most : std::max(covered, some), n);
         if (rc && asked) return rc;
         if (rc) {
-            // no room, or none to be had in a caller's capture: the walk gives the same image
+            // no room: the walk gives the same image
             seg = false;
             ctx->err.clear();
             set_thread_error("");
         }
     }
     p->seg_now = seg;
-    p->staged_tile = frame ? (int)p->render_tile : -1;
+    p->staged_tile = frame || asked ? (int)p->render_tile : -1;
     std::memcpy(p->cover_pinned, cover, sizeof(cover));
     *p->view_pinned = *view;
     S3R_CUDA(ctx, cudaMemcpyAsync(p->stage_dev, p->stage_pinned, p->stage_bytes, cudaMemcpyHostToDevice, s));
@@ -992,8 +1001,16 @@ int plan_launch_interp(s3r_plan* p, const float* sparse, cudaStream_t s, uint32_
     return S3R_OK;
 }
 
+// Whether a frame of the staged view queued on `s` goes block-major.  What a caller captures in the default form walks:
+// the graph may be replayed after other views, for which the results and items are allocated and cut anew, while the
+// walk reads only memory that lives as long as the plan.
+bool plan_block_major(const s3r_plan* p, cudaStream_t s)
+{
+    return p->seg_now && (p->render_tile >= (uint32_t)kRenderWalkTiles || !capturing(s));
+}
+
 int plan_launch_render(s3r_plan* p, const float* tf, float* rgba, uint32_t* argb, unsigned long long* samples,
-                       cudaStream_t s, uint32_t* kernels, int slot = 0)
+                       bool seg, cudaStream_t s, uint32_t* kernels, int slot = 0)
 {
     FrameArgs fa{};
     fa.view = p->view_dev;
@@ -1007,7 +1024,7 @@ int plan_launch_render(s3r_plan* p, const float* tf, float* rgba, uint32_t* argb
     fa.cover = p->cover_dev;
     if (p->staged_tile != (int)p->render_tile)
         return fail(p->ctx, S3R_ERR_INVALID, "view not staged for this render tile");
-    if (p->seg_now) {
+    if (seg) {
         const int data = slot ? 1 : 0;
         if (!p->seg_buf[data])
             return fail(p->ctx, S3R_ERR_INVALID, "block-major render buffers not allocated for this view");
@@ -1975,7 +1992,7 @@ int s3r_frame_render(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const f
     cudaStream_t s = as_stream(stream);
     if ((rc = plan_stage_view(plan, view, s, true))) return rc;
     uint32_t k = 0;
-    rc = plan_launch_render(plan, tf, rgba, argb, samples, s, &k);
+    rc = plan_launch_render(plan, tf, rgba, argb, samples, plan_block_major(plan, s), s, &k);
     ctx->launches += k;
     return rc;
 }
@@ -2035,7 +2052,8 @@ static int plan_launch_frame(s3r_plan* plan, int slot, const s3r_view* view, con
     s3r_ctx* ctx = plan->ctx;
     FrameGraph& G = plan->graphs[slot];
     const void* key[5] = {sparse, tf, rgba, argb, samples};
-    const uint32_t dims[5] = {view->W, view->H, view->tf_n, view->filter, (plan->seg_now ? 2u : 0u) | (plan->seg_lanes ? 1u : 0u)};
+    const bool seg = plan_block_major(plan, s);
+    const uint32_t dims[5] = {view->W, view->H, view->tf_n, view->filter, seg ? (plan->seg_lanes ? 2u : 1u) : 0u};
     const bool same = G.exec && std::memcmp(key, G.key, sizeof(key)) == 0 && std::memcmp(dims, G.dims, sizeof(dims)) == 0;
     if (!same) {
         if (G.exec) cudaGraphExecDestroy(G.exec);
@@ -2045,7 +2063,7 @@ static int plan_launch_frame(s3r_plan* plan, int slot, const s3r_view* view, con
         uint32_t k = 0;
         const int data = slot == 2 ? 1 : 0; // the host pipeline's second slot has its own bricks
         int r1 = plan_launch_interp(plan, sparse, cs, &k, data);
-        int r3 = r1 ? r1 : plan_launch_render(plan, tf, rgba, argb, samples, cs, &k, data);
+        int r3 = r1 ? r1 : plan_launch_render(plan, tf, rgba, argb, samples, seg, cs, &k, data);
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(cs, &graph);
         if (r3) {
@@ -2314,7 +2332,7 @@ int s3r_plan_autotune(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const 
             continue;
         }
         float ms = 0;
-        rc = timed([&](uint32_t* kk) { return plan_launch_render(plan, tf, img, nullptr, nullptr, s, kk); }, ms);
+        rc = timed([&](uint32_t* kk) { return plan_launch_render(plan, tf, img, nullptr, nullptr, plan_block_major(plan, s), s, kk); }, ms);
         if (rc) return cleanup(rc);
         if (ms < best) {
             best = ms;

@@ -51,3 +51,73 @@ def test_host_pipeline_orders_the_items(m, tile):
     assert m.calls("segments") == k
     assert m.trouble() == []
     m.ok(m.lib.s3r_plan_destroy(plan))
+
+
+def _captured(m, plan, view, tf, image, run):
+    """A caller's graph of one frame of the staged view; run: (sparse values) interpolation and render."""
+    s = m.stream()
+    args = (C.byref(view), *([run] if run else []), tf, None, image, None, s)
+    f = m.lib.s3r_frame_run if run else m.lib.s3r_frame_render
+    return m.capture(s, lambda: m.ok(f(m.h, plan, *args))), s
+
+
+@pytest.mark.parametrize("run", [False, True])
+def test_captured_default_render_outlives_every_view(m, run):
+    """A default render captured by the caller is replayed after closer views, views that walk, larger and smaller
+    images, a field mode's view and the host pipeline: only memory that lives as long as the plan is in it, and each
+    replay shows the view that is staged then."""
+    w = _level2()
+    plan = m.plan(w)
+    sparse, tf, image = m.buffer(w.nodes), m.buffer(4 * 256), m.buffer(1500 * 1100, np.uint32)
+    view = hf.view_of(w, eye=FAR)
+    assert _block_major(m, view, plan)
+    graph, s = _captured(m, plan, view, tf, image, sparse if run else None)
+    w.W, w.H = 1500, 1100
+    large = hf.view_of(w, eye=NEAR)
+    w.W, w.H = 160, 120
+    stop = hf.view_of(w, eye=NEAR)
+    stop.alpha_stop = 0.9
+    for other in (hf.view_of(w, eye=NEAR), large, stop, view):
+        m.render(plan, other)
+        m.lib.cudaDeviceSynchronize()
+        m.launch(graph, s)
+        m.lib.cudaDeviceSynchronize()
+    near = hf.view_of(w, eye=NEAR)
+    pres = hf.host.presentation(_lib.MODE_MAX_INTENSITY, near)
+    m.ok(m.lib.s3r_frame_render_mode(m.h, plan, C.byref(near), C.byref(pres), tf, None, None, image, None))
+    m.lib.cudaDeviceSynchronize()
+    m.launch(graph, s)
+    for _ in range(2):
+        m.ok(m.lib.s3r_frame_run_host(m.h, plan, C.byref(view), sparse, tf, m.buffer(w.W * w.H, np.uint32), None))
+    m.ok(m.lib.s3r_frame_host_sync(m.h, plan))
+    m.launch(graph, s)
+    m.lib.cudaDeviceSynchronize()
+    assert m.trouble() == []
+    assert m.calls("walk") >= 5  # the replays among them
+    m.ok(m.lib.s3r_plan_destroy(plan))
+
+
+def test_captured_block_major_render_keeps_its_buffers(m):
+    """A render in a block-major form by its id, captured: replays follow the views of the same image size and at most
+    as many work items, a field mode's view and the first use of the host pipeline."""
+    w = _level2()
+    plan = m.plan(w, 16)
+    sparse, tf, image = m.buffer(w.nodes), m.buffer(4 * 256), m.buffer(w.W * w.H, np.uint32)
+    near = hf.view_of(w, eye=NEAR)
+    m.render(plan, near)
+    graph, s = _captured(m, plan, near, tf, image, None)
+    far = hf.view_of(w, eye=FAR)
+    m.render(plan, far)
+    m.lib.cudaDeviceSynchronize()
+    m.launch(graph, s)
+    m.lib.cudaDeviceSynchronize()
+    pres = hf.host.presentation(_lib.MODE_MAX_INTENSITY, near)
+    m.ok(m.lib.s3r_frame_render_mode(m.h, plan, C.byref(near), C.byref(pres), tf, None, None, image, None))
+    m.lib.cudaDeviceSynchronize()
+    m.launch(graph, s)
+    m.lib.cudaDeviceSynchronize()
+    m.ok(m.lib.s3r_frame_run_host(m.h, plan, C.byref(far), sparse, tf, m.buffer(w.W * w.H, np.uint32), None))
+    m.ok(m.lib.s3r_frame_host_sync(m.h, plan))
+    m.launch(graph, s)
+    assert m.trouble() == []
+    m.ok(m.lib.s3r_plan_destroy(plan))
