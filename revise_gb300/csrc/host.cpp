@@ -133,6 +133,9 @@ struct s3r_plan {
     uint64_t seg_items_cap = 0;
     uint64_t seg_pixels[2] = {0, 0};    // pixels the buffers hold
     uint32_t seg_words = 0;
+    // a data slot's block-major frames, on whatever streams, take its results, masks and queue counter in turn
+    cudaEvent_t seg_done[2] = {nullptr, nullptr};
+    std::mutex seg_turn;
     // s3r_frame_run_host: per slot a device copy of the frame's sparse values and its image, and the
     // streams and events that overlap frame k's copies with frames k-1 and k+1
     float* hs_sparse[2] = {nullptr, nullptr};
@@ -999,6 +1002,19 @@ int plan_launch_interp(s3r_plan* p, const float* sparse, cudaStream_t s, uint32_
     S3R_CUDA(ctx, launch_interp_plan(a, p->fmt, p->tile_log2, p->grid_ctas, s));
     ++*kernels;
     return S3R_OK;
+}
+
+// Queues a frame's work on `s` by body(): a block-major one after the frames that used the data slot's results, masks
+// and queue counter before it, whichever streams and threads they came from.  (A block-major render by its id in the
+// caller's capture is ordered by the caller, its graph being launched where this cannot see it.)
+template <class F> int plan_in_turn(s3r_plan* p, bool seg, int data, cudaStream_t s, F&& body)
+{
+    if (!seg || capturing(s)) return body();
+    std::lock_guard<std::mutex> lock(p->seg_turn);
+    S3R_CUDA(p->ctx, cudaStreamWaitEvent(s, p->seg_done[data], 0));
+    const int rc = body();
+    S3R_CUDA(p->ctx, cudaEventRecord(p->seg_done[data], s));
+    return rc;
 }
 
 // Whether a frame of the staged view queued on `s` goes block-major.  What a caller captures in the default form walks:
@@ -1875,8 +1891,9 @@ int s3r_frame_plan(s3r_ctx* ctx, const s3r_frame_desc* desc, s3r_plan** out)
         place(p->stage_dev, p->table_dev, p->view_dev, p->cover_dev, p->seg_list_dev);
         place(p->stage_pinned, p->table_pinned, p->view_pinned, p->cover_pinned, p->seg_list_pinned);
     }
-    if ((e = cudaEventCreateWithFlags(&p->staged, cudaEventDisableTiming)) != cudaSuccess)
-        return bail(cuda_fail(ctx, e, "cudaEventCreate"));
+    for (cudaEvent_t* ev : {&p->staged, &p->seg_done[0], &p->seg_done[1]})
+        if ((e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming)) != cudaSuccess)
+            return bail(cuda_fail(ctx, e, "cudaEventCreate"));
     // block-major render: blocks deepest first (most samples per ray), so that the longest work items start first
     {
         std::vector<uint32_t> idx(desc->nblocks);
@@ -1918,7 +1935,8 @@ int s3r_plan_destroy(s3r_plan* p)
     f(p->dtf_part);
     f(p->seg_queue);
     plan_free_segments(p);
-    if (p->staged) cudaEventDestroy(p->staged);
+    for (cudaEvent_t ev : {p->staged, p->seg_done[0], p->seg_done[1]})
+        if (ev) cudaEventDestroy(ev);
     delete p;
     return S3R_OK;
 }
@@ -1992,7 +2010,8 @@ int s3r_frame_render(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const f
     cudaStream_t s = as_stream(stream);
     if ((rc = plan_stage_view(plan, view, s, true))) return rc;
     uint32_t k = 0;
-    rc = plan_launch_render(plan, tf, rgba, argb, samples, plan_block_major(plan, s), s, &k);
+    const bool seg = plan_block_major(plan, s);
+    rc = plan_in_turn(plan, seg, 0, s, [&] { return plan_launch_render(plan, tf, rgba, argb, samples, seg, s, &k); });
     ctx->launches += k;
     return rc;
 }
@@ -2081,7 +2100,11 @@ static int plan_launch_frame(s3r_plan* plan, int slot, const s3r_view* view, con
         std::memcpy(G.dims, dims, sizeof(dims));
         G.kernels = k;
     }
-    S3R_CUDA(ctx, cudaGraphLaunch(G.exec, s));
+    if (int rc = plan_in_turn(plan, seg, slot == 2 ? 1 : 0, s, [&]() -> int {
+            S3R_CUDA(ctx, cudaGraphLaunch(G.exec, s));
+            return S3R_OK;
+        }))
+        return rc;
     ctx->launches += G.kernels;
     return S3R_OK;
 }
@@ -2332,7 +2355,10 @@ int s3r_plan_autotune(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const 
             continue;
         }
         float ms = 0;
-        rc = timed([&](uint32_t* kk) { return plan_launch_render(plan, tf, img, nullptr, nullptr, plan_block_major(plan, s), s, kk); }, ms);
+        const bool seg = plan_block_major(plan, s);
+        rc = plan_in_turn(plan, seg, 0, s, [&] {
+            return timed([&](uint32_t* kk) { return plan_launch_render(plan, tf, img, nullptr, nullptr, seg, s, kk); }, ms);
+        });
         if (rc) return cleanup(rc);
         if (ms < best) {
             best = ms;

@@ -1,4 +1,4 @@
-"""Default-form renders inside a caller's CUDA graph, replayed after other views."""
+"""Default-form renders inside a caller's CUDA graph, replayed after other views, and on two streams at once."""
 import numpy as np
 import pytest
 
@@ -53,4 +53,30 @@ def test_captured_default_render_follows_the_view(ctx, run):
         plan.run_host(view, torch.from_numpy(w.sparse).pin_memory(), tf, out)
         plan.host_sync()
     del graph
+    plan.close()
+
+
+@pytest.mark.parametrize("tile", [0, 16])
+def test_two_streams_of_one_plan(ctx, tile):
+    """One staged view with two transfer functions, on two streams without order between them: both images, every time."""
+    import torch
+    from revise_gb300.api import FramePlan
+    w = workloads.small(seed=42, level=2, depths=(4, 5, 6), W=200, H=150)
+    sp = torch.from_numpy(w.sparse).cuda()
+    plan = FramePlan(ctx, w, render_tile=tile)
+    plan.interp(sp)
+    view = host.view_for(w)
+    tfs = [torch.from_numpy(np.ascontiguousarray(t)).cuda() for t in (w.tf, w.tf[::-1])]
+    want = [_image(plan, walked(view), tf) for tf in tfs]
+    _image(plan, view, tfs[0])  # staged
+    streams = [torch.cuda.Stream() for _ in tfs]
+    got = [[torch.full_like(want[0], -1.0) for _ in range(16)] for _ in tfs]
+    torch.cuda.synchronize()
+    for k in range(16):
+        for q, s in enumerate(streams):
+            plan.render(view, tfs[q], got[q][k], stream=s)
+    torch.cuda.synchronize()
+    for q in range(2):
+        for k in range(16):
+            assert torch.equal(got[q][k].view(torch.int32), want[q].view(torch.int32)), (q, k)
     plan.close()

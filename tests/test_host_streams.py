@@ -121,3 +121,23 @@ def test_captured_block_major_render_keeps_its_buffers(m):
     m.launch(graph, s)
     assert m.trouble() == []
     m.ok(m.lib.s3r_plan_destroy(plan))
+
+
+@pytest.mark.parametrize("tile", [0, 16])
+def test_two_streams_take_turns(m, tile):
+    """Frames of one staged view on two streams, and of s3r_frame_run's graph beside them: the block-major form's
+    results, masks and work queue serve one at a time."""
+    w = _level2()
+    plan = m.plan(w, tile)
+    view = hf.view_of(w, eye=NEAR)
+    sparse, tf = m.buffer(w.nodes), m.buffer(4 * 256)
+    assert _block_major(m, view, plan)
+    m.lib.cudaDeviceSynchronize()
+    streams = [m.stream() for _ in range(3)]
+    for k in range(6):
+        m.render(plan, view, streams[k % 3])
+    m.lib.cudaDeviceSynchronize()
+    m.ok(m.lib.s3r_frame_run(m.h, plan, C.byref(view), sparse, tf, None, m.buffer(w.W * w.H, np.uint32), None, streams[0]))
+    m.render(plan, view, streams[1])
+    assert m.trouble() == []
+    m.ok(m.lib.s3r_plan_destroy(plan))
