@@ -2064,7 +2064,8 @@ int s3r_frame_run(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const floa
     return plan_launch_frame(plan, 0, view, sparse, tf, rgba, argb, samples, s);
 }
 
-// The frame as a CUDA graph in cache slot `slot`, captured again when its arguments change.
+// The frame as a CUDA graph in cache slot `slot`, captured again when its arguments change; into a caller's capture its
+// kernels go one by one (a graph cannot be instantiated there).
 static int plan_launch_frame(s3r_plan* plan, int slot, const s3r_view* view, const float* sparse, const float* tf,
                       float* rgba, uint32_t* argb, unsigned long long* samples, cudaStream_t s)
 {
@@ -2073,6 +2074,14 @@ static int plan_launch_frame(s3r_plan* plan, int slot, const s3r_view* view, con
     const void* key[5] = {sparse, tf, rgba, argb, samples};
     const bool seg = plan_block_major(plan, s);
     const uint32_t dims[5] = {view->W, view->H, view->tf_n, view->filter, seg ? (plan->seg_lanes ? 2u : 1u) : 0u};
+    const int data = slot == 2 ? 1 : 0; // the host pipeline's second slot has its own bricks
+    if (capturing(s)) {
+        uint32_t k = 0;
+        int rc = plan_launch_interp(plan, sparse, s, &k, data);
+        if (!rc) rc = plan_launch_render(plan, tf, rgba, argb, samples, seg, s, &k, data);
+        ctx->launches += k;
+        return rc;
+    }
     const bool same = G.exec && std::memcmp(key, G.key, sizeof(key)) == 0 && std::memcmp(dims, G.dims, sizeof(dims)) == 0;
     if (!same) {
         if (G.exec) cudaGraphExecDestroy(G.exec);
@@ -2080,7 +2089,6 @@ static int plan_launch_frame(s3r_plan* plan, int slot, const s3r_view* view, con
         cudaStream_t cs = ctx->capture;
         S3R_CUDA(ctx, cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
         uint32_t k = 0;
-        const int data = slot == 2 ? 1 : 0; // the host pipeline's second slot has its own bricks
         int r1 = plan_launch_interp(plan, sparse, cs, &k, data);
         int r3 = r1 ? r1 : plan_launch_render(plan, tf, rgba, argb, samples, seg, cs, &k, data);
         cudaGraph_t graph = nullptr;
@@ -2100,7 +2108,7 @@ static int plan_launch_frame(s3r_plan* plan, int slot, const s3r_view* view, con
         std::memcpy(G.dims, dims, sizeof(dims));
         G.kernels = k;
     }
-    if (int rc = plan_in_turn(plan, seg, slot == 2 ? 1 : 0, s, [&]() -> int {
+    if (int rc = plan_in_turn(plan, seg, data, s, [&]() -> int {
             S3R_CUDA(ctx, cudaGraphLaunch(G.exec, s));
             return S3R_OK;
         }))
