@@ -766,39 +766,42 @@ uint64_t seg_pixel_bytes(const s3r_plan* p) { return (3ull * (1u << p->level) - 
 
 // The block-major render's per-rank results and rank masks for `npix` pixels, in the second data slot too once there is
 // a host-buffer pipeline, and behind those of the first slot room for `items` work items.  Called before a frame is
-// launched (or captured) in the block-major form.  A slot that is too small is allocated again, which drops the plan's
-// captured frames (they hold the old buffers).
-int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t items)
+// launched in the block-major form.  A slot that is too small is allocated again, in the order of stream `s` and of the
+// frames that use the slots: no call of a render waits for the device.  The plan's captured frames are dropped with it
+// (they hold the old buffers).
+int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t items, cudaStream_t s)
 {
     s3r_ctx* ctx = p->ctx;
     const uint32_t words = (3 * (1u << p->level) - 2 + 63) / 64;
+    p->seg_words = words;
     for (int b = 0; b < (p->hs_h2d ? 2 : 1); ++b) {
         if (p->seg_buf[b] && p->seg_pixels[b] >= npix && (b || p->seg_items_cap >= items)) continue;
-        S3R_CUDA(ctx, cudaDeviceSynchronize()); // frames in flight
+        if (capturing(s)) return fail(ctx, S3R_ERR_UNSUPPORTED, "allocation in a stream capture");
+        std::lock_guard<std::mutex> lock(p->seg_turn);
         plan_drop_graph(p);
-        if (p->seg_buf[b]) cudaFree(p->seg_buf[b]);
+        for (cudaEvent_t done : p->seg_done) S3R_CUDA(ctx, cudaStreamWaitEvent(s, done, 0)); // both slots read the items
+        if (p->seg_buf[b]) S3R_CUDA(ctx, cudaFreeAsync(p->seg_buf[b], s));
         p->seg_buf[b] = nullptr;
         const uint64_t pixels = std::max(npix, p->seg_pixels[b]),
                        room = b ? 0 : (p->seg_items_cap >= items ? p->seg_items_cap : items + items / 4);
         p->seg_pixels[b] = 0;
+        if (b == 0) p->seg_items_cap = 0;
         const size_t results = pixels * seg_pixel_bytes(p), masks = (size_t)words * pixels * sizeof(unsigned long long);
-        cudaError_t e = cudaMalloc(&p->seg_buf[b], results + masks + room * sizeof(uint2));
-        if (e == cudaSuccess) {
-            char* mask = reinterpret_cast<char*>(p->seg_buf[b]) + results;
-            p->seg_mask[b] = reinterpret_cast<unsigned long long*>(mask);
-            if (b == 0) p->seg_items_dev = reinterpret_cast<uint2*>(mask + masks);
-            e = cudaMemset(mask, 0, masks);
-        }
+        const cudaError_t e =
+            cudaMallocAsync(reinterpret_cast<void**>(&p->seg_buf[b]), results + masks + room * sizeof(uint2), s);
         if (e != cudaSuccess) {
-            plan_free_segments(p);
+            p->seg_buf[b] = nullptr;
             (void)cudaGetLastError(); // an allocation failure leaves no error behind for later launches
-            return cuda_fail(ctx, e, "cudaMalloc(block-major render buffers)");
+            return cuda_fail(ctx, e, "cudaMallocAsync(block-major render buffers)");
         }
-        S3R_CUDA(ctx, cudaDeviceSynchronize());
+        char* mask = reinterpret_cast<char*>(p->seg_buf[b]) + results;
+        p->seg_mask[b] = reinterpret_cast<unsigned long long*>(mask);
+        if (b == 0) p->seg_items_dev = reinterpret_cast<uint2*>(mask + masks);
+        S3R_CUDA(ctx, cudaMemsetAsync(mask, 0, masks, s));
+        S3R_CUDA(ctx, cudaEventRecord(p->seg_done[b], s)); // frames on other streams find it cleared
         p->seg_pixels[b] = pixels;
         if (b == 0) p->seg_items_cap = room;
     }
-    p->seg_words = words;
     return S3R_OK;
 }
 
@@ -941,7 +944,7 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
         // cover more of it: room for the whole viewport.  Else some room to move closer in.
         const uint64_t most = (uint64_t)view->W * view->H,
                        some = std::min({covered + covered / 2, most, kSegAutoBytes / seg_pixel_bytes(p)});
-        const int rc = plan_ensure_segments(p, asked ? most : std::max(covered, some), n);
+        const int rc = plan_ensure_segments(p, asked ? most : std::max(covered, some), n, s);
         if (rc && asked) return rc;
         if (rc) {
             // no room: the walk gives the same image

@@ -87,6 +87,7 @@ def test_captured_default_render_outlives_every_view(m, run):
     m.ok(m.lib.s3r_frame_render_mode(m.h, plan, C.byref(near), C.byref(pres), tf, None, None, image, None))
     m.lib.cudaDeviceSynchronize()
     m.launch(graph, s)
+    m.lib.cudaDeviceSynchronize()  # (views are staged in the caller's order)
     for _ in range(2):
         m.ok(m.lib.s3r_frame_run_host(m.h, plan, C.byref(view), sparse, tf, m.buffer(w.W * w.H, np.uint32), None))
     m.ok(m.lib.s3r_frame_host_sync(m.h, plan))
@@ -115,7 +116,7 @@ def test_captured_block_major_render_keeps_its_buffers(m):
     m.ok(m.lib.s3r_frame_render_mode(m.h, plan, C.byref(near), C.byref(pres), tf, None, None, image, None))
     m.lib.cudaDeviceSynchronize()
     m.launch(graph, s)
-    m.lib.cudaDeviceSynchronize()
+    m.lib.cudaDeviceSynchronize()  # (as above)
     m.ok(m.lib.s3r_frame_run_host(m.h, plan, C.byref(far), sparse, tf, m.buffer(w.W * w.H, np.uint32), None))
     m.ok(m.lib.s3r_frame_host_sync(m.h, plan))
     m.launch(graph, s)
@@ -139,5 +140,39 @@ def test_two_streams_take_turns(m, tile):
     m.lib.cudaDeviceSynchronize()
     m.ok(m.lib.s3r_frame_run(m.h, plan, C.byref(view), sparse, tf, None, m.buffer(w.W * w.H, np.uint32), None, streams[0]))
     m.render(plan, view, streams[1])
+    assert m.trouble() == []
+    m.ok(m.lib.s3r_plan_destroy(plan))
+
+
+def test_growing_views_wait_for_nothing(m):
+    """Default renders whose views cover more and more, on alternating streams with frames in flight: the buffers grow
+    in stream order, without a device-wide wait or a blocking allocation inside the call."""
+    w = _level2()
+    plan = m.plan(w)
+    streams = [m.stream(), m.stream()]
+    waits = ("cudaMalloc", "cudaFree", "cudaDeviceSynchronize", "cudaStreamSynchronize")
+    for k, (W, H, eye) in enumerate([(100, 80, FAR), (160, 120, FAR), (160, 120, NEAR), (400, 300, NEAR)]):
+        w.W, w.H = W, H
+        view = hf.view_of(w, eye=eye)
+        before = [m.calls(n) for n in waits]
+        m.render(plan, view, streams[k % 2])
+        assert [m.calls(n) for n in waits] == before
+        m.lib.cudaStreamSynchronize(streams[k % 2])  # the caller's own order between views
+        m.render(plan, view, streams[1 - k % 2])
+    assert m.calls("segments") == 8
+    assert m.trouble() == []
+    m.ok(m.lib.s3r_plan_destroy(plan))
+
+
+def test_no_room_for_results_walks(m):
+    """Without memory for the block results the default form walks, and what other calls then queue is clean."""
+    w = _level2(W=640, H=480)
+    plan = m.plan(w)
+    view = hf.view_of(w, eye=NEAR)
+    m.lib.fake_limit(1 << 20)
+    assert not _block_major(m, view, plan) and m.calls("walk") == 1
+    m.lib.fake_limit(2 ** 64 - 1)
+    assert not _block_major(m, view, plan)  # as staged
+    assert _block_major(m, hf.view_of(w, eye=FAR), plan)
     assert m.trouble() == []
     m.ok(m.lib.s3r_plan_destroy(plan))
