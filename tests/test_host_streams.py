@@ -176,3 +176,22 @@ def test_no_room_for_results_walks(m):
     assert _block_major(m, hf.view_of(w, eye=FAR), plan)
     assert m.trouble() == []
     m.ok(m.lib.s3r_plan_destroy(plan))
+
+
+@pytest.mark.parametrize("level,eye", [(3, (0.1, 0.2, 0.3)), (4, (0.3, 0.2, 1.0)), (4, (0.0, 0.0, -6.0))])
+def test_default_form_inside_the_level_walks(m, level, eye):
+    """A camera inside the level or facing away from it: blocks with a corner behind the eye have the whole viewport for
+    their rectangle, hundreds of times the rays that meet a block.  The default form walks and allocates nothing; seen
+    from outside the same plan goes block-major."""
+    w = hf.coarse_set(level, depth=1, W=300, H=200, quality=16.0)
+    plan = m.plan(w)
+    outside = hf.view_of(w, eye=NEAR)
+    assert _block_major(m, outside, plan)
+    inside = hf.view_of(w, eye=eye)
+    if eye[2] < -5:  # the level behind the camera
+        w.center = (0.0, 0.0, -9.0)
+        inside = hf.view_of(w, eye=eye)
+    before = m.lib.fake_used()
+    assert not _block_major(m, inside, plan) and m.calls("walk") == 1
+    assert m.lib.fake_used() == before and m.trouble() == []
+    m.ok(m.lib.s3r_plan_destroy(plan))
