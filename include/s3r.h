@@ -396,8 +396,8 @@ int s3r_make_color_transfer(const double* xs, const double* rgba, uint32_t npoin
  *     blocks' view rectangles (deepest blocks first) and march one block each, a deep block's rays with several
  *     lanes where few of them would set the time; the per-block results are blended per pixel in front-to-back
  *     order afterwards.  The same image bit for bit as id 0 but on rays that run in a plane between two blocks
- *     (the walk takes one of them, this form both); for levels up to 7, at the cost of (3 * 2^level - 2) x W x H
- *     x 16 bytes of device memory per data slot.
+ *     (the walk takes one of them, this form both); for levels up to 7, at the cost of (3 * 2^level - 2) x 16
+ *     bytes of device memory per pixel that the blocks cover (and half as many more) and data slot.
  *   One thread per ray (ids 0-3): a view for which block-major is the faster one (64 blocks and more with rays of
  *     some length in each; at most 1 GB of results; alpha_stop of 1 or more) renders in that form, restricted to
  *     the blocks that the walk meets -- the walk's image bit for bit.  A render that is captured by the caller
@@ -406,7 +406,7 @@ int s3r_make_color_transfer(const double* xs, const double* rgba, uint32_t npoin
  *     allocated in stream order (cudaMallocAsync) by the first view that needs them and again by one that needs more,
  *     without waiting for the device; where there is no room, ids 0-3 walk and the others fail.  Frames of a plan on
  *     several streams use them in turn.  A captured block-major render (ids 16-18) holds them: capture it again after
- *     a view of more pixels or more work items.
+ *     a view that covers more or looks from closer.
  * The autotuner times every form. */
 #define S3R_RENDER_TILES_WALK 16u
 #define S3R_RENDER_TILES 19u

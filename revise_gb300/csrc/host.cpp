@@ -951,11 +951,10 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
         if (!asked && covered * seg_pixel_bytes(p) + n * sizeof(uint2) > kSegAutoBytes) seg = false;
     }
     if (seg) {
-        // Asked for by its id, the form may be in a caller's graph, which is replayed after views of the same size that
-        // cover more of it: room for the whole viewport.  Else some room to move closer in.
+        // some room to move closer in
         const uint64_t most = (uint64_t)view->W * view->H,
-                       some = std::min({covered + covered / 2, most, kSegAutoBytes / seg_pixel_bytes(p)});
-        const int rc = plan_ensure_segments(p, asked ? most : std::max(covered, some), n, s);
+                       some = std::min(covered + covered / 2, asked ? most : std::min(most, kSegAutoBytes / seg_pixel_bytes(p)));
+        const int rc = plan_ensure_segments(p, std::max({covered, some, (uint64_t)1}), n, s);
         if (rc && asked) return rc;
         if (rc) {
             // no room: the walk gives the same image
