@@ -1189,14 +1189,15 @@ template <int Fmt> struct Texels {
     float f[3];
 };
 
-// Sample kf (a whole number) of the ray in its block.  kTogether (the rays of a warp march one block): inside the
+// Sample k of the ray in its block.  kTogether (the rays of a warp march one block): inside the
 // brick the cell's 8 texels are four pairs in four rows, and a sample in the outer half texel (a ray's first one, on
 // the block's face) takes the clamped indices.  Rays in different blocks meet their faces at different times, so
 // there every sample takes the clamped indices (320 x 240 pixels of a level-2 set: 109 us against 115 us).
 template <int Fmt, bool kTogether>
-__device__ __forceinline__ void fetch_texels(const void* brick, const BlockRay& r, float kf, Texels<Fmt>& x)
+__device__ __forceinline__ void fetch_texels(const void* brick, const BlockRay& r, int k, Texels<Fmt>& x)
 {
     const uint32_t hi = r.n - 1;
+    const float kf = (float)k;
     int a[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -1268,14 +1269,14 @@ __device__ __forceinline__ Premul march_block(const s3r_view& v, const BlockRay&
             if (Fmt != S3R_BRICK_F32) val = __fmaf_rn(scale, val, offset);
             return blend(tf_colour(tf, v.tf_n, rel(val)));
         };
-        fetch_texels<Fmt, kTogether>(brick, r, 0.f, ca);
-        const float last = (float)(r.samples - 1); // samples 0 .. last-1
-        float k = 0.f; // the samples taken, a whole number
+        fetch_texels<Fmt, kTogether>(brick, r, 0, ca);
+        const int last = r.samples - 1; // samples 0 .. last-1
+        int k = 0;                      // the samples taken (a float would stop counting at 2^24)
         while (true) {
-            k += 1.f;
+            ++k;
             if (k < last) fetch_texels<Fmt, kTogether>(brick, r, k, cb);
             if (sample(ca) || k >= last) break;
-            k += 1.f;
+            ++k;
             if (k < last) fetch_texels<Fmt, kTogether>(brick, r, k, ca);
             if (sample(cb) || k >= last) break;
         }
@@ -1298,29 +1299,28 @@ __device__ __forceinline__ Premul march_block(const s3r_view& v, const BlockRay&
 // order, so the result is march_block's bit for bit.  A ray's chain of samples is that much shorter, for a third more
 // instructions in all; a warp's 32 lanes call it together (last: samples to take, 0 for no ray).
 template <int Fmt, bool kTex>
-__device__ __forceinline__ Premul march_block_lanes(const s3r_view& v, const BlockRay& r, float last, const void* brick,
+__device__ __forceinline__ Premul march_block_lanes(const s3r_view& v, const BlockRay& r, int last, const void* brick,
                                                     float scale, float offset, uint32_t depth, const TfTable& tf,
                                                     const Relative& rel, float of, uint32_t lanes, uint32_t sub,
                                                     uint32_t& taken)
 {
     const float il = layer_exponent(depth, v.level, v.quality);
     Premul acc{0.f, 0.f, 0.f, 0.f};
-    bool open = last > 0.f;
-    float k0 = 0.f; // the group's first sample
-    const float fsub = (float)sub, flanes = (float)lanes;
+    bool open = last > 0;
+    int k0 = 0; // the group's first sample
     Texels<Fmt> cur, nxt;
     if constexpr (!kTex)
-        if (fsub < last) fetch_texels<Fmt, true>(brick, r, fsub, cur);
+        if ((int)sub < last) fetch_texels<Fmt, true>(brick, r, (int)sub, cur);
     while (__any_sync(0xffffffffu, open)) {
-        const float k = k0 + fsub;
+        const int k = k0 + (int)sub, next = k + (int)lanes;
         if constexpr (!kTex)
-            if (open && k + flanes < last) fetch_texels<Fmt, true>(brick, r, k + flanes, nxt);
+            if (open && next < last) fetch_texels<Fmt, true>(brick, r, next, nxt);
         // a sample outside the domain blends as nothing: all zero
         float4 col = make_float4(0.f, 0.f, 0.f, 0.f);
         if (open && k < last) {
             float val;
             bool in;
-            if constexpr (kTex) in = tex_trilinear<Fmt>(brick, r, (int)k, val);
+            if constexpr (kTex) in = tex_trilinear<Fmt>(brick, r, k, val);
             else in = filter_texels<Fmt>(cur, val);
             if (in) {
                 if (Fmt != S3R_BRICK_F32) val = __fmaf_rn(scale, val, offset);
@@ -1338,7 +1338,7 @@ __device__ __forceinline__ Premul march_block_lanes(const s3r_view& v, const Blo
                 acc.g = __fmaf_rn(w, cg, acc.g);
                 acc.b = __fmaf_rn(w, cb, acc.b);
                 acc.a = __fadd_rn(acc.a, w);
-                k0 += 1.f;
+                ++k0;
                 if (sub == 0) ++taken;
                 open = !(acc.a > kAlphaThreshold) && k0 < last;
             }
@@ -1592,7 +1592,7 @@ __global__ void __launch_bounds__(kSegThreads, 2) frame_segments_kernel(FrameArg
         Premul acc{0.f, 0.f, 0.f, 0.f};
         if (kLanes && log_lanes) {
             const uint32_t lanes = 1u << log_lanes, sub = lane & (lanes - 1);
-            acc = march_block_lanes<Fmt, kTex>(v, r, hit ? (float)(r.samples - 1) : 0.f, brick, scale, offset,
+            acc = march_block_lanes<Fmt, kTex>(v, r, hit ? r.samples - 1 : 0, brick, scale, offset,
                                                rb->depth, tf, rel, of, lanes, sub, taken);
             hit = hit && sub == 0;
         } else if (hit) {
@@ -1768,8 +1768,9 @@ __device__ __forceinline__ uint32_t clamped_corner(const int a[3], Dim g, int q)
     return ((uint32_t)z * g.n + (uint32_t)y) * g.pitch + (uint32_t)x;
 }
 
-__device__ __forceinline__ void fetch_grad_cell(const float* brick, const BlockRay& r, float kf, GradCell& c)
+__device__ __forceinline__ void fetch_grad_cell(const float* brick, const BlockRay& r, int k, GradCell& c)
 {
+    const float kf = (float)k;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         const float p = __fmaf_rn(r.step[d], kf, r.p0[d]);
@@ -2047,15 +2048,15 @@ __global__ void __launch_bounds__(kBackwardThreads, 8) frame_backward_kernel(Fra
             // software-pipelined as the forward march, unrolled by two with two
             // buffers: sample i's texels load while sample i-1's gradients form
             GradCell ca, cb;
-            if (r.samples > 1) fetch_grad_cell(brick, r, 0.f, ca);
-            const float last = (float)(r.samples - 1);
-            for (float k = 1.f; k <= last;) {
+            if (r.samples > 1) fetch_grad_cell(brick, r, 0, ca);
+            const int last = r.samples - 1;
+            for (int k = 1; k <= last;) {
                 if (k < last) fetch_grad_cell(brick, r, k, cb);
                 if (!step_sample(ca) || k >= last) break;
-                k += 1.f;
+                ++k;
                 if (k < last) fetch_grad_cell(brick, r, k, ca);
                 if (!step_sample(cb)) break;
-                k += 1.f;
+                ++k;
             }
             cg.put(0xffu);
             // block composite exactly as the forward kernel forms it
