@@ -343,6 +343,13 @@ struct Relative {
         const float a = __fsub_rn(val, lo);
         return fast ? div_by(a, span, y) : __fdiv_rn(a, span);
     }
+    // The texture unit's rule clamps the lookup of an infinite relative value to the table's end, which the kept
+    // reciprocal's residual would make a NaN.  (The exact filter's fraction of an infinite value is a NaN either way.)
+    __device__ __forceinline__ float clamped(float val) const
+    {
+        const float q = (*this)(val);
+        return fabsf(q) <= 3.402823466e38f ? q : __fdiv_rn(__fsub_rn(val, lo), span);
+    }
 };
 __device__ __forceinline__ Relative relative_of(const s3r_view& v)
 {
@@ -494,6 +501,7 @@ __device__ __forceinline__ F3 blinn(F3 N, F3 V, F3 L, const s3r_light& light, F3
 // kContracted: the crossing positions of the isosurface modes written as the
 // reference writes them (pos + step * t, which nvcc fuses into one fma), else
 // rounded twice as the oracle rounds them.
+// kTexRule: filtered as the texture unit does, the transfer function too.
 // kAhead: sample k + 1 is fetched before sample k is used.  The texture unit's
 // rule in software filters in its fetch, and a sample ahead only costs it
 // registers (lit volume, 64 blocks of depth 6: 10.0 against 11.0 ms).
@@ -503,7 +511,7 @@ template <bool kTex> struct BrickSampler {
     Dim n;
     TfTable tf;
     uint32_t tfn;
-    static constexpr bool kStepwise = kTex, kContracted = false, kAhead = !kTex;
+    static constexpr bool kStepwise = kTex, kTexRule = kTex, kContracted = false, kAhead = !kTex;
     using Sample = std::conditional_t<kTex, float, FieldCell>;
     __device__ void fetch(int second, F3 p, Sample& x) const
     {
@@ -520,7 +528,7 @@ template <bool kTex> struct BrickSampler {
 
 struct TextureSampler {
     cudaTextureObject_t t1, t2, tf;
-    static constexpr bool kStepwise = true, kContracted = true, kAhead = true;
+    static constexpr bool kStepwise = true, kTexRule = true, kContracted = true, kAhead = true;
     using Sample = float;
     __device__ void fetch(int second, F3 p, Sample& x) const { x = tex3D<float>(second ? t2 : t1, p.x, p.y, p.z); }
     static __device__ float value(const Sample& x) { return x; }
@@ -706,7 +714,7 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
             if (mode == S3R_MODE_DOMAIN_VOXELS) {
                 col = dom;
             } else {
-                col = smp.colour(rel(val));
+                col = smp.colour(S::kTexRule ? rel.clamped(val) : rel(val));
                 col.w = 1.f - powf(1.f - col.w * of, il);
                 if (mode == S3R_MODE_ARGB_LIGHT) {
                     // renderArgbLight.hpp:44-56: only visible enough samples are lit
@@ -1288,7 +1296,7 @@ __device__ __forceinline__ Premul march_block(const s3r_view& v, const BlockRay&
             float val;
             if (!tex_trilinear<Fmt>(brick, r, i - 1, val)) continue;
             if (Fmt != S3R_BRICK_F32) val = __fmaf_rn(scale, val, offset);
-            if (blend(tex_tf_lookup(tf.raw(), v.tf_n, rel(val)))) break;
+            if (blend(tex_tf_lookup(tf.raw(), v.tf_n, rel.clamped(val)))) break;
         }
         return acc;
     }
@@ -1324,7 +1332,7 @@ __device__ __forceinline__ Premul march_block_lanes(const s3r_view& v, const Blo
             else in = filter_texels<Fmt>(cur, val);
             if (in) {
                 if (Fmt != S3R_BRICK_F32) val = __fmaf_rn(scale, val, offset);
-                col = kTex ? tex_tf_lookup(tf.raw(), v.tf_n, rel(val)) : tf_colour(tf, v.tf_n, rel(val));
+                col = kTex ? tex_tf_lookup(tf.raw(), v.tf_n, rel.clamped(val)) : tf_colour(tf, v.tf_n, rel(val));
                 col.w = __fsub_rn(1.f, __powf(__fmaf_rn(-col.w, of, 1.f), il));
             }
         }
