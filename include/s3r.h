@@ -403,8 +403,8 @@ int s3r_make_color_transfer(const double* xs, const double* rgba, uint32_t npoin
  *     the blocks that the walk meets -- the walk's image bit for bit.  A render that is captured by the caller
  *     always walks: the graph may be replayed after other views and shows the view staged last.
  *   Block results belong to the plan: up to 1 GB per data slot (the second one with s3r_frame_run_host) for ids 0-3,
- *     allocated in stream order (cudaMallocAsync) by the first view that needs them and again by one that needs more,
- *     without waiting for the device; where there is no room, ids 0-3 walk and the others fail.  Frames of a plan on
+ *     allocated by the first view that needs them and again by one that needs more, which waits for the device;
+ *     where there is no room, ids 0-3 walk and the others fail.  Frames of a plan on
  *     several streams use them in turn.  A captured block-major render (ids 16-18) holds them: capture it again after
  *     a view that covers more or looks from closer.
  * The autotuner times every form. */

@@ -766,9 +766,10 @@ uint64_t seg_pixel_bytes(const s3r_plan* p) { return (3ull * (1u << p->level) - 
 
 // The block-major render's per-rank results and rank masks for `npix` pixels, in the second data slot too once there is
 // a host-buffer pipeline, and behind those of the first slot room for `items` work items.  Called before a frame is
-// launched in the block-major form.  A slot that is too small is allocated again, in the order of stream `s` and of the
-// frames that use the slots: no call of a render waits for the device.  The plan's captured frames are dropped with it
-// (they hold the old buffers).
+// launched in the block-major form.  The first allocation waits for nothing; a slot that has become too small waits for
+// the frames that use it and is allocated again, which drops the plan's captured frames (they hold the old buffers).
+// (In stream order, by cudaMallocAsync and cudaFreeAsync, a larger view's first frame takes 290 instead of 360 us, but a
+// plan's first one, which maps new memory, 730 instead of 520: 512 mixed blocks at 1920x1080.)
 int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t items, cudaStream_t s)
 {
     s3r_ctx* ctx = p->ctx;
@@ -779,20 +780,21 @@ int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t items, cudaStream_
         if (capturing(s)) return fail(ctx, S3R_ERR_UNSUPPORTED, "allocation in a stream capture");
         std::lock_guard<std::mutex> lock(p->seg_turn);
         plan_drop_graph(p);
-        for (cudaEvent_t done : p->seg_done) S3R_CUDA(ctx, cudaStreamWaitEvent(s, done, 0)); // both slots read the items
-        if (p->seg_buf[b]) S3R_CUDA(ctx, cudaFreeAsync(p->seg_buf[b], s));
+        if (p->seg_buf[b]) {
+            for (cudaEvent_t done : p->seg_done) S3R_CUDA(ctx, cudaEventSynchronize(done)); // both slots read the items
+            cudaFree(p->seg_buf[b]);
+        }
         p->seg_buf[b] = nullptr;
         const uint64_t pixels = std::max(npix, p->seg_pixels[b]),
                        room = b ? 0 : (p->seg_items_cap >= items ? p->seg_items_cap : items + items / 4);
         p->seg_pixels[b] = 0;
         if (b == 0) p->seg_items_cap = 0;
         const size_t results = pixels * seg_pixel_bytes(p), masks = (size_t)words * pixels * sizeof(unsigned long long);
-        const cudaError_t e =
-            cudaMallocAsync(reinterpret_cast<void**>(&p->seg_buf[b]), results + masks + room * sizeof(uint2), s);
+        const cudaError_t e = cudaMalloc(&p->seg_buf[b], results + masks + room * sizeof(uint2));
         if (e != cudaSuccess) {
             p->seg_buf[b] = nullptr;
             (void)cudaGetLastError(); // an allocation failure leaves no error behind for later launches
-            return cuda_fail(ctx, e, "cudaMallocAsync(block-major render buffers)");
+            return cuda_fail(ctx, e, "cudaMalloc(block-major render buffers)");
         }
         char* mask = reinterpret_cast<char*>(p->seg_buf[b]) + results;
         p->seg_mask[b] = reinterpret_cast<unsigned long long*>(mask);

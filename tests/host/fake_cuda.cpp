@@ -210,30 +210,17 @@ cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return allocate(p, n, 
 cudaError_t cudaFree(void* p)
 {
     ++g_calls["cudaFree"];
+    // (waits for the device, but a caller that leaves it to that is told)
+    auto it = g_memory.find(static_cast<const char*>(p));
+    if (p && it != g_memory.end())
+        for (const Past& b : it->second.past) {
+            auto over = g_host.find(b.stream);
+            if (over == g_host.end() || over->second < b.time) trouble("memory freed that " + b.name + " may still use");
+        }
     join_all(g_host);
     return release(p);
 }
 cudaError_t cudaFreeHost(void* p) { return release(p); }
-cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t s)
-{
-    if (g_streams[s].capturing) trouble("cudaMallocAsync in a capture");
-    const cudaError_t e = allocate(p, n, false);
-    if (e == cudaSuccess) {
-        const Access a{*p, n, true};
-        run(Op{"cudaMallocAsync", [a] { return std::vector<Access>{a}; }, nullptr}, s);
-    }
-    return e;
-}
-cudaError_t cudaFreeAsync(void* p, cudaStream_t s)
-{
-    if (g_streams[s].capturing) trouble("cudaFreeAsync in a capture");
-    auto it = g_memory.find(static_cast<const char*>(p));
-    if (it == g_memory.end()) return cudaSuccess;
-    const Access a{p, it->second.bytes, true};
-    run(Op{"cudaFreeAsync", [a] { return std::vector<Access>{a}; }, nullptr}, s);
-    return release(p);
-}
-
 cudaError_t cudaDeviceSynchronize()
 {
     ++g_calls["cudaDeviceSynchronize"];
