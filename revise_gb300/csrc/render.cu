@@ -1985,7 +1985,11 @@ __global__ void __launch_bounds__(kBackwardThreads, 8) frame_backward_kernel(Fra
                 // the forward's v01 up to the last ulp (a reciprocal instead of the division), and its colour
                 const float u = __fmaf_rn(__fmul_rn(__fsub_rn(val, v.field_min), inv_span), (float)v.tf_n, -0.5f);
                 int j;
-                const float f = u - floor_small(fminf(fmaxf(u, -1.f), (float)v.tf_n - 0.5f), j);
+                // the fraction of the clamped u: beyond the table the pair is one entry twice, and a fraction that grew with
+                // the distance would leave the entry's gradient to the difference of two large sums (the product by
+                // zero passes the NaN of an infinite value on, as the forward does)
+                const float uc = fminf(fmaxf(u, -1.f), (float)v.tf_n - 0.5f);
+                const float f = __fmaf_rn(0.f, u, uc) - floor_small(uc, j);
                 const float4 p = tf.p[j + 1];
                 float4 d;
                 if (tf.d) {
