@@ -1500,13 +1500,17 @@ __device__ __forceinline__ uint32_t ray_rank(const float dir[3], uint32_t ix, ui
 }
 
 // Whether the per-ray walk (walk_blocks) meets this block on the ray, block_ray having found that the ray passes it.
-// It does wherever the middle of the ray's segment lies inside the block by more than the walk's rounding (its
-// crossing times are summed up over as many blocks as it has passed); only a ray that grazes the block -- along a
-// face, past an edge -- is walked to see which of the blocks around it the walk takes.
+// It does wherever the middle of the ray's segment lies inside the block by more than the walk's rounding; only a ray
+// that grazes the block -- along a face, past an edge -- is walked to see which of the blocks around it the walk takes.
+// A crossing time is a quotient (two roundings, and one of its numerator) and up to m sums of a period: off by at most
+// (m + 4) 2^-24 of the time itself; two of them are compared, which is as far along the ray as |dir| times that, and
+// twice as much is asked for.
 __device__ __forceinline__ bool on_walk(const s3r_view& v, const float org[3], const float dir[3], const float inv[3],
                                         const RenderBlock& rb, const BlockRay& r, uint32_t cell)
 {
-    const float tm = 0.5f * (r.tau_enter + r.tau_exit), room = rb.half - (2e-4f + 1e-5f * (float)(1u << v.level));
+    const float way = fmaxf(fmaxf(fabsf(dir[0]), fabsf(dir[1])), fabsf(dir[2])) * r.tau_exit;
+    const float tm = 0.5f * (r.tau_enter + r.tau_exit),
+                room = rb.half - (1e-5f + (float)((1u << v.level) + 4u) * 2.3841858e-7f * way); // 2^-22
     bool inside = true;
 #pragma unroll
     for (int d = 0; d < 3; ++d) inside &= fabsf(__fmaf_rn(dir[d], tm, org[d]) - rb.center[d]) < room;
