@@ -528,7 +528,7 @@ class VsWorker:
         self.ctx._check(self.lib.s3r_render_scene_part(self.ctx.h, C.byref(s.view),
                                                        C.byref(pres) if pres is not None else None, C.byref(wb),
                                                        bmin, bmax, ptr(self.renderer._tf), ptr(self.viewport), rect,
-                                                       None))
+                                                       _stream(None)))
         if rect[2] == 0:
             return (0, 0), (0, 0), torch.zeros(1, dtype=torch.int32, device="cuda")
         crop = torch.empty(rect[2] * rect[3], dtype=torch.int32, device="cuda")
@@ -551,7 +551,7 @@ class VsWorker:
         self.ctx._check(self.lib.s3r_render_scene_part_bricks(self.ctx.h, plan.h, C.byref(s.view),
                                                               C.byref(pres) if pres is not None else None,
                                                               ptr(bricks2), bmin, bmax, ptr(self.renderer._tf),
-                                                              ptr(self.viewport), rect, None))
+                                                              ptr(self.viewport), rect, _stream(None)))
         if rect[2] == 0:
             return (0, 0), (0, 0), torch.zeros(1, dtype=torch.int32, device="cuda")
         crop = torch.empty(rect[2] * rect[3], dtype=torch.int32, device="cuda")
