@@ -11,7 +11,9 @@ Mirrors the reference's interfaces for this path:
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
+import threading
 from dataclasses import dataclass
 
 import numpy as np
@@ -452,6 +454,8 @@ class RenderSharedState:
         self.blocks = workload.blocks
         self.block_index = {(int(b[0]), int(b[1]), int(b[2])): i for i, b in enumerate(workload.blocks)}
         self._dev = {}
+        self._boxes = collections.OrderedDict()
+        self._boxes_lock = threading.Lock()
 
     def device_all(self):
         """All blocks' nodes and values as single device arrays (n2i as int16 bits, values float32),
@@ -463,6 +467,33 @@ class RenderSharedState:
                                 np.ascontiguousarray(w.node_off, dtype=np.uint64), to_device_n2i(w.n2i),
                                 torch.from_numpy(np.ascontiguousarray(w.sparse, dtype=np.float32)).cuda())
         return self._dev["all"]
+
+    def device_box(self, bmin, bmax):
+        """device_all for the blocks of an index box, which alone go to the device; the last boxes are kept, of as many
+        nodes together as the level has at most."""
+        if "all" in self._dev:
+            return self._dev["all"]
+        key = (*bmin, *bmax)
+        with self._boxes_lock:
+            if key in self._boxes:
+                self._boxes.move_to_end(key)
+                return self._boxes[key]
+            torch = _torch()
+            inside = ((self.blocks[:, :3] >= np.array(bmin)) & (self.blocks[:, :3] < np.array(bmax))).all(1)
+            if inside.all():
+                return self.device_all()
+            picked = np.flatnonzero(inside)
+            nodes = [self.w.block_nodes(int(b)) for b in picked]
+            counts = np.array([v.shape[0] for _, v in nodes], dtype=np.uint64)
+            node_off = np.concatenate([[0], np.cumsum(counts)]).astype(np.uint64)
+            n2i = np.concatenate([x for x, _ in nodes]) if nodes else np.zeros((0, 3), np.uint16)
+            values = np.concatenate([v for _, v in nodes]) if nodes else np.zeros(0, np.float32)
+            held = int(node_off[-1]) + sum(int(b[1][-1]) for b in self._boxes.values())
+            while self._boxes and held > self.w.nodes:
+                held -= int(self._boxes.popitem(last=False)[1][1][-1])
+            self._boxes[key] = (np.ascontiguousarray(self.blocks[picked], dtype=np.uint32), node_off,
+                                to_device_n2i(n2i), torch.from_numpy(values.astype(np.float32, copy=False)).cuda())
+            return self._boxes[key]
 
     def device_nodes(self, b: int):
         if b not in self._dev:
@@ -504,15 +535,19 @@ class VsWorker:
         return ImagePartResult(origin, size, pix)
 
     def render_scene_part_native(self, level: int, index_box_min, index_box_max, pres=None, sparse2_dev=None):
-        """renderScenePart as one native call (s3r_render_scene_part): clear, back-to-front block loop
-        (interpolate + render per block), bounding rectangle; the cropped part stays in device memory:
-        (origin, size, int32 tensor), size (0, 0) when nothing was drawn."""
+        """renderScenePart as one native call (s3r_render_scene_part): clear, the box's blocks interpolated and
+        rendered, blended back to front, bounding rectangle; the cropped part stays in device memory:
+        (origin, size, int32 tensor), size (0, 0) when nothing was drawn.  sparse2_dev: the secondary field's
+        values of the whole level."""
+        return self._render_native(self.state.device_all(), index_box_min, index_box_max, pres, sparse2_dev)
+
+    def _render_native(self, level_data, index_box_min, index_box_max, pres=None, sparse2_dev=None):
         torch = _torch()
         s = self.state
         W, H = s.view.W, s.view.H
         if self.viewport is None or self.viewport.numel() != W * H:
             self.viewport = torch.empty(W * H, dtype=torch.int32, device="cuda")
-        blocks, node_off, n2i_dev, sparse_dev = s.device_all()
+        blocks, node_off, n2i_dev, sparse_dev = level_data
         wb = WorkerBlocks()
         wb.nblocks = blocks.shape[0]
         wb.blocks = arr(blocks, C.c_uint32)
@@ -536,8 +571,8 @@ class VsWorker:
         return (int(rect[0]), int(rect[1])), (int(rect[2]), int(rect[3])), crop
 
     def render_scene_part_plan(self, plan, level: int, index_box_min, index_box_max, pres=None, bricks2=None):
-        """renderScenePart from a FramePlan's brick store (interpolated with plan.interp for all blocks):
-        one render launch per block of the box, back to front; the cropped part in device memory."""
+        """renderScenePart from a FramePlan's brick store (interpolated with plan.interp for all blocks): the box's
+        blocks marched by one launch and blended back to front; the cropped part in device memory."""
         torch = _torch()
         s = self.state
         W, H = s.view.W, s.view.H
@@ -561,11 +596,13 @@ class VsWorker:
     def render_scene_part_device(self, level: int, index_box_min, index_box_max, cancelled=_never):
         """renderScenePart with the cropped part left in device memory: (origin, size, int32 tensor),
         size (0, 0) when nothing was drawn; None when cancelled.  A render that nothing can cancel is one native
-        call; `cancelled` is asked between blocks, so with it they go one by one."""
-        if cancelled is _never:
-            return self.render_scene_part_native(level, index_box_min, index_box_max)
-        torch = _torch()
+        call; `cancelled` is asked between blocks, so with it they go one by one.  (One by one too where the view is
+        not the workload's own: of another level, or from another eye, by which the native call would order.)"""
         s = self.state
+        if cancelled is _never and level == s.view.level and s.view.cam.eye[:] == [C.c_float(x).value for x in s.w.eye]:
+            return self._render_native(s.device_box([int(x) for x in index_box_min], [int(x) for x in index_box_max]),
+                                       index_box_min, index_box_max)
+        torch = _torch()
         W, H = s.view.W, s.view.H
         if self.viewport is None or self.viewport.numel() != W * H:
             self.viewport = torch.empty(W * H, dtype=torch.int32, device="cuda")
