@@ -28,6 +28,7 @@ thread_local std::string g_last_error;
 struct s3r_ctx {
     int device = 0;
     std::string err;
+    cudaError_t last_cuda = cudaSuccess; // behind the last S3R_ERR_CUDA
     float* grid = nullptr; // block interpolation scratch: scattered node values, and their mask (rows of whole words)
     size_t grid_cap = 0;   // floats
     uint32_t* grid_bits = nullptr;
@@ -187,6 +188,7 @@ int fail(s3r_ctx* ctx, int code, const std::string& msg)
 
 int cuda_fail(s3r_ctx* ctx, cudaError_t e, const char* what)
 {
+    if (ctx) ctx->last_cuda = e;
     return fail(ctx, S3R_ERR_CUDA, std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")");
 }
 
@@ -2598,6 +2600,33 @@ int part_textures(s3r_ctx* ctx, const uint32_t need[S3R_MAX_DEPTH + 1], int fiel
     return S3R_OK;
 }
 
+// After a part's launches failed with `rc`: whether there was no room for what they need at once.  The part's memory is
+// given back then, for the block-by-block loop, which needs one block's.
+bool part_no_room(s3r_ctx* ctx, int rc, cudaStream_t s)
+{
+    cudaStreamSynchronize(s); // the staged tables may still be read
+    if (rc != S3R_ERR_CUDA || ctx->last_cuda != cudaErrorMemoryAllocation) return false;
+    for (auto& per_field : ctx->worker_tex)
+        for (auto& per_depth : per_field) {
+            for (s3r_texture* t : per_depth) s3r_texture_destroy(t);
+            per_depth.clear();
+        }
+    ctx->worker_tex_bytes = 0;
+    auto give = [](auto*& p, size_t& cap) {
+        if (p) cudaFree(p);
+        p = nullptr;
+        cap = 0;
+    };
+    for (int f = 0; f < 2; ++f) give(ctx->worker_dense[f], ctx->worker_cap[f]);
+    give(ctx->part_lists, ctx->part_lists_cap);
+    give(ctx->grid, ctx->grid_cap);
+    give(ctx->grid_bits, ctx->grid_bits_cap);
+    (void)cudaGetLastError(); // the failure leaves no error behind for later launches
+    ctx->err.clear();
+    set_thread_error("");
+    return true;
+}
+
 // A block of the part: its index in the caller's list and its view rectangle.
 struct PartBlock {
     uint32_t b;
@@ -2809,12 +2838,10 @@ int s3r_render_scene_part(s3r_ctx* ctx, const s3r_view* view, const s3r_presenta
         s3r_presentation argb{};
         argb.mode = S3R_MODE_ARGB;
         ctx->part_used = 0; // every call ends with its stream drained
-        if ((rc = part_from_nodes(ctx, view, pres ? pres : &argb, wb, list, span, tf, viewport, s))) {
-            cudaStreamSynchronize(s); // the staged tables may still be read
-            return rc;
-        }
+        rc = part_from_nodes(ctx, view, pres ? pres : &argb, wb, list, span, tf, viewport, s);
+        if (rc && !part_no_room(ctx, rc, s)) return rc;
         int32_t overflow = 0;
-        if ((rc = bound_rect(ctx, viewport, view->W, view->H, rect, &overflow, s)) || !overflow) return rc;
+        if (!rc && ((rc = bound_rect(ctx, viewport, view->W, view->H, rect, &overflow, s)) || !overflow)) return rc;
         if ((rc = s3r_clear_viewport(ctx, viewport, view->W, view->H, clear, stream))) return rc;
     }
     for (const PartBlock& p : list) {
@@ -2910,12 +2937,10 @@ int s3r_render_scene_part_bricks(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* v
             r.src2 = secondary ? (unsigned long long)(uintptr_t)(b2 + o) : 0;
         }
         ctx->part_used = 0; // every call ends with its stream drained
-        if ((rc = part_blend(ctx, view, pres ? pres : &argb, refs, span, tf, 0, false, viewport, s))) {
-            cudaStreamSynchronize(s); // the staged tables may still be read
-            return rc;
-        }
+        rc = part_blend(ctx, view, pres ? pres : &argb, refs, span, tf, 0, false, viewport, s);
+        if (rc && !part_no_room(ctx, rc, s)) return rc;
         int32_t overflow = 0;
-        if ((rc = bound_rect(ctx, viewport, view->W, view->H, rect, &overflow, s)) || !overflow) return rc;
+        if (!rc && ((rc = bound_rect(ctx, viewport, view->W, view->H, rect, &overflow, s)) || !overflow)) return rc;
         if ((rc = s3r_clear_viewport(ctx, viewport, view->W, view->H, clear, stream))) return rc;
     }
     for (const PartBlock& p : list) {

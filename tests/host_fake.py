@@ -83,6 +83,19 @@ class Machine:
         self.ok(self.lib.s3r_frame_plan(self.h, C.byref(d), C.byref(h)))
         return h
 
+    def part(self, w, view, pres=None, stream=None):
+        """s3r_render_scene_part of the whole level; returns the rectangle."""
+        wb = _lib.WorkerBlocks()
+        blocks, off = np.ascontiguousarray(w.blocks, np.uint32), np.ascontiguousarray(w.node_off, np.uint64)
+        self._keep += [blocks, off]
+        wb.nblocks, wb.blocks, wb.node_off = blocks.shape[0], _lib.arr(blocks, C.c_uint32), _lib.arr(off, C.c_uint64)
+        wb.n2i, wb.sparse, wb.sparse2 = self.buffer(3 * w.nodes, np.uint16), self.buffer(w.nodes), self.buffer(w.nodes)
+        lo, hi, rect = (C.c_uint32 * 3)(0, 0, 0), (C.c_uint32 * 3)(*[1 << w.level] * 3), (C.c_int32 * 4)()
+        self.ok(self.lib.s3r_render_scene_part(self.h, C.byref(view), C.byref(pres) if pres is not None else None,
+                                               C.byref(wb), lo, hi, self.buffer(4 * view.tf_n),
+                                               self.buffer(view.W * view.H, np.uint32), rect, stream))
+        return rect[:]
+
     def render(self, plan, view, stream=None, image=None):
         self.ok(self.lib.s3r_frame_render(self.h, plan, C.byref(view), self.buffer(4 * view.tf_n),
                                           None, image or self.buffer(view.W * view.H, np.uint32), None, stream))

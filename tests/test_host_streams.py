@@ -195,3 +195,36 @@ def test_default_form_inside_the_level_walks(m, level, eye):
     assert not _block_major(m, inside, plan) and m.calls("walk") == 1
     assert m.lib.fake_used() == before and m.trouble() == []
     m.ok(m.lib.s3r_plan_destroy(plan))
+
+
+@pytest.mark.parametrize("filt", [_lib.FILTER_EXACT, _lib.FILTER_TEXTURE])
+@pytest.mark.parametrize("secondary", [False, True])
+@pytest.mark.parametrize("room", [3 << 20, 12 << 20, 60 << 20])
+def test_part_without_room_goes_block_by_block(m, filt, secondary, room):
+    """A part whose textures, dense fields or pixel lists do not fit is rendered block by block, in one block's memory; a
+    later part with room is not."""
+    w = _level2(W=640, H=480)
+    w.blocks[:, 3] = 5
+    view = hf.view_of(w, eye=NEAR, filter=filt)
+    pres = hf.host.presentation(_lib.MODE_VALUE_ON_ISOSURFACE, view, secondary_range=(0.0, 1.0)) if secondary else None
+    m.lib.fake_limit(room)
+    assert m.part(w, view, pres) == [0, 0, 640, 480]
+    assert m.calls("render_block") == 64 and m.trouble() == []
+    m.lib.fake_limit(2 ** 64 - 1)
+    assert m.part(w, view, pres) == [0, 0, 640, 480]
+    assert m.calls("render_block") == 64 and m.calls("part") == 1 and m.trouble() == []
+
+
+@pytest.mark.parametrize("room", [1 << 20, 2 ** 64 - 1])
+def test_part_of_bricks_without_room(m, room):
+    w = _level2(W=640, H=480)
+    plan = m.plan(w)
+    view = hf.view_of(w, eye=NEAR)
+    m.lib.fake_limit(room)
+    lo, hi, rect = (C.c_uint32 * 3)(0, 0, 0), (C.c_uint32 * 3)(4, 4, 4), (C.c_int32 * 4)()
+    m.ok(m.lib.s3r_render_scene_part_bricks(m.h, plan, C.byref(view), None, None, lo, hi, m.buffer(4 * 256),
+                                            m.buffer(w.W * w.H, np.uint32), rect, None))
+    assert rect[:] == [0, 0, 640, 480]
+    assert m.calls("render_block") == (64 if room < 2 ** 63 else 0) and m.trouble() == []
+    m.lib.fake_limit(2 ** 64 - 1)
+    m.ok(m.lib.s3r_plan_destroy(plan))
