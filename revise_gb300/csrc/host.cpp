@@ -766,13 +766,14 @@ void plan_free_segments(s3r_plan* p)
 
 uint64_t seg_pixel_bytes(const s3r_plan* p) { return (3ull * (1u << p->level) - 2) * sizeof(float4); }
 
-// The block-major render's per-rank results and rank masks for `npix` pixels, in the second data slot too once there is
-// a host-buffer pipeline, and behind those of the first slot room for `items` work items.  Called before a frame is
+// The block-major render's per-rank results and rank masks for `npix` pixels (`roomy` where they are allocated), in the
+// second data slot too once there is a host-buffer pipeline, and behind those of the first slot room for `items` work
+// items.  Called before a frame is
 // launched in the block-major form.  The first allocation waits for nothing; a slot that has become too small waits for
 // the frames that use it and is allocated again, which drops the plan's captured frames (they hold the old buffers).
 // (In stream order, by cudaMallocAsync and cudaFreeAsync, a larger view's first frame takes 290 instead of 360 us, but a
 // plan's first one, which maps new memory, 730 instead of 520: 512 mixed blocks at 1920x1080.)
-int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t items, cudaStream_t s)
+int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t roomy, uint64_t items, cudaStream_t s)
 {
     s3r_ctx* ctx = p->ctx;
     const uint32_t words = (3 * (1u << p->level) - 2 + 63) / 64;
@@ -787,7 +788,7 @@ int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t items, cudaStream_
             cudaFree(p->seg_buf[b]);
         }
         p->seg_buf[b] = nullptr;
-        const uint64_t pixels = std::max(npix, p->seg_pixels[b]),
+        const uint64_t pixels = p->seg_pixels[b] >= npix ? p->seg_pixels[b] : std::max(npix, roomy),
                        room = b ? 0 : (p->seg_items_cap >= items ? p->seg_items_cap : items + items / 4);
         p->seg_pixels[b] = 0;
         if (b == 0) p->seg_items_cap = 0;
@@ -873,8 +874,8 @@ double seg_lanes_by_depth(const s3r_plan* p, const RenderBlock* table, uint32_t 
 // too: block-major marches what lies behind opaque blocks (64 FP16 blocks of depth 6, 233x238: 74 against 157 us), and
 // how opaque the data are is not known here.
 // rects: the pixels of all view rectangles, each a ray and block that block-major sets up where the walk meets at most
-// 3m - 2 blocks a ray.  Seen from outside they are 0.3 to 0.9 times as many; inside the level a block with a corner behind the eye
-// has the whole viewport for its rectangle.  From 1.0 times on (1.3 in small views) the empty rays cost more than the
+// 3m - 2 blocks a ray.  Seen from outside they are 0.3 to 0.9 times as many; inside the level a block with a corner
+// behind the eye has the whole viewport for its rectangle.  From 1.0 times on (1.3 in small views) the empty rays cost more than the
 // march gains: level 3 of depths 3-5, 1280x720, 0.8 times: 670 against 668 us, 1.1: 781 against 712, 3.4: 1755 against
 // 590; level 4 of depths 2-4, 320x200, 1.3: 133 against 157, 1.7: 152 against 117, 46 times: 2818 against 75.
 constexpr uint64_t kSegAutoBytes = 1ull << 30; // of block results and items
@@ -899,6 +900,8 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
     const bool asked = p->render_tile >= (uint32_t)kRenderWalkTiles; // block-major by its id
     if (asked && (3 * (1u << p->level) - 2 + 63) / 64 > kSegMaskWords)
         return fail(ctx, S3R_ERR_UNSUPPORTED, "the block-major render covers levels up to 7");
+    // 8x4-pixel items unless asked: 16x2 take 293 against 306 us on 4096 mixed blocks (475 against 511 close up), and 1 to
+    // 4 % more on 64 and 512 (64 of depth 6: 119 against 116); 4x8 take 0 to 18 % more than 8x4
     const int shape = asked ? (int)(p->render_tile - (uint32_t)kRenderWalkTiles) : 0;
     // a view staged for another form (the autotuner's) or, since then, for fewer data slots is staged again
     const bool same = p->have_view && std::memcmp(&p->last_view, view, sizeof(s3r_view)) == 0 &&
@@ -956,9 +959,9 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
     }
     if (seg) {
         // some room to move closer in
-        const uint64_t most = (uint64_t)view->W * view->H,
-                       some = std::min(covered + covered / 2, asked ? most : std::min(most, kSegAutoBytes / seg_pixel_bytes(p)));
-        const int rc = plan_ensure_segments(p, std::max({covered, some, (uint64_t)1}), n, s);
+        uint64_t roomy = std::min(covered + covered / 2, (uint64_t)view->W * view->H);
+        if (!asked) roomy = std::min(roomy, kSegAutoBytes / seg_pixel_bytes(p));
+        const int rc = plan_ensure_segments(p, std::max<uint64_t>(covered, 1), roomy, n, s);
         if (rc && asked) return rc;
         if (rc) {
             // no room: the walk gives the same image
@@ -1026,7 +1029,7 @@ int plan_launch_interp(s3r_plan* p, const float* sparse, cudaStream_t s, uint32_
 // caller's capture is ordered by the caller, its graph being launched where this cannot see it.)
 template <class F> int plan_in_turn(s3r_plan* p, bool seg, int data, cudaStream_t s, F&& body)
 {
-    if (!seg || capturing(s)) return body();
+    if (!seg || (p->render_tile >= (uint32_t)kRenderWalkTiles && capturing(s))) return body();
     std::lock_guard<std::mutex> lock(p->seg_turn);
     S3R_CUDA(p->ctx, cudaStreamWaitEvent(s, p->seg_done[data], 0));
     const int rc = body();

@@ -164,6 +164,19 @@ def test_growing_views(m):
     m.ok(m.lib.s3r_plan_destroy(plan))
 
 
+@pytest.mark.parametrize("tile", [0, 16])
+def test_a_little_more_fits(m, tile):
+    """Views that cover up to half as many pixels again as a plan's first one reuse its buffers."""
+    w = _level2()
+    plan = m.plan(w, tile)
+    m.render(plan, hf.view_of(w, eye=FAR))
+    before = m.calls("cudaMalloc")
+    for z in (39.0, 38.0, 40.0):
+        m.render(plan, hf.view_of(w, eye=(6.0, 12.0, z)))
+    assert m.calls("cudaMalloc") == before and m.calls("segments") == 4
+    m.ok(m.lib.s3r_plan_destroy(plan))
+
+
 def test_no_room_for_results_walks(m):
     """Without memory for the block results the default form walks, and what other calls then queue is clean."""
     w = _level2(W=640, H=480)
