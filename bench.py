@@ -412,6 +412,10 @@ def run_gb300(a):
     samples.zero_()
     render_ms = timed(lambda: plan.render(view, tf, rgba, None, samples), max(5, a.steps // 2))
     nsamp = int(samples.item()) / max(5, a.steps // 2)
+    # the form that ran: ids below RENDER_TILES_WALK go block-major (a march and a composite) where that pays
+    before = ctx.launches
+    plan.render(view, tf, rgba)
+    render_form = "block-major" if ctx.launches - before > 1 else "per-ray walk"
     t_interp = statistics.median(interp_ms)
     t_render = statistics.median(render_ms)
 
@@ -473,8 +477,8 @@ def run_gb300(a):
     tp = ROOT / "profiles" / "interp_tiles_cfg3_traffic.json"
     if tp.exists() and a.config == "cfg3":
         traffic = json.loads(tp.read_text()).get("dram_bytes_per_launch")
-    # the render: DRAM bytes per frame and L2 hit rate from the committed ncu capture of the same
-    # render form on this workload, over this run's CUDA-event time
+    # the render: DRAM bytes per frame and L2 hit rate from the committed ncu capture of the same render tile (a
+    # block-major id: form and item shape) on this workload, over this run's CUDA-event time
     render_roof = None
     rp = ROOT / "profiles" / "frame_render_cfg3_traffic.json"
     if rp.exists() and a.config == "cfg3":
@@ -512,7 +516,7 @@ def run_gb300(a):
                        "l2": "L2 flushed (2x129 MB write) between timed steps; 2.5 GB brick store per step",
                        "tile_cells": int(info.tile_cells), "tile_cells_by_depth": tiles_by_depth,
                        "render_tile": int(info.render_tile),
-                       "render_form": "block-major" if int(info.render_tile) >= _lib.RENDER_TILES_WALK else "per-ray walk"},
+                       "render_form": render_form},
             "ms_per_frame": ms, "frames_per_s": 1e3 / ms,
             "interp": {"ms": t_interp, "gvertices_per_s": V / (t_interp * 1e-3) / 1e9,
                        "algorithmic_bytes": alg_bytes},

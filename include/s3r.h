@@ -356,21 +356,23 @@ typedef struct s3r_worker_blocks {
 
 /* VsWorker_cu::renderScenePart (src/s3vs_worker/cuda/VsWorker_cu.cpp:225-313) natively, for the index box
  * [box_min, box_max) of view->level: the viewport (device, W*H ARGB32) cleared as clearViewport clears it,
- * the box's blocks visited back to front for the view's eye (BackToFrontOrder over the box, blocks missing
- * from wb skipped), each block's dense field interpolated from its nodes into the context's scratch
- * (s3r_interp_dense; the secondary field too for the value-on-isosurface modes) and ray-cast into the
- * viewport (s3r_render_block, or s3r_render_block_argb when pres is NULL) -- with S3R_FILTER_TEXTURE into
- * context-owned field textures per depth and a transfer-function texture filled from tf at the start of the
- * call (s3r_interp_dense_texture, s3r_render_block_texture), as the reference samples; then rect = the bounding
- * rectangle of the non-transparent pixels (s3r_bound_rect; {0,0,0,0} when empty) -- the part s3r_crop
- * cuts out.  Allocates the scratch on the first call for a depth; synchronizes the stream at the end. */
+ * the box's blocks (those missing from wb skipped) blended into it back to front for the view's eye
+ * (BackToFrontOrder over the box), byte for byte as one call per block would: s3r_interp_dense (the secondary
+ * field too for the value-on-isosurface modes) and s3r_render_block, or s3r_render_block_argb when pres is NULL --
+ * with S3R_FILTER_TEXTURE s3r_interp_dense_texture and s3r_render_block_texture, the transfer-function texture
+ * filled from tf at the start of the call, as the reference samples; then rect = the bounding rectangle of the
+ * non-transparent pixels (s3r_bound_rect; {0,0,0,0} when empty) -- the part s3r_crop cuts out.
+ * Up to 256 blocks at a time are interpolated by one set of launches and marched by one, each pixel's results blended
+ * in order afterwards; boxes of one block or of more than 64 blocks along their axes together, a pixel that more blocks
+ * contribute to than lie on a path, and parts that the memory does not suffice for go block by block.  The context
+ * keeps what a part used for the next one: up to 512 MB of dense fields per field, or 1 GB of field textures, 256 MB
+ * of results, and the scattered values of a chunk's blocks of depth 5 and up.  Allocates; synchronizes the stream. */
 int s3r_render_scene_part(s3r_ctx* ctx, const s3r_view* view, const s3r_presentation* pres,
                           const s3r_worker_blocks* wb, const uint32_t box_min[3], const uint32_t box_max[3],
                           const float* tf, uint32_t* viewport, int32_t rect[4], void* stream);
 
 /* s3r_render_scene_part with the blocks' dense fields taken from a plan's brick store (F32; interpolated
- * for all of the plan's blocks at once by s3r_frame_interp) instead of interpolated block by block:
- * per block of the box (back to front) only the render launch.  bricks2: the secondary field's brick
+ * for all of the plan's blocks at once by s3r_frame_interp) instead of interpolated for the part.  bricks2: the secondary field's brick
  * store in the plan's layout (value-on-isosurface modes). */
 int s3r_render_scene_part_bricks(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view, const s3r_presentation* pres,
                                  const void* bricks2, const uint32_t box_min[3], const uint32_t box_max[3],

@@ -688,7 +688,7 @@ __device__ __forceinline__ void run_tile(const TileArgs& a, float* s, uint32_t* 
 // ---------------------------------------------------------------- blocks from their node lists
 //
 // A subtree's dense grid from its nodes as the caller holds them (vertex indices and values in any order), tile by
-// tile as above.  A block of up to kGridDirectTiles tiles and few nodes has every tile read the whole node list; else
+// tile as above.  A block of one tile, or of 8 and up to kGridDirectNodes nodes, has every tile read the whole node list; else
 // the nodes were scattered beforehand, each value to its vertex's place in a grid and one bit into a mask of the
 // block's vertices (rows of whole words), so that a tile reads 17^2 mask rows and the values of the nodes it holds
 // instead of 17^3 grid values, and the grid itself is never cleared.

@@ -144,8 +144,8 @@ struct FrameArgs {
     float* dtf_part;      // kDtfParts zeroed copies of dtf (tf_n RGBA float4 each), summed into dtf afterwards
 };
 
-// The block-major frame render (render tile ids kRenderWalkTiles and up): its work
-// items and per-pixel block results.
+// The block-major frame render (render tile ids kRenderWalkTiles and up, and the
+// default ids where it pays): its work items and per-pixel block results.
 constexpr uint32_t kTfPlain = 3072; // table entries that the renders other than block-major and adjoint take
 constexpr uint32_t kSegMaskWords = 6; // rank masks of up to 384 ranks: levels <= 7
 constexpr uint32_t kSegLanesShift = 28, kSegCellMask = (1u << kSegLanesShift) - 1;
@@ -294,9 +294,10 @@ cudaError_t launch_compose(const s3r_image_part* parts, const s3r_image_part* pa
 
 // Render CTA pixel shapes the autotuner chooses from: {x, y} pixels.  A render
 // tile id below kRenderWalkTiles is a per-ray walk (frame_render_kernel), shape +
-// kRenderShapes * log2(lanes per ray), lanes per ray 1..8; the kSegShapes ids
-// from kRenderWalkTiles up are the block-major form with item footprint
-// kSegShapeX x kSegShapeY pixels.
+// kRenderShapes * log2(lanes per ray), lanes per ray 1..8 -- with one lane (ids
+// below kRenderShapes, the default) only where block-major does not pay; the
+// kSegShapes ids from kRenderWalkTiles up are the block-major form with item
+// footprint kSegShapeX x kSegShapeY pixels.
 constexpr int kRenderShapes = 4;
 constexpr int kRenderWalkTiles = kRenderShapes * 4;
 constexpr int kSegShapes = 3;
