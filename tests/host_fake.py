@@ -14,9 +14,11 @@ vp = C.c_void_p
 
 
 def build(out: Path) -> C.CDLL:
-    cmd = ["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-ffp-contract=off", "-I", str(ROOT / "include"), "-I",
-           str(ROOT / "revise_gb300" / "csrc"), "-I", str(cuda_home() / "include"),
-           str(ROOT / "tests" / "host" / "fake_cuda.cpp"), str(ROOT / "revise_gb300" / "csrc" / "host.cpp"), "-o", str(out)]
+    csrc = ROOT / "revise_gb300" / "csrc"
+    # -Bsymbolic: the stand-in's own functions, whatever runtime the process has loaded besides
+    cmd = ["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-ffp-contract=off", "-Wl,-Bsymbolic",
+           "-I", str(ROOT / "include"), "-I", str(csrc), "-I", str(cuda_home() / "include"),
+           str(ROOT / "tests" / "host" / "fake_cuda.cpp"), str(csrc / "host.cpp"), "-o", str(out)]
     subprocess.run(cmd, check=True)
     lib = _lib.load(out)
     lib.fake_trouble.restype = C.c_char_p
