@@ -1340,9 +1340,7 @@ static int render_block_argb_pitched(s3r_ctx* ctx, const s3r_view* view, const f
     block_sampling(view->level, idx, depth, rb);
     rb.pitch = pitch;
     for (int i = 0; i < 4; ++i) rb.rect[i] = rect[i];
-    s3r_presentation argb{};
-    argb.mode = S3R_MODE_ARGB;
-    S3R_CUDA(ctx, launch_render_block_mode(view, &argb, brick, nullptr, rb, tf, viewport, as_stream(stream)));
+    S3R_CUDA(ctx, launch_render_block_mode(view, nullptr, brick, nullptr, rb, tf, viewport, as_stream(stream)));
     if (rect[2] > 0 && rect[3] > 0) ++ctx->launches;
     return S3R_OK;
 }
@@ -2548,7 +2546,7 @@ int part_blend(s3r_ctx* ctx, const s3r_view* view, const s3r_presentation* pres,
         for (uint32_t i = 0; i < n; ++i)
             if (refs[i].rb.depth == (uint32_t)d) sorted[put++] = refs[i];
     uint32_t tw, th;
-    part_tile(pres->mode, texture, tw, th);
+    part_tile(pres ? pres->mode : S3R_MODE_ARGB, texture, tw, th);
     for (uint32_t k = 0; k < strips; ++k) {
         uint32_t* first = reinterpret_cast<uint32_t*>(host + refs_bytes + k * first_bytes);
         const int32_t s0 = y0 + (int32_t)k * rows, s1 = std::min(s0 + rows, y1);
@@ -2838,10 +2836,8 @@ int s3r_render_scene_part(s3r_ctx* ctx, const s3r_view* view, const s3r_presenta
     if (part_at_once(box_min, box_max, list.size())) {
         uint32_t span = 0;
         for (int a = 0; a < 3; ++a) span += box_max[a] - box_min[a];
-        s3r_presentation argb{};
-        argb.mode = S3R_MODE_ARGB;
         ctx->part_used = 0; // every call ends with its stream drained
-        rc = part_from_nodes(ctx, view, pres ? pres : &argb, wb, list, span, tf, viewport, s);
+        rc = part_from_nodes(ctx, view, pres, wb, list, span, tf, viewport, s);
         if (rc && !part_no_room(ctx, rc, s)) return rc;
         int32_t overflow = 0;
         if (!rc && ((rc = bound_rect(ctx, viewport, view->W, view->H, rect, &overflow, s)) || !overflow)) return rc;
@@ -2927,8 +2923,6 @@ int s3r_render_scene_part_bricks(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* v
     if (part_at_once(box_min, box_max, list.size())) {
         uint32_t span = 0;
         for (int a = 0; a < 3; ++a) span += box_max[a] - box_min[a];
-        s3r_presentation argb{};
-        argb.mode = S3R_MODE_ARGB;
         std::vector<PartRef> refs(list.size());
         for (size_t i = 0; i < list.size(); ++i) {
             const uint32_t* bl = &plan->blocks[4 * list[i].b];
@@ -2940,7 +2934,7 @@ int s3r_render_scene_part_bricks(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* v
             r.src2 = secondary ? (unsigned long long)(uintptr_t)(b2 + o) : 0;
         }
         ctx->part_used = 0; // every call ends with its stream drained
-        rc = part_blend(ctx, view, pres ? pres : &argb, refs, span, tf, 0, false, viewport, s);
+        rc = part_blend(ctx, view, pres, refs, span, tf, 0, false, viewport, s);
         if (rc && !part_no_room(ctx, rc, s)) return rc;
         int32_t overflow = 0;
         if (!rc && ((rc = bound_rect(ctx, viewport, view->W, view->H, rect, &overflow, s)) || !overflow)) return rc;

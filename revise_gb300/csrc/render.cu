@@ -620,6 +620,11 @@ struct ModeOut {
     float t;    // kMax: (max value - field min) / span
 };
 
+// s3r_render_block_argb's march: MODE_ARGB, but a sample is left out where one of its texels is NaN, not where its value
+// is (infinite texels filter to a NaN, which shows).  The two are told apart by the NaN that stands for "outside".
+constexpr int kPlainArgb = 8;
+__device__ __forceinline__ bool is_outside(float v) { return __float_as_uint(v) == 0x7fc00000u; }
+
 // The per-pixel march of one block in a field mode (renderKernel<mode>,
 // DenseFieldRenderer_cu.cu:62-215 and render*.hpp): max intensity gives the
 // block's maximum above the threshold; the colour modes (Argb, ArgbLight,
@@ -673,7 +678,7 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
     constexpr float kMax = 0.996f; // AlphaThreshold / AlphaMaxThreshold
     // kMode >= 0: the mode is fixed at compile time (one kernel per mode, as renderKernel<mode> is), so
     // only its branch is compiled in and the registers are that mode's
-    const uint32_t mode = kMode >= 0 ? (uint32_t)kMode : pr.mode;
+    const uint32_t mode = kMode == kPlainArgb ? (uint32_t)S3R_MODE_ARGB : kMode >= 0 ? (uint32_t)kMode : pr.mode;
     if (mode == S3R_MODE_MAX_INTENSITY) {
         // renderMaxIntensityProjection.hpp:30-50; the pixel holds float bits
         float maxv = v.field_min - span;
@@ -709,7 +714,7 @@ __device__ __forceinline__ ModeOut march_block_mode(const s3r_view& v, const s3r
                 open(i);
             }
             const float val = value(x, p);
-            if (isnan(val)) continue;
+            if (kMode == kPlainArgb ? is_outside(val) : isnan(val)) continue;
             float4 col;
             if (mode == S3R_MODE_DOMAIN_VOXELS) {
                 col = dom;
@@ -2135,11 +2140,21 @@ template <class F> auto with_mode(uint32_t mode, F&& f)
     }
 }
 
+inline s3r_presentation argb_presentation()
+{
+    s3r_presentation p{};
+    p.mode = S3R_MODE_ARGB;
+    return p;
+}
+
 cudaError_t launch_render_block_mode(const s3r_view* view_host, const s3r_presentation* pres, const float* brick,
                                      const float* brick2, const RenderBlock& rb, const float* tf, uint32_t* viewport,
                                      cudaStream_t s)
 {
     if (rb.rect[2] <= 0 || rb.rect[3] <= 0) return cudaSuccess;
+    const bool plain = !pres;
+    const s3r_presentation argb = argb_presentation();
+    if (plain) pres = &argb;
     dim3 block(16, 8);
     dim3 grid((rb.rect[2] + 15) / 16, (rb.rect[3] + 7) / 8);
     const size_t smem = tf_smem_entries(view_host->tf_n, false) * sizeof(float4);
@@ -2149,7 +2164,11 @@ cudaError_t launch_render_block_mode(const s3r_view* view_host, const s3r_presen
         kernel<<<grid, block, smem, s>>>(*view_host, *pres, brick, brick2, rb, tf, viewport);
         return cudaGetLastError();
     };
-    if (view_host->filter == S3R_FILTER_TEXTURE) return launch(render_block_mode_kernel<true, -1>);
+    const bool tex = view_host->filter == S3R_FILTER_TEXTURE;
+    if (plain)
+        return tex ? launch(render_block_mode_kernel<true, kPlainArgb>)
+                   : launch(render_block_mode_kernel<false, kPlainArgb>);
+    if (tex) return launch(render_block_mode_kernel<true, -1>);
     if (pres->mode == S3R_MODE_ARGB) return launch(render_block_mode_kernel<false, S3R_MODE_ARGB>);
     return launch(render_block_mode_kernel<false, -1>);
 }
@@ -2166,6 +2185,9 @@ cudaError_t launch_part(const s3r_view* view_host, const s3r_presentation* pres,
 {
     cudaError_t err = cudaMemsetAsync(a.count, 0, (size_t)a.w * a.h * sizeof(uint32_t), s);
     if (err != cudaSuccess || ctas == 0) return err;
+    const bool plain = !pres && !texture;
+    const s3r_presentation argb = argb_presentation();
+    if (!pres) pres = &argb;
     uint32_t tw, th;
     part_tile(pres->mode, texture, tw, th);
     const dim3 block(tw, th);
@@ -2176,8 +2198,10 @@ cudaError_t launch_part(const s3r_view* view_host, const s3r_presentation* pres,
         kernel<<<ctas, block, smem, s>>>(*view_host, *pres, a);
         return cudaGetLastError();
     };
+    const bool rule = view_host->filter == S3R_FILTER_TEXTURE;
     err = with_mode(pres->mode, [&](auto mode) {
         constexpr int m = decltype(mode)::value;
+        if (plain) return rule ? launch(part_blocks_kernel<1, kPlainArgb>) : launch(part_blocks_kernel<0, kPlainArgb>);
         if (texture) return launch(part_blocks_kernel<2, m>);
         return view_host->filter != S3R_FILTER_TEXTURE ? launch(part_blocks_kernel<0, m>)
                                                        : launch(part_blocks_kernel<1, -1>);

@@ -239,6 +239,7 @@ cudaError_t launch_block_prep(const PrepArgs& a, uint32_t nblocks, uint32_t max_
 cudaError_t launch_render_block_texture(const s3r_view* view_host, const s3r_presentation* pres, uint64_t field,
                                        uint64_t field2, uint64_t tf_tex, const RenderBlock& rb, uint32_t* viewport,
                                        cudaStream_t s);
+// pres nullptr, here and for a part: s3r_render_block_argb.
 cudaError_t launch_render_block_mode(const s3r_view* view_host, const s3r_presentation* pres, const float* brick,
                                      const float* brick2, const RenderBlock& rb, const float* tf, uint32_t* viewport,
                                      cudaStream_t s);

@@ -1,4 +1,4 @@
-"""Values whose relative value overflows -- infinite, or finite but far outside a narrow field range -- under the texture
+"""Infinite values in bricks; values whose relative value overflows -- infinite, or finite but far outside a narrow field range -- under the texture
 unit's filtering rule: they take the transfer function's end entries, as any value beyond the range does."""
 import numpy as np
 import pytest
@@ -66,3 +66,45 @@ def test_blocks(ctx, mode, value):
     assert mode == _lib.MODE_ARGB_LIGHT or int((got[0][0] != 0).sum()) > 0
     for a, b in zip(*(g if np.isfinite(value) else g[:1] for g in got)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("via", ["block", "part"])
+def test_infinite_texels_show_in_the_argb_call(ctx, via):
+    """s3r_render_block_argb leaves a sample out where a texel is NaN; infinite texels, whose weighted sum is a NaN, make
+    its pixel transparent (a NaN as a byte is 0).  The Argb field mode leaves out what filters to a NaN."""
+    import torch
+    from revise_gb300.api import FramePlan, RenderSharedState, VsWorker
+    w, view = _scene()
+    view.filter = _lib.FILTER_EXACT
+    tf = torch.from_numpy(np.ascontiguousarray(w.tf)).cuda()
+    plan = FramePlan(ctx, w)
+    signs = torch.ones_like(plan.bricks()[0])
+    signs[::2] = -1.0
+    plan.bricks()[0].copy_(signs * float("inf"))
+    pres = host.presentation(_lib.MODE_ARGB, view)
+    seen = []
+    for p in (None, pres):
+        if via == "part":
+            st = RenderSharedState(w, filter=_lib.FILTER_EXACT)
+            st.view = view
+            wk = VsWorker(ctx)
+            wk.set_render_shared_state(st)
+            wk.render_scene_part_plan(plan, w.level, (0, 0, 0), (2, 2, 2), p)
+            seen.append(wk.viewport.clone())
+            continue
+        vp = torch.full((w.W * w.H,), -1, dtype=torch.int32, device="cuda")  # opaque white
+        dense = plan.block_dense(0).contiguous()
+        idx = w.blocks[0, :3]
+        rect = host.block_view_rect(view, idx)
+        if p is None:
+            ctx.render_block_argb(view, dense, 3, idx, rect, tf, vp)
+        else:
+            ctx.render_block(view, p, dense, 3, idx, rect, tf, vp)
+        seen.append(vp)
+    torch.cuda.synchronize()
+    if via == "block":
+        assert int((seen[0] == 0x00ffffff).sum()) > 100  # transparent, its colour kept
+        assert int((seen[1] != -1).sum()) == 0
+    else:
+        assert int((seen[0] != 0).sum()) == 0 and int((seen[1] != 0).sum()) == 0
+    plan.close()
