@@ -849,6 +849,7 @@ double seg_lanes_by_depth(const s3r_plan* p, const RenderBlock* table, uint32_t 
             double work = 0, top = 0;
             for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d) {
                 l[d] = 0;
+                if (items[d] == 0) continue;
                 while (l[d] < 3 && chain[d] / (1u << l[d]) > limit * 1.001) ++l[d];
                 const double own = chain[d] / (1u << l[d]);
                 work += items[d] * (1u << l[d]) * (kSetup + kHit * own * (l[d] ? kShared : kSlower));

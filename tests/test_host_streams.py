@@ -241,3 +241,15 @@ def test_part_of_bricks_without_room(m, room):
     assert m.calls("render_block") == (64 if room < 2 ** 63 else 0) and m.trouble() == []
     m.lib.fake_limit(2 ** 64 - 1)
     m.ok(m.lib.s3r_plan_destroy(plan))
+
+
+def test_few_shallow_blocks_walk(m):
+    """8 blocks of depths 2 to 4 go block-major for no view: their rays have too few samples to share, whatever deeper
+    blocks would do."""
+    w = hf.coarse_set(1, depth=4, W=407, H=407)
+    w.blocks[:, 3] = [2, 3, 4, 2, 3, 4, 2, 3]
+    w.n2i = np.concatenate([np.array([[q & 1, q >> 1 & 1, q >> 2] for q in range(8)], np.uint16) << d for d in w.blocks[:, 3]])
+    plan = m.plan(w)
+    for distance in (9.0, 14.0, 30.0, 60.0):
+        assert not _block_major(m, hf.view_of(w, eye=(0.3 * distance, 0.2 * distance, distance)), plan)
+    m.ok(m.lib.s3r_plan_destroy(plan))
