@@ -876,15 +876,21 @@ double seg_lanes_by_depth(const s3r_plan* p, const RenderBlock* table, uint32_t 
 // how opaque the data are is not known here.
 // rects: the pixels of all view rectangles, each a ray and block that block-major sets up where the walk meets at most
 // 3m - 2 blocks a ray.  Seen from outside they are 0.3 to 0.9 times as many; inside the level a block with a corner
-// behind the eye has the whole viewport for its rectangle.  From 1.0 times on (1.3 in small views) the empty rays cost more than the
-// march gains: level 3 of depths 3-5, 1280x720, 0.8 times: 670 against 668 us, 1.1: 781 against 712, 3.4: 1755 against
-// 590; level 4 of depths 2-4, 320x200, 1.3: 133 against 157, 1.7: 152 against 117, 46 times: 2818 against 75.
+// behind the eye has the whole viewport for its rectangle.  From 1.0 times on (1.3 in small views) the empty rays cost
+// more than the march gains: level 3 of depths 3-5, 1280x720, 0.8 times: 670 against 668 us, 1.1: 781 against 712, 3.4:
+// 1755 against 590; level 4 of depths 2-4, 320x200, 1.3: 133 against 157, 1.7: 152 against 117, 46 times: 2818 against
+// 75.  Only views so small that their rays' chains set the time hide them: the walk takes about m (1.5 + 0.16 samples)
+// us there, of which block-major saves half, and 1000 empty rays 0.027 us (64 blocks of depth 6, 50x50 pixels, 4.9
+// times: 55 against 90 us; 240x160: 79 against 77; 64 of depths 2 and 3, 90x60: 24 against 21).
 constexpr uint64_t kSegAutoBytes = 1ull << 30; // of block results and items
 bool seg_pays(const s3r_plan* p, uint64_t covered, uint64_t rects, double samples, float quality,
               const uint32_t log_lanes[S3R_MAX_DEPTH + 1])
 {
     if (p->level < 1 || p->level > 7 || covered == 0 || covered * seg_pixel_bytes(p) > kSegAutoBytes) return false;
-    if ((double)rects > (covered < 100000 ? 1.3 : 1.0) * (double)covered * (3.0 * (1u << p->level) - 2)) return false;
+    const double m = 1u << p->level;
+    if ((double)rects > (covered < 100000 ? 1.3 : 1.0) * (double)covered * (3 * m - 2) &&
+        (double)rects * 2.7e-5 > 0.5 * m * (1.5 + 0.16 * samples))
+        return false;
     if (p->level == 1) {
         bool lanes = false; // shared rays of at least 32 samples
         for (uint32_t d = 0; d <= S3R_MAX_DEPTH; ++d) lanes |= log_lanes[d] > 0 && 1.3 * quality * (1u << d) >= 32;

@@ -253,3 +253,13 @@ def test_few_shallow_blocks_walk(m):
     for distance in (9.0, 14.0, 30.0, 60.0):
         assert not _block_major(m, hf.view_of(w, eye=(0.3 * distance, 0.2 * distance, distance)), plan)
     m.ok(m.lib.s3r_plan_destroy(plan))
+
+
+def test_small_views_inside_the_level_go_block_major(m):
+    """A camera inside the level, but so few pixels that empty rays cost nothing beside the chains of samples."""
+    w = hf.coarse_set(2, depth=6, W=50, H=50)
+    plan = m.plan(w)
+    assert _block_major(m, hf.view_of(w, eye=(0.1, 0.2, 0.3)), plan)
+    w.W, w.H = 500, 400
+    assert not _block_major(m, hf.view_of(w, eye=(0.1, 0.2, 0.3)), plan)
+    m.ok(m.lib.s3r_plan_destroy(plan))
