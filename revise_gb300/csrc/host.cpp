@@ -114,7 +114,8 @@ struct s3r_plan {
     s3r_view* view_pinned = nullptr;
     int32_t* cover_pinned = nullptr;
     uint2* seg_list_pinned = nullptr;
-    cudaEvent_t staged = nullptr;
+    cudaEvent_t staged = nullptr;   // the staging copy
+    cudaEvent_t expanded = nullptr; // the work items expanded from it
     bool have_view = false;
     s3r_view last_view{};
     // frame graphs: slot 0 for s3r_frame_run, slots 1 and 2 for the two buffers of s3r_frame_run_host
@@ -136,6 +137,7 @@ struct s3r_plan {
     uint32_t seg_words = 0;
     // a data slot's block-major frames, on whatever streams, take its results, masks and queue counter in turn
     cudaEvent_t seg_done[2] = {nullptr, nullptr};
+    unsigned long long seg_user[2] = {~0ull, ~0ull}; // the stream of the last one (its id: a handle may come again)
     std::mutex seg_turn;
     // s3r_frame_run_host: per slot a device copy of the frame's sparse values and its image, and the
     // streams and events that overlap frame k's copies with frames k-1 and k+1
@@ -804,6 +806,7 @@ int plan_ensure_segments(s3r_plan* p, uint64_t npix, uint64_t roomy, uint64_t it
         if (b == 0) p->seg_items_dev = reinterpret_cast<uint2*>(mask + masks);
         S3R_CUDA(ctx, cudaMemsetAsync(mask, 0, masks, s));
         S3R_CUDA(ctx, cudaEventRecord(p->seg_done[b], s)); // frames on other streams find it cleared
+        p->seg_user[b] = ~0ull;
         p->seg_pixels[b] = pixels;
         if (b == 0) p->seg_items_cap = room;
     }
@@ -982,12 +985,12 @@ int plan_stage_view(s3r_plan* p, const s3r_view* view, cudaStream_t s, bool fram
     std::memcpy(p->cover_pinned, cover, sizeof(cover));
     *p->view_pinned = *view;
     S3R_CUDA(ctx, cudaMemcpyAsync(p->stage_dev, p->stage_pinned, p->stage_bytes, cudaMemcpyHostToDevice, s));
+    S3R_CUDA(ctx, cudaEventRecord(p->staged, s)); // the pinned buffers may be filled again
     if (seg) {
         S3R_CUDA(ctx, launch_seg_items(p->seg_list_dev, p->nblocks, p->seg_items_dev, s));
         ++ctx->launches;
+        S3R_CUDA(ctx, cudaEventRecord(p->expanded, s));
     }
-    // after the expansion: the host pipeline orders its other slot's stream by this event alone
-    S3R_CUDA(ctx, cudaEventRecord(p->staged, s));
     p->last_view = *view;
     p->have_view = true;
     return S3R_OK;
@@ -1037,10 +1040,14 @@ int plan_launch_interp(s3r_plan* p, const float* sparse, cudaStream_t s, uint32_
 template <class F> int plan_in_turn(s3r_plan* p, bool seg, int data, cudaStream_t s, F&& body)
 {
     if (!seg || (p->render_tile >= (uint32_t)kRenderWalkTiles && capturing(s))) return body();
+    unsigned long long id = 0;
+    S3R_CUDA(p->ctx, cudaStreamGetId(s, &id));
     std::lock_guard<std::mutex> lock(p->seg_turn);
-    S3R_CUDA(p->ctx, cudaStreamWaitEvent(s, p->seg_done[data], 0));
+    if (p->seg_user[data] != id) S3R_CUDA(p->ctx, cudaStreamWaitEvent(s, p->seg_done[data], 0));
+    p->seg_user[data] = ~0ull;
     const int rc = body();
     S3R_CUDA(p->ctx, cudaEventRecord(p->seg_done[data], s));
+    p->seg_user[data] = id;
     return rc;
 }
 
@@ -1916,7 +1923,7 @@ int s3r_frame_plan(s3r_ctx* ctx, const s3r_frame_desc* desc, s3r_plan** out)
         place(p->stage_dev, p->table_dev, p->view_dev, p->cover_dev, p->seg_list_dev);
         place(p->stage_pinned, p->table_pinned, p->view_pinned, p->cover_pinned, p->seg_list_pinned);
     }
-    for (cudaEvent_t* ev : {&p->staged, &p->seg_done[0], &p->seg_done[1]})
+    for (cudaEvent_t* ev : {&p->staged, &p->expanded, &p->seg_done[0], &p->seg_done[1]})
         if ((e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming)) != cudaSuccess)
             return bail(cuda_fail(ctx, e, "cudaEventCreate"));
     // block-major render: blocks deepest first (most samples per ray), so that the longest work items start first
@@ -1960,7 +1967,7 @@ int s3r_plan_destroy(s3r_plan* p)
     f(p->dtf_part);
     f(p->seg_queue);
     plan_free_segments(p);
-    for (cudaEvent_t ev : {p->staged, p->seg_done[0], p->seg_done[1]})
+    for (cudaEvent_t ev : {p->staged, p->expanded, p->seg_done[0], p->seg_done[1]})
         if (ev) cudaEventDestroy(ev);
     delete p;
     return S3R_OK;
@@ -2217,8 +2224,8 @@ static int frame_host_submit(s3r_ctx* ctx, s3r_plan* plan, const s3r_view* view,
         for (int q = 0; q < 2; ++q) S3R_CUDA(ctx, cudaStreamSynchronize(plan->hs_comp[q]));
     }
     if ((rc = plan_stage_view(plan, view, cb, true))) return rc;
-    // the table upload may have been queued on the other slot's stream
-    S3R_CUDA(ctx, cudaStreamWaitEvent(cb, plan->staged, 0));
+    // the table upload, and the expansion of the work items after it, may have been queued on the other slot's stream
+    S3R_CUDA(ctx, cudaStreamWaitEvent(cb, plan->seg_now ? plan->expanded : plan->staged, 0));
     if ((rc = plan_launch_frame(plan, 1 + b, view, plan->hs_sparse[b], plan->hs_tf[b], nullptr, plan->hs_argb[b],
                                 nullptr, cb)))
         return rc;

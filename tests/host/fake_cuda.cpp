@@ -234,6 +234,11 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned)
     return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long* id)
+{
+    *id = reinterpret_cast<unsigned long long>(s);
+    return cudaSuccess;
+}
 cudaError_t cudaStreamSynchronize(cudaStream_t s)
 {
     ++g_calls["cudaStreamSynchronize"];
