@@ -401,7 +401,8 @@ int s3r_make_color_transfer(const double* xs, const double* rgba, uint32_t npoin
  *     (the walk takes one of them, this form both); for levels up to 7, at the cost of (3 * 2^level - 2) x 16
  *     bytes of device memory per pixel that the blocks cover (and half as many more) and data slot.
  *   One thread per ray (ids 0-3): a view for which block-major is the faster one (64 blocks and more with rays of
- *     some length in each; at most 1 GB of results; alpha_stop of 1 or more) renders in that form, restricted to
+ *     some length in each, or a small view of 8 deep ones; seen from outside the level or in few pixels; at most 1 GB of
+ *     results and items; alpha_stop of 1 or more) renders in that form, restricted to
  *     the blocks that the walk meets -- the walk's image bit for bit.  A render that is captured by the caller
  *     always walks: the graph may be replayed after other views and shows the view staged last.
  *   Block results belong to the plan: up to 1 GB per data slot (the second one with s3r_frame_run_host) for ids 0-3,
